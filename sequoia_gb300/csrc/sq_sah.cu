@@ -19,16 +19,21 @@
 // result is record-for-record the oracle's.
 //
 // Schedule:
-//   large nodes (> kSmall triangles): level by level.  Chunks of 256 or
-//     2048 triangles (by mesh size) bin into per-warp shared bins (shared-memory atomics on
-//     order-preserving integer encodings, or full-warp reductions when a
-//     warp's 32 triangles share one bin), then one atomic per bin value and
-//     block; one warp per node sweeps the planes; a count / scan / scatter
-//     triple partitions stably into the other id buffer.
+//   large nodes (> kSmall triangles): level by level, two kernels a level.
+//     k_large_split  one warp per node picks the plane from the node's bins,
+//                    places the children and scans the left counts of the
+//                    node's chunks;
+//     k_large_move   one block per chunk (256 or 2048 triangles, by mesh
+//                    size) moves the chunk's triangles to their side, stably,
+//                    and bins each one for the child that it goes to, so the
+//                    next level's split finds its bins ready.
+//     A triangle's box is read once a level: the bin it falls in is kept as a
+//     byte beside its id, and the next partition needs only that byte.
 //   small nodes: one warp per subtree, smaller child first (stack depth
 //     O(log n)), binning and partitioning with warp intrinsics only.
 #include "sq_common.cuh"
 
+#include <type_traits>
 #include <utility>
 
 namespace {
@@ -49,8 +54,9 @@ constexpr int kStackDepth = 24;
 // round trip): deeper work is finished by the small phase.
 constexpr uint32_t kBatchLargeLevels = 24;
 // Large-phase levels a single build queues between two host reads of the
-// task count (even, so the count read is always the next level's).
+// task count, after a first group sized to the mesh (build_sah).
 constexpr uint32_t kSahLevelsPerCheck = 4;
+constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 struct __align__(16) Task {
     uint32_t begin, count, slot, flags;  // flags: bit0 = ids live in buffer B, bit1 = root-like record
@@ -65,23 +71,31 @@ struct LeafRange {
 };
 static_assert(sizeof(LeafRange) == 48, "LeafRange is 48 bytes");
 
-struct Split {
-    int plane;   // -1: no split (leaf)
-    int axis;
-    float k1, cmin;
-    uint32_t nl;
-    uint32_t pad[3];
+// What k_large_move needs to move one task's chunks: the task's own range
+// and plane (a bin at or below it goes left; -1: the task became a leaf and
+// its triangles stay), and for each side that is a large task the bins and
+// chunks it collects into and how it bins.
+struct __align__(16) Part {
+    uint32_t begin, count, nl, chunk0;
+    int plane;
+    uint32_t flags;  // bit 0: ids in buffer B; bit 1: several chunks
+    int axis[2];     // binning axis of the large children
+    uint32_t task[2], child_chunk0[2];  // kNone: the side is not a large task
+    float k1[2], cmin[2];
 };
+static_assert(sizeof(Part) == 64, "Part is 64 bytes");
 
-// Task counts.  n_large[l & 1] holds the large tasks of level l: level l
-// reads it and appends its large children to n_large[(l + 1) & 1], which
-// the level's prep kernel clears first; the kernels read the counts on the
-// device, so a level needs no host round trip.
+// Task counts.  level[l % 3] holds the tasks (low word) and chunks (high
+// word) of level l: k_large_split of level l reads it and adds its large
+// children to level[(l + 1) % 3]; k_large_move of level l, which runs while
+// neither is needed, clears level[(l + 2) % 3].  The kernels read the counts
+// on the device, so a level needs no host round trip.
 struct Ctl {
-    uint32_t n_large[2], n_small, n_leaf;
-    uint32_t small_pop, err_bits, big_pop, pad;  // pop counters of the staged and the unstaged small kernels
+    unsigned long long level[3];
+    uint32_t n_small, n_leaf;
+    uint32_t small_pop, big_pop;  // pop counters of the staged and the unstaged small kernels
 };
-static_assert(sizeof(Ctl) == 32, "Ctl is 32 bytes");
+static_assert(sizeof(Ctl) == 40, "Ctl is 40 bytes");
 
 __device__ __forceinline__ float box_sa(const float* mn, const float* mx)
 {
@@ -172,40 +186,110 @@ __global__ void __launch_bounds__(256) k_sah_setup(const float* __restrict__ tri
 __device__ __forceinline__ float dec_neg(uint32_t u) { return -ordered_to_float(u); }
 __device__ __forceinline__ float dec_pos(uint32_t u) { return ordered_to_float(u); }
 
-// Place a task: leaf (recorded in the leaf list), large (appended to
-// large_next, counted in *large_cnt), or small.
-__device__ void classify(const Task& t, uint32_t leaf_size, Task* __restrict__ large_next, uint32_t* large_cnt,
-                         Task* __restrict__ small, LeafRange* __restrict__ leaves, Ctl* ctl)
+// Where the large tasks of one level are listed: the tasks, each task's
+// first chunk, the task of each chunk, and the bins and per-chunk bin counts
+// that k_large_move fills.
+struct LevelLists {
+    Task* tasks;
+    uint32_t *chunk0, *chunk_task, *bins, *counts;
+};
+
+// 32-bit words of a chunk's bin counts (16 bits a bin: a chunk holds at most
+// 2048 triangles)
+__host__ __device__ __forceinline__ uint32_t count_words(int nb) { return ((uint32_t)nb + 1u) >> 1; }
+
+// Place a task (all lanes of a warp call it with the same task): leaf
+// (recorded in the leaf list), large (listed for the level counted by *cnt),
+// or small.  side: which child of `part` it is, for the large case.  zero:
+// the bins are collected with atomics and must start from zero (else one
+// block stores them whole).
+template <uint32_t CHUNK>
+__device__ void place_task(const Task& t, uint32_t leaf_size, int nb, const LevelLists& next, unsigned long long* cnt,
+                           bool zero, Task* __restrict__ small, LeafRange* __restrict__ leaves, Ctl* ctl, Part& part,
+                           int side)
 {
+    const uint32_t lane = threadIdx.x & 31u;
+    part.task[side] = kNone;
     const bool leaf = t.count <= leaf_size || !(box_sa(t.cmn, t.cmx) > 0.0f);
     if (leaf) {
-        const uint32_t k = atomicAdd(&ctl->n_leaf, 1u);
-        LeafRange lr;
-        lr.begin = t.begin; lr.count = t.count; lr.slot = t.slot; lr.flags = t.flags;
-        for (int a = 0; a < 3; ++a) { lr.pmn[a] = t.pmn[a]; lr.pmx[a] = t.pmx[a]; }
-        lr.pad[0] = lr.pad[1] = 0;
-        leaves[k] = lr;
-    } else if (t.count > kSmall) {
-        large_next[atomicAdd(large_cnt, 1u)] = t;
-    } else {
-        small[atomicAdd(&ctl->n_small, 1u)] = t;
+        if (lane == 0) {
+            const uint32_t k = atomicAdd(&ctl->n_leaf, 1u);
+            LeafRange lr;
+            lr.begin = t.begin; lr.count = t.count; lr.slot = t.slot; lr.flags = t.flags;
+            for (int a = 0; a < 3; ++a) { lr.pmn[a] = t.pmn[a]; lr.pmx[a] = t.pmx[a]; }
+            lr.pad[0] = lr.pad[1] = 0;
+            leaves[k] = lr;
+        }
+        return;
     }
+    if (t.count <= kSmall) {
+        if (lane == 0) small[atomicAdd(&ctl->n_small, 1u)] = t;
+        return;
+    }
+    const uint32_t chunks = (t.count + CHUNK - 1) / CHUNK;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(cnt, ((unsigned long long)chunks << 32) | 1ull);
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    const uint32_t k = (uint32_t)at, c0 = (uint32_t)(at >> 32);
+    if (lane == 0) {
+        next.tasks[k] = t;
+        next.chunk0[k] = c0;
+    }
+    for (uint32_t c = lane; c < chunks; c += 32) next.chunk_task[c0 + c] = k;
+    if (zero) {
+        uint32_t* b = next.bins + (size_t)k * kMaxBins * kBinWords;
+        for (int j = lane; j < nb * kBinWords; j += 32) b[j] = 0;
+        if (chunks > 1) {
+            const uint32_t cw = count_words(nb);
+            uint32_t* cc = next.counts + (size_t)c0 * cw;
+            for (uint32_t j = lane; j < chunks * cw; j += 32) cc[j] = 0;
+        }
+    }
+    part.task[side] = k;
+    part.child_chunk0[side] = c0;
+    part.axis[side] = choose_axis(t.cmn, t.cmx);
+    part.cmin[side] = sel(t.cmn, part.axis[side]);
+    part.k1[side] = bin_k1(nb, sel(t.cmx, part.axis[side]) - part.cmin[side]);
 }
 
-__global__ void k_root_task(const uint32_t* __restrict__ root_ord, uint32_t n, uint32_t leaf_size, Task* large,
-                            Task* small, LeafRange* leaves, Ctl* ctl, float* scene_out)
+// A root task: placed, and where it is large its Part makes k_large_move
+// bin it in place (everything on side 0).
+template <uint32_t CHUNK>
+__device__ void place_root(const Task& t, uint32_t leaf_size, int nb, const LevelLists& l0, Part* __restrict__ parts,
+                           Task* __restrict__ small, LeafRange* __restrict__ leaves, Ctl* ctl)
 {
-    Task t;
+    Part p;
+    place_task<CHUNK>(t, leaf_size, nb, l0, &ctl->level[0], true, small, leaves, ctl, p, 0);
+    if (p.task[0] == kNone) return;
+    p.begin = t.begin;
+    p.count = p.nl = t.count;
+    p.chunk0 = p.child_chunk0[0];
+    p.plane = kMaxBins;
+    p.flags = (t.flags & 1u) | 2u;
+    p.axis[1] = 0;
+    p.task[1] = kNone;
+    p.child_chunk0[1] = 0;
+    p.k1[1] = p.cmin[1] = 0.0f;
+    if ((threadIdx.x & 31u) == 0) parts[p.task[0]] = p;
+}
+
+template <uint32_t CHUNK>
+__global__ void k_root_task(const uint32_t* __restrict__ root_ord, uint32_t n, uint32_t leaf_size, int nb,
+                            LevelLists l0, Part* parts, Task* small, LeafRange* leaves, Ctl* ctl, float* scene_out)
+{
+    Task t;  // one warp
     t.begin = 0; t.count = n; t.slot = 0; t.flags = 2u;
     for (int k = 0; k < 3; ++k) {
         t.pmn[k] = dec_neg(root_ord[k]);
         t.pmx[k] = dec_pos(root_ord[3 + k]);
         t.cmn[k] = dec_neg(root_ord[6 + k]);
         t.cmx[k] = dec_pos(root_ord[9 + k]);
-        scene_out[k] = t.pmn[k];
-        scene_out[3 + k] = t.pmx[k];
+        if (threadIdx.x == 0) {
+            scene_out[k] = t.pmn[k];
+            scene_out[3 + k] = t.pmx[k];
+        }
     }
-    classify(t, leaf_size, large, &ctl->n_large[0], small, leaves, ctl);
+    place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
 }
 
 // ---------------------------------------------------------------------------
@@ -261,24 +345,23 @@ __global__ void __launch_bounds__(256) k_grid_bin(const float4* __restrict__ tb,
     }
 }
 
+// One warp per cell, in Morton order; cell m covers [begin_m, begin_m +
+// count_m), begin_m summed by the warp from the earlier cells' counts.
+template <uint32_t CHUNK>
 __global__ void k_grid_tasks(const uint32_t* __restrict__ cell_ord, const uint32_t* __restrict__ root_ord, uint32_t n,
-                             uint32_t leaf_size, uint32_t scene_box_cells, Task* large, Task* small,
-                             LeafRange* leaves, Ctl* ctl, float* scene_out)
+                             uint32_t leaf_size, uint32_t scene_box_cells, int nb, LevelLists l0, Part* parts,
+                             Task* small, LeafRange* leaves, Ctl* ctl, float* scene_out)
 {
-    // one thread per cell, in Morton order; cell m covers [begin_m, begin_m + count_m)
-    __shared__ uint32_t s_begin[65];
-    const uint32_t m = threadIdx.x;
-    if (m == 0) {
-        uint32_t sum = 0;
-        for (int j = 0; j < 64; ++j) { s_begin[j] = sum; sum += cell_ord[j * kBinWords + 12]; }
-        s_begin[64] = sum;
-        for (int k = 0; k < 3; ++k) { scene_out[k] = dec_neg(root_ord[k]); scene_out[3 + k] = dec_pos(root_ord[3 + k]); }
-    }
-    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (m >= 64) return;
+    if (m == 0 && lane == 0)
+        for (int k = 0; k < 3; ++k) { scene_out[k] = dec_neg(root_ord[k]); scene_out[3 + k] = dec_pos(root_ord[3 + k]); }
+    uint32_t before = lane < m ? cell_ord[lane * kBinWords + 12] : 0u;
+    if (lane + 32u < m) before += cell_ord[(lane + 32u) * kBinWords + 12];
     const uint32_t* cb = cell_ord + m * kBinWords;
     Task t;
-    t.begin = s_begin[m];
+    t.begin = __reduce_add_sync(0xFFFFFFFFu, before);
     t.count = cb[12];
     t.slot = 63u + m;
     t.flags = 2u;
@@ -294,7 +377,7 @@ __global__ void k_grid_tasks(const uint32_t* __restrict__ cell_ord, const uint32
         // the plain grid builder gives every cell node the scene box (src/builder.cpp:2173-2174)
         for (int k = 0; k < 3; ++k) { t.pmn[k] = dec_neg(root_ord[k]); t.pmx[k] = dec_pos(root_ord[3 + k]); }
     }
-    classify(t, leaf_size, large, &ctl->n_large[0], small, leaves, ctl);
+    place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
 }
 
 // heap of 63 inner nodes above the 64 cell nodes (src/builder.cpp:2181-2188)
@@ -457,303 +540,259 @@ __device__ __forceinline__ Task child_task(uint32_t begin, uint32_t count, uint3
 // ---------------------------------------------------------------------------
 // large phase
 //
-// Every kernel reads the level's task count *ntp on the device and loops
-// over its work (chunks per block, tasks per warp), so the same kernels run
-// with an exact grid when the host knows the count and with a fixed grid in
-// the graph-captured batch build, where it does not.
+// Every kernel reads the level's task and chunk counts on the device and
+// loops over its work (tasks per warp, chunks per block), so a fixed grid
+// serves any level, with or without the host knowing the counts.
 
-__global__ void k_large_zero(uint32_t* __restrict__ bins, const uint32_t* __restrict__ ntp, int nb)
+// Sum of the counts of bins [0, plane] of one chunk's count row.
+__device__ __forceinline__ uint32_t left_count(const uint32_t* __restrict__ row, int plane)
 {
-    chain_wait();  // a chained launch (enqueue_level_chunks)
-    chain_release();
-    const size_t per = (size_t)nb * kBinWords;
-    const size_t words = (size_t)(*ntp) * per;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += (size_t)gridDim.x * blockDim.x)
-        bins[(i / per) * (kMaxBins * kBinWords) + i % per] = 0;
+    const int full = (plane + 1) >> 1;
+    uint32_t n = 0;
+    for (int w = 0; w < full; ++w) {
+        const uint32_t v = row[w];
+        n += (v & 0xFFFFu) + (v >> 16);
+    }
+    if ((plane + 1) & 1) n += row[full] & 0xFFFFu;
+    return n;
 }
 
+// One warp per task: the plane, the node record, the two children, and the
+// number of left triangles before each of the task's chunks.
 template <uint32_t CHUNK>
-__global__ void k_large_prep(const Task* __restrict__ tasks, const uint32_t* __restrict__ ntp, uint32_t* next_cnt,
-                             int nb, Split* __restrict__ split, uint32_t* __restrict__ chunk_start)
+__global__ void __launch_bounds__(128) k_large_split(LevelLists cur, LevelLists next, const Ctl* __restrict__ ctl_in,
+                                                     uint32_t cur_i, uint32_t next_i, int nb, uint32_t base,
+                                                     uint32_t leaf_size, Node* __restrict__ nodes,
+                                                     Part* __restrict__ parts, uint32_t* __restrict__ chunk_left,
+                                                     Task* small, LeafRange* leaves, Ctl* ctl)
 {
-    chain_wait();  // a chained launch (enqueue_level_chunks)
+    chain_wait();  // a chained launch (enqueue_levels)
     chain_release();
-    // single block: chunk counts and their exclusive scan
-    __shared__ uint32_t s_sum[1024];
-    const uint32_t nt = *ntp;
-    if (threadIdx.x == 0) *next_cnt = 0;  // this level's large children are counted from 0
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < nt; base += blockDim.x) {
-        const uint32_t t = base + threadIdx.x;
-        uint32_t ch = 0;
-        if (t < nt) {
-            const Task& tk = tasks[t];
-            ch = (tk.count + CHUNK - 1) / CHUNK;
-            Split s;
-            s.axis = choose_axis(tk.cmn, tk.cmx);
-            s.cmin = sel(tk.cmn, s.axis);
-            s.k1 = bin_k1(nb, sel(tk.cmx, s.axis) - s.cmin);
-            s.plane = -1;
-            s.nl = 0;
-            s.pad[0] = s.pad[1] = s.pad[2] = 0;
-            split[t] = s;
-        }
-        s_sum[threadIdx.x] = ch;
-        __syncthreads();
-        for (uint32_t o = 1; o < blockDim.x; o <<= 1) {
-            const uint32_t v = threadIdx.x >= o ? s_sum[threadIdx.x - o] : 0u;
-            __syncthreads();
-            s_sum[threadIdx.x] += v;
-            __syncthreads();
-        }
-        if (t < nt) chunk_start[t] = carry + s_sum[threadIdx.x] - ch;
-        carry += s_sum[blockDim.x - 1];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) chunk_start[nt] = carry;
-}
-
-__device__ __forceinline__ uint32_t task_of_chunk(const uint32_t* __restrict__ chunk_start, uint32_t nt, uint32_t c)
-{
-    uint32_t lo = 0, hi = nt;  // largest t with chunk_start[t] <= c
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(chunk_start + mid) <= c) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
-template <uint32_t CHUNK>
-__global__ void __launch_bounds__(256) k_large_bin(const Task* __restrict__ tasks, const uint32_t* __restrict__ ntp,
-                                                   const Split* __restrict__ split, const uint32_t* __restrict__ chunk_start,
-                                                   const uint32_t* __restrict__ ids_a, const uint32_t* __restrict__ ids_b,
-                                                   const float4* __restrict__ tb, int nb, uint32_t* __restrict__ bins_g)
-{
-    chain_wait();  // a chained launch (enqueue_level_chunks)
-    chain_release();
-    __shared__ uint32_t s_wb[8][kMaxBins * kBinWords];
-    const uint32_t nt = *ntp;
-    const uint32_t chunks = chunk_start[nt];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t* wb = s_wb[warp];
-    for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-        const uint32_t t = task_of_chunk(chunk_start, nt, c);
-        const Task tk = tasks[t];
-        const Split sp = split[t];
-        const uint32_t off = (c - chunk_start[t]) * CHUNK;
-        const uint32_t len = min(CHUNK, tk.count - off);
-        const uint32_t* ids = (tk.flags & 1u) ? ids_b : ids_a;
-        for (int j = lane; j < kMaxBins * kBinWords; j += 32) wb[j] = 0;
-        __syncwarp();
-        for (uint32_t base = warp * 32; base < len; base += 256) {
-            const uint32_t j = base + lane;
-            float mn[3], mx[3], cc[3];
-            int bin = nb;
-            if (j < len) {
-                load_box(tb, ids[tk.begin + off + j], mn, mx);
-                for (int a = 0; a < 3; ++a) cc[a] = (mn[a] + mx[a]) * 0.5f;
-                bin = bin_of(sp.k1, sel(cc, sp.axis), sp.cmin, nb);
-            } else {
-                for (int a = 0; a < 3; ++a) { mn[a] = mx[a] = cc[a] = 0.0f; }
-            }
-            warp_bin_add(wb, bin, nb, mn, mx, cc);
-        }
-        __syncthreads();
-        uint32_t* g = bins_g + (size_t)t * kMaxBins * kBinWords;
-        for (int j = threadIdx.x; j < nb * kBinWords; j += blockDim.x) {
-            uint32_t v = s_wb[0][j];
-            const bool is_count = (j % kBinWords) == 12;
-            for (int w = 1; w < 8; ++w) v = is_count ? v + s_wb[w][j] : max(v, s_wb[w][j]);
-            if (v) {
-                if (is_count) atomicAdd(g + j, v); else atomicMax(g + j, v);
-            }
-        }
-        __syncthreads();  // every warp's bins read before the next chunk clears them
-    }
-}
-
-__global__ void k_large_split(const Task* __restrict__ tasks, const uint32_t* __restrict__ ntp, Split* __restrict__ split,
-                              const uint32_t* __restrict__ bins_g, int nb, uint32_t base, uint32_t leaf_size,
-                              Node* __restrict__ nodes, Task* large_next, uint32_t* next_cnt, Task* small,
-                              LeafRange* leaves, Ctl* ctl)
-{
-    chain_wait();  // a chained launch (enqueue_level_chunks)
-    chain_release();
-    const uint32_t nt = *ntp;
-    const int lane = threadIdx.x & 31;
+    const uint32_t nt = (uint32_t)ctl_in->level[cur_i];
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t cw = count_words(nb);
     for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += warps) {
-        const Task tk = tasks[t];
-        const PlaneResult r = warp_choose_plane(bins_g + (size_t)t * kMaxBins * kBinWords, nb);
-        if (lane != 0) continue;
+        const Task tk = cur.tasks[t];
+        const uint32_t chunk0 = cur.chunk0[t];
+        const uint32_t chunks = (tk.count + CHUNK - 1) / CHUNK;
+        const PlaneResult r = warp_choose_plane(cur.bins + (size_t)t * kMaxBins * kBinWords, nb);
+        Part p;
+        p.begin = tk.begin;
+        p.count = tk.count;
+        p.nl = r.nl;
+        p.chunk0 = chunk0;
+        p.plane = r.plane;
+        p.flags = (tk.flags & 1u) | (chunks > 1 ? 2u : 0u);
+        p.task[0] = p.task[1] = kNone;
+        p.axis[0] = p.axis[1] = 0;
+        p.child_chunk0[0] = p.child_chunk0[1] = 0;
+        p.k1[0] = p.k1[1] = p.cmin[0] = p.cmin[1] = 0.0f;
         if (r.plane < 0 || r.nl == 0 || r.nl == tk.count) {
             // no plane scored below FLT_MAX: the node becomes a leaf
-            const uint32_t k = atomicAdd(&ctl->n_leaf, 1u);
-            LeafRange lr;
-            lr.begin = tk.begin; lr.count = tk.count; lr.slot = tk.slot; lr.flags = tk.flags;
-            for (int a = 0; a < 3; ++a) { lr.pmn[a] = tk.pmn[a]; lr.pmx[a] = tk.pmx[a]; }
-            lr.pad[0] = lr.pad[1] = 0;
-            leaves[k] = lr;
+            p.plane = -1;
+            if (lane == 0) {
+                const uint32_t k = atomicAdd(&ctl->n_leaf, 1u);
+                LeafRange lr;
+                lr.begin = tk.begin; lr.count = tk.count; lr.slot = tk.slot; lr.flags = tk.flags;
+                for (int a = 0; a < 3; ++a) { lr.pmn[a] = tk.pmn[a]; lr.pmx[a] = tk.pmx[a]; }
+                lr.pad[0] = lr.pad[1] = 0;
+                leaves[k] = lr;
+                parts[t] = p;
+            }
             continue;
         }
-        Split s = split[t];
-        s.plane = r.plane;
-        s.nl = r.nl;
-        split[t] = s;
         const uint32_t q = tk.begin + r.nl;
-        Box pb;
-        for (int a = 0; a < 3; ++a) { pb.mn[a] = tk.pmn[a]; pb.mx[a] = tk.pmx[a]; }
-        store_node(nodes + tk.slot, pb, base + 2u * q, 2u, 0);
+        if (lane == 0) {
+            Box pb;
+            for (int a = 0; a < 3; ++a) { pb.mn[a] = tk.pmn[a]; pb.mx[a] = tk.pmx[a]; }
+            store_node(nodes + tk.slot, pb, base + 2u * q, 2u, 0);
+        }
         const uint32_t buf = (tk.flags & 1u) ^ 1u;
-        classify(child_task(tk.begin, r.nl, base + 2u * q, buf, r.lp, r.lc), leaf_size, large_next, next_cnt, small,
-                 leaves, ctl);
-        classify(child_task(q, tk.count - r.nl, base + 2u * q + 1u, buf, r.rp, r.rc), leaf_size, large_next, next_cnt,
-                 small, leaves, ctl);
-    }
-}
-
-template <uint32_t CHUNK>
-__global__ void __launch_bounds__(256) k_large_count(const Task* __restrict__ tasks, const uint32_t* __restrict__ ntp,
-                                                     const Split* __restrict__ split,
-                                                     const uint32_t* __restrict__ chunk_start,
-                                                     const uint32_t* __restrict__ ids_a, const uint32_t* __restrict__ ids_b,
-                                                     const float4* __restrict__ tb, int nb,
-                                                     uint32_t* __restrict__ chunk_left)
-{
-    chain_wait();  // a chained launch (enqueue_level_chunks)
-    chain_release();
-    __shared__ uint32_t s[8];
-    const uint32_t nt = *ntp;
-    const uint32_t chunks = chunk_start[nt];
-    for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-        const uint32_t t = task_of_chunk(chunk_start, nt, c);
-        const Split sp = split[t];
-        if (sp.plane < 0) continue;  // block-uniform
-        const Task tk = tasks[t];
-        const uint32_t off = (c - chunk_start[t]) * CHUNK;
-        const uint32_t len = min(CHUNK, tk.count - off);
-        const uint32_t* ids = (tk.flags & 1u) ? ids_b : ids_a;
-        uint32_t cnt = 0;
-        for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) {
-            float mn[3], mx[3];
-            load_box(tb, ids[tk.begin + off + j], mn, mx);
-            const float cc = (sel(mn, sp.axis) + sel(mx, sp.axis)) * 0.5f;
-            cnt += bin_of(sp.k1, cc, sp.cmin, nb) <= sp.plane;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
-        if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = cnt;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t total = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) total += s[w];
-            chunk_left[c] = total;
-        }
-        __syncthreads();
-    }
-}
-
-// exclusive scan of the left counts over each task's chunks (one warp per task)
-__global__ void k_large_scan(const Split* __restrict__ split, const uint32_t* __restrict__ ntp,
-                             const uint32_t* __restrict__ chunk_start, uint32_t* __restrict__ chunk_left)
-{
-    chain_wait();  // a chained launch (enqueue_level_chunks)
-    chain_release();
-    const uint32_t nt = *ntp;
-    const int lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += warps) {
-        if (split[t].plane < 0) continue;  // warp-uniform
+        const bool zero = chunks > 1;
+        place_task<CHUNK>(child_task(tk.begin, r.nl, base + 2u * q, buf, r.lp, r.lc), leaf_size, nb, next,
+                          &ctl->level[next_i], zero, small, leaves, ctl, p, 0);
+        place_task<CHUNK>(child_task(q, tk.count - r.nl, base + 2u * q + 1u, buf, r.rp, r.rc), leaf_size, nb, next,
+                          &ctl->level[next_i], zero, small, leaves, ctl, p, 1);
+        if (lane == 0) parts[t] = p;
+        // exclusive scan of the chunks' left counts, 128 chunks a round
         uint32_t carry = 0;
-        for (uint32_t c0 = chunk_start[t]; c0 < chunk_start[t + 1]; c0 += 32) {
-            const uint32_t c = c0 + lane;
-            const uint32_t v = c < chunk_start[t + 1] ? chunk_left[c] : 0u;
-            uint32_t x = v;
+        if (chunks > 1)
+            for (uint32_t c0 = 0; c0 < chunks; c0 += 128) {
+                const uint32_t c = c0 + 4u * lane;
+                uint32_t v[4], sum = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-                if (lane >= o) x += y;
+                for (int k = 0; k < 4; ++k) {
+                    v[k] = c + k < chunks ? left_count(cur.counts + (size_t)(chunk0 + c + k) * cw, r.plane) : 0u;
+                    sum += v[k];
+                }
+                uint32_t x = sum;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                    if (lane >= (uint32_t)o) x += y;
+                }
+                uint32_t run = carry + x - sum;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (c + k < chunks) chunk_left[chunk0 + c + k] = run;
+                    run += v[k];
+                }
+                carry += __shfl_sync(0xFFFFFFFFu, x, 31);
             }
-            if (c < chunk_start[t + 1]) chunk_left[c] = carry + x - v;
-            carry += __shfl_sync(0xFFFFFFFFu, x, 31);
-        }
     }
 }
 
-template <uint32_t CHUNK>
-__global__ void __launch_bounds__(256) k_large_scatter(const Task* __restrict__ tasks, const uint32_t* __restrict__ ntp,
-                                                       const Split* __restrict__ split,
-                                                       const uint32_t* __restrict__ chunk_start,
-                                                       uint32_t* __restrict__ ids_a, uint32_t* __restrict__ ids_b,
-                                                       const float4* __restrict__ tb, int nb,
-                                                       const uint32_t* __restrict__ chunk_left)
+// One block per chunk: the chunk's triangles move to their side of the
+// task's plane, in order, and each is binned for the large child it joins:
+// its bin is stored as a byte beside its id, its boxes go into the child's
+// bins, and where the task has several chunks the bin counts of the child's
+// chunks are counted too (a side's run of one chunk lands in at most two).
+// ROOT: the level's tasks are binned in place, nothing moves.
+//
+// The blocks share one set of bins per side: shared-memory atomics on
+// order-preserving integers (13 a triangle), or full-warp reductions when 32
+// triangles share one side and bin.
+template <uint32_t CHUNK, bool ROOT>
+__global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ parts, LevelLists cur, LevelLists next,
+                                                    uint32_t cur_i, uint32_t* __restrict__ ids_a,
+                                                    uint32_t* __restrict__ ids_b, uint8_t* __restrict__ bin_a,
+                                                    uint8_t* __restrict__ bin_b, const uint32_t* __restrict__ chunk_left,
+                                                    const float4* __restrict__ tb, int nb, Ctl* ctl)
 {
-    chain_wait();  // a chained launch (enqueue_level_chunks)
+    chain_wait();  // a chained launch (enqueue_levels)
     chain_release();
-    constexpr int kPer = CHUNK / 256;  // consecutive elements per thread
+    __shared__ uint32_t s_bins[2 * kMaxBins * kBinWords];
+    __shared__ uint32_t s_cnt[2][2][kMaxBins];
     __shared__ uint32_t s_w[8];
-    const uint32_t nt = *ntp;
-    const uint32_t chunks = chunk_start[nt];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!ROOT && blockIdx.x == 0 && threadIdx.x == 0) ctl->level[(cur_i + 2u) % 3u] = 0;
+    const uint32_t chunks = (uint32_t)(ctl->level[cur_i] >> 32);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t cw = count_words(nb);
     for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-        const uint32_t t = task_of_chunk(chunk_start, nt, c);
-        const Split sp = split[t];
-        if (sp.plane < 0) continue;  // block-uniform
-        const Task tk = tasks[t];
-        const uint32_t off = (c - chunk_start[t]) * CHUNK;
-        const uint32_t len = min(CHUNK, tk.count - off);
-        const uint32_t* in = (tk.flags & 1u) ? ids_b : ids_a;
-        uint32_t* out = (tk.flags & 1u) ? ids_a : ids_b;
-        uint32_t idv[kPer];
-        bool left[kPer];
-        uint32_t cnt = 0;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const uint32_t j = threadIdx.x * kPer + k;
-            left[k] = false;
-            idv[k] = 0;
-            if (j < len) {
-                idv[k] = in[tk.begin + off + j];
-                float mn[3], mx[3];
-                load_box(tb, idv[k], mn, mx);
-                const float cc = (sel(mn, sp.axis) + sel(mx, sp.axis)) * 0.5f;
-                left[k] = bin_of(sp.k1, cc, sp.cmin, nb) <= sp.plane;
-                cnt += left[k];
+        const Part P = parts[cur.chunk_task[c]];
+        if (P.plane < 0) continue;  // block-uniform
+        const uint32_t off = (c - P.chunk0) * CHUNK;
+        const uint32_t len = min(CHUNK, P.count - off);
+        const bool from_b = P.flags & 1u;
+        const uint32_t* in = (from_b ? ids_b : ids_a) + P.begin + off;
+        const uint8_t* bin_in = (from_b ? bin_b : bin_a) + P.begin + off;
+        uint32_t* out = ROOT ? nullptr : (from_b ? ids_a : ids_b) + P.begin;
+        uint8_t* bin_out = (from_b != ROOT ? bin_a : bin_b) + P.begin;
+        const bool large0 = P.task[0] != kNone, large1 = P.task[1] != kNone;
+        for (int j = threadIdx.x; j < 2 * kMaxBins * kBinWords; j += 256) s_bins[j] = 0;
+        if (threadIdx.x < 4 * kMaxBins) (&s_cnt[0][0][0])[threadIdx.x] = 0;
+        // the warp's rows of 32 triangles
+        const uint32_t rows = (len + 31u) >> 5, per = (rows + 7u) >> 3;
+        const uint32_t r0 = warp * per, r1 = min(rows, r0 + per);
+        uint32_t left_before = 0, lrun = 0;
+        if (!ROOT) {
+            uint32_t nl = 0;
+            for (uint32_t r = r0; r < r1; ++r) {
+                const uint32_t j = r * 32u + lane;
+                nl += __popc(__ballot_sync(0xFFFFFFFFu, j < len && (int)bin_in[j] <= P.plane));
             }
+            if (lane == 0) s_w[warp] = nl;
+            left_before = (P.flags & 2u) ? chunk_left[c] : 0u;
         }
-        // block exclusive scan of per-thread left counts
-        uint32_t x = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) s_w[warp] = x;
         __syncthreads();
-        uint32_t wsum = 0;
-        for (int w = 0; w < warp; ++w) wsum += s_w[w];
-        uint32_t lrank = wsum + x - cnt;                    // left elements before this thread in the chunk
-        const uint32_t left_before = chunk_left[c];          // left elements before this chunk in the task
-        const uint32_t lbase = tk.begin + left_before;
-        const uint32_t rbase = tk.begin + sp.nl + (off - left_before);
+        if (!ROOT)
+            for (uint32_t w = 0; w < warp; ++w) lrun += s_w[w];
+        lrun += left_before;  // left triangles of the task before this warp's row
+        const uint32_t first[2] = {ROOT ? c - P.chunk0 : left_before / CHUNK,
+                                   (off - left_before) / CHUNK};  // first chunk of each side's run
+        for (uint32_t r = r0; r < r1; ++r) {
+            const uint32_t j = r * 32u + lane;
+            const bool valid = j < len;
+            bool left = true;
+            uint32_t id = 0, pos = off + j;  // pos: place in the task's range
+            if (valid) id = in[j];
+            if (!ROOT) {
+                left = valid && (int)bin_in[j] <= P.plane;
+                const uint32_t lb = __ballot_sync(0xFFFFFFFFu, left);
+                const uint32_t lrank = lrun + __popc(lb & lt);
+                lrun += __popc(lb);
+                // a right triangle's rank is its index less the left ones before it
+                pos = left ? lrank : off + j - lrank;
+            }
+            const uint32_t side = left ? 0u : 1u;
+            const bool binned = valid && (left ? large0 : large1);
+            const uint32_t to = pos + (left ? 0u : P.nl);
+            if (!ROOT && valid) out[to] = id;
+            uint32_t key = 0xFFu;
+            uint32_t e[12];
+            if (binned) {
+                float mn[3], mx[3], cc[3];
+                load_box(tb, id, mn, mx);
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const uint32_t j = threadIdx.x * kPer + k;
-            if (j < len) {
-                if (left[k]) { out[lbase + lrank] = idv[k]; lrank++; }
-                else out[rbase + (j - lrank)] = idv[k];
+                for (int a = 0; a < 3; ++a) cc[a] = (mn[a] + mx[a]) * 0.5f;
+                const int b = bin_of(left ? P.k1[0] : P.k1[1], sel(cc, left ? P.axis[0] : P.axis[1]),
+                                     left ? P.cmin[0] : P.cmin[1], nb);
+                bin_out[to] = (uint8_t)b;
+                key = side * kMaxBins + (uint32_t)b;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    e[a] = float_to_ordered(-mn[a]);
+                    e[3 + a] = float_to_ordered(mx[a]);
+                    e[6 + a] = float_to_ordered(-cc[a]);
+                    e[9 + a] = float_to_ordered(cc[a]);
+                }
+                atomicAdd(&s_cnt[side][pos / CHUNK - (left ? first[0] : first[1])][b], 1u);
+            }
+            const uint32_t key0 = __shfl_sync(0xFFFFFFFFu, key, 0);
+            if (__all_sync(0xFFFFFFFFu, key == key0)) {
+                if (key0 != 0xFFu) {
+#pragma unroll
+                    for (int k = 0; k < 12; ++k) e[k] = __reduce_max_sync(0xFFFFFFFFu, e[k]);
+                    if (lane == 0) {
+#pragma unroll
+                        for (int k = 0; k < 12; ++k) atomicMax(&s_bins[key * kBinWords + k], e[k]);
+                    }
+                }
+            } else if (binned) {
+#pragma unroll
+                for (int k = 0; k < 12; ++k) atomicMax(&s_bins[key * kBinWords + k], e[k]);
             }
         }
-        __syncthreads();  // s_w read by every warp before the next chunk writes it
+        __syncthreads();
+        const bool several = P.flags & 2u;
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            if (P.task[side] == kNone) continue;  // block-uniform
+            uint32_t* g = next.bins + (size_t)P.task[side] * kMaxBins * kBinWords;
+            const uint32_t* sb = s_bins + side * kMaxBins * kBinWords;
+            for (int j = threadIdx.x; j < nb * kBinWords; j += 256) {
+                const int b = j / kBinWords;
+                const bool is_count = j - b * kBinWords == 12;
+                const uint32_t v = is_count ? s_cnt[side][0][b] + s_cnt[side][1][b] : sb[j];
+                if (!several) g[j] = v;
+                else if (v) {
+                    if (is_count) atomicAdd(g + j, v); else atomicMax(g + j, v);
+                }
+            }
+            if (several && (side ? P.count - P.nl : P.nl) > CHUNK) {
+                // the counts of the run's one or two chunks, two bins a word
+                for (uint32_t j = threadIdx.x; j < 2u * cw; j += 256) {
+                    const uint32_t slot = j >= cw ? 1u : 0u, w = j - slot * cw;
+                    const uint32_t v = s_cnt[side][slot][2 * w] |
+                                       (2 * w + 1 < (uint32_t)nb ? s_cnt[side][slot][2 * w + 1] << 16 : 0u);
+                    if (v) atomicAdd(next.counts + (size_t)(P.child_chunk0[side] + first[side] + slot) * cw + w, v);
+                }
+            }
+        }
+        __syncthreads();  // the shared bins are cleared for the next chunk
     }
 }
 
 // After the last fixed level of the batch build: large tasks still left go
 // to the small phase, whose warps split subtrees of any size.
-__global__ void k_large_to_small(const Task* __restrict__ large, const uint32_t* __restrict__ ntp,
+__global__ void k_large_to_small(const Task* __restrict__ large, const unsigned long long* __restrict__ level,
                                  Task* __restrict__ small, Ctl* ctl)
 {
-    const uint32_t nt = *ntp;
+    chain_wait();  // a chained launch (enqueue_levels)
+    chain_release();
+    const uint32_t nt = (uint32_t)*level;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x)
         small[atomicAdd(&ctl->n_small, 1u)] = large[t];
 }
@@ -999,101 +1038,99 @@ int sms() { return sm_count(); }
 struct SahWs {
     float4* tb;
     uint32_t *ids_a, *ids_b;
-    Task *lists[2], *small;
+    uint8_t *bin_a, *bin_b;
+    LevelLists lists[2];
+    Task* small;
     LeafRange* leaves;
-    Split* split;
-    uint32_t *chunk_start, *chunk_left, *bins, *cells, *hist, *root_ord;
+    Part* parts;
+    uint32_t *chunk_left, *cells, *hist, *root_ord;
     Ctl* ctl;
 };
 
+// Most large tasks a level can have, and most chunks.
 size_t sah_tasks(uint32_t n) { return n / kSmall + 2; }
+size_t sah_chunks(uint32_t n) { return (size_t)n / (n < kChunkSmallBelow ? kChunkSmall : kChunk) + sah_tasks(n) + 1; }
+
+// Lays the workspace out at p (null: only the size is wanted) and returns its size.
+size_t sah_layout(char* p, uint32_t n, uint32_t meshes, SahWs& w)
+{
+    const size_t tasks = sah_tasks(n), chunks = sah_chunks(n);
+    size_t used = 0;
+    auto take = [&](auto*& ptr, size_t count) {
+        using T = std::remove_reference_t<decltype(*ptr)>;
+        ptr = reinterpret_cast<T*>(p + used);
+        used += (sizeof(T) * count + 255) / 256 * 256;
+    };
+    take(w.tb, 2ull * n);  // triangle boxes
+    take(w.ids_a, n);
+    take(w.ids_b, n);
+    take(w.bin_a, n);
+    take(w.bin_b, n);
+    for (LevelLists& l : w.lists) {
+        take(l.tasks, tasks);
+        take(l.chunk0, tasks);
+        take(l.chunk_task, chunks);
+        take(l.bins, (size_t)kMaxBins * kBinWords * tasks);
+        take(l.counts, (size_t)(kMaxBins / 2) * chunks);
+    }
+    take(w.small, (size_t)n / 2 + 2);
+    take(w.leaves, (size_t)n + 66 + meshes);  // + 64 empty grid cells, + empty meshes
+    take(w.parts, tasks);
+    take(w.chunk_left, chunks);
+    take(w.cells, 64 * kBinWords);
+    take(w.hist, 64);
+    take(w.root_ord, 16ull * (meshes ? meshes : 1));  // 12 words per mesh
+    take(w.ctl, 1);
+    return used;
+}
 
 size_t sah_ws_bytes(uint32_t n, uint32_t meshes)
 {
-    const size_t tasks = sah_tasks(n);
-    size_t b = 0;
-    auto add = [&](size_t bytes) { b += (bytes + 255) / 256 * 256; };
-    add(sizeof(float4) * 2ull * n);               // triangle boxes
-    add(sizeof(uint32_t) * (size_t)n);            // ids A
-    add(sizeof(uint32_t) * (size_t)n);            // ids B
-    add(sizeof(Task) * tasks);                    // large lists (two levels)
-    add(sizeof(Task) * tasks);
-    add(sizeof(Task) * ((size_t)n / 2 + 2));      // small list
-    add(sizeof(LeafRange) * ((size_t)n + 66 + meshes));  // leaf list (+64 empty grid cells, + empty meshes)
-    add(sizeof(Split) * tasks);
-    add(sizeof(uint32_t) * (tasks + 1));          // chunk starts
-    add(sizeof(uint32_t) * ((size_t)n / kChunkSmall + tasks + 1));  // chunk left counts
-    add(sizeof(uint32_t) * (size_t)kMaxBins * kBinWords * tasks);  // bins
-    add(sizeof(uint32_t) * 64 * kBinWords);       // grid cells
-    add(sizeof(uint32_t) * 64);                   // grid histogram
-    add(sizeof(uint32_t) * 16ull * (meshes ? meshes : 1));  // root boxes (12 words per mesh)
-    add(sizeof(Ctl));
-    return b;
+    SahWs w;
+    return sah_layout(nullptr, n, meshes, w);
 }
 
 SahWs carve(void* ws, uint32_t n, uint32_t meshes)
 {
-    const size_t tasks = sah_tasks(n);
-    char* p = static_cast<char*>(ws);
-    auto take = [&](size_t bytes) { char* r = p; p += (bytes + 255) / 256 * 256; return r; };
     SahWs w;
-    w.tb = reinterpret_cast<float4*>(take(sizeof(float4) * 2ull * n));
-    w.ids_a = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (size_t)n));
-    w.ids_b = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (size_t)n));
-    w.lists[0] = reinterpret_cast<Task*>(take(sizeof(Task) * tasks));
-    w.lists[1] = reinterpret_cast<Task*>(take(sizeof(Task) * tasks));
-    w.small = reinterpret_cast<Task*>(take(sizeof(Task) * ((size_t)n / 2 + 2)));
-    w.leaves = reinterpret_cast<LeafRange*>(take(sizeof(LeafRange) * ((size_t)n + 66 + meshes)));
-    w.split = reinterpret_cast<Split*>(take(sizeof(Split) * tasks));
-    w.chunk_start = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (tasks + 1)));
-    w.chunk_left = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * ((size_t)n / kChunkSmall + tasks + 1)));
-    w.bins = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * (size_t)kMaxBins * kBinWords * tasks));
-    w.cells = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * 64 * kBinWords));
-    w.hist = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * 64));
-    w.root_ord = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * 16ull * (meshes ? meshes : 1)));
-    w.ctl = reinterpret_cast<Ctl*>(take(sizeof(Ctl)));
+    sah_layout(static_cast<char*>(ws), n, meshes, w);
     return w;
 }
 
-// One level of the large phase on the tasks in w.lists[level & 1], whose
-// count is ctl->n_large[level & 1] on the device.  chunk_grid / task_blocks:
-// exact grids when the host knows the count, fixed ones otherwise (the
-// kernels loop over whatever the count holds).
-template <uint32_t CHUNK>
-void enqueue_level_chunks(const SahWs& w, uint32_t level, int nb, uint32_t base, uint32_t leaf_size, Node* nodes,
-                          uint32_t chunk_grid, uint32_t task_blocks, cudaStream_t s)
+// Calls f(std::integral_constant<uint32_t, CHUNK>) with the chunk size of a
+// build over n triangles.
+template <class F>
+void with_chunk(uint32_t n, F f)
 {
-    const Task* proc = w.lists[level & 1];
-    Task* outl = w.lists[(level + 1) & 1];
-    const uint32_t* ntp = &w.ctl->n_large[level & 1];
-    uint32_t* next = &w.ctl->n_large[(level + 1) & 1];
-    // seven short kernels per level, chained: each may launch while the one
-    // before it runs and waits for it on the device (chain_wait)
-    launch_chained(k_large_zero, dim3(task_blocks), dim3(256), 0, s, w.bins, ntp, nb);
-    launch_chained(k_large_prep<CHUNK>, dim3(1), dim3(1024), 0, s, proc, ntp, next, nb, w.split, w.chunk_start);
-    launch_chained(k_large_bin<CHUNK>, dim3(chunk_grid), dim3(256), 0, s, proc, ntp, (const Split*)w.split,
-                   (const uint32_t*)w.chunk_start, (const uint32_t*)w.ids_a, (const uint32_t*)w.ids_b,
-                   (const float4*)w.tb, nb, w.bins);
-    launch_chained(k_large_split, dim3(task_blocks), dim3(128), 0, s, proc, ntp, w.split, (const uint32_t*)w.bins, nb,
-                   base, leaf_size, nodes, outl, next, w.small, w.leaves, w.ctl);
-    launch_chained(k_large_count<CHUNK>, dim3(chunk_grid), dim3(256), 0, s, proc, ntp, (const Split*)w.split,
-                   (const uint32_t*)w.chunk_start, (const uint32_t*)w.ids_a, (const uint32_t*)w.ids_b,
-                   (const float4*)w.tb, nb, w.chunk_left);
-    launch_chained(k_large_scan, dim3(task_blocks), dim3(128), 0, s, (const Split*)w.split, ntp,
-                   (const uint32_t*)w.chunk_start, w.chunk_left);
-    launch_chained(k_large_scatter<CHUNK>, dim3(chunk_grid), dim3(256), 0, s, proc, ntp, (const Split*)w.split,
-                   (const uint32_t*)w.chunk_start, w.ids_a, w.ids_b, (const float4*)w.tb, nb,
-                   (const uint32_t*)w.chunk_left);
+    if (n < kChunkSmallBelow) f(std::integral_constant<uint32_t, kChunkSmall>());
+    else f(std::integral_constant<uint32_t, kChunk>());
 }
 
-// one large level of a build over n triangles (chunk size by n)
-void enqueue_large_level(const SahWs& w, uint32_t level, int nb, uint32_t base, uint32_t leaf_size, Node* nodes,
-                         uint32_t chunk_grid, uint32_t task_blocks, uint32_t n, cudaStream_t s)
+// The bins of the root tasks in w.lists[0].
+template <uint32_t CHUNK>
+void enqueue_root_bins(const SahWs& w, int nb, cudaStream_t s)
 {
-    if (n < kChunkSmallBelow)
-        enqueue_level_chunks<kChunkSmall>(w, level, nb, base, leaf_size, nodes, chunk_grid, task_blocks, s);
-    else
-        enqueue_level_chunks<kChunk>(w, level, nb, base, leaf_size, nodes, chunk_grid, task_blocks, s);
+    launch_chained(k_large_move<CHUNK, true>, dim3(sms() * 8), dim3(256), 0, s, (const Part*)w.parts, w.lists[0],
+                   w.lists[0], 0u, w.ids_a, w.ids_b, w.bin_a, w.bin_b, (const uint32_t*)w.chunk_left,
+                   (const float4*)w.tb, nb, w.ctl);
+}
+
+// Levels [level, level + count) of the large phase: two chained launches a
+// level, each may launch while the one before it runs and waits for it on
+// the device (chain_wait).  Levels past the tree's depth find no tasks.
+template <uint32_t CHUNK>
+void enqueue_levels(const SahWs& w, uint32_t level, uint32_t count, int nb, uint32_t base, uint32_t leaf_size,
+                    Node* nodes, cudaStream_t s)
+{
+    const uint32_t grid = (uint32_t)sms() * 8u;
+    for (uint32_t l = level; l < level + count; ++l) {
+        const LevelLists &cur = w.lists[l & 1], &next = w.lists[(l + 1) & 1];
+        launch_chained(k_large_split<CHUNK>, dim3(grid), dim3(128), 0, s, cur, next, (const Ctl*)w.ctl, l % 3u,
+                       (l + 1) % 3u, nb, base, leaf_size, nodes, w.parts, w.chunk_left, w.small, w.leaves, w.ctl);
+        launch_chained(k_large_move<CHUNK, false>, dim3(grid), dim3(256), 0, s, (const Part*)w.parts, cur, next, l % 3u,
+                       w.ids_a, w.ids_b, w.bin_a, w.bin_b, (const uint32_t*)w.chunk_left, (const float4*)w.tb, nb,
+                       w.ctl);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1145,31 +1182,33 @@ __global__ void __launch_bounds__(256) k_sah_setup_seg(const float* __restrict__
     }
 }
 
-// One root task per mesh: triangles [off[m], off[m + 1]), record root0 + m.
+// One root task per mesh (one warp each): triangles [off[m], off[m + 1]),
+// record root0 + m.
+template <uint32_t CHUNK>
 __global__ void k_root_tasks_seg(const uint32_t* __restrict__ root_ord, const uint32_t* __restrict__ off, uint32_t M,
-                                 uint32_t leaf_size, uint32_t root0, Task* large, Task* small, LeafRange* leaves,
-                                 Ctl* ctl)
+                                 uint32_t leaf_size, uint32_t root0, int nb, LevelLists l0, Part* parts, Task* small,
+                                 LeafRange* leaves, Ctl* ctl)
 {
-    for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-        Task t;
-        t.begin = off[m];
-        t.count = off[m + 1] - off[m];
-        t.slot = root0 + m;
-        t.flags = 2u;
-        const uint32_t* ro = root_ord + 16ull * m;
-        for (int k = 0; k < 3; ++k) {
-            if (t.count) {
-                t.pmn[k] = dec_neg(ro[k]);
-                t.pmx[k] = dec_pos(ro[3 + k]);
-                t.cmn[k] = dec_neg(ro[6 + k]);
-                t.cmx[k] = dec_pos(ro[9 + k]);
-            } else {
-                t.pmn[k] = t.cmn[k] = FLT_MAX;
-                t.pmx[k] = t.cmx[k] = -FLT_MAX;
-            }
+    const uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (m >= M) return;
+    Task t;
+    t.begin = off[m];
+    t.count = off[m + 1] - off[m];
+    t.slot = root0 + m;
+    t.flags = 2u;
+    const uint32_t* ro = root_ord + 16ull * m;
+    for (int k = 0; k < 3; ++k) {
+        if (t.count) {
+            t.pmn[k] = dec_neg(ro[k]);
+            t.pmx[k] = dec_pos(ro[3 + k]);
+            t.cmn[k] = dec_neg(ro[6 + k]);
+            t.cmx[k] = dec_pos(ro[9 + k]);
+        } else {
+            t.pmn[k] = t.cmn[k] = FLT_MAX;
+            t.pmx[k] = t.cmx[k] = -FLT_MAX;
         }
-        classify(t, leaf_size, large, &ctl->n_large[0], small, leaves, ctl);
     }
+    place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
 }
 
 }  // namespace
@@ -1193,15 +1232,13 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
     const uint32_t leaf0 = base + 2u * n + 2u;
     cudaError_t e;
 #define SQ_TRY(x) do { if ((e = (x)) != cudaSuccess) return (int)e; } while (0)
-    SQ_TRY(cudaMemsetAsync(w.cells, 0, sizeof(uint32_t) * 64 * kBinWords, s));
-    SQ_TRY(cudaMemsetAsync(w.hist, 0, sizeof(uint32_t) * 64, s));
+    if (grid) SQ_TRY(cudaMemsetAsync(w.cells, 0, sizeof(uint32_t) * 64 * kBinWords, s));
+    if (grid) SQ_TRY(cudaMemsetAsync(w.hist, 0, sizeof(uint32_t) * 64, s));
     SQ_TRY(cudaMemsetAsync(w.root_ord, 0, sizeof(uint32_t) * 16, s));
     SQ_TRY(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), s));
     const uint32_t g = min((n + 255) / 256, (uint32_t)sms() * 8u);
     k_sah_setup<<<g, 256, 0, s>>>(tris, n, w.tb, w.ids_a, w.root_ord);
-    if (!grid) {
-        k_root_task<<<1, 1, 0, s>>>(w.root_ord, n, leaf_size, w.lists[0], w.small, w.leaves, w.ctl, scene_out);
-    } else {
+    if (grid) {
         // bin into 64 cells keyed by Morton slot, then stable sort by slot
         k_grid_bin<<<g, 256, 0, s>>>(w.tb, n, w.root_ord, sort_keys, w.cells, w.hist);
         SQ_TRY(cudaMemcpyAsync(sort_vals, w.ids_a, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s));
@@ -1209,23 +1246,34 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
                                       sort_counters, 6, 1, err, s);
         SQ_TRY(cudaMemcpyAsync(w.ids_a, which ? sort_alt_vals : sort_vals, sizeof(uint32_t) * (size_t)n,
                                cudaMemcpyDeviceToDevice, s));
-        k_grid_tasks<<<1, 64, 0, s>>>(w.cells, w.root_ord, n, leaf_size, scene_box_cells, w.lists[0], w.small,
-                                      w.leaves, w.ctl, scene_out);
     }
-    // large phase: the level kernels read their task counts on the device
-    // and stride over them with fixed grids, so levels are queued
-    // kSahLevelsPerCheck at a time and the host reads a count (and waits)
-    // only between such groups; levels past the tree's depth find no tasks
-    // and do nothing.  One host round trip per level left the GPU idle for
-    // most of a small mesh's build.
-    const uint32_t grid_fixed = (uint32_t)sms() * 8u;
-    for (uint32_t level = 0;; level += kSahLevelsPerCheck) {
-        SQ_TRY(cudaMemcpyAsync(host_ctl, &w.ctl->n_large[level & 1], sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        SQ_TRY(cudaStreamSynchronize(s));
-        if (host_ctl[0] == 0) break;
-        for (uint32_t j = 0; j < kSahLevelsPerCheck; ++j)
-            enqueue_large_level(w, level + j, (int)nb, base, leaf_size, nodes, grid_fixed, grid_fixed, n, s);
-    }
+    with_chunk(n, [&](auto chunk) {
+        constexpr uint32_t CHUNK = decltype(chunk)::value;
+        if (grid)
+            k_grid_tasks<CHUNK><<<16, 128, 0, s>>>(w.cells, w.root_ord, n, leaf_size, scene_box_cells, (int)nb,
+                                                   w.lists[0], w.parts, w.small, w.leaves, w.ctl, scene_out);
+        else
+            k_root_task<CHUNK><<<1, 32, 0, s>>>(w.root_ord, n, leaf_size, (int)nb, w.lists[0], w.parts, w.small,
+                                                w.leaves, w.ctl, scene_out);
+        if (n > kSmall) enqueue_root_bins<CHUNK>(w, (int)nb, s);
+    });
+    // large phase: levels are queued in groups and the host reads the next
+    // level's task count (and waits) only between groups; levels past the
+    // tree's depth find no tasks and cost two empty launches.  The first
+    // group is a balanced tree's depth and two levels more, which is all of
+    // most meshes' large phase; a mesh of at most kSmall triangles has none.
+    uint32_t group = 2;
+    while (((uint64_t)kSmall << (group - 2)) < n) ++group;
+    if (n > kSmall)
+        for (uint32_t level = 0;; group = kSahLevelsPerCheck) {
+            with_chunk(n, [&](auto chunk) {
+                enqueue_levels<decltype(chunk)::value>(w, level, group, (int)nb, base, leaf_size, nodes, s);
+            });
+            level += group;
+            SQ_TRY(cudaMemcpyAsync(host_ctl, &w.ctl->level[level % 3u], sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            SQ_TRY(cudaStreamSynchronize(s));
+            if (host_ctl[0] == 0) break;
+        }
     // small phase and leaves
     const uint32_t sg = (uint32_t)sms() * 8u;
     // a single build's small tasks all have at most kSmall = kStage triangles
@@ -1260,12 +1308,15 @@ int build_sah_batch(const float* tris, uint32_t n, const uint32_t* off, uint32_t
         const uint32_t g = min((n + 255) / 256, sm * 8u);
         k_sah_setup_seg<<<g, 256, 0, s>>>(tris, n, off, M, w.tb, w.ids_a, w.root_ord);
     }
-    k_root_tasks_seg<<<(M + 127) / 128, 128, 0, s>>>(w.root_ord, off, M, leaf_size, root0, w.lists[0], w.small,
-                                                      w.leaves, w.ctl);
-    for (uint32_t level = 0; level < kBatchLargeLevels; ++level)
-        enqueue_large_level(w, level, (int)nb, 0u, leaf_size, nodes, sm * 8u, sm * 8u, n, s);
-    k_large_to_small<<<sm, 256, 0, s>>>(w.lists[kBatchLargeLevels & 1], &w.ctl->n_large[kBatchLargeLevels & 1],
-                                       w.small, w.ctl);
+    with_chunk(n, [&](auto chunk) {
+        constexpr uint32_t CHUNK = decltype(chunk)::value;
+        k_root_tasks_seg<CHUNK><<<(M + 3) / 4, 128, 0, s>>>(w.root_ord, off, M, leaf_size, root0, (int)nb, w.lists[0],
+                                                            w.parts, w.small, w.leaves, w.ctl);
+        enqueue_root_bins<CHUNK>(w, (int)nb, s);
+        enqueue_levels<CHUNK>(w, 0, kBatchLargeLevels, (int)nb, 0u, leaf_size, nodes, s);
+    });
+    launch_chained(k_large_to_small, dim3(sm), dim3(256), 0, s, (const Task*)w.lists[kBatchLargeLevels & 1].tasks,
+                   (const unsigned long long*)&w.ctl->level[kBatchLargeLevels % 3], w.small, w.ctl);
     k_small<true><<<sm * 8u, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0,
                                           err);
     k_small<false><<<sm * 8u, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0,
