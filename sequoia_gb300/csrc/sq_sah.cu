@@ -439,92 +439,144 @@ struct PlaneResult {
     float lp[6], rp[6], lc[6], rc[6];  // min xyz, max xyz
 };
 
-// choose_plane (src/builder.cpp:488-523) over nb bins held as encoded words
-// (one bin per lane); every lane returns the result.
-__device__ PlaneResult warp_choose_plane(const uint32_t* __restrict__ bins, int nb)
+__device__ __forceinline__ float redux_min(float v)
 {
-    const int lane = threadIdx.x & 31;
-    float p[6], c[6];
-    uint32_t cnt = 0;
-    if (lane < nb) {
-        const uint32_t* b = bins + lane * kBinWords;
-        cnt = b[12];
-        if (cnt) {
-            for (int a = 0; a < 3; ++a) {
-                p[a] = dec_neg(b[a]); p[3 + a] = dec_pos(b[3 + a]);
-                c[a] = dec_neg(b[6 + a]); c[3 + a] = dec_pos(b[9 + a]);
-            }
-        }
-    }
-    if (lane >= nb || !cnt) {
-        for (int a = 0; a < 3; ++a) { p[a] = FLT_MAX; p[3 + a] = -FLT_MAX; c[a] = FLT_MAX; c[3 + a] = -FLT_MAX; }
-    }
-    // inclusive prefix (l2r) and suffix unions
-    float lp[6], lc[6], sp[6], sc[6];
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float redux_max(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// choose_plane (src/builder.cpp:488-523) for 32 / NBP nodes at once: lane =
+// (node g, bin b), `cnt` and the boxes p of the lane's bin (FLT_MAX boxes
+// where it is empty or b >= nb), c its centroid box.  Every lane of a group
+// returns its node's plane (-1: none), left count, and both sides' boxes.
+// The primitive boxes are scanned from both ends; the centroid boxes are
+// needed at the chosen plane alone and are reduced once it is known.
+template <int NBP>
+__device__ __forceinline__ void choose_planes(int nb, uint32_t cnt, const float* p, const float* c, int& plane,
+                                              uint32_t& nl, float* lp, float* rp, float* lc, float* rc)
+{
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, b = lane & (NBP - 1), g0 = lane - b;
+    float l[6], s[6];
     uint32_t lcnt = cnt, scnt = cnt;
-    for (int k = 0; k < 6; ++k) { lp[k] = p[k]; lc[k] = c[k]; sp[k] = p[k]; sc[k] = c[k]; }
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        float yp[6], yc[6], zp[6], zc[6];
+    for (int k = 0; k < 6; ++k) l[k] = s[k] = p[k];
+    // below 32 bins an empty bin follows the last one: its FLT_MAX box is
+    // part of every right side's union
+    const bool cap = nb < kMaxBins && b == NBP - 1;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (cap) { s[k] = fminf(s[k], FLT_MAX); s[3 + k] = fmaxf(s[3 + k], -FLT_MAX); }
+    }
+#pragma unroll
+    for (int o = 1; o < NBP; o <<= 1) {
+#pragma unroll
         for (int k = 0; k < 6; ++k) {
-            yp[k] = __shfl_up_sync(0xFFFFFFFFu, lp[k], o);
-            yc[k] = __shfl_up_sync(0xFFFFFFFFu, lc[k], o);
-            zp[k] = __shfl_down_sync(0xFFFFFFFFu, sp[k], o);
-            zc[k] = __shfl_down_sync(0xFFFFFFFFu, sc[k], o);
+            const float y = __shfl_up_sync(FULL, l[k], o, NBP), z = __shfl_down_sync(FULL, s[k], o, NBP);
+            if (b >= o) l[k] = k < 3 ? fminf(l[k], y) : fmaxf(l[k], y);
+            if (b + o < NBP) s[k] = k < 3 ? fminf(s[k], z) : fmaxf(s[k], z);
         }
-        const uint32_t ycnt = __shfl_up_sync(0xFFFFFFFFu, lcnt, o);
-        const uint32_t zcnt = __shfl_down_sync(0xFFFFFFFFu, scnt, o);
-        if (lane >= o) {
-            for (int k = 0; k < 3; ++k) {
-                lp[k] = fminf(lp[k], yp[k]); lp[3 + k] = fmaxf(lp[3 + k], yp[3 + k]);
-                lc[k] = fminf(lc[k], yc[k]); lc[3 + k] = fmaxf(lc[3 + k], yc[3 + k]);
-            }
-            lcnt += ycnt;
-        }
-        if (lane + o < 32) {
-            for (int k = 0; k < 3; ++k) {
-                sp[k] = fminf(sp[k], zp[k]); sp[3 + k] = fmaxf(sp[3 + k], zp[3 + k]);
-                sc[k] = fminf(sc[k], zc[k]); sc[3 + k] = fmaxf(sc[3 + k], zc[3 + k]);
-            }
-            scnt += zcnt;
-        }
+        const uint32_t yc = __shfl_up_sync(FULL, lcnt, o, NBP), zc = __shfl_down_sync(FULL, scnt, o, NBP);
+        if (b >= o) lcnt += yc;
+        if (b + o < NBP) scnt += zc;
     }
-    // right side of plane i = suffix(i + 1)
-    float rp[6], rc[6];
-    for (int k = 0; k < 6; ++k) {
-        rp[k] = __shfl_down_sync(0xFFFFFFFFu, sp[k], 1);
-        rc[k] = __shfl_down_sync(0xFFFFFFFFu, sc[k], 1);
-    }
-    const uint32_t rcnt = __shfl_down_sync(0xFFFFFFFFu, scnt, 1);
+    // right side of plane b = suffix(b + 1)
+    float r[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) r[k] = __shfl_down_sync(FULL, s[k], 1, NBP);
+    const uint32_t rcnt = __shfl_down_sync(FULL, scnt, 1, NBP);
     bool valid = false;
     float score = 0.0f;
-    if (lane <= nb - 2) {
-        const float sl = box_sa(lp, lp + 3) * (float)lcnt;
-        const float sr = box_sa(rp, rp + 3) * (float)rcnt;
+    if (b <= nb - 2) {
+        const float sl = box_sa(l, l + 3) * (float)lcnt;
+        const float sr = box_sa(r, r + 3) * (float)rcnt;
         score = sl + sr;
         valid = score < FLT_MAX;
     }
-    // best: smallest score, ties to the highest plane
-    int best = valid ? lane : -1;
-    float bs = score;
+    // smallest score, ties to the highest plane
+    int best = valid ? b : -1;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-        const float os = __shfl_xor_sync(0xFFFFFFFFu, bs, o);
-        if (ob >= 0 && (best < 0 || os < bs || (os == bs && ob > best))) { best = ob; bs = os; }
+    for (int o = NBP / 2; o > 0; o >>= 1) {
+        const int ob = __shfl_xor_sync(FULL, best, o);
+        const float os = __shfl_xor_sync(FULL, score, o);
+        if (ob >= 0 && (best < 0 || os < score || (os == score && ob > best))) { best = ob; score = os; }
     }
-    PlaneResult r;
-    r.plane = best;
-    r.nl = 0;
-    if (best >= 0) {
-        r.nl = __shfl_sync(0xFFFFFFFFu, lcnt, best);
+    plane = best;
+    const int at = g0 + (best < 0 ? 0 : best);
+    nl = __shfl_sync(FULL, lcnt, at);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) { lp[k] = __shfl_sync(FULL, l[k], at); rp[k] = __shfl_sync(FULL, r[k], at); }
+    // centroid boxes of bins [0, best] and (best, ...]
+    const bool in_left = b <= best;
+    if (NBP > 8) {
+        // whole-warp reductions, once per node
+#pragma unroll
+        for (int q = 0; q < 32 / NBP; ++q) {
+            const bool mine = NBP == 32 || g0 == q * NBP;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float x0 = redux_min(mine && in_left ? c[k] : INFINITY);
+                const float x1 = redux_max(mine && in_left ? c[3 + k] : -INFINITY);
+                const float x2 = redux_min(mine && !in_left ? c[k] : INFINITY);
+                const float x3 = redux_max(mine && !in_left ? c[3 + k] : -INFINITY);
+                if (mine) { lc[k] = x0; lc[3 + k] = x1; rc[k] = x2; rc[3 + k] = x3; }
+            }
+        }
+    } else {
+#pragma unroll
         for (int k = 0; k < 6; ++k) {
-            r.lp[k] = __shfl_sync(0xFFFFFFFFu, lp[k], best);
-            r.lc[k] = __shfl_sync(0xFFFFFFFFu, lc[k], best);
-            r.rp[k] = __shfl_sync(0xFFFFFFFFu, rp[k], best);
-            r.rc[k] = __shfl_sync(0xFFFFFFFFu, rc[k], best);
+            const float none = k < 3 ? INFINITY : -INFINITY;
+            lc[k] = in_left ? c[k] : none;
+            rc[k] = in_left ? none : c[k];
+        }
+#pragma unroll
+        for (int o = NBP / 2; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const float y = __shfl_xor_sync(FULL, lc[k], o), z = __shfl_xor_sync(FULL, rc[k], o);
+                lc[k] = k < 3 ? fminf(lc[k], y) : fmaxf(lc[k], y);
+                rc[k] = k < 3 ? fminf(rc[k], z) : fmaxf(rc[k], z);
+            }
         }
     }
+    if (nb < kMaxBins) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { rc[k] = fminf(rc[k], FLT_MAX); rc[3 + k] = fmaxf(rc[3 + k], -FLT_MAX); }
+    }
+}
+
+// A bin's boxes from its encoded words (FLT_MAX boxes when it is empty).
+__device__ __forceinline__ uint32_t load_bin(const uint32_t* bin, bool in_range, float* p, float* c)
+{
+    const uint32_t cnt = in_range ? bin[12] : 0u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        p[a] = c[a] = FLT_MAX;
+        p[3 + a] = c[3 + a] = -FLT_MAX;
+        if (cnt) {
+            p[a] = dec_neg(bin[a]); p[3 + a] = dec_pos(bin[3 + a]);
+            c[a] = dec_neg(bin[6 + a]); c[3 + a] = dec_pos(bin[9 + a]);
+        }
+    }
+    return cnt;
+}
+
+// The plane of one node whose nb bins are given, one bin per lane; every lane
+// returns the result.
+__device__ __forceinline__ PlaneResult warp_choose_plane(const uint32_t* __restrict__ bins, int nb)
+{
+    const int lane = threadIdx.x & 31;
+    PlaneResult r;
+    float p[6], c[6];
+    const uint32_t cnt = load_bin(bins + lane * kBinWords, lane < nb, p, c);
+    choose_planes<32>(nb, cnt, p, c, r.plane, r.nl, r.lp, r.rp, r.lc, r.rc);
     return r;
 }
 
@@ -838,80 +890,264 @@ __global__ void k_emit_leaves(const LeafRange* __restrict__ leaves, const Ctl* _
 //
 // A subtree of at most kStage triangles (every small task of a single build:
 // a task turns small at kSmall or fewer) is staged once in the warp's shared
-// memory -- each triangle's box and id -- and its nodes are binned,
-// partitioned and emitted from there: only 16-bit local indices move between
-// the two orders (the buffer parity of the global ids, which the staged
-// subtree no longer writes), and leaves read their boxes from the stage.  A
-// node then costs shared-memory latency instead of two dependent global
-// round trips per 32 triangles.  Larger small tasks (leftovers of the
-// batched build's fixed large levels) read and write the global buffers.
+// memory -- each triangle's box and id -- and built from there: only local
+// indices move, and leaves read their boxes from the stage.
+//
+// The warp's nodes wait on a stack and are split G = 32 / NBP at a time (NBP:
+// the bin count rounded up to 8, 16 or 32), lane = (node, bin) while the
+// planes are swept and lane = triangle while the nodes' triangles are binned
+// and partitioned, four rounds of 32 at most for all of them together.  A
+// node holds 5 to 30 triangles mostly, so one node at a time left most lanes
+// idle in the binning and 24 of 32 in a sweep of 8 bins; the sweep, a chain
+// of shuffles, was what bounded a node.  The order of the stack does not
+// matter: a node's records go to slots that its range gives.
+//
+// Larger small tasks (leftovers of the batched build's fixed large levels)
+// are split by k_small_big, one node at a time, in the global buffers.
 constexpr uint32_t kStage = 128;
 
+struct SmallNode {
+    float p[6], c[6];  // primitive and centroid boxes (min xyz, max xyz)
+    uint32_t slot;
+    uint16_t begin, count;  // positions in the subtree
+};
+static_assert(sizeof(SmallNode) == 56, "SmallNode is 56 bytes");
+
 struct SmallStage {
-    float4 box[kStage][2];      // min xyz, max xyz of local triangle k
-    uint32_t gid[kStage];       // its triangle id
-    uint16_t loc[2][kStage];    // local triangles in the order of buffer parity p
+    float4 box[kStage][2];                   // min xyz, id; max xyz
+    uint32_t bins[kMaxBins * kBinWords];
+    SmallNode stack[kStage / 2];             // waiting nodes are disjoint and hold two triangles or more
+    uint8_t loc[kStage];                     // the triangle at each position
 };
 
-template <bool STAGED>
-__device__ void small_subtree(Task cur, SmallStage& sg, Task* st, uint32_t* wb, uint32_t* __restrict__ ids_a,
-                              uint32_t* __restrict__ ids_b, const float4* __restrict__ tb, int nb, uint32_t leaf_size,
-                              uint32_t base, Node* __restrict__ nodes, uint32_t leaf0, uint32_t* err)
+// One small task from the stage.
+template <int NBP>
+__device__ void staged_subtree(const Task& root, SmallStage& sg, const uint32_t* __restrict__ ids,
+                               const float4* __restrict__ tb, int nb, uint32_t leaf_size, uint32_t base,
+                               Node* __restrict__ nodes, uint32_t leaf0)
 {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t root_begin = cur.begin;
-    // triangle at position `pos` (global) of the order of parity p
-    auto get = [&](uint32_t p, uint32_t pos, uint32_t& id, uint16_t& li, float* mn, float* mx) {
-        if (STAGED) {
-            li = sg.loc[p][pos - root_begin];
-            const float4 a = sg.box[li][0], b = sg.box[li][1];
-            mn[0] = a.x; mn[1] = a.y; mn[2] = a.z;
-            mx[0] = b.x; mx[1] = b.y; mx[2] = b.z;
-            id = sg.gid[li];
-        } else {
-            li = 0;
-            id = (p ? ids_b : ids_a)[pos];
-            load_box(tb, id, mn, mx);
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    constexpr int G = 32 / NBP;
+    constexpr int kRounds = kStage / 32;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t b = lane & (NBP - 1), g = lane / NBP;
+    const uint32_t rb = root.begin;
+    for (uint32_t j = lane; j < root.count; j += 32) {
+        const uint32_t id = ids[rb + j];
+        float4 lo = __ldg(tb + 2ull * id);
+        lo.w = __uint_as_float(id);
+        sg.box[j][0] = lo;
+        sg.box[j][1] = __ldg(tb + 2ull * id + 1);
+        sg.loc[j] = (uint8_t)j;
+    }
+    if (lane == 0) {
+        SmallNode& s = sg.stack[0];
+        for (int k = 0; k < 3; ++k) {
+            s.p[k] = root.pmn[k]; s.p[3 + k] = root.pmx[k];
+            s.c[k] = root.cmn[k]; s.c[3 + k] = root.cmx[k];
         }
-    };
-    auto put = [&](uint32_t p, uint32_t pos, uint32_t id, uint16_t li) {
-        if (STAGED) sg.loc[p][pos - root_begin] = li;
-        else (p ? ids_b : ids_a)[pos] = id;
-    };
-    // leaf records of positions [b, b + c) of parity p (warp_emit_leaf's records)
-    auto emit_leaf = [&](uint32_t p, uint32_t b, uint32_t c, uint32_t slot, uint32_t flags, const float* pmn,
-                         const float* pmx) {
-        for (uint32_t j = lane; j < c; j += 32) {
-            uint32_t id;
-            uint16_t li;
-            Box bb;
-            get(p, b + j, id, li, bb.mn, bb.mx);
-            store_node(nodes + leaf0 + b + j, bb, id, 1u, kLeafFlag);
-            if (c == 1 && !(flags & 2u)) store_node(nodes + slot, bb, id, 1u, kLeafFlag);
+        s.slot = root.slot; s.begin = 0; s.count = (uint16_t)root.count;
+    }
+    __syncwarp();
+    uint32_t sp = 1;
+    while (sp) {
+        // the top m nodes of the stack, one per lane group (every one is
+        // splittable: more than leaf_size triangles, centroid area > 0)
+        const uint32_t m = min((uint32_t)G, sp);
+        const bool act = g < m;
+        const SmallNode& nd = sg.stack[sp - m + (act ? g : 0u)];
+        const uint32_t begin = nd.begin, count = act ? nd.count : 0u, slot = nd.slot;
+        float np[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) np[k] = nd.p[k];
+        const int axis = choose_axis(nd.c, nd.c + 3);
+        const float cmin = sel(nd.c, axis);
+        const float k1 = bin_k1(nb, sel(nd.c + 3, axis) - cmin);
+        // the group's triangles are [start, start + count) of the warp's total
+        uint32_t starts[G], total = 0, start = 0;
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            starts[q] = total;
+            if (g == (uint32_t)q) start = total;
+            total += __shfl_sync(FULL, count, q * NBP);
         }
-        if (lane == 0 && (c != 1 || (flags & 2u))) {
-            if (c > 65535u) { raise_error(err, SQ_DEVERR_NODE_COUNT); return; }
+        for (uint32_t j = lane; j < (uint32_t)(kMaxBins * kBinWords / 4); j += 32)
+            reinterpret_cast<uint4*>(sg.bins)[j] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+        // bin: lane = triangle
+        uint32_t el[kRounds];  // the triangle's place in the stage, its bin and its node's group
+#pragma unroll
+        for (int it = 0; it < kRounds; ++it) {
+            el[it] = 0;
+            if (32u * it < total) {  // warp-uniform
+                const uint32_t e = 32u * it + lane;
+                uint32_t ge = 0;
+#pragma unroll
+                for (int q = 1; q < G; ++q) ge += ((uint32_t)q < m && e >= starts[q]) ? 1u : 0u;
+                const int src = (int)ge * NBP;
+                const uint32_t at = __shfl_sync(FULL, (begin - start) & 0xFFFFu, src);
+                const int ax = __shfl_sync(FULL, axis, src);
+                const float cm = __shfl_sync(FULL, cmin, src), kk = __shfl_sync(FULL, k1, src);
+                if (e < total) {
+                    const uint32_t li = sg.loc[(at + e) & 0xFFFFu];
+                    const float4 lo = sg.box[li][0], hi = sg.box[li][1];
+                    const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
+                    float cc[3];
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) cc[a] = (mn[a] + mx[a]) * 0.5f;
+                    const uint32_t bin = (uint32_t)bin_of(kk, sel(cc, ax), cm, nb);
+                    el[it] = li | (bin << 8) | (ge << 16);
+                    uint32_t* w = sg.bins + (ge * NBP + bin) * kBinWords;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        atomicMax(w + a, float_to_ordered(-mn[a]));
+                        atomicMax(w + 3 + a, float_to_ordered(mx[a]));
+                        atomicMax(w + 6 + a, float_to_ordered(-cc[a]));
+                        atomicMax(w + 9 + a, float_to_ordered(cc[a]));
+                    }
+                    atomicAdd(w + 12, 1u);
+                }
+            }
+        }
+        __syncwarp();
+        // sweep: lane = (node, bin)
+        int plane;
+        uint32_t nl;
+        float lp[6], rp[6], lc[6], rc[6];
+        {
+            float p[6], c[6];
+            const uint32_t cnt = load_bin(sg.bins + lane * kBinWords, act && (int)b < nb, p, c);
+            choose_planes<NBP>(nb, cnt, p, c, plane, nl, lp, rp, lc, rc);
+        }
+        // the node's records and its children: lane 0 of a group has the
+        // node, lanes 1 and 2 the left and the right child
+        const bool has = act && plane >= 0 && nl != 0 && nl != count;
+        const uint32_t nr = count - nl, q = rb + begin + nl;
+        const bool leaf_l = has && (nl <= leaf_size || !(box_sa(lc, lc + 3) > 0.0f));
+        const bool leaf_r = has && (nr <= leaf_size || !(box_sa(rc, rc + 3) > 0.0f));
+        const bool right = b == 2;
+        const bool push = has && (b == 1 || right) && !(right ? leaf_r : leaf_l);
+        const uint32_t pushes = __ballot_sync(FULL, push);
+        sp -= m;
+        if (act && b <= 2) {
+            const uint32_t cn = b == 0 ? count : (right ? nr : nl);
             Box pb;
-            for (int a = 0; a < 3; ++a) { pb.mn[a] = pmn[a]; pb.mx[a] = pmx[a]; }
-            store_node(nodes + slot, pb, leaf0 + b, c, 0);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                pb.mn[a] = b == 0 ? np[a] : (right ? rp[a] : lp[a]);
+                pb.mx[a] = b == 0 ? np[3 + a] : (right ? rp[3 + a] : lp[3 + a]);
+            }
+            const uint32_t cslot = b == 0 ? slot : base + 2u * q + (right ? 1u : 0u);
+            if (push) {
+                SmallNode& s = sg.stack[sp + __popc(pushes & lt)];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    s.p[a] = pb.mn[a]; s.p[3 + a] = pb.mx[a];
+                    s.c[a] = right ? rc[a] : lc[a]; s.c[3 + a] = right ? rc[3 + a] : lc[3 + a];
+                }
+                s.slot = cslot;
+                s.begin = (uint16_t)(begin + (right ? nl : 0u));
+                s.count = (uint16_t)cn;
+            } else if (b == 0 && has) {
+                store_node(nodes + slot, pb, base + 2u * q, 2u, 0);
+            } else if (b == 0 || (has && cn != 1)) {
+                // a leaf's range: this node's when no plane scored below
+                // FLT_MAX, else the child's (a leaf child of one triangle has
+                // that triangle's record at its slot)
+                store_node(nodes + cslot, pb, leaf0 + rb + begin + (right ? nl : 0u), cn, 0);
+            }
         }
-    };
-    if (STAGED) {
-        const uint32_t* in0 = (cur.flags & 1u) ? ids_b : ids_a;
-        for (uint32_t j = lane; j < cur.count; j += 32) {
-            const uint32_t id = in0[cur.begin + j];
-            sg.box[j][0] = __ldg(tb + 2ull * id);
-            sg.box[j][1] = __ldg(tb + 2ull * id + 1);
-            sg.gid[j] = id;
-            sg.loc[cur.flags & 1u][j] = (uint16_t)j;
+        sp += __popc(pushes);
+        // partition, stably: lane = triangle again
+        uint32_t lb[kRounds], before[kRounds];
+        const uint32_t say = (has ? 1u : 0u) | (leaf_l ? 2u : 0u) | (leaf_r ? 4u : 0u) | ((uint32_t)(plane & 31) << 3) |
+                             (nl << 8) | (begin << 16) | (start << 24);
+        uint32_t sum = 0;
+#pragma unroll
+        for (int it = 0; it < kRounds; ++it) {
+            lb[it] = 0;
+            before[it] = sum;
+            if (32u * it < total) {
+                const uint32_t x = __shfl_sync(FULL, say, (int)(el[it] >> 16) * NBP);
+                lb[it] = __ballot_sync(FULL, 32u * it + lane < total && (x & 1u) && ((el[it] >> 8) & 0xFFu) <= ((x >> 3) & 31u));
+                sum += __popc(lb[it]);
+            }
+        }
+        // left triangles before this group's first
+        uint32_t lstart = 0;
+#pragma unroll
+        for (int it = 0; it < kRounds; ++it)
+            if (start >= 32u * it && start < 32u * it + 32u) lstart = before[it] + __popc(lb[it] & ((1u << (start & 31u)) - 1u));
+        const uint32_t say2 = lstart | (count << 8);
+#pragma unroll
+        for (int it = 0; it < kRounds; ++it) {
+            if (32u * it >= total) break;
+            const uint32_t e = 32u * it + lane;
+            const int src = (int)(el[it] >> 16) * NBP;
+            const uint32_t x = __shfl_sync(FULL, say, src), y = __shfl_sync(FULL, say2, src);
+            if (e < total) {
+                const bool split = x & 1u, left = (lb[it] >> lane) & 1u;
+                const uint32_t xnl = (x >> 8) & 0xFFu, xbegin = (x >> 16) & 0xFFu, rel = e - (x >> 24);
+                const uint32_t lr = before[it] + __popc(lb[it] & lt) - (y & 0xFFu);
+                const uint32_t pos = xbegin + (split ? (left ? lr : xnl + rel - lr) : rel);
+                const uint32_t li = el[it] & 0xFFu;
+                sg.loc[pos] = (uint8_t)li;
+                if (!split || (x & (left ? 2u : 4u))) {
+                    const float4 lo = sg.box[li][0], hi = sg.box[li][1];
+                    Box bb;
+                    bb.mn[0] = lo.x; bb.mn[1] = lo.y; bb.mn[2] = lo.z;
+                    bb.mx[0] = hi.x; bb.mx[1] = hi.y; bb.mx[2] = hi.z;
+                    const uint32_t id = __float_as_uint(lo.w);
+                    store_node(nodes + leaf0 + rb + pos, bb, id, 1u, kLeafFlag);
+                    if (split && (left ? xnl : (y >> 8) - xnl) == 1u)
+                        store_node(nodes + base + 2u * (rb + xbegin + xnl) + (left ? 0u : 1u), bb, id, 1u, kLeafFlag);
+                }
+            }
         }
         __syncwarp();
     }
+}
+
+// One warp per small task of at most kStage triangles (k_small_big takes the
+// others; each kernel pops the shared list with its own counter).
+template <int NBP>
+__global__ void __launch_bounds__(128) k_small(const Task* __restrict__ small, Ctl* ctl,
+                                               const uint32_t* __restrict__ ids_a, const uint32_t* __restrict__ ids_b,
+                                               const float4* __restrict__ tb, int nb, uint32_t leaf_size, uint32_t base,
+                                               Node* __restrict__ nodes, uint32_t leaf0)
+{
+    __shared__ __align__(16) SmallStage s_stage[4];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t total = ctl->n_small;
+    for (;;) {
+        uint32_t ti = 0;
+        if (lane == 0) ti = atomicAdd(&ctl->small_pop, 1u);
+        ti = __shfl_sync(0xFFFFFFFFu, ti, 0);
+        if (ti >= total) return;
+        const Task t = small[ti];
+        if (t.count > kStage) continue;  // warp-uniform
+        staged_subtree<NBP>(t, s_stage[warp], (t.flags & 1u) ? ids_b : ids_a, tb, nb, leaf_size, base, nodes, leaf0);
+    }
+}
+
+// A small task of more than kStage triangles: one warp, one node at a time,
+// smaller child first (stack depth O(log n)), in the global buffers.
+__device__ void big_subtree(Task cur, Task* st, uint32_t* wb, uint32_t* __restrict__ ids_a, uint32_t* __restrict__ ids_b,
+                            const float4* __restrict__ tb, int nb, uint32_t leaf_size, uint32_t base,
+                            Node* __restrict__ nodes, uint32_t leaf0, uint32_t* err)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    auto emit_leaf = [&](const Task& t) {
+        warp_emit_leaf((t.flags & 1u) ? ids_b : ids_a, t.begin, t.count, t.slot, t.flags, t.pmn, t.pmx, tb, nodes, leaf0,
+                       err);
+    };
     int sp = 0;
     for (;;) {
         // cur is splittable (count > leaf_size, centroid area > 0)
         const uint32_t pin = cur.flags & 1u, pout = pin ^ 1u;
+        const uint32_t* in = pin ? ids_b : ids_a;
+        uint32_t* out = pin ? ids_a : ids_b;
         const int axis = choose_axis(cur.cmn, cur.cmx);
         const float cmin = sel(cur.cmn, axis);
         const float k1 = bin_k1(nb, sel(cur.cmx, axis) - cmin);
@@ -922,9 +1158,7 @@ __device__ void small_subtree(Task cur, SmallStage& sg, Task* st, uint32_t* wb, 
             float mn[3], mx[3], cc[3];
             int bin = nb;
             if (j < cur.count) {
-                uint32_t id;
-                uint16_t li;
-                get(pin, cur.begin + j, id, li, mn, mx);
+                load_box(tb, in[cur.begin + j], mn, mx);
                 for (int a = 0; a < 3; ++a) cc[a] = (mn[a] + mx[a]) * 0.5f;
                 bin = bin_of(k1, sel(cc, axis), cmin, nb);
             } else {
@@ -937,7 +1171,7 @@ __device__ void small_subtree(Task cur, SmallStage& sg, Task* st, uint32_t* wb, 
         bool have_next = false;
         if (r.plane < 0 || r.nl == 0 || r.nl == cur.count) {
             // no plane scored below FLT_MAX: leaf
-            emit_leaf(pin, cur.begin, cur.count, cur.slot, cur.flags, cur.pmn, cur.pmx);
+            emit_leaf(cur);
         } else {
             const uint32_t q = cur.begin + r.nl;
             if (lane == 0) {
@@ -951,19 +1185,19 @@ __device__ void small_subtree(Task cur, SmallStage& sg, Task* st, uint32_t* wb, 
                 const uint32_t j = j0 + lane;
                 const bool valid = j < cur.count;
                 uint32_t id = 0;
-                uint16_t li = 0;
                 bool left = false;
                 if (valid) {
                     float mn[3], mx[3];
-                    get(pin, cur.begin + j, id, li, mn, mx);
+                    id = in[cur.begin + j];
+                    load_box(tb, id, mn, mx);
                     const float cc = (sel(mn, axis) + sel(mx, axis)) * 0.5f;
                     left = bin_of(k1, cc, cmin, nb) <= r.plane;
                 }
                 const uint32_t lb = __ballot_sync(0xFFFFFFFFu, valid && left);
                 const uint32_t rb = __ballot_sync(0xFFFFFFFFu, valid && !left);
                 if (valid) {
-                    if (left) put(pout, cur.begin + lc + __popc(lb & lt), id, li);
-                    else put(pout, q + rc + __popc(rb & lt), id, li);
+                    if (left) out[cur.begin + lc + __popc(lb & lt)] = id;
+                    else out[q + rc + __popc(rb & lt)] = id;
                 }
                 lc += __popc(lb);
                 rc += __popc(rb);
@@ -974,7 +1208,7 @@ __device__ void small_subtree(Task cur, SmallStage& sg, Task* st, uint32_t* wb, 
             bool split_ch[2];
             for (int k = 0; k < 2; ++k) {
                 split_ch[k] = !(ch[k].count <= leaf_size || !(box_sa(ch[k].cmn, ch[k].cmx) > 0.0f));
-                if (!split_ch[k]) emit_leaf(pout, ch[k].begin, ch[k].count, ch[k].slot, ch[k].flags, ch[k].pmn, ch[k].pmx);
+                if (!split_ch[k]) emit_leaf(ch[k]);
             }
             if (split_ch[0] && split_ch[1]) {
                 const int small_k = ch[0].count <= ch[1].count ? 0 : 1;
@@ -1000,35 +1234,25 @@ __device__ void small_subtree(Task cur, SmallStage& sg, Task* st, uint32_t* wb, 
             __syncwarp();
         }
     }
-    __syncwarp();  // the stage is reused by the warp's next subtree
 }
 
-// One warp per small task: STAGED takes the tasks of at most kStage
-// triangles (all of a single build's), the other kernel the rest (leftovers
-// of the batched build's fixed large levels); each kernel pops the shared
-// list with its own counter and skips the other's tasks.  Two kernels, so
-// the staged one keeps its own, smaller register count.
-template <bool STAGED>
-__global__ void __launch_bounds__(128) k_small(const Task* __restrict__ small, Ctl* ctl, uint32_t* __restrict__ ids_a,
-                                               uint32_t* __restrict__ ids_b, const float4* __restrict__ tb, int nb,
-                                               uint32_t leaf_size, uint32_t base, Node* __restrict__ nodes,
-                                               uint32_t leaf0, uint32_t* err)
+__global__ void __launch_bounds__(128) k_small_big(const Task* __restrict__ small, Ctl* ctl, uint32_t* __restrict__ ids_a,
+                                                   uint32_t* __restrict__ ids_b, const float4* __restrict__ tb, int nb,
+                                                   uint32_t leaf_size, uint32_t base, Node* __restrict__ nodes,
+                                                   uint32_t leaf0, uint32_t* err)
 {
     __shared__ uint32_t s_bins[4][kMaxBins * kBinWords];
     __shared__ Task s_stack[4][kStackDepth];
-    __shared__ SmallStage s_stage[STAGED ? 4 : 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t total = ctl->n_small;
-    uint32_t* pop = STAGED ? &ctl->small_pop : &ctl->big_pop;
     for (;;) {
         uint32_t ti = 0;
-        if (lane == 0) ti = atomicAdd(pop, 1u);
+        if (lane == 0) ti = atomicAdd(&ctl->big_pop, 1u);
         ti = __shfl_sync(0xFFFFFFFFu, ti, 0);
         if (ti >= total) return;
         const Task cur = small[ti];
-        if ((cur.count <= kStage) != STAGED) continue;  // warp-uniform
-        small_subtree<STAGED>(cur, s_stage[STAGED ? warp : 0], s_stack[warp], s_bins[warp], ids_a, ids_b, tb, nb,
-                              leaf_size, base, nodes, leaf0, err);
+        if (cur.count <= kStage) continue;  // warp-uniform
+        big_subtree(cur, s_stack[warp], s_bins[warp], ids_a, ids_b, tb, nb, leaf_size, base, nodes, leaf0, err);
     }
 }
 
@@ -1131,6 +1355,13 @@ void enqueue_levels(const SahWs& w, uint32_t level, uint32_t count, int nb, uint
                        w.ids_a, w.ids_b, w.bin_a, w.bin_b, (const uint32_t*)w.chunk_left, (const float4*)w.tb, nb,
                        w.ctl);
     }
+}
+
+void launch_small(const SahWs& w, int nb, uint32_t leaf_size, uint32_t base, Node* nodes, uint32_t leaf0, cudaStream_t s)
+{
+    const uint32_t grid = (uint32_t)sms() * 8u;
+    auto kernel = nb <= 8 ? k_small<8> : nb <= 16 ? k_small<16> : k_small<32>;
+    kernel<<<grid, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, nb, leaf_size, base, nodes, leaf0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1278,8 +1509,7 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
     const uint32_t sg = (uint32_t)sms() * 8u;
     // a single build's small tasks all have at most kSmall = kStage triangles
     static_assert(kSmall <= kStage, "every small task of a single build is staged");
-    k_small<true><<<sg, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, base, nodes, leaf0,
-                                     err);
+    launch_small(w, (int)nb, leaf_size, base, nodes, leaf0, s);
     k_emit_leaves<<<sg, 256, 0, s>>>(w.leaves, w.ctl, w.ids_a, w.ids_b, w.tb, nodes, leaf0, err);
     if (grid) k_grid_heap<<<1, 32, 0, s>>>(nodes);
     return (int)cudaGetLastError();
@@ -1317,10 +1547,9 @@ int build_sah_batch(const float* tris, uint32_t n, const uint32_t* off, uint32_t
     });
     launch_chained(k_large_to_small, dim3(sm), dim3(256), 0, s, (const Task*)w.lists[kBatchLargeLevels & 1].tasks,
                    (const unsigned long long*)&w.ctl->level[kBatchLargeLevels % 3], w.small, w.ctl);
-    k_small<true><<<sm * 8u, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0,
-                                          err);
-    k_small<false><<<sm * 8u, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0,
-                                           err);
+    launch_small(w, (int)nb, leaf_size, 0u, nodes, leaf0, s);
+    k_small_big<<<sm * 8u, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0,
+                                        err);
     k_emit_leaves<<<sm * 8u, 256, 0, s>>>(w.leaves, w.ctl, w.ids_a, w.ids_b, w.tb, nodes, leaf0, err);
     return (int)cudaGetLastError();
 #undef SQ_TRY
