@@ -248,16 +248,19 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
     }
     __syncwarp();
     if (active && k == 0) {
-        uint32_t counts = 0;
+        uint32_t counts = 0, ranks = 0;  // a rank at an empty or leaf slot is not read
 #pragma unroll
-        for (int q = 0; q < 8; ++q) counts |= sm.cnt[g][q] << (4 * q);
+        for (int q = 0; q < 8; ++q) {
+            counts |= sm.cnt[g][q] << (4 * q);
+            ranks |= (uint32_t)__popc(imask & ((1u << q) - 1u)) << (8 + 3 * q);
+        }
         sn.ox = self.mnx; sn.oy = self.mny; sn.oz = self.mnz;
         sn.exps_imask = (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) |
                         (imask << 24);
         sn.child_base = child_base;
-        sn.tri_base = tri_base;
+        sn.tri_base = (tri_base & kTriBaseMask) | ((uint32_t)__popc(valid) << 27);
         sn.counts = counts;
-        sn.valid = valid;
+        sn.valid = valid | ranks;
     }
     __syncwarp();
     if (active) {

@@ -228,22 +228,21 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
     return r;
 }
 
-// Sum of the 4-bit triangle counts of slots [0, k) of a node's count word.
-__device__ __forceinline__ uint32_t slots_below(uint32_t counts, int k)
-{
-    const uint32_t x = k >= 8 ? counts : counts & ((1u << (4 * k)) - 1u);
-    const uint32_t s = (x & 0x0F0F0F0Fu) + ((x >> 4) & 0x0F0F0F0Fu);
-    return (s * 0x01010101u) >> 24;
-}
+// What a visit keeps of a node's header words.
+struct Head8 {
+    uint32_t imask, child_base, tri_base, counts, valid;
+};
 
 // Stack entry of child slot k: an inner child's node index, or a leaf
 // child's triangle range (bit 31, count in bits 27-30, first triangle).
 // Computed only for children that pass their box test.
-__device__ __forceinline__ uint32_t child_entry(uint32_t imask, uint32_t child_base, uint32_t counts, uint32_t tri_base,
-                                                int k)
+__device__ __forceinline__ uint32_t child_entry(const Head8& h, int k)
 {
-    if ((imask >> k) & 1u) return child_base + __popc(imask & ((1u << k) - 1u));
-    return 0x80000000u | (((counts >> (4 * k)) & 0xFu) << 27) | (tri_base + slots_below(counts, k));
+    if ((h.imask >> k) & 1u) return h.child_base + ((h.valid >> (8 + 3 * k)) & 7u);
+    // triangles of the slots below k
+    const uint32_t x = h.counts & ((1u << (4 * k)) - 1u);
+    const uint32_t s = (((x & 0x0F0F0F0Fu) + ((x >> 4) & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
+    return 0x80000000u | (((h.counts >> (4 * k)) & 0xFu) << 27) | ((h.tri_base & kTriBaseMask) + s);
 }
 
 // Entry and exit distances of child slot k (word w = k / 4, byte j = k % 4).
@@ -289,6 +288,121 @@ __device__ __forceinline__ void child_span(const uint32_t* qa, const uint32_t* q
     }
 }
 
+// Node `cur` as the box tests take it: header, origin and steps, and the
+// packed planes of each axis, near and far (SIGNED) or low and high.
+struct Node8Regs {
+    Head8 h;
+    float org[3], sc[3];
+    uint32_t qa[6], qb[6];
+};
+
+template <bool SIGNED>
+__device__ __forceinline__ void load_node8(const Node8* __restrict__ nodes, uint32_t cur, const Pre8& rp, Node8Regs& d)
+{
+    const float4* p = reinterpret_cast<const float4*>(nodes + cur);
+    const float4 w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2), w3 = __ldg(p + 3), w4 = __ldg(p + 4);
+    d.org[0] = w0.x; d.org[1] = w0.y; d.org[2] = w0.z;
+    const uint32_t ei = __float_as_uint(w0.w);
+    d.sc[0] = pow2f((int)(ei & 0xFFu) - 127);
+    d.sc[1] = pow2f((int)((ei >> 8) & 0xFFu) - 127);
+    d.sc[2] = pow2f((int)((ei >> 16) & 0xFFu) - 127);
+    d.h.imask = ei >> 24;
+    d.h.child_base = __float_as_uint(w1.x);
+    d.h.tri_base = __float_as_uint(w1.y);
+    d.h.counts = __float_as_uint(w1.z);
+    d.h.valid = __float_as_uint(w1.w);
+    // q words: qlo x (2 words: slots 0-3, 4-7), qlo y, qlo z, qhi x, qhi y, qhi z
+    const uint32_t q[12] = {__float_as_uint(w2.x), __float_as_uint(w2.y), __float_as_uint(w2.z), __float_as_uint(w2.w),
+                            __float_as_uint(w3.x), __float_as_uint(w3.y), __float_as_uint(w3.z), __float_as_uint(w3.w),
+                            __float_as_uint(w4.x), __float_as_uint(w4.y), __float_as_uint(w4.z), __float_as_uint(w4.w)};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const bool neg = SIGNED && rp.inv[a] < 0.0f;
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const uint32_t lo = q[a * 2 + w], hi = q[6 + a * 2 + w];
+            d.qa[a * 2 + w] = neg ? hi : lo;
+            d.qb[a * 2 + w] = neg ? lo : hi;
+        }
+    }
+}
+
+// Mask of the hit child slots (entry not beyond `lim`); each slot's entry
+// distance goes to s_n[32 * slot], a column of the warp's shared memory.
+template <bool AFF, bool SIGNED>
+__device__ __forceinline__ uint32_t test_children(const Node8Regs& d, const Pre8& rp, const float* A, const float* Cn,
+                                                  const float* Cf, float lim, float* __restrict__ s_n)
+{
+    uint32_t mask = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float n, f;
+        child_span<AFF, SIGNED>(d.qa, d.qb, k >> 2, (uint32_t)(k & 3), A, Cn, Cf, d.sc, d.org, rp, n, f);
+        s_n[32 * k] = n;
+        if (n <= f && n <= lim) mask |= 1u << k;
+    }
+    return mask & d.h.valid & 0xFFu;
+}
+
+// One more hit child, of a larger slot than those before it: the nearest is
+// kept aside, the others go onto the stack above `seg`, far (bottom) to near
+// (top); equal distances keep slot order.  A new nearest displaces the old
+// one, which is then the nearest of the pushed (and of a smaller slot than
+// any of its distance): it goes on top.  Any other hit goes below the
+// entries that are not farther.
+__device__ __forceinline__ void add_hit(uint32_t ent, float n, uint32_t& near_e, float& near_t, uint2* st, int seg,
+                                        int& sp)
+{
+    if (near_e == kNoHit) {
+        near_e = ent;
+        near_t = n;
+    } else if (n < near_t) {
+        st[sp++] = make_uint2(near_e, __float_as_uint(near_t));
+        near_e = ent;
+        near_t = n;
+    } else {
+        int b = sp - 1;
+        while (b >= seg) {
+            const uint2 o = st[b];
+            if (__uint_as_float(o.y) > n) break;
+            st[b + 1] = o;
+            --b;
+        }
+        st[b + 1] = make_uint2(ent, __float_as_uint(n));
+        ++sp;
+    }
+}
+
+// Tests and orders node `cur`'s children: returns the nearest hit (kNoHit:
+// none), the others are on the stack.  The tests only make a mask and the
+// hits are ordered in a loop over its bits, one iteration per hit of the lane
+// with the most: incoherent rays hit about one slot each, but together nearly
+// every slot, so ordering in the unrolled test loop ran eight bodies a visit
+// with two or three lanes in each.
+template <bool SIGNED>
+__device__ __forceinline__ uint32_t visit_children(const Node8* __restrict__ nodes, uint32_t cur, const Pre8& rp,
+                                                   float lim, float* __restrict__ s_n, uint2* st, int& sp,
+                                                   uint32_t& tests)
+{
+    Node8Regs d;
+    load_node8<SIGNED>(nodes, cur, rp, d);
+    tests += d.h.tri_base >> 27;
+    float A[3], Cn[3], Cf[3];
+    const bool aff = SIGNED && node_affine(d.org, d.sc, rp, A, Cn, Cf);
+    uint32_t mask = aff ? test_children<true, SIGNED>(d, rp, A, Cn, Cf, lim, s_n)
+                        : test_children<false, SIGNED>(d, rp, A, Cn, Cf, lim, s_n);
+    uint32_t near_e = kNoHit;
+    float near_t = 0.0f;
+    const int seg = sp;
+    while (mask) {
+        const int k = __ffs(mask) - 1;
+        mask &= mask - 1u;
+        add_hit(child_entry(d.h, k), s_n[32 * k], near_e, near_t, st,
+                seg, sp);
+    }
+    return near_e;
+}
+
 struct Res8 {
     uint32_t id;
     float t;
@@ -307,43 +421,19 @@ __device__ Res8 trace8_impl(const Node8* __restrict__ nodes, uint32_t root, cons
     uint32_t best = kNoHit;
     uint32_t tests = 0, ttests = 0, nvis = 0;
     bool overflow = false;
-    uint32_t st_e[kStack8];
-    float st_t[kStack8];
+    uint2 st[kStack8];
     int sp = 0;
     uint32_t cur = root;
     bool have = true;
-    // SIGNED: which of the (lo, hi) word pairs holds the near plane, per axis
-    const bool neg[3] = {rp.inv[0] < 0.0f, rp.inv[1] < 0.0f, rp.inv[2] < 0.0f};
     while (have) {
-        const float4* p = reinterpret_cast<const float4*>(nodes + cur);
-        const float4 w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2), w3 = __ldg(p + 3), w4 = __ldg(p + 4);
+        Node8Regs d;
+        load_node8<SIGNED>(nodes, cur, rp, d);
         nvis++;
-        const float org[3] = {w0.x, w0.y, w0.z};
-        const uint32_t ei = __float_as_uint(w0.w);
-        const float sc[3] = {pow2f((int)(ei & 0xFFu) - 127), pow2f((int)((ei >> 8) & 0xFFu) - 127),
-                             pow2f((int)((ei >> 16) & 0xFFu) - 127)};
-        const uint32_t imask = ei >> 24;
-        const uint32_t child_base = __float_as_uint(w1.x), tri_base = __float_as_uint(w1.y);
-        const uint32_t counts = __float_as_uint(w1.z), valid = __float_as_uint(w1.w);
-        // q words: qlo x (2 words: slots 0-3, 4-7), qlo y, qlo z, qhi x, qhi y, qhi z
-        const uint32_t q[12] = {__float_as_uint(w2.x), __float_as_uint(w2.y), __float_as_uint(w2.z), __float_as_uint(w2.w),
-                                __float_as_uint(w3.x), __float_as_uint(w3.y), __float_as_uint(w3.z), __float_as_uint(w3.w),
-                                __float_as_uint(w4.x), __float_as_uint(w4.y), __float_as_uint(w4.z), __float_as_uint(w4.w)};
-        uint32_t qa[6], qb[6];  // SIGNED: near and far words; otherwise lo and hi
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const uint32_t lo = q[a * 2 + w], hi = q[6 + a * 2 + w];
-                qa[a * 2 + w] = (SIGNED && neg[a]) ? hi : lo;
-                qb[a * 2 + w] = (SIGNED && neg[a]) ? lo : hi;
-            }
-        }
         uint32_t hn[8];
         float ht[8];
         int nh = 0;
         float A[3], Cn[3], Cf[3];
-        const bool aff = SIGNED && node_affine(org, sc, rp, A, Cn, Cf);
+        const bool aff = SIGNED && node_affine(d.org, d.sc, rp, A, Cn, Cf);
         // the child loop, compiled once per distance form (branching per node,
         // not per child, keeps one form's registers live at a time).  Every
         // slot is tested without a branch (lanes at different nodes have
@@ -352,31 +442,29 @@ __device__ Res8 trace8_impl(const Node8* __restrict__ nodes, uint32_t root, cons
             constexpr bool AFF = decltype(form)::value;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                {
-                    float n, f;
-                    child_span<AFF, SIGNED, true>(qa, qb, k >> 2, (uint32_t)(k & 3), A, Cn, Cf, sc, org, rp, n, f);
-                    if (((valid >> k) & 1u) && n <= f && n <= best_t * kRobust) {
-                        const uint32_t ent = child_entry(imask, child_base, counts, tri_base, k);
-                        int b = nh - 1;
-                        while (b >= 0 && ht[b] > n) { hn[b + 1] = hn[b]; ht[b + 1] = ht[b]; --b; }
-                        hn[b + 1] = ent;
-                        ht[b + 1] = n;
-                        nh++;
-                    }
+                float n, f;
+                child_span<AFF, SIGNED, true>(d.qa, d.qb, k >> 2, (uint32_t)(k & 3), A, Cn, Cf, d.sc, d.org, rp, n, f);
+                if (((d.h.valid >> k) & 1u) && n <= f && n <= best_t * kRobust) {
+                    const uint32_t ent = child_entry(d.h, k);
+                    int b = nh - 1;
+                    while (b >= 0 && ht[b] > n) { hn[b + 1] = hn[b]; ht[b + 1] = ht[b]; --b; }
+                    hn[b + 1] = ent;
+                    ht[b + 1] = n;
+                    nh++;
                 }
             }
         };
-        tests += __popc(valid);
+        tests += d.h.tri_base >> 27;
         if (aff) scan(std::true_type{});
         else scan(std::false_type{});
         if (sp + nh > kStack8) { overflow = true; break; }
-        for (int a = nh - 1; a >= 0; --a) { st_e[sp] = hn[a]; st_t[sp] = ht[a]; sp++; }
+        for (int a = nh - 1; a >= 0; --a) st[sp++] = make_uint2(hn[a], __float_as_uint(ht[a]));
         have = false;
         bool done = false;
         while (sp > 0) {
-            --sp;
-            const uint32_t e = st_e[sp];
-            if (st_t[sp] > best_t * kRobust) continue;
+            const uint2 o = st[--sp];
+            const uint32_t e = o.x;
+            if (__uint_as_float(o.y) > best_t * kRobust) continue;
             if (e & 0x80000000u) {
                 const uint32_t cnt = (e >> 27) & 0xFu, first = e & 0x07FFFFFFu;
                 for (uint32_t j = 0; j < cnt; ++j) {
@@ -415,7 +503,6 @@ __device__ Res8 trace8(const Node8* __restrict__ nodes, uint32_t root, const flo
     if (no_nan_slabs(rp)) return trace8_impl<ANY, true>(nodes, root, t8, rp);
     return trace8_impl<ANY, false>(nodes, root, t8, rp);
 }
-
 
 // ---------------------------------------------------------------------------
 // Persistent traversal kernels hand out rays in one of two ways (persistent
@@ -471,99 +558,26 @@ __device__ __forceinline__ bool leaf8(Lane8& L, const float4* __restrict__ t8, u
 }
 
 // Visit node L.cur; afterwards L.cur is the next node, or kNoHit when the
-// ray has finished (stack empty, any-hit found, or stack overflow).
+// ray has finished (stack empty, any-hit found, or stack overflow: of a
+// node's hits all but the nearest are pushed).
 template <bool ANY, bool SIGNED>
 __device__ __forceinline__ void visit8(Lane8& L, const Node8* __restrict__ nodes, const float4* __restrict__ t8,
-                                       uint32_t* st_e, float* st_t)
+                                       uint2* st, float* __restrict__ s_n)
 {
-    const Pre8& rp = L.rp;
-    const float4* p = reinterpret_cast<const float4*>(nodes + L.cur);
-    const float4 w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2), w3 = __ldg(p + 3), w4 = __ldg(p + 4);
-    L.nvis++;
-    const float org[3] = {w0.x, w0.y, w0.z};
-    const uint32_t ei = __float_as_uint(w0.w);
-    const float sc[3] = {pow2f((int)(ei & 0xFFu) - 127), pow2f((int)((ei >> 8) & 0xFFu) - 127),
-                         pow2f((int)((ei >> 16) & 0xFFu) - 127)};
-    const uint32_t imask = ei >> 24;
-    const uint32_t child_base = __float_as_uint(w1.x), tri_base = __float_as_uint(w1.y);
-    const uint32_t counts = __float_as_uint(w1.z), valid = __float_as_uint(w1.w);
-    const uint32_t q[12] = {__float_as_uint(w2.x), __float_as_uint(w2.y), __float_as_uint(w2.z), __float_as_uint(w2.w),
-                            __float_as_uint(w3.x), __float_as_uint(w3.y), __float_as_uint(w3.z), __float_as_uint(w3.w),
-                            __float_as_uint(w4.x), __float_as_uint(w4.y), __float_as_uint(w4.z), __float_as_uint(w4.w)};
-    uint32_t qa[6], qb[6];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const bool ng = SIGNED && rp.inv[a] < 0.0f;
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-            const uint32_t lo = q[a * 2 + w], hi = q[6 + a * 2 + w];
-            qa[a * 2 + w] = ng ? hi : lo;
-            qb[a * 2 + w] = ng ? lo : hi;
-        }
-    }
-    const float lim = L.best_t * kRobust;
-    // nearest hit child (kept in registers) and the others pushed onto the
-    // stack, sorted far (bottom) to near (top) within this node's pushes
-    uint32_t near_e = kNoHit;
-    float near_t = 0.0f;
-    const int seg = L.sp;
-    float A[3], Cn[3], Cf[3];
-    const bool aff = SIGNED && node_affine(org, sc, rp, A, Cn, Cf);
-    // the child loop, compiled once per distance form (see the tiles path)
-    auto scan = [&](auto form) {
-        constexpr bool AFF = decltype(form)::value;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            {
-                float n, f;
-                child_span<AFF, SIGNED>(qa, qb, k >> 2, (uint32_t)(k & 3), A, Cn, Cf, sc, org, rp, n, f);
-                if (((valid >> k) & 1u) && n <= f && n <= lim) {
-                    uint32_t ent = child_entry(imask, child_base, counts, tri_base, k);
-                    float et = n;
-                    if (near_e == kNoHit) {
-                        near_e = ent;
-                        near_t = n;
-                    } else {
-                        // Children are visited in ascending (entry distance, slot)
-                        // order.  The pushed entries keep that order from the top;
-                        // a new child has the largest slot so far and goes below
-                        // entries of equal distance, a displaced nearest has the
-                        // smallest and goes above them.
-                        bool displaced = false;
-                        if (n < near_t) {
-                            const uint32_t te = near_e; const float tt = near_t;
-                            near_e = ent; near_t = n;
-                            ent = te; et = tt;
-                            displaced = true;
-                        }
-                        if (L.sp >= kStack8) {
-                            L.overflow = true;
-                        } else {
-                            int b = L.sp - 1;
-                            while (b >= seg && (st_t[b] < et || (!displaced && st_t[b] == et))) {
-                                st_e[b + 1] = st_e[b]; st_t[b + 1] = st_t[b]; --b;
-                            }
-                            st_e[b + 1] = ent;
-                            st_t[b + 1] = et;
-                            L.sp++;
-                        }
-                    }
-                }
-            }
-        }
-    };
-    L.tests += __popc(valid);
-    if (aff) scan(std::true_type{});
-    else scan(std::false_type{});
-    if (L.overflow) { L.cur = kNoHit; return; }
     // the next node: the nearest child, else the stack (leaves tested on the way)
-    uint32_t e = near_e;
+    uint32_t e = visit_children<SIGNED>(nodes, L.cur, L.rp, L.best_t * kRobust, s_n, st, L.sp, L.tests);
+    L.nvis++;
+    if (L.sp > kStack8) {
+        L.overflow = true;
+        L.cur = kNoHit;
+        return;
+    }
     for (;;) {
         if (e == kNoHit) {
             if (L.sp == 0) { L.cur = kNoHit; return; }
-            --L.sp;
-            if (st_t[L.sp] > L.best_t * kRobust) continue;
-            e = st_e[L.sp];
+            const uint2 o = st[--L.sp];
+            if (__uint_as_float(o.y) > L.best_t * kRobust) continue;
+            e = o.x;
         }
         if (e & 0x80000000u) {
             if (leaf8<ANY>(L, t8, e)) { L.cur = kNoHit; return; }
@@ -577,14 +591,19 @@ __device__ __forceinline__ void visit8(Lane8& L, const Node8* __restrict__ nodes
 
 // Camera rays, tiles: a warp takes one 8x4 pixel tile, each lane runs its
 // ray to the end (trace8), then the warp takes the next tile.
+//
+// One warp per block: a block's SM slot is free as soon as its warp finds no
+// tile left, so the next kernel on the GPU (the next band of a banded image)
+// fills it at once instead of waiting for the slowest of four warps.
+constexpr int kTilesBlock = 32;
+
 template <int MODE>
-__global__ void __launch_bounds__(128) k_trace8_tiles(const sqk::Trace8Args a, uint32_t batches)
+__global__ void __launch_bounds__(kTilesBlock, 32) k_trace8_tiles(const sqk::Trace8Args a, uint32_t batches)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const bool camera = a.ray_kind != SQ_RAYS_EXPLICIT;
     const uint32_t tiles_x = (a.width + 7u) >> 3;
-    __shared__ WarpStats s_stats[4];
-    WarpStats& ws = s_stats[threadIdx.x >> 5];
+    __shared__ WarpStats ws;
     ws.reset(lane);
     for (;;) {
         uint32_t b = 0;
@@ -681,19 +700,19 @@ __global__ void __launch_bounds__(128) k_trace8_tiles(const sqk::Trace8Args a, u
     if (a.stats) ws.flush(lane, a.stats);
 }
 
-// Launch bounds of six blocks per SM: the register count stays at 72 (seven
-// blocks resident), but the code scheduled under this cap runs 2-3% faster
-// on incoherent rays than under the default.
+// Seven blocks per SM (72 registers): one bounce off the 4.2M-triangle
+// terrain took 0.62 ms against 0.65-0.67 ms with six (80 registers) and 0.63
+// ms with eight (64).
 template <int MODE>
-__global__ void __launch_bounds__(128, 6) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
+__global__ void __launch_bounds__(128, 7) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
 {
     constexpr bool ANY = MODE == SQ_TRACE_ANYHIT;
     const uint32_t lane = threadIdx.x & 31u;
     const bool camera = a.ray_kind != SQ_RAYS_EXPLICIT;
     const uint32_t tiles_x = (a.width + 7u) >> 3;
     const Node8* nodes = static_cast<const Node8*>(a.nodes);
-    uint32_t st_e[kStack8];
-    float st_t[kStack8];
+    uint2 st[kStack8 + 8];  // a visit pushes up to seven before it looks
+    __shared__ float s_n[128 / 32][8 * 32];
     Lane8 L;
     L.cur = kNoHit;
     bool has = false, exhausted = false;
@@ -746,8 +765,8 @@ __global__ void __launch_bounds__(128, 6) k_trace8_refill(const sqk::Trace8Args 
             // slab form chosen per ray, as trace8 does (sign-selected planes
             // for a ray that cannot produce NaN), so a ray's box tests do not
             // depend on the rays it shares a warp with
-            if (no_nan_slabs(L.rp)) visit8<ANY, true>(L, nodes, a.tris8, st_e, st_t);
-            else visit8<ANY, false>(L, nodes, a.tris8, st_e, st_t);
+            if (no_nan_slabs(L.rp)) visit8<ANY, true>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
+            else visit8<ANY, false>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
             if (L.cur == kNoHit) {
                 has = false;
                 if (L.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
@@ -791,11 +810,6 @@ void launch8(const sqk::Trace8Args& a, cudaStream_t s)
     if (a.ray_kind == SQ_RAYS_EXPLICIT) batches = (a.ray_count + 31u) / 32u;
     else batches = ((a.width + 7u) / 8u) * ((a.height + 3u) / 4u);
     if (batches == 0) return;
-    // The tiles kernel runs one warp per block: a block's SM slot is free as
-    // soon as its warp finds no tile left, so the next kernel on the GPU (the
-    // next band of a banded image) fills it at once instead of waiting for
-    // the slowest of four warps.
-    constexpr int kTilesBlock = 32;
     static PerDevice<std::array<int, 2>> cache;
     const std::array<int, 2> per_sm = cache.get([] {
         return std::array<int, 2>{blocks_per_sm(k_trace8_tiles<MODE>, kTilesBlock),
@@ -890,8 +904,8 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(cons
     const uint32_t lane = threadIdx.x & 31u;
     const Node8* nodes = static_cast<const Node8*>(a.nodes8);
     const uint32_t total = a.total_batches * 32u;
-    uint32_t st_e[kStack8];
-    float st_t[kStack8];
+    uint2 st[kStack8 + 8];  // a visit pushes up to seven before it looks
+    __shared__ float s_n[BLOCK / 32][8 * 32];
     Lane8 L;
     L.cur = kNoHit;
     bool has = false, exhausted = false, explicit_rays = false;
@@ -958,8 +972,8 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(cons
             continue;
         }
         if (has) {
-            if (no_nan_slabs(L.rp)) visit8<ANY, true>(L, nodes, a.tris8, st_e, st_t);
-            else visit8<ANY, false>(L, nodes, a.tris8, st_e, st_t);
+            if (no_nan_slabs(L.rp)) visit8<ANY, true>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
+            else visit8<ANY, false>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
             if (L.cur == kNoHit) {
                 has = false;
                 if (L.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
