@@ -344,9 +344,9 @@ sq_status build_sah(sq_ctx* c, sq_bvh* b, const sq_build_params& p, int grid)
 sq_status build_wide(sq_ctx* c, sq_bvh* b)
 {
     const uint32_t n = b->n;
-    b->nodes8 = dalloc(c, sqk::bvh8_node_bytes(n));
+    b->nodes8 = dalloc(c, sqk::bvh8_node_bytes(n, 1u));
     b->tris8 = dalloc(c, sqk::bvh8_tri_bytes(n));
-    b->ws8 = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * sqk::bvh8_ws_words(n)));
+    b->ws8 = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * sqk::bvh8_ws_words(n, 1u)));
     if (!b->nodes8 || !b->tris8 || !b->ws8) return fail(c, SQ_ERR_OOM, "8-wide BVH allocation failed (n=%u)", n);
     b->meta8 = static_cast<uint32_t*>(dalloc(c, 2 * sizeof(uint32_t)));
     if (!b->meta8) return fail(c, SQ_ERR_OOM, "8-wide BVH allocation failed (n=%u)", n);

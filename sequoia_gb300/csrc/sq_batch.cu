@@ -11,9 +11,8 @@
 //   climb            the LBVH climb of sq_lbvh.cu (k_lbvh_climb and
 //                    k_lbvh_global over mesh segments): nothing merges across
 //                    a mesh boundary; mesh m's root record is slot 3N + 2 + m
-//   8-wide collapse  (optional) seeded with all mesh roots, a fixed number
-//                    of level kernels with device-side task counts: 8-wide
-//                    node m is mesh m's root
+//   8-wide collapse  (optional) of all meshes' trees at once: 8-wide node m
+//                    is mesh m's root
 // SAH builder: sqk::build_sah_batch (sq_sah.cu) -- per-mesh root boxes and
 // root tasks, then the binned SAH's level kernels over all meshes' tasks at
 // once, a fixed number of levels with device-side task counts, the small
@@ -47,7 +46,6 @@ struct sq_batch {
     uint32_t* d_off = nullptr;        // mesh m: triangles [off[m], off[m + 1])
     float* d_rays = nullptr;          // concatenated explicit rays
     sqk::BatchJob* d_jobs = nullptr;
-    uint32_t* d_roots = nullptr;      // binary root record of each mesh
     Node* d_nodes = nullptr;          // 3N + 2 + M records
     void* d_nodes8 = nullptr;
     void* d_tris8 = nullptr;
@@ -247,7 +245,7 @@ sq_status enqueue_run(sq_batch* b)
                    3u * N + 2u, 2u * N + 2u);
     const bool wide = b->params.wide != 0;
     if (wide) {
-        const int rc = sqk::build_bvh8_queue(b->d_nodes, b->d_roots, M, 2u * N + 2u, b->d_tris, N, b->d_nodes8,
+        const int rc = sqk::build_bvh8_queue(b->d_nodes, 3u * N + 2u, M, 2u * N + 2u, b->d_tris, N, b->d_nodes8,
                                              b->d_tris8, b->d_ws8, c->ctrl, s);
         if (rc) return fail(c, SQ_ERR_CUDA, "batch collapse: %s", cudaGetErrorString((cudaError_t)rc));
     }
@@ -397,11 +395,10 @@ sq_status sq_batch_create(sq_ctx* c, const sq_batch_mesh* meshes, uint32_t mesh_
     b->d_off = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * (M + 1)));
     b->d_rays = static_cast<float*>(dalloc(c, sizeof(sq_ray) * (xrays ? xrays : 1)));
     b->d_jobs = static_cast<sqk::BatchJob*>(dalloc(c, sizeof(sqk::BatchJob) * M));
-    b->d_roots = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * M));
     b->d_nodes = static_cast<Node*>(dalloc(c, sizeof(Node) * (3ull * N + 2 + M)));
-    b->d_nodes8 = dalloc(c, 80ull * (sqk::bvh8_capacity(N) + M));
+    b->d_nodes8 = dalloc(c, sqk::bvh8_node_bytes(N, M));
     b->d_tris8 = dalloc(c, sqk::bvh8_tri_bytes(N));
-    b->d_ws8 = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * (sqk::bvh8_ws_words(N) + 4ull * M)));
+    b->d_ws8 = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * sqk::bvh8_ws_words(N, M)));
     b->d_zero = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * zero));
     b->d_keys = static_cast<uint32_t*>(dalloc(c, sizeof(uint32_t) * 7ull * (N ? N : 1)));
     b->d_info = static_cast<float4*>(dalloc(c, sizeof(float4) * 6ull * (N ? N : 1)));
@@ -414,7 +411,7 @@ sq_status sq_batch_create(sq_ctx* c, const sq_batch_mesh* meshes, uint32_t mesh_
             return fail(c, SQ_ERR_OOM, "batch allocation failed");
         }
     }
-    if (!b->d_tris || !b->d_off || !b->d_rays || !b->d_jobs || !b->d_roots || !b->d_nodes || !b->d_nodes8 ||
+    if (!b->d_tris || !b->d_off || !b->d_rays || !b->d_jobs || !b->d_nodes || !b->d_nodes8 ||
         !b->d_tris8 || !b->d_ws8 || !b->d_zero || !b->d_keys || !b->d_info || !b->d_hits || !b->d_heat) {
         sq_batch_free(b);
         return fail(c, SQ_ERR_OOM, "batch allocation failed");
@@ -429,9 +426,6 @@ sq_status sq_batch_create(sq_ctx* c, const sq_batch_mesh* meshes, uint32_t mesh_
                                        sizeof(sq_ray) * meshes[m].rays.ray_count, cudaMemcpyDefault, s));
     }
     SQ_CUDA(c, cudaMemcpyAsync(b->d_off, off.data(), sizeof(uint32_t) * (M + 1), cudaMemcpyHostToDevice, s));
-    std::vector<uint32_t> roots(M);
-    for (uint32_t m = 0; m < M; ++m) roots[m] = 3u * N + 2u + m;
-    SQ_CUDA(c, cudaMemcpyAsync(b->d_roots, roots.data(), sizeof(uint32_t) * M, cudaMemcpyHostToDevice, s));
     SQ_CUDA(c, cudaStreamSynchronize(s));
     const sq_status st = prepare(b);
     if (st != SQ_OK) {
@@ -492,7 +486,7 @@ sq_status sq_batch_free(sq_batch* b)
     Guard g(c->device);
     cudaStreamSynchronize(c->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    void* bufs[] = {b->d_tris, b->d_off, b->d_rays, b->d_jobs, b->d_roots, b->d_nodes, b->d_nodes8, b->d_tris8,
+    void* bufs[] = {b->d_tris, b->d_off, b->d_rays, b->d_jobs, b->d_nodes, b->d_nodes8, b->d_tris8,
                     b->d_ws8, b->d_zero, b->d_keys, b->d_info, b->d_hits, b->d_heat, b->d_sah_ws};
     for (void* p : bufs) dfree(c, p);
     delete b;

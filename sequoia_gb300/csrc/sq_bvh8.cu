@@ -15,7 +15,14 @@
 // children or no inner child is left.  Leaf-cluster records (and single leaf
 // records) become leaf children; their triangles are copied into a 48-byte
 // triangle array in leaf order, with the original triangle index in the
-// fourth float of the first vertex.
+// fourth float of the first vertex.  A cluster that does not fit its parent
+// becomes a node of its own, one triangle per slot.
+//
+// Schedule: the nodes that open records depend on their parents, level by
+// level (k_collapse_coop).  The cluster nodes -- five in six of all nodes --
+// depend on nothing but their place, so a parent only leaves a placeholder
+// (record, first triangle slot) in the cluster's node, and k_collapse_clusters
+// writes them all in one pass afterwards.
 #include "sq_bvh8_dev.cuh"
 
 #include <algorithm>
@@ -71,6 +78,78 @@ __device__ __forceinline__ uint8_t quant_hi(float v, float origin, int e)
 }
 
 
+// One warp's staging area: a node per group of eight lanes.
+struct GroupSmem {
+    Node8 node[4];
+    uint32_t off[4][8], cnt[4][8], child[4][8];
+};
+
+// A cluster node that k_collapse_clusters is still to write: the cluster's
+// record and its first triangle slot stand in the node's second 16 bytes,
+// marked by a `valid` word no node has (slot 0's rank is 0).
+constexpr uint32_t kPlaceholder = 0xFFFFFFFFu;
+
+__device__ __forceinline__ uint4* placeholder_of(Node8* node) { return reinterpret_cast<uint4*>(node) + 1; }
+
+// Quantise and write a node, eight lanes per node (all 32 lanes call this):
+// lane k holds slot k's child box (ok: the slot is used), `self` the node's
+// own box.  Each lane quantises its slot's six planes; the exponents take one
+// lane per axis.
+__device__ __forceinline__ void write_node8(bool active, int k, int g, const Node& self, const Node& child, bool ok,
+                                            uint32_t imask, uint32_t valid, uint32_t child_base, uint32_t tri_base,
+                                            GroupSmem& sm, Node8* __restrict__ dst)
+{
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    Node8& sn = sm.node[g];
+    const float lo[3] = {self.mnx, self.mny, self.mnz}, hi[3] = {self.mxx, self.mxy, self.mxz};
+    const int ea = active ? quant_exp(k == 0 ? lo[0] : (k == 1 ? lo[1] : lo[2]), k == 0 ? hi[0] : (k == 1 ? hi[1] : hi[2]))
+                          : 0;
+    int e[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) e[a] = __shfl_sync(FULL, ea, a, 8);
+    if (active) {
+        uint32_t ql[3] = {255u, 255u, 255u}, qh[3] = {0u, 0u, 0u};
+        if (ok) {
+            const float cl[3] = {child.mnx, child.mny, child.mnz}, ch[3] = {child.mxx, child.mxy, child.mxz};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                ql[a] = quant_lo(cl[a], lo[a], e[a]);
+                qh[a] = quant_hi(ch[a], lo[a], e[a]);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) { sn.qlo[a][k] = (uint8_t)ql[a]; sn.qhi[a][k] = (uint8_t)qh[a]; }
+    }
+    __syncwarp();
+    if (active && k == 0) {
+        uint32_t counts = 0, ranks = 0;  // a rank at an empty or leaf slot is not read
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            counts |= sm.cnt[g][q] << (4 * q);
+            ranks |= (uint32_t)__popc(imask & ((1u << q) - 1u)) << (8 + 3 * q);
+        }
+        sn.ox = self.mnx; sn.oy = self.mny; sn.oz = self.mnz;
+        sn.exps_imask = (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) |
+                        (imask << 24);
+        sn.child_base = child_base;
+        sn.tri_base = (tri_base & kTriBaseMask) | ((uint32_t)__popc(valid) << 27);
+        sn.counts = counts;
+        sn.valid = valid | ranks;
+    }
+    __syncwarp();
+    // the node: five 16-byte words
+    if (active && k < 5) reinterpret_cast<float4*>(dst)[k] = reinterpret_cast<const float4*>(&sn)[k];
+}
+
+__device__ __forceinline__ void write_tri8(float4* __restrict__ d, const float* __restrict__ tris, uint32_t id)
+{
+    float tv[9];
+    load_tri(tris, id, tv);
+    d[0] = make_float4(tv[0], tv[1], tv[2], __uint_as_float(id));
+    d[1] = make_float4(tv[3], tv[4], tv[5], 0.0f);
+    d[2] = make_float4(tv[6], tv[7], tv[8], 0.0f);
+}
+
 // Build 8-wide nodes from binary records, eight lanes per node and four
 // nodes per warp.  Lane k of a group holds candidate child slot k (its binary
 // record in registers), so the records a step opens are loaded in parallel
@@ -80,24 +159,21 @@ __device__ __forceinline__ uint8_t quant_hi(float v, float origin, int e)
 // All 32 lanes must call this; a group whose `active` is false only takes
 // part in the warp-wide shuffles.  Inner children become nodes
 // [child_base, child_base + n) and leaf triangles take the triangle slots
-// [tri_base, ...).
+// [tri_base, ...), those of the cluster children after the node's own.
 // The warp's four groups allocate together: lane 0 calls
-// alloc(nodes, tris, node_base, tri_base, task_base) once with the warp's
-// totals (one atomic per warp instead of one per node and one per child:
-// same-address atomics serialise in L2), and each group takes its share in
-// group order.  publish(task, node, record) is called by the child's lane
-// with task = task_base + the child's rank in the warp.  sm: this warp's
-// staging area (one GroupSmem per warp).
-struct GroupSmem {
-    Node8 node[4];
-    uint32_t off[4][8], cnt[4][8], child[4][8];
-};
-
-template <class Alloc, class Publish>
+// alloc(nodes, tris, tasks, node_base, tri_base, task_base) once with the
+// warp's totals (same-address atomics serialise in L2), and each group takes
+// its share in group order.  publish(task, node, record) is called by the
+// lane of each child that opens records itself, with task = task_base + the
+// child's rank among those; cluster children get a placeholder.  published()
+// is called by the whole warp once that is done: what follows (the node's
+// planes and the triangle copies) is of no matter to the next level.  sm: this
+// warp's staging area.
+template <class Alloc, class Publish, class Published>
 __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0, const float* __restrict__ tris,
                                     bool active, uint32_t rec_i, uint32_t node_i, Node8* __restrict__ nodes8,
-                                    float4* __restrict__ tris8, uint32_t* err, GroupSmem& sm, Alloc alloc,
-                                    Publish publish)
+                                    float4* __restrict__ tris8, uint32_t capacity, uint32_t* err, GroupSmem& sm,
+                                    Alloc alloc, Publish publish, Published published)
 {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const int lane = (int)(threadIdx.x & 31u);
@@ -183,7 +259,8 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
     // a cluster of 2..8 triangles that did not fit becomes a wide child node
     // of its own (its triangles one per slot), so every triangle keeps its own
     // box; larger clusters stay leaf children of up to 15 triangles
-    if (k < nc && e_kind == 1 && e_cnt >= 2 && e_cnt <= 8) e_kind = 0;
+    const bool own_node = k < nc && e_kind == 1 && e_cnt >= 2 && e_cnt <= 8;
+    if (own_node) e_kind = 0;
     // children with an empty box (empty grid cells and subtrees of them) take
     // no slot
     const bool ok = k < nc && e_node.mnx <= e_node.mxx && e_node.mny <= e_node.mxy && e_node.mnz <= e_node.mxz;
@@ -193,79 +270,52 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
         if (active && k == 0) raise_error(err, SQ_DEVERR_NODE_COUNT);
         active = false;
     }
+    // triangle slots: the leaf children's in the low half, the cluster
+    // children's in the high half (at most 64 and 120)
     const uint32_t cntk = leafc ? e_cnt : 0u;
+    const uint32_t both = cntk | (inner && own_node ? e_cnt << 16 : 0u);
     const uint32_t imask = gballot(inner);
     const uint32_t valid = gballot(ok);
+    const uint32_t tmask = gballot(inner && !own_node);
     const uint32_t leafrec = gballot(k < nc && node_is_leaf(e_node.count_flags));
-    uint32_t incl = cntk;
+    uint32_t incl = both;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
         const uint32_t y = __shfl_up_sync(FULL, incl, o, 8);
         if (k >= o) incl += y;
     }
-    const uint32_t n_tris = __shfl_sync(FULL, incl, 7, 8);
-    const uint32_t tri_off = incl - cntk;
-    const uint32_t n_inner = active ? __popc(imask) : 0u, n_place = active ? n_tris : 0u;
-    // the warp's totals and this group's offsets (groups in lane order)
-    uint32_t pre_i = 0, pre_t = 0, sum_i = 0, sum_t = 0;
+    const uint32_t all = __shfl_sync(FULL, incl, 7, 8);
+    const uint32_t n_tris = all & 0xFFFFu;
+    const uint32_t tri_off = (incl - both) & 0xFFFFu;
+    // the warp's totals and this group's offsets (groups in lane order):
+    // tasks and nodes (at most 32 each) in one word
+    const uint32_t n_nt = active ? __popc(imask) | (__popc(tmask) << 16) : 0u;
+    const uint32_t n_place = active ? n_tris + (all >> 16) : 0u;
+    uint32_t pre_nt = 0, pre_t = 0, sum_nt = 0, sum_t = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const uint32_t a = __shfl_sync(FULL, n_inner, 8 * q), b = __shfl_sync(FULL, n_place, 8 * q);
-        if (q < g) { pre_i += a; pre_t += b; }
-        sum_i += a;
+        const uint32_t a = __shfl_sync(FULL, n_nt, 8 * q), b = __shfl_sync(FULL, n_place, 8 * q);
+        if (q < g) { pre_nt += a; pre_t += b; }
+        sum_nt += a;
         sum_t += b;
     }
     uint32_t node_base = 0, tri_base = 0, task_base = 0;
-    if (lane == 0 && (sum_i | sum_t)) alloc(sum_i, sum_t, node_base, tri_base, task_base);
-    const uint32_t child_base = __shfl_sync(FULL, node_base, 0) + pre_i;
+    if (lane == 0 && (sum_nt | sum_t)) alloc(sum_nt & 0xFFFFu, sum_t, sum_nt >> 16, node_base, tri_base, task_base);
+    const uint32_t child_base = __shfl_sync(FULL, node_base, 0) + (pre_nt & 0xFFFFu);
     tri_base = __shfl_sync(FULL, tri_base, 0) + pre_t;
-    task_base = __shfl_sync(FULL, task_base, 0) + pre_i;
-    // quantised child planes, one slot per lane, staged in shared memory
-    Node8& sn = sm.node[g];
-    int e[3] = {0, 0, 0};
-    if (active) {
-        const float lo[3] = {self.mnx, self.mny, self.mnz}, hi[3] = {self.mxx, self.mxy, self.mxz};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) e[a] = quant_exp(lo[a], hi[a]);
-        uint32_t ql[3] = {255u, 255u, 255u}, qh[3] = {0u, 0u, 0u};
-        if (ok) {
-            const float cl[3] = {e_node.mnx, e_node.mny, e_node.mnz}, ch[3] = {e_node.mxx, e_node.mxy, e_node.mxz};
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                ql[a] = quant_lo(cl[a], lo[a], e[a]);
-                qh[a] = quant_hi(ch[a], lo[a], e[a]);
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) { sn.qlo[a][k] = (uint8_t)ql[a]; sn.qhi[a][k] = (uint8_t)qh[a]; }
-        sm.off[g][k] = tri_off;
-        sm.cnt[g][k] = cntk;
-        sm.child[g][k] = e_node.child;
-        if (inner) {
-            const uint32_t r = __popc(imask & ((1u << k) - 1u));
-            publish(task_base + r, child_base + r, e_rec);
-        }
+    task_base = __shfl_sync(FULL, task_base, 0) + (pre_nt >> 16);
+    sm.off[g][k] = tri_off;
+    sm.cnt[g][k] = cntk;
+    sm.child[g][k] = e_node.child;
+    if (active && inner) {
+        const uint32_t node = child_base + __popc(imask & ((1u << k) - 1u));
+        if (!own_node) publish(task_base + __popc(tmask & ((1u << k) - 1u)), node, e_rec);
+        else if (node < capacity)
+            *placeholder_of(nodes8 + node) = make_uint4(e_rec, tri_base + n_tris + ((incl - both) >> 16), 0u, kPlaceholder);
     }
-    __syncwarp();
-    if (active && k == 0) {
-        uint32_t counts = 0, ranks = 0;  // a rank at an empty or leaf slot is not read
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            counts |= sm.cnt[g][q] << (4 * q);
-            ranks |= (uint32_t)__popc(imask & ((1u << q) - 1u)) << (8 + 3 * q);
-        }
-        sn.ox = self.mnx; sn.oy = self.mny; sn.oz = self.mnz;
-        sn.exps_imask = (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) |
-                        (imask << 24);
-        sn.child_base = child_base;
-        sn.tri_base = (tri_base & kTriBaseMask) | ((uint32_t)__popc(valid) << 27);
-        sn.counts = counts;
-        sn.valid = valid | ranks;
-    }
-    __syncwarp();
+    published();
+    write_node8(active, k, g, self, e_node, ok, imask, valid, child_base, tri_base, sm, nodes8 + node_i);
     if (active) {
-        // the node: five 16-byte words
-        if (k < 5) reinterpret_cast<float4*>(nodes8 + node_i)[k] = reinterpret_cast<const float4*>(&sn)[k];
         // leaf triangles, spread over the group: triangle t of the node
         // belongs to the leaf slot whose [off, off + cnt) holds it
         for (uint32_t t = (uint32_t)k; t < n_tris; t += 8u) {
@@ -275,28 +325,61 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
                 if (sm.cnt[g][r] && sm.off[g][r] <= t) q = r;
             const uint32_t j = t - sm.off[g][q], qc = sm.child[g][q];
             // a leaf record is its own triangle; a cluster's are its leaves
-            const uint32_t id = ((leafrec >> q) & 1u) ? qc + j : rec[qc + j].child;
-            float tv[9];
-            load_tri(tris, id, tv);
-            float4* d = tris8 + 3ull * (tri_base + t);
-            d[0] = make_float4(tv[0], tv[1], tv[2], __uint_as_float(id));
-            d[1] = make_float4(tv[3], tv[4], tv[5], 0.0f);
-            d[2] = make_float4(tv[6], tv[7], tv[8], 0.0f);
+            write_tri8(tris8 + 3ull * (tri_base + t), tris, ((leafrec >> q) & 1u) ? qc + j : rec[qc + j].child);
         }
     }
     __syncwarp();  // the staging area is reused by the warp's next nodes
 }
 
+// The cluster nodes, four per warp: lane k of a group has the cluster's
+// triangle k, its box from its leaf record.  One pass over the node array
+// (80 B a node read or written, the leaf records and the triangles gathered):
+// bound by those gathers.
+__global__ void __launch_bounds__(256) k_collapse_clusters(const Node* __restrict__ rec, const float* __restrict__ tris,
+                                                           const uint32_t* __restrict__ count,
+                                                           Node8* __restrict__ nodes8, float4* __restrict__ tris8)
+{
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    __shared__ GroupSmem s_group[8];
+    GroupSmem& sm = s_group[threadIdx.x >> 5];
+    const int lane = (int)(threadIdx.x & 31u), k = lane & 7, g = lane >> 3, gs = lane & ~7;
+    const uint32_t n = *count;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t base = 4u * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < n; base += 4u * warps) {
+        const uint32_t i = base + (uint32_t)g;
+        uint4 ph = make_uint4(0u, 0u, 0u, 0u);
+        if (i < n) ph = *placeholder_of(nodes8 + i);
+        const bool active = i < n && ph.w == kPlaceholder;
+        if (!__any_sync(FULL, active)) continue;
+        Node self, child;
+        bool ok = false;
+        uint32_t id = 0;
+        if (active) {
+            self = rec[ph.x];
+            if (k < (int)node_count(self.count_flags)) {
+                child = rec[self.child + (uint32_t)k];
+                id = child.child;
+                ok = child.mnx <= child.mxx && child.mny <= child.mxy && child.mnz <= child.mxz;
+            }
+        }
+        const uint32_t valid = (__ballot_sync(FULL, ok) >> gs) & 0xFFu;
+        sm.cnt[g][k] = ok ? 1u : 0u;
+        write_node8(active, k, g, self, child, ok, 0u, valid, 0u, ph.y, sm, nodes8 + i);
+        if (ok) write_tri8(tris8 + 3ull * (ph.y + __popc(valid & ((1u << k) - 1u))), tris, id);
+        __syncwarp();  // the staging area is reused by the warp's next nodes
+    }
+}
+
 // Nodes and triangle slots of one warp from the counter pair at ctr (nodes
-// in word 0, triangles in word 1: one 64-bit atomic).  On overflow of the
-// node capacity the error word is set and the nodes land at `capacity`, where
-// nothing is written.
-__device__ __forceinline__ void alloc_nodes_tris(uint32_t* ctr, uint32_t kn, uint32_t kt, uint32_t capacity,
-                                                 uint32_t* err, uint32_t& nb, uint32_t& tb)
+// after the roots in word 0, triangles in word 1: one 64-bit atomic).  On
+// overflow of the node capacity the error word is set and the nodes land at
+// `capacity`, where nothing is written.
+__device__ __forceinline__ void alloc_nodes_tris(uint32_t* ctr, uint32_t kn, uint32_t kt, uint32_t nroots,
+                                                 uint32_t capacity, uint32_t* err, uint32_t& nb, uint32_t& tb)
 {
     const unsigned long long v =
         atomicAdd(reinterpret_cast<unsigned long long*>(ctr), ((unsigned long long)kt << 32) | kn);
-    nb = (uint32_t)v;
+    nb = (uint32_t)v + nroots;
     tb = (uint32_t)(v >> 32);
     if ((unsigned long long)nb + kn > capacity) {
         raise_error(err, SQ_DEVERR_SAH_QUEUE);
@@ -304,202 +387,215 @@ __device__ __forceinline__ void alloc_nodes_tris(uint32_t* ctr, uint32_t kn, uin
     }
 }
 
-// One level of the collapse: group i (four per warp) builds node
-// task_node[i] from binary record tasks[i]; inner children are allocated
-// contiguously from the node counter and appended to the next level's list.
+// Workspace words: the counters, then two task lists (record and node of
+// each task), `capacity` words a list half.
+struct CollapseWs {
+    uint32_t* head;  // see the indices below
+    uint32_t *rec[2], *node[2];
+};
+constexpr uint32_t kMaxLevels = 64;
+// Words that atomics go to and words that are stored stand on lines of their
+// own: with the level's cluster mark stored beside the counters the collapse
+// of the 2M soup took 858 us instead of 215.
+constexpr uint32_t kWsNodes = 0;               // a 64-bit pair: nodes beyond the roots, triangle slots
+constexpr uint32_t kWsBarrier = 32;            // arrivals, generation
+constexpr uint32_t kWsCount = 64;              // final node count, then the number of levels
+constexpr uint32_t kWsClusters = 66;           // levels that the deepest cluster node makes
+constexpr uint32_t kWsBefore = 67;             // nodes before the level
+constexpr uint32_t kWsLevel = 96;              // tasks of level l at kWsLevel + l
+constexpr uint32_t kWsHead = kWsLevel + kMaxLevels + 32;
+
+__host__ __device__ inline CollapseWs collapse_ws(uint32_t* ws, uint32_t capacity)
+{
+    CollapseWs w;
+    w.head = ws;
+    uint32_t* p = ws + kWsHead;
+    for (int i = 0; i < 2; ++i) {
+        w.rec[i] = p;
+        w.node[i] = p + capacity;
+        p += 2ull * capacity;
+    }
+    return w;
+}
+
+// The work of one task group of level `level`: allocation from the head's
+// counters, open-record children to the next level's list.  Wide node r
+// (r < nroots) is the tree of record root + r; the other nodes follow.
+template <class Published>
+__device__ __forceinline__ void collapse_task(const Node* __restrict__ rec, uint32_t leaf0,
+                                              const float* __restrict__ tris, bool active, uint32_t rec_i,
+                                              uint32_t node_i, uint32_t level, uint32_t nroots, const CollapseWs& w,
+                                              Node8* __restrict__ nodes8, float4* __restrict__ tris8, uint32_t capacity,
+                                              uint32_t* err, GroupSmem& sm, Published published)
+{
+    uint32_t* head = w.head;
+    uint32_t *next_rec = w.rec[(level + 1) & 1], *next_node = w.node[(level + 1) & 1];
+    auto alloc = [&](uint32_t kn, uint32_t kt, uint32_t kj, uint32_t& nb, uint32_t& tb, uint32_t& jb) {
+        if (kj) jb = atomicAdd(head + kWsLevel + level + 1, kj);
+        alloc_nodes_tris(head + kWsNodes, kn, kt, nroots, capacity, err, nb, tb);
+    };
+    auto publish = [&](uint32_t j, uint32_t node, uint32_t record) {
+        if (node >= capacity || j >= capacity) return;
+        next_rec[j] = record;
+        next_node[j] = node;
+    };
+    collapse_node_group(rec, leaf0, tris, active, rec_i, node_i, nodes8, tris8, capacity, err, sm, alloc, publish,
+                        published);
+}
+
+// One level per launch (where a cooperative launch is not possible): group i
+// (four per warp) takes task i of the level's list.
 constexpr int kCollapseBlock = 128;
 
 __global__ void __launch_bounds__(kCollapseBlock) k_collapse_level(
-    const Node* __restrict__ rec, uint32_t leaf0, const float* __restrict__ tris, const uint32_t* __restrict__ tasks,
-    const uint32_t* __restrict__ task_node, uint32_t ntasks, Node8* __restrict__ nodes8, float4* __restrict__ tris8,
-    uint32_t* __restrict__ counters, uint32_t* __restrict__ next_tasks, uint32_t* __restrict__ next_node,
-    uint32_t capacity, uint32_t* err)
+    const Node* __restrict__ rec, uint32_t leaf0, const float* __restrict__ tris, uint32_t root, uint32_t nroots,
+    uint32_t level, uint32_t ntasks, CollapseWs w, uint32_t capacity, Node8* __restrict__ nodes8,
+    float4* __restrict__ tris8, uint32_t* err)
 {
     __shared__ GroupSmem s_group[kCollapseBlock / 32];
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (4u * w >= ntasks) return;  // whole warps
-    const uint32_t i = 4u * w + ((threadIdx.x & 31u) >> 3);
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (4u * warp >= ntasks) return;  // whole warps
+    const uint32_t i = 4u * warp + ((threadIdx.x & 31u) >> 3);
     const bool active = i < ntasks;
-    auto alloc = [&](uint32_t kn, uint32_t kt, uint32_t& nb, uint32_t& tb, uint32_t& jb) {
-        alloc_nodes_tris(counters, kn, kt, capacity, err, nb, tb);
-        jb = kn ? atomicAdd(counters + 2, kn) : 0u;
-    };
-    auto publish = [&](uint32_t j, uint32_t node, uint32_t record) {
-        if (node >= capacity) return;
-        next_tasks[j] = record;
-        next_node[j] = node;
-    };
-    collapse_node_group(rec, leaf0, tris, active, active ? tasks[i] : 0u, active ? task_node[i] : 0u, nodes8, tris8,
-                        err, s_group[threadIdx.x >> 5], alloc, publish);
+    const uint32_t rec_i = !active ? 0u : (level ? w.rec[level & 1][i] : root + i);
+    const uint32_t node_i = !active ? 0u : (level ? w.node[level & 1][i] : i);
+    collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
+                  s_group[threadIdx.x >> 5], [] {});
 }
 
-// Collapse without host synchronisation (so it can be captured in a CUDA
-// graph): a fixed number of level kernels, each a grid-stride loop over the
-// task count its predecessor left in device memory (counts[level]); a level
-// with no tasks returns at once.  Nothing waits on anything.  If the tree is
-// deeper than the launched levels, the last level raises SQ_DEVERR_SAH_QUEUE.
-constexpr uint32_t kFixedLevels = 64;
-
-__global__ void __launch_bounds__(128) k_collapse_fixed(const Node* __restrict__ rec, uint32_t leaf0,
-                                                        const float* __restrict__ tris, uint32_t level,
-                                                        uint32_t* __restrict__ counts, const uint32_t* __restrict__ tasks,
-                                                        const uint32_t* __restrict__ task_node,
-                                                        uint32_t* __restrict__ next_tasks, uint32_t* __restrict__ next_node,
-                                                        uint32_t* __restrict__ counters2, Node8* __restrict__ nodes8,
-                                                        float4* __restrict__ tris8, uint32_t capacity, uint32_t* err)
+// After level `level`, before anything of the next one: a level that made
+// more nodes than tasks made cluster nodes, one level below its own.
+__device__ __forceinline__ void collapse_level_end(uint32_t* head, uint32_t level)
 {
-    chain_wait();  // a chained launch: the levels follow one another
-    chain_release();
-    const uint32_t ntasks = counts[level];
-    if (ntasks == 0) return;
-    if (level + 1 >= kFixedLevels) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(err, SQ_DEVERR_SAH_QUEUE);
-        return;
+    const uint32_t nodes = ld_acquire_u32(head + kWsNodes), tasks = ld_acquire_u32(head + kWsLevel + level + 1);
+    if (nodes - ld_acquire_u32(head + kWsBefore) > tasks) st_relaxed_u32(head + kWsClusters, level + 2u);
+    st_relaxed_u32(head + kWsBefore, nodes);
+}
+
+// The final counts: nodes, and levels (levels of tasks, or one more where the
+// deepest nodes are clusters).
+__device__ __forceinline__ void collapse_done(uint32_t* head, uint32_t levels, uint32_t nroots, uint32_t capacity,
+                                              uint32_t* meta)
+{
+    const uint32_t nodes = ld_acquire_u32(head + kWsNodes) + nroots, deep = ld_acquire_u32(head + kWsClusters);
+    head[kWsCount] = nodes < capacity ? nodes : capacity;
+    head[kWsCount + 1] = deep > levels ? deep : levels;
+    if (meta) {
+        meta[0] = head[kWsCount];
+        meta[1] = head[kWsCount + 1];
     }
-    __shared__ GroupSmem s_group[4];
-    uint32_t* next_count = counts + level + 1;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t base = 4u * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < ntasks; base += 4u * warps) {
-        const uint32_t i = base + ((threadIdx.x & 31u) >> 3);
-        const bool active = i < ntasks;
-        auto alloc = [&](uint32_t kn, uint32_t kt, uint32_t& nb, uint32_t& tb, uint32_t& jb) {
-            alloc_nodes_tris(counters2, kn, kt, capacity, err, nb, tb);
-            jb = kn ? atomicAdd(next_count, kn) : 0u;
-        };
-        auto publish = [&](uint32_t j, uint32_t node, uint32_t record) {
-            if (node >= capacity) return;
-            next_tasks[j] = record;
-            next_node[j] = node;
-        };
-        collapse_node_group(rec, leaf0, tris, active, active ? tasks[i] : 0u, active ? task_node[i] : 0u, nodes8,
-                            tris8, err, s_group[threadIdx.x >> 5], alloc, publish);
-    }
+}
+
+__global__ void k_collapse_level_end(CollapseWs w, uint32_t level) { collapse_level_end(w.head, level); }
+
+__global__ void k_collapse_done(CollapseWs w, uint32_t levels, uint32_t nroots, uint32_t capacity)
+{
+    collapse_done(w.head, levels, nroots, capacity, nullptr);
 }
 
 // All levels in one cooperative launch (every block is resident): a
 // grid-stride loop over a level's tasks, a grid barrier, the next level.  No
-// host round trip per level.  The barrier's wait is bounded: a block that
-// polls more than kBarrierSpins times raises SQ_DEVERR_SAH_QUEUE and returns
-// (the other blocks then time out at their next barrier too).  Task lists
-// are read through L2 (__ldcg): the same lists are rewritten every other
-// level, so an SM's L1 may hold stale lines of them.  The failure-detection
-// tests pass a small poll limit and one phantom block (barrier_extra = 1)
-// that never arrives: every block then gives up at the first barrier.
+// host round trip per level, and a CUDA graph can hold it.  The barrier's
+// wait is bounded: a block that polls more than kBarrierSpins times raises
+// SQ_DEVERR_SAH_QUEUE and returns (the other blocks then time out at their
+// next barrier too).  Task lists are read through L2 (__ldcg): the same lists
+// are rewritten every other level, so an SM's L1 may hold stale lines of
+// them.  The failure-detection tests pass a small poll limit and one phantom
+// block (barrier_extra = 1) that never arrives: every block then gives up at
+// the first barrier.
 constexpr uint32_t kBarrierSpins = 1u << 24;
 
-// Grid barrier; the last block to arrive runs on_last() (thread 0 only)
-// after every other block's writes before the barrier are visible to it and
-// before any block leaves.
+// Grid barrier in two halves.  barrier_arrive: every warp calls it once, when
+// its writes before the barrier are done; the block's last warp arrives for
+// the block, and the grid's last block runs on_last() before any block
+// leaves, with every write of before the barrier visible to it.
+// barrier_wait: the block waits (thread 0 polls), and every thread gets the
+// value of *word, which the blocks changed before the barrier; false when the
+// wait gave up.  s_warps: a shared counter, zero before the first use.
 template <class OnLast>
-__device__ bool grid_barrier(uint32_t* bar, uint32_t nblocks, uint32_t spin_limit, uint32_t* err, OnLast on_last)
+__device__ __forceinline__ void barrier_arrive(uint32_t* bar, uint32_t nblocks, uint32_t* s_warps, OnLast on_last)
 {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const uint32_t gen = ld_acquire_u32(bar + 1);
+    __syncwarp();
+    if ((threadIdx.x & 31u) != 0) return;
+    __threadfence();
+    if (atomicAdd(s_warps, 1u) + 1u != (blockDim.x >> 5)) return;
+    __threadfence();
+    *s_warps = 0;  // every warp of the block has counted; the next use is after barrier_wait's block barrier
+    if (atomicAdd(bar, 1u) + 1u == nblocks) {
+        // last arrival: reset the count, then open the next generation
         __threadfence();
-        if (atomicAdd(bar, 1u) + 1u == nblocks) {
-            // last arrival: reset the count, then open the next generation
-            __threadfence();
-            on_last();
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            uint32_t spins = 0;
-            while (ld_acquire_u32(bar + 1) == gen) {
-                if (++spins > spin_limit) {
-                    raise_error(err, SQ_DEVERR_SAH_QUEUE);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        s_ok = ok;
+        on_last();
+        atomicExch(bar, 0u);
+        __threadfence();
+        atomicAdd(bar + 1, 1u);
     }
-    __syncthreads();
-    return s_ok != 0;
 }
 
-// The tasks of a level are the nodes [lo, hi) that the previous level
-// allocated, in allocation order: task j builds node lo + j from the binary
-// record in the level's task list at j.  A warp's allocation at node base b
-// therefore also places its children's tasks at b - hi in the next list, and
-// the next level's end is the node counter once the level is done (read by
-// the barrier's last block).
+__device__ __forceinline__ bool barrier_wait(const uint32_t* bar, uint32_t gen, uint32_t spin_limit, const uint32_t* word,
+                                             uint32_t* err, uint32_t& value)
+{
+    __shared__ uint32_t s_ok, s_value;
+    if (threadIdx.x == 0) {
+        uint32_t ok = 1, spins = 0;
+        while (ld_acquire_u32(bar + 1) == gen) {
+            if (++spins > spin_limit) {
+                raise_error(err, SQ_DEVERR_SAH_QUEUE);
+                ok = 0;
+                break;
+            }
+            __nanosleep(32);
+        }
+        s_ok = ok;
+        s_value = ld_acquire_u32(word);
+    }
+    __syncthreads();
+    const bool ok = s_ok != 0;
+    value = s_value;
+    __syncthreads();  // read by every thread before the next wait writes them
+    return ok;
+}
+
+// A warp arrives at a level's barrier as soon as its last task's children are
+// published and writes that task's node and triangles while it waits: a thin
+// level (the top and the bottom of the tree, most levels) is a chain of
+// dependent loads, and what the next level does not need is off it.
 __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ rec, uint32_t leaf0,
-                                                       const float* __restrict__ tris, uint32_t* __restrict__ ws,
-                                                       uint32_t capacity, Node8* __restrict__ nodes8,
-                                                       float4* __restrict__ tris8, uint32_t* err,
+                                                       const float* __restrict__ tris, uint32_t root, uint32_t nroots,
+                                                       CollapseWs w, uint32_t capacity, Node8* __restrict__ nodes8,
+                                                       float4* __restrict__ tris8, uint32_t* meta, uint32_t* err,
                                                        uint32_t barrier_extra, uint32_t spin_limit)
 {
-    // ws: [0] node counter, [1] triangle counter (one 64-bit pair), [2..3]
-    // barrier, [4] levels done, [5] end of the next level's nodes, then the
-    // task lists of even and odd levels (`capacity` records each, at the
-    // offsets the seed uses)
-    uint32_t* bar = ws + 2;
-    uint32_t* ta = ws + 8 + kFixedLevels + 8;
-    uint32_t* tb = ta + 2ull * capacity;
     __shared__ GroupSmem s_group[8];
+    __shared__ uint32_t s_warps;
+    if (threadIdx.x == 0) s_warps = 0;
+    __syncthreads();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t lo = 0, hi = 1;  // the root task
-    for (uint32_t level = 0;; ++level) {
-        const uint32_t ntasks = hi - lo;
-        if (ntasks == 0) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) ws[4] = level;
-            return;
-        }
-        if (level + 1 >= kFixedLevels) {
+    uint32_t* bar = w.head + kWsBarrier;
+    uint32_t ntasks = nroots;
+    // (an overflow of the node capacity has raised the error word; the lists
+    // hold no more than `capacity` tasks)
+    for (uint32_t level = 0; ntasks; ++level, ntasks = min(ntasks, capacity)) {
+        if (level + 1 >= kMaxLevels) {
             if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(err, SQ_DEVERR_SAH_QUEUE);
             return;
         }
-        const uint32_t* tasks = (level & 1) ? tb : ta;
-        uint32_t* next_tasks = (level & 1) ? ta : tb;
+        // the generations are the levels: nobody has opened this one yet
+        auto arrive = [&] {
+            barrier_arrive(bar, gridDim.x + barrier_extra, &s_warps, [&] { collapse_level_end(w.head, level); });
+        };
+        if (4u * wid >= ntasks) arrive();
         for (uint32_t base = 4u * wid; base < ntasks; base += 4u * warps) {
             const uint32_t i = base + ((threadIdx.x & 31u) >> 3);
             const bool active = i < ntasks;
-            auto alloc = [&](uint32_t kn, uint32_t kt, uint32_t& nb, uint32_t& tb_, uint32_t& jb) {
-                alloc_nodes_tris(ws, kn, kt, capacity, err, nb, tb_);
-                jb = nb - hi;
-            };
-            auto publish = [&](uint32_t j, uint32_t node, uint32_t record) {
-                if (node >= capacity) return;
-                next_tasks[j] = record;
-            };
-            collapse_node_group(rec, leaf0, tris, active, active ? __ldcg(tasks + i) : 0u, lo + i, nodes8, tris8, err,
-                                s_group[threadIdx.x >> 5], alloc, publish);
+            const uint32_t rec_i = !active ? 0u : (level ? __ldcg(w.rec[level & 1] + i) : root + i);
+            const uint32_t node_i = !active ? 0u : (level ? __ldcg(w.node[level & 1] + i) : i);
+            const bool last = ntasks - base <= 4u * warps;
+            collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
+                          s_group[threadIdx.x >> 5], [&] { if (last) arrive(); });
         }
-        const bool ok = grid_barrier(bar, gridDim.x + barrier_extra, spin_limit, err, [&]() {
-            const uint32_t end = ld_acquire_u32(ws);
-            st_relaxed_u32(ws + 5, end < capacity ? end : capacity);
-        });
-        if (!ok) return;
-        lo = hi;
-        hi = ld_acquire_u32(ws + 5);
-    }
-}
-
-// Seed of the cooperative collapse: one root task (record `root`, node 0).
-__global__ void k_coop_seed(uint32_t* __restrict__ ws, uint32_t root)
-{
-    ws[0] = 1u;  // node 0 is the root
-    ws[8 + kFixedLevels + 8] = root;  // the first task list
-}
-
-__global__ void k_fixed_seed(const uint32_t* __restrict__ roots, uint32_t nroots, uint32_t* __restrict__ tasks,
-                             uint32_t* __restrict__ task_node, uint32_t* __restrict__ counts,
-                             uint32_t* __restrict__ node_counter)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nroots; i += gridDim.x * blockDim.x) {
-        tasks[i] = roots[i];
-        task_node[i] = i;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        counts[0] = nroots;
-        *node_counter = nroots;
+        if (!barrier_wait(bar, level, spin_limit, w.head + kWsLevel + level + 1, err, ntasks)) return;
+        if (!ntasks && blockIdx.x == 0 && threadIdx.x == 0) collapse_done(w.head, level + 1, nroots, capacity, meta);
     }
 }
 
@@ -507,80 +603,96 @@ __global__ void k_fixed_seed(const uint32_t* __restrict__ roots, uint32_t nroots
 
 namespace sqk {
 
-int build_bvh8_queue(const Node* rec, const uint32_t* roots_dev, uint32_t nroots, uint32_t leaf0, const float* tris,
-                     uint32_t n, void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s)
+// A wide node has at least two children except the root and nodes next to
+// empty grid cells (at most 64 of those), so n + 130 nodes beside the roots
+// always suffice.
+uint32_t bvh8_capacity(uint32_t n) { return n + 130u; }
+size_t bvh8_node_bytes(uint32_t n, uint32_t nroots) { return sizeof(Node8) * ((size_t)bvh8_capacity(n) + nroots); }
+size_t bvh8_ws_words(uint32_t n, uint32_t nroots) { return 4ull * (bvh8_capacity(n) + nroots) + kWsHead; }
+size_t bvh8_tri_bytes(uint32_t n) { return sizeof(float4) * 3ull * ((size_t)n + 1); }
+
+// Blocks per SM of the cooperative collapse: every block must be resident
+// (0: no cooperative launch on this device).
+static int coop_blocks()
 {
-    // ws: [0] node counter, [1] triangle counter, [8 .. 8+kFixedLevels] level
-    // counts, then two (record, node) task lists of `capacity` entries
-    const uint32_t capacity = bvh8_capacity(n) + nroots;
-    uint32_t* node_counter = ws;
-    uint32_t* counts = ws + 8;
-    uint32_t* ta = counts + kFixedLevels + 8;
-    uint32_t* na = ta + capacity;
-    uint32_t* tb = na + capacity;
-    uint32_t* nb = tb + capacity;
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * (16 + kFixedLevels), s)) != cudaSuccess) return (int)e;
-    k_fixed_seed<<<(nroots + 255) / 256, 256, 0, s>>>(roots_dev, nroots, ta, na, counts, node_counter);
     static PerDevice<int> cache;
-    const int grid = cache.get([] { return blocks_per_sm(k_collapse_fixed, 128) * sm_count(); });
-    for (uint32_t level = 0; level < kFixedLevels; ++level) {
-        uint32_t* in_t = (level & 1) ? tb : ta;
-        uint32_t* in_n = (level & 1) ? nb : na;
-        uint32_t* out_t = (level & 1) ? ta : tb;
-        uint32_t* out_n = (level & 1) ? na : nb;
-        launch_chained(k_collapse_fixed, dim3(grid), dim3(128), 0, s, rec, leaf0, tris, level, counts,
-                       (const uint32_t*)in_t, (const uint32_t*)in_n, out_t, out_n, ws, static_cast<Node8*>(nodes8),
-                       static_cast<float4*>(tris8), capacity, err);
+    return cache.get([] {
+        int coop = 0, occ = 0;
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, current_device());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_collapse_coop, 256, 0);
+        return (coop && occ > 0) ? occ : 0;
+    });
+}
+
+static cudaError_t launch_clusters(const Node* rec, const float* tris, const CollapseWs& w, void* nodes8, void* tris8,
+                                   cudaStream_t s)
+{
+    static PerDevice<int> cache;
+    const int grid = cache.get([] { return blocks_per_sm(k_collapse_clusters, 256) * sm_count(); });
+    k_collapse_clusters<<<grid, 256, 0, s>>>(rec, tris, w.head + kWsCount, static_cast<Node8*>(nodes8),
+                                             static_cast<float4*>(tris8));
+    return cudaGetLastError();
+}
+
+// The collapse as one kernel launch per level of tasks (the host reads each
+// level's task count), where a cooperative launch does not fit.  The node
+// count is host_ctl[0] and the number of levels host_ctl[3].
+static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n,
+                             void* nodes8, void* tris8, const CollapseWs& w, uint32_t* host_ctl, uint32_t* err,
+                             cudaStream_t s)
+{
+    const uint32_t capacity = bvh8_capacity(n) + 1u;
+    cudaError_t e;
+    uint32_t ntasks = 1, level = 0;
+    for (; ntasks && level + 1 < kMaxLevels; ++level) {
+        k_collapse_level<<<(ntasks + 15) / 16, kCollapseBlock, 0, s>>>(rec, leaf0, tris, root, 1u, level, ntasks, w, capacity,
+                                                               static_cast<Node8*>(nodes8), static_cast<float4*>(tris8),
+                                                               err);
+        k_collapse_level_end<<<1, 1, 0, s>>>(w, level);
+        if ((e = cudaMemcpyAsync(host_ctl, w.head + kWsLevel + level + 1, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+            return (int)e;
+        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
+        ntasks = std::min(host_ctl[0], capacity);
     }
+    k_collapse_done<<<1, 1, 0, s>>>(w, level, 1u, capacity);
+    if ((e = launch_clusters(rec, tris, w, nodes8, tris8, s)) != cudaSuccess) return (int)e;
+    uint32_t m[2];
+    if ((e = cudaMemcpyAsync(m, w.head + kWsCount, sizeof m, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
+    host_ctl[0] = m[0];
+    host_ctl[3] = m[1];
+    host_ctl[4] = 2 * level + 2;  // launches
     return (int)cudaGetLastError();
 }
 
-
-
-// A wide node has at least two children except the root and nodes next to
-// empty grid cells (at most 64 of those), so n + 130 nodes always suffice.
-uint32_t bvh8_capacity(uint32_t n) { return n + 130u; }
-size_t bvh8_node_bytes(uint32_t n) { return sizeof(Node8) * (size_t)bvh8_capacity(n); }
-size_t bvh8_ws_words(uint32_t n) { return 4ull * bvh8_capacity(n) + 16 + 2 * kFixedLevels; }
-size_t bvh8_tri_bytes(uint32_t n) { return sizeof(float4) * 3ull * ((size_t)n + 1); }
-
-// Collapse the binary tree rooted at record `root` (an inner record) into
-// nodes8 / tris8, one kernel launch per level of the 8-wide tree (the host
-// reads each level's task count from pinned memory).  ws: bvh8_ws_words(n)
-// words; host_ctl: pinned, 4 words.  Returns 0 or a cudaError_t; the node
-// count is host_ctl[0] and the number of levels host_ctl[3].
-static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n, void* nodes8, void* tris8,
-               uint32_t* ws, uint32_t* host_ctl, uint32_t* err, cudaStream_t s)
+// The cooperative collapse and the cluster pass of the trees of records
+// root .. root + nroots - 1 over n triangles: nothing waits on the host, so a
+// CUDA graph can hold it.  meta (device, 2 words, may be null): node and level
+// counts.
+static cudaError_t enqueue_collapse(const Node* rec, uint32_t root, uint32_t nroots, uint32_t leaf0, const float* tris,
+                                    uint32_t n, void* nodes8, void* tris8, uint32_t* ws, uint32_t* meta, uint32_t* err,
+                                    int per_sm, const BarrierStall* stall, cudaStream_t s)
 {
-    const uint32_t capacity = bvh8_capacity(n);
-    uint32_t* counters = ws;  // [0] nodes allocated, [1] triangles placed, [2] next-level tasks
-    uint32_t* ta = ws + 8;    // task lists (record, node), two levels
-    uint32_t* na = ta + capacity;
-    uint32_t* tb = na + capacity;
-    uint32_t* nb = tb + capacity;
+    uint32_t capacity = bvh8_capacity(n) + nroots;
+    CollapseWs w = collapse_ws(ws, capacity);
+    const uint32_t extra = stall ? 1u : 0u;
+    const uint32_t spins = stall ? stall->spin_limit : kBarrierSpins;
+    void* args[] = {(void*)&rec, (void*)&leaf0, (void*)&tris, (void*)&root, (void*)&nroots, (void*)&w, (void*)&capacity,
+                    (void*)&nodes8, (void*)&tris8, (void*)&meta, (void*)&err, (void*)&extra, (void*)&spins};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_collapse_coop, dim3(per_sm * sm_count()), dim3(256),
+                                                      args, 0, s);
+    if (e != cudaSuccess) return e;
+    return launch_clusters(rec, tris, w, nodes8, tris8, s);
+}
+
+int build_bvh8_queue(const Node* rec, uint32_t root0, uint32_t nroots, uint32_t leaf0, const float* tris, uint32_t n,
+                     void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s)
+{
+    const int per_sm = coop_blocks();
+    if (per_sm == 0) return (int)cudaErrorCooperativeLaunchTooLarge;
     cudaError_t e;
-    const uint32_t init[4] = {1u, 0u, 0u, 0u};
-    if ((e = cudaMemcpyAsync(counters, init, sizeof init, cudaMemcpyHostToDevice, s)) != cudaSuccess) return (int)e;
-    const uint32_t first[2] = {root, 0u};
-    if ((e = cudaMemcpyAsync(ta, &first[0], 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemcpyAsync(na, &first[1], 4, cudaMemcpyHostToDevice, s)) != cudaSuccess) return (int)e;
-    uint32_t ntasks = 1, levels = 0;
-    while (ntasks) {
-        ++levels;
-        if ((e = cudaMemsetAsync(counters + 2, 0, 4, s)) != cudaSuccess) return (int)e;
-        k_collapse_level<<<(ntasks + 15) / 16, kCollapseBlock, 0, s>>>(rec, leaf0, tris, ta, na, ntasks,
-                                                               static_cast<Node8*>(nodes8), static_cast<float4*>(tris8),
-                                                               counters, tb, nb, capacity, err);
-        if ((e = cudaMemcpyAsync(host_ctl, counters, 12, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
-        ntasks = host_ctl[2];
-        std::swap(ta, tb);
-        std::swap(na, nb);
-    }
-    host_ctl[3] = levels;
-    host_ctl[4] = levels;  // one launch per level
-    return (int)cudaGetLastError();
+    if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * kWsHead, s)) != cudaSuccess) return (int)e;
+    return (int)enqueue_collapse(rec, root0, nroots, leaf0, tris, n, nodes8, tris8, ws, nullptr, err, per_sm, nullptr, s);
 }
 
 int build_bvh8(const Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n, void* nodes8, void* tris8,
@@ -588,45 +700,18 @@ int build_bvh8(const Node* rec, uint32_t root, uint32_t leaf0, const float* tris
                const BarrierStall* stall)
 {
     host_ctl[5] = 0;
-    // every block of the cooperative collapse must be resident: at most the
-    // occupancy limit per SM (0: no cooperative launch, use the per-level
-    // path).  From 5M triangles up, four blocks per SM instead of the limit
-    // (five): on Gaussian soups the 6M and 8M collapses took 0.61 / 0.76 ms
-    // with four against 0.64 / 0.86 ms with five, while at 1-4M (and the 4M
-    // terrain) five were as fast or faster.
-    static PerDevice<int> cache;
-    const int per_sm = cache.get([] {
-        int coop = 0, occ = 0;
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, current_device());
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_collapse_coop, 256, 0);
-        return (coop && occ > 0) ? occ : 0;
-    });
-    const int grid = (n >= 5000000u && per_sm > 4 ? 4 : per_sm) * sm_count();
-    if (grid == 0) return build_bvh8_levels(rec, root, leaf0, tris, n, nodes8, tris8, ws, host_ctl, err, s);
-    const uint32_t capacity = bvh8_capacity(n);
     cudaError_t e;
-    if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * (16 + kFixedLevels), s)) != cudaSuccess) return (int)e;
-    k_coop_seed<<<1, 1, 0, s>>>(ws, root);
-    const uint32_t extra = stall ? 1u : 0u;
-    const uint32_t spins = stall ? stall->spin_limit : kBarrierSpins;
-    void* args[] = {(void*)&rec, (void*)&leaf0, (void*)&tris, (void*)&ws, (void*)&capacity, (void*)&nodes8,
-                    (void*)&tris8, (void*)&err, (void*)&extra, (void*)&spins};
-    if ((e = cudaLaunchCooperativeKernel((const void*)k_collapse_coop, dim3(grid), dim3(256), args, 0, s)) !=
+    if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * kWsHead, s)) != cudaSuccess) return (int)e;
+    const int per_sm = coop_blocks();
+    if (per_sm == 0)
+        return build_bvh8_levels(rec, root, leaf0, tris, n, nodes8, tris8, collapse_ws(ws, bvh8_capacity(n) + 1u),
+                                 host_ctl, err, s);
+    if ((e = enqueue_collapse(rec, root, 1u, leaf0, tris, n, nodes8, tris8, ws, meta, err, per_sm, stall, s)) !=
         cudaSuccess)
         return (int)e;
-    host_ctl[4] = 2;  // the seed and the cooperative kernel
-    if (meta) {
-        // node count and levels stay on the device until asked for
-        if ((e = cudaMemcpyAsync(meta, ws, 4, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return (int)e;
-        if ((e = cudaMemcpyAsync(meta + 1, ws + 4, 4, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return (int)e;
-        host_ctl[5] = 1;
-        return (int)cudaGetLastError();
-    }
-    // node count -> host_ctl[0], levels -> host_ctl[3]
-    if ((e = cudaMemcpyAsync(host_ctl, ws, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemcpyAsync(host_ctl + 3, ws + 4, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
-    return (int)cudaGetLastError();
+    host_ctl[4] = 2;  // the cooperative kernel and the cluster pass
+    host_ctl[5] = 1;  // node count and levels stay in meta until asked for
+    return 0;
 }
 
 }  // namespace sqk

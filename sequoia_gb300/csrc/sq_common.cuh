@@ -437,14 +437,13 @@ struct Trace8Args {
 // first triangle of a leaf range in 27 bits (and its count in 4).
 constexpr uint32_t kWide8MaxTris = 1u << 27;
 uint32_t bvh8_capacity(uint32_t n);
-size_t bvh8_node_bytes(uint32_t n);
-size_t bvh8_ws_words(uint32_t n);
+size_t bvh8_node_bytes(uint32_t n, uint32_t nroots);
+size_t bvh8_ws_words(uint32_t n, uint32_t nroots);
 size_t bvh8_tri_bytes(uint32_t n);
-// meta (device, 2 words, may be null): when given and the cooperative
-// collapse runs, the node count and level count are copied there on the
-// stream instead of being read back (no host synchronisation); host_ctl[4]
-// then holds 2 and host_ctl[0] / [3] are not written.  Returns 1 in
-// host_ctl[5] when meta was filled that way, else 0.
+// meta (device, 2 words): the cooperative collapse leaves its node and level
+// counts there (no host synchronisation) and sets host_ctl[5] to 1; the
+// per-level fallback reads them back to host_ctl[0] and [3] and sets it to 0.
+// host_ctl[4]: kernel launches.
 // Fault injection for the failure-detection tests: the cooperative
 // collapse's grid barrier waits for one block more than the grid, so every
 // block gives up after spin_limit polls (SQ_DEVERR_SAH_QUEUE) and returns.
@@ -452,7 +451,7 @@ struct BarrierStall {
     uint32_t spin_limit;
 };
 int build_bvh8(const sq::Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n, void* nodes8,
-               void* tris8, uint32_t* ws, uint32_t* host_ctl, uint32_t* err, cudaStream_t s, uint32_t* meta = nullptr,
+               void* tris8, uint32_t* ws, uint32_t* host_ctl, uint32_t* err, cudaStream_t s, uint32_t* meta,
                const BarrierStall* stall = nullptr);
 void trace8(const Trace8Args& a, cudaStream_t s);
 
@@ -492,11 +491,10 @@ struct BatchTraceArgs {
 void trace_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);
 void trace8_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);
 
-// 8-wide collapse seeded with several roots, with no host synchronisation
-// (a fixed number of level kernels with device-side task counts), so it can
-// be captured in a CUDA graph.  ws: bvh8_ws_words(n) + 4 * nroots words.
-// Wide node k (k < nroots) is the tree of roots[k].
-int build_bvh8_queue(const sq::Node* rec, const uint32_t* roots_dev, uint32_t nroots, uint32_t leaf0, const float* tris,
+// 8-wide collapse of several trees, with no host synchronisation, so it can
+// be captured in a CUDA graph.  ws: bvh8_ws_words(n, nroots) words.  Wide node
+// k (k < nroots) is the tree of record root0 + k.
+int build_bvh8_queue(const sq::Node* rec, uint32_t root0, uint32_t nroots, uint32_t leaf0, const float* tris,
                      uint32_t n, void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s);
 
 }  // namespace sqk
