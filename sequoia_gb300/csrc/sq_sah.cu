@@ -93,7 +93,7 @@ static_assert(sizeof(Part) == 64, "Part is 64 bytes");
 struct Ctl {
     unsigned long long level[3];
     uint32_t n_small, n_leaf;
-    uint32_t small_pop, big_pop;  // pop counters of the staged and the unstaged small kernels
+    uint32_t small_pop, pad;  // tasks taken by k_small's warps
 };
 static_assert(sizeof(Ctl) == 40, "Ctl is 40 bytes");
 
@@ -380,16 +380,20 @@ __global__ void k_grid_tasks(const uint32_t* __restrict__ cell_ord, const uint32
     place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
 }
 
-// heap of 63 inner nodes above the 64 cell nodes (src/builder.cpp:2181-2188)
+// heap of 63 inner nodes above the 64 cell nodes (src/builder.cpp:2181-2188),
+// a level at a time, one lane per node
 __global__ void k_grid_heap(Node* __restrict__ nodes)
 {
-    if (threadIdx.x != 0) return;
-    for (int i = 62; i >= 0; --i) {
-        const Node a = nodes[2 * i + 1], b = nodes[2 * i + 2];
-        Box u;
-        u.mn[0] = ref_min(a.mnx, b.mnx); u.mn[1] = ref_min(a.mny, b.mny); u.mn[2] = ref_min(a.mnz, b.mnz);
-        u.mx[0] = ref_max(a.mxx, b.mxx); u.mx[1] = ref_max(a.mxy, b.mxy); u.mx[2] = ref_max(a.mxz, b.mxz);
-        store_node(nodes + i, u, 2u * i + 1u, 2u, 0);
+    for (uint32_t width = 32; width; width >>= 1) {
+        if (threadIdx.x < width) {
+            const uint32_t i = width - 1u + threadIdx.x;
+            const Node a = nodes[2 * i + 1], b = nodes[2 * i + 2];
+            Box u;
+            u.mn[0] = ref_min(a.mnx, b.mnx); u.mn[1] = ref_min(a.mny, b.mny); u.mn[2] = ref_min(a.mnz, b.mnz);
+            u.mx[0] = ref_max(a.mxx, b.mxx); u.mx[1] = ref_max(a.mxy, b.mxy); u.mx[2] = ref_max(a.mxz, b.mxz);
+            store_node(nodes + i, u, 2u * i + 1u, 2u, 0);
+        }
+        __syncwarp();
     }
 }
 
@@ -702,10 +706,15 @@ __global__ void __launch_bounds__(128) k_large_split(LevelLists cur, LevelLists 
 // chunks are counted too (a side's run of one chunk lands in at most two).
 // ROOT: the level's tasks are binned in place, nothing moves.
 //
-// The blocks share one set of bins per side: shared-memory atomics on
-// order-preserving integers (13 a triangle), or full-warp reductions when 32
-// triangles share one side and bin.
-template <uint32_t CHUNK, bool ROOT>
+// The block's warps share kSlots / NBP copies of a side's bins (NBP: the bin count
+// rounded up to 8, 16 or 32), a lane's copy by its number: shared-memory
+// atomics on order-preserving integers, 13 a triangle, which were what bounded
+// the kernel (half of all shared-memory cycles) while lanes of one bin waited
+// for one another; full-warp reductions when 32 triangles share one side and
+// bin.
+constexpr int kSlots = 32;
+
+template <uint32_t CHUNK, int NBP, bool ROOT>
 __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ parts, LevelLists cur, LevelLists next,
                                                     uint32_t cur_i, uint32_t* __restrict__ ids_a,
                                                     uint32_t* __restrict__ ids_b, uint8_t* __restrict__ bin_a,
@@ -714,13 +723,14 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
 {
     chain_wait();  // a chained launch (enqueue_levels)
     chain_release();
-    __shared__ uint32_t s_bins[2 * kMaxBins * kBinWords];
-    __shared__ uint32_t s_cnt[2][2][kMaxBins];
+    __shared__ uint32_t s_bins[2 * kSlots * kBinWords];
+    __shared__ uint32_t s_cnt[2][2][kSlots];
     __shared__ uint32_t s_w[8];
     if (!ROOT && blockIdx.x == 0 && threadIdx.x == 0) ctl->level[(cur_i + 2u) % 3u] = 0;
     const uint32_t chunks = (uint32_t)(ctl->level[cur_i] >> 32);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t copy = (lane * NBP) & (kSlots - 1);  // first bin of the lane's copy
     const uint32_t cw = count_words(nb);
     for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {
         const Part P = parts[cur.chunk_task[c]];
@@ -733,8 +743,8 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
         uint32_t* out = ROOT ? nullptr : (from_b ? ids_a : ids_b) + P.begin;
         uint8_t* bin_out = (from_b != ROOT ? bin_a : bin_b) + P.begin;
         const bool large0 = P.task[0] != kNone, large1 = P.task[1] != kNone;
-        for (int j = threadIdx.x; j < 2 * kMaxBins * kBinWords; j += 256) s_bins[j] = 0;
-        if (threadIdx.x < 4 * kMaxBins) (&s_cnt[0][0][0])[threadIdx.x] = 0;
+        for (int j = threadIdx.x; j < 2 * kSlots * kBinWords; j += 256) s_bins[j] = 0;
+        for (int j = threadIdx.x; j < 4 * kSlots; j += 256) (&s_cnt[0][0][0])[j] = 0;
         // the warp's rows of 32 triangles
         const uint32_t rows = (len + 31u) >> 5, per = (rows + 7u) >> 3;
         const uint32_t r0 = warp * per, r1 = min(rows, r0 + per);
@@ -772,7 +782,7 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
             const bool binned = valid && (left ? large0 : large1);
             const uint32_t to = pos + (left ? 0u : P.nl);
             if (!ROOT && valid) out[to] = id;
-            uint32_t key = 0xFFu;
+            uint32_t key = kNone;
             uint32_t e[12];
             if (binned) {
                 float mn[3], mx[3], cc[3];
@@ -782,7 +792,7 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
                 const int b = bin_of(left ? P.k1[0] : P.k1[1], sel(cc, left ? P.axis[0] : P.axis[1]),
                                      left ? P.cmin[0] : P.cmin[1], nb);
                 bin_out[to] = (uint8_t)b;
-                key = side * kMaxBins + (uint32_t)b;
+                key = side * kSlots + (uint32_t)b;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     e[a] = float_to_ordered(-mn[a]);
@@ -790,11 +800,11 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
                     e[6 + a] = float_to_ordered(-cc[a]);
                     e[9 + a] = float_to_ordered(cc[a]);
                 }
-                atomicAdd(&s_cnt[side][pos / CHUNK - (left ? first[0] : first[1])][b], 1u);
+                atomicAdd(&s_cnt[side][pos / CHUNK - (left ? first[0] : first[1])][copy + (uint32_t)b], 1u);
             }
             const uint32_t key0 = __shfl_sync(0xFFFFFFFFu, key, 0);
             if (__all_sync(0xFFFFFFFFu, key == key0)) {
-                if (key0 != 0xFFu) {
+                if (key0 != kNone) {
 #pragma unroll
                     for (int k = 0; k < 12; ++k) e[k] = __reduce_max_sync(0xFFFFFFFFu, e[k]);
                     if (lane == 0) {
@@ -804,7 +814,7 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
                 }
             } else if (binned) {
 #pragma unroll
-                for (int k = 0; k < 12; ++k) atomicMax(&s_bins[key * kBinWords + k], e[k]);
+                for (int k = 0; k < 12; ++k) atomicMax(&s_bins[(key + copy) * kBinWords + k], e[k]);
             }
         }
         __syncthreads();
@@ -813,11 +823,14 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
         for (int side = 0; side < 2; ++side) {
             if (P.task[side] == kNone) continue;  // block-uniform
             uint32_t* g = next.bins + (size_t)P.task[side] * kMaxBins * kBinWords;
-            const uint32_t* sb = s_bins + side * kMaxBins * kBinWords;
+            const uint32_t* sb = s_bins + side * kSlots * kBinWords;
             for (int j = threadIdx.x; j < nb * kBinWords; j += 256) {
                 const int b = j / kBinWords;
                 const bool is_count = j - b * kBinWords == 12;
-                const uint32_t v = is_count ? s_cnt[side][0][b] + s_cnt[side][1][b] : sb[j];
+                uint32_t v = 0;
+#pragma unroll
+                for (int q = 0; q < kSlots; q += NBP)
+                    v = is_count ? v + s_cnt[side][0][b + q] + s_cnt[side][1][b + q] : max(v, sb[j + q * kBinWords]);
                 if (!several) g[j] = v;
                 else if (v) {
                     if (is_count) atomicAdd(g + j, v); else atomicMax(g + j, v);
@@ -827,26 +840,17 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
                 // the counts of the run's one or two chunks, two bins a word
                 for (uint32_t j = threadIdx.x; j < 2u * cw; j += 256) {
                     const uint32_t slot = j >= cw ? 1u : 0u, w = j - slot * cw;
-                    const uint32_t v = s_cnt[side][slot][2 * w] |
-                                       (2 * w + 1 < (uint32_t)nb ? s_cnt[side][slot][2 * w + 1] << 16 : 0u);
+                    uint32_t v = 0;
+#pragma unroll
+                    for (int q = 0; q < kSlots; q += NBP)
+                        v += s_cnt[side][slot][2 * w + q] +
+                             (2 * w + 1 < (uint32_t)nb ? s_cnt[side][slot][2 * w + 1 + q] << 16 : 0u);
                     if (v) atomicAdd(next.counts + (size_t)(P.child_chunk0[side] + first[side] + slot) * cw + w, v);
                 }
             }
         }
         __syncthreads();  // the shared bins are cleared for the next chunk
     }
-}
-
-// After the last fixed level of the batch build: large tasks still left go
-// to the small phase, whose warps split subtrees of any size.
-__global__ void k_large_to_small(const Task* __restrict__ large, const unsigned long long* __restrict__ level,
-                                 Task* __restrict__ small, Ctl* ctl)
-{
-    chain_wait();  // a chained launch (enqueue_levels)
-    chain_release();
-    const uint32_t nt = (uint32_t)*level;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x)
-        small[atomicAdd(&ctl->n_small, 1u)] = large[t];
 }
 
 // ---------------------------------------------------------------------------
@@ -902,9 +906,10 @@ __global__ void k_emit_leaves(const LeafRange* __restrict__ leaves, const Ctl* _
 // of shuffles, was what bounded a node.  The order of the stack does not
 // matter: a node's records go to slots that its range gives.
 //
-// Larger small tasks (leftovers of the batched build's fixed large levels)
-// are split by k_small_big, one node at a time, in the global buffers.
+// The large tasks left after a batch's fixed levels are split by k_small_big,
+// one node at a time, in the global buffers.
 constexpr uint32_t kStage = 128;
+static_assert(kSmall <= kStage, "every small task is staged");
 
 struct SmallNode {
     float p[6], c[6];  // primitive and centroid boxes (min xyz, max xyz)
@@ -1108,8 +1113,8 @@ __device__ void staged_subtree(const Task& root, SmallStage& sg, const uint32_t*
     }
 }
 
-// One warp per small task of at most kStage triangles (k_small_big takes the
-// others; each kernel pops the shared list with its own counter).
+// One warp per small task of at most kStage triangles (the tasks
+// left after the last level of a batch, larger ones, are k_small_big's).
 template <int NBP>
 __global__ void __launch_bounds__(128) k_small(const Task* __restrict__ small, Ctl* ctl,
                                                const uint32_t* __restrict__ ids_a, const uint32_t* __restrict__ ids_b,
@@ -1125,12 +1130,11 @@ __global__ void __launch_bounds__(128) k_small(const Task* __restrict__ small, C
         ti = __shfl_sync(0xFFFFFFFFu, ti, 0);
         if (ti >= total) return;
         const Task t = small[ti];
-        if (t.count > kStage) continue;  // warp-uniform
         staged_subtree<NBP>(t, s_stage[warp], (t.flags & 1u) ? ids_b : ids_a, tb, nb, leaf_size, base, nodes, leaf0);
     }
 }
 
-// A small task of more than kStage triangles: one warp, one node at a time,
+// A task of more than kStage triangles: one warp, one node at a time,
 // smaller child first (stack depth O(log n)), in the global buffers.
 __device__ void big_subtree(Task cur, Task* st, uint32_t* wb, uint32_t* __restrict__ ids_a, uint32_t* __restrict__ ids_b,
                             const float4* __restrict__ tb, int nb, uint32_t leaf_size, uint32_t base,
@@ -1236,22 +1240,19 @@ __device__ void big_subtree(Task cur, Task* st, uint32_t* wb, uint32_t* __restri
     }
 }
 
-__global__ void __launch_bounds__(128) k_small_big(const Task* __restrict__ small, Ctl* ctl, uint32_t* __restrict__ ids_a,
+__global__ void __launch_bounds__(128) k_small_big(const Task* __restrict__ tasks,
+                                                   const unsigned long long* __restrict__ level,
+                                                   uint32_t* __restrict__ ids_a,
                                                    uint32_t* __restrict__ ids_b, const float4* __restrict__ tb, int nb,
                                                    uint32_t leaf_size, uint32_t base, Node* __restrict__ nodes,
                                                    uint32_t leaf0, uint32_t* err)
 {
     __shared__ uint32_t s_bins[4][kMaxBins * kBinWords];
     __shared__ Task s_stack[4][kStackDepth];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t total = ctl->n_small;
-    for (;;) {
-        uint32_t ti = 0;
-        if (lane == 0) ti = atomicAdd(&ctl->big_pop, 1u);
-        ti = __shfl_sync(0xFFFFFFFFu, ti, 0);
-        if (ti >= total) return;
-        const Task cur = small[ti];
-        if (cur.count <= kStage) continue;  // warp-uniform
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t total = (uint32_t)*level;
+    for (uint32_t ti = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ti < total; ti += (gridDim.x * blockDim.x) >> 5) {
+        const Task cur = tasks[ti];
         big_subtree(cur, s_stack[warp], s_bins[warp], ids_a, ids_b, tb, nb, leaf_size, base, nodes, leaf0, err);
     }
 }
@@ -1330,13 +1331,21 @@ void with_chunk(uint32_t n, F f)
     else f(std::integral_constant<uint32_t, kChunk>());
 }
 
+// One k_large_move launch over the chunks of level `level` (in w.lists[cur]).
+template <uint32_t CHUNK, bool ROOT>
+void enqueue_move(const SahWs& w, uint32_t cur, uint32_t next, uint32_t cur_i, int nb, cudaStream_t s)
+{
+    auto kernel = nb <= 8 ? k_large_move<CHUNK, 8, ROOT> : nb <= 16 ? k_large_move<CHUNK, 16, ROOT>
+                                                                    : k_large_move<CHUNK, 32, ROOT>;
+    launch_chained(kernel, dim3(sms() * 8), dim3(256), 0, s, (const Part*)w.parts, w.lists[cur], w.lists[next], cur_i,
+                   w.ids_a, w.ids_b, w.bin_a, w.bin_b, (const uint32_t*)w.chunk_left, (const float4*)w.tb, nb, w.ctl);
+}
+
 // The bins of the root tasks in w.lists[0].
 template <uint32_t CHUNK>
 void enqueue_root_bins(const SahWs& w, int nb, cudaStream_t s)
 {
-    launch_chained(k_large_move<CHUNK, true>, dim3(sms() * 8), dim3(256), 0, s, (const Part*)w.parts, w.lists[0],
-                   w.lists[0], 0u, w.ids_a, w.ids_b, w.bin_a, w.bin_b, (const uint32_t*)w.chunk_left,
-                   (const float4*)w.tb, nb, w.ctl);
+    enqueue_move<CHUNK, true>(w, 0, 0, 0, nb, s);
 }
 
 // Levels [level, level + count) of the large phase: two chained launches a
@@ -1348,12 +1357,10 @@ void enqueue_levels(const SahWs& w, uint32_t level, uint32_t count, int nb, uint
 {
     const uint32_t grid = (uint32_t)sms() * 8u;
     for (uint32_t l = level; l < level + count; ++l) {
-        const LevelLists &cur = w.lists[l & 1], &next = w.lists[(l + 1) & 1];
-        launch_chained(k_large_split<CHUNK>, dim3(grid), dim3(128), 0, s, cur, next, (const Ctl*)w.ctl, l % 3u,
-                       (l + 1) % 3u, nb, base, leaf_size, nodes, w.parts, w.chunk_left, w.small, w.leaves, w.ctl);
-        launch_chained(k_large_move<CHUNK, false>, dim3(grid), dim3(256), 0, s, (const Part*)w.parts, cur, next, l % 3u,
-                       w.ids_a, w.ids_b, w.bin_a, w.bin_b, (const uint32_t*)w.chunk_left, (const float4*)w.tb, nb,
-                       w.ctl);
+        launch_chained(k_large_split<CHUNK>, dim3(grid), dim3(128), 0, s, w.lists[l & 1], w.lists[(l + 1) & 1],
+                       (const Ctl*)w.ctl, l % 3u, (l + 1) % 3u, nb, base, leaf_size, nodes, w.parts, w.chunk_left,
+                       w.small, w.leaves, w.ctl);
+        enqueue_move<CHUNK, false>(w, l & 1, (l + 1) & 1, l % 3u, nb, s);
     }
 }
 
@@ -1507,8 +1514,6 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
         }
     // small phase and leaves
     const uint32_t sg = (uint32_t)sms() * 8u;
-    // a single build's small tasks all have at most kSmall = kStage triangles
-    static_assert(kSmall <= kStage, "every small task of a single build is staged");
     launch_small(w, (int)nb, leaf_size, base, nodes, leaf0, s);
     k_emit_leaves<<<sg, 256, 0, s>>>(w.leaves, w.ctl, w.ids_a, w.ids_b, w.tb, nodes, leaf0, err);
     if (grid) k_grid_heap<<<1, 32, 0, s>>>(nodes);
@@ -1545,11 +1550,9 @@ int build_sah_batch(const float* tris, uint32_t n, const uint32_t* off, uint32_t
         enqueue_root_bins<CHUNK>(w, (int)nb, s);
         enqueue_levels<CHUNK>(w, 0, kBatchLargeLevels, (int)nb, 0u, leaf_size, nodes, s);
     });
-    launch_chained(k_large_to_small, dim3(sm), dim3(256), 0, s, (const Task*)w.lists[kBatchLargeLevels & 1].tasks,
-                   (const unsigned long long*)&w.ctl->level[kBatchLargeLevels % 3], w.small, w.ctl);
     launch_small(w, (int)nb, leaf_size, 0u, nodes, leaf0, s);
-    k_small_big<<<sm * 8u, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0,
-                                        err);
+    k_small_big<<<sm * 8u, 128, 0, s>>>(w.lists[kBatchLargeLevels & 1].tasks, &w.ctl->level[kBatchLargeLevels % 3],
+                                        w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0, err);
     k_emit_leaves<<<sm * 8u, 256, 0, s>>>(w.leaves, w.ctl, w.ids_a, w.ids_b, w.tb, nodes, leaf0, err);
     return (int)cudaGetLastError();
 #undef SQ_TRY
