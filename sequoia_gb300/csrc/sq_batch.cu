@@ -2,7 +2,7 @@
 // sequence that is captured once in a CUDA graph and replayed.
 //
 // Build (all meshes together, no host synchronisation), Morton builder:
-//   k_seg_bounds     every mesh's box (warp-aggregated atomics per mesh)
+//   k_seg_bounds     every mesh's box
 //   k_seg_morton     30-bit Morton codes in each mesh's own box (as if the
 //                    reference's setup_morton, src/builder.cpp:2204-2237, ran
 //                    per mesh) + the code digit histograms
@@ -86,24 +86,13 @@ __global__ void __launch_bounds__(256) k_seg_bounds(const float* __restrict__ tr
 {
     chain_wait();  // a chained launch (the batch build's kernels follow one another)
     chain_release();
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < n;
-        uint32_t m = 0xFFFFFFFFu;
-        uint32_t e[6] = {0, 0, 0, 0, 0, 0};
-        if (valid) {
-            m = mesh_of(off, M, i);
-            float t[9];
-            load_tri(tris, i, t);
-            const Box b = tri_box(t);
-            for (int k = 0; k < 3; ++k) { e[k] = float_to_ordered(-b.mn[k]); e[3 + k] = float_to_ordered(b.mx[k]); }
-        }
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, m);
+    seg_maxima<6>(n, off, M, box_ord, 8u, [&](uint32_t i, uint32_t* e) {
+        float t[9];
+        load_tri(tris, i, t);
+        const Box b = tri_box(t);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) e[k] = __reduce_max_sync(peers, e[k]);
-        if (valid && (threadIdx.x & 31) == (uint32_t)(__ffs(peers) - 1))
-            for (int k = 0; k < 6; ++k) atomicMax(box_ord + 8ull * m + k, e[k]);
-    }
+        for (int k = 0; k < 3; ++k) { e[k] = float_to_ordered(-b.mn[k]); e[3 + k] = float_to_ordered(b.mx[k]); }
+    });
 }
 
 __global__ void __launch_bounds__(256) k_seg_morton(const float* __restrict__ tris, uint32_t n,
@@ -146,12 +135,17 @@ __global__ void __launch_bounds__(256) k_seg_morton(const float* __restrict__ tr
     }
 }
 
-// mesh id of each sorted element, as the key of the second sort
+// mesh id of each sorted element, as the key of the second sort, and the
+// digit histograms of that sort (the meshes' sizes)
 __global__ void k_mesh_keys(const uint32_t* __restrict__ vals, uint32_t n, const uint32_t* __restrict__ off, uint32_t M,
-                            uint32_t* __restrict__ mkeys)
+                            uint32_t* __restrict__ mkeys, uint32_t* __restrict__ hist, uint32_t passes)
 {
     chain_wait();  // a chained launch (the batch build's kernels follow one another)
     chain_release();
+    for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
+        const uint32_t c = off[m + 1] - off[m];
+        for (uint32_t p = 0; p < passes && c; ++p) atomicAdd(hist + 256u * p + ((m >> (8u * p)) & 255u), c);
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         mkeys[i] = mesh_of(off, M, vals[i]);
 }
@@ -230,8 +224,8 @@ sq_status enqueue_run(sq_batch* b)
         uint32_t* mk = w ? ka : kb;   // free key buffer for the mesh keys
         uint32_t* ok = w ? kb : ka;
         uint32_t* ov = w ? va : vb;
-        launch_chained(k_mesh_keys, dim3(g), dim3(256), 0, s, (const uint32_t*)sv, N, (const uint32_t*)b->d_off, M, mk);
-        sqk::sort_histogram(mk, N, hist_m, 8, mp, s);
+        launch_chained(k_mesh_keys, dim3(g), dim3(256), 0, s, (const uint32_t*)sv, N, (const uint32_t*)b->d_off, M, mk,
+                       hist_m, mp);
         const int w2 = sqk::sort_passes(mk, sv, ok, ov, N, hist_m, lb_m, ctr + 8, 8, mp, c->ctrl, s);
         uint32_t* perm = w2 ? ov : sv;
         launch_chained(k_gather_codes, dim3(g), dim3(256), 0, s, (const uint32_t*)perm, N, (const uint32_t*)code_by_tri,

@@ -18,6 +18,61 @@ __device__ __forceinline__ uint32_t mesh_of(const uint32_t* __restrict__ off, ui
     return lo;
 }
 
+// Per-mesh maxima of K order-preserving words per triangle, into
+// out[stride * mesh + k] (zeroed; atomics).  Each block of 256 threads takes a
+// run of consecutive 256-triangle tiles and keeps the maxima of its current
+// mesh in registers, so the atomics are one set per warp and mesh of a block's
+// run; a tile that holds a mesh boundary merges its lanes by mesh instead.
+// (With that merge for every 32 triangles and a set of atomics after each,
+// 2.8M triangles of 64 meshes took 308 us, most of it waiting on the same few
+// words.)  load(i, e) fills e for triangle i.
+template <int K, class Load>
+__device__ __forceinline__ void seg_maxima(uint32_t n, const uint32_t* __restrict__ off, uint32_t M,
+                                           uint32_t* __restrict__ out, uint32_t stride, Load load)
+{
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t tiles = (n + 255u) / 256u, per = (tiles + gridDim.x - 1u) / gridDim.x;
+    const uint32_t t0 = blockIdx.x * per, t1 = min(tiles, t0 + per);
+    if (t0 >= t1) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t acc[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k] = 0u;
+    uint32_t m = mesh_of(off, M, t0 * 256u), end = __ldg(off + m + 1);
+    auto flush = [&] {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t v = __reduce_max_sync(FULL, acc[k]);
+            if (lane == 0 && v) atomicMax(out + (size_t)stride * m + k, v);
+            acc[k] = 0u;
+        }
+    };
+    for (uint32_t t = t0; t < t1; ++t) {
+        const uint32_t i = t * 256u + threadIdx.x, last = min(n, t * 256u + 256u);
+        uint32_t e[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) e[k] = 0u;
+        if (i < n) load(i, e);
+        if (last <= end) {  // block-uniform: the tile lies in mesh m
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc[k] = max(acc[k], e[k]);
+            continue;
+        }
+        flush();
+        const uint32_t mi = i < n ? mesh_of(off, M, i) : FULL;
+        const uint32_t peers = __match_any_sync(FULL, mi);
+#pragma unroll
+        for (int k = 0; k < K; ++k) e[k] = __reduce_max_sync(peers, e[k]);
+        if (i < n && lane == (uint32_t)(__ffs(peers) - 1))
+            for (int k = 0; k < K; ++k) atomicMax(out + (size_t)stride * mi + k, e[k]);
+        if (t + 1 < t1) {
+            m = mesh_of(off, M, last);
+            end = __ldg(off + m + 1);
+        }
+    }
+    flush();
+}
+
 struct RunFrame {
     uint32_t b, e, slot, state;
     Box acc;

@@ -32,6 +32,7 @@
 //   small nodes: one warp per subtree, smaller child first (stack depth
 //     O(log n)), binning and partitioning with warp intrinsics only.
 #include "sq_common.cuh"
+#include "sq_lbvh_dev.cuh"
 
 #include <type_traits>
 #include <utility>
@@ -1375,49 +1376,28 @@ void launch_small(const SahWs& w, int nb, uint32_t leaf_size, uint32_t base, Nod
 // batch: many meshes in one build
 
 // Boxes, ids and every mesh's root boxes (order-preserving words, 12 per
-// mesh at a stride of 16): triangle i belongs to the mesh m with
-// off[m] <= i < off[m + 1]; lanes of one mesh merge through the warp before
-// one atomic per word.
+// mesh at a stride of 16).
 __global__ void __launch_bounds__(256) k_sah_setup_seg(const float* __restrict__ tris, uint32_t n,
                                                        const uint32_t* __restrict__ off, uint32_t M,
                                                        float4* __restrict__ tb, uint32_t* __restrict__ ids,
                                                        uint32_t* __restrict__ root_ord)
 {
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < n;
-        uint32_t m = 0xFFFFFFFFu;
-        uint32_t e[12];
+    seg_maxima<12>(n, off, M, root_ord, 16u, [&](uint32_t i, uint32_t* e) {
+        float t[9];
+        load_tri(tris, i, t);
+        const Box b = tri_box(t);
+        tb[2ull * i] = make_float4(b.mn[0], b.mn[1], b.mn[2], 0.0f);
+        tb[2ull * i + 1] = make_float4(b.mx[0], b.mx[1], b.mx[2], 0.0f);
+        ids[i] = i;
 #pragma unroll
-        for (int k = 0; k < 12; ++k) e[k] = 0u;
-        if (valid) {
-            uint32_t lo = 0, hi = M;  // largest m with off[m] <= i
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (__ldg(off + mid) <= i) lo = mid; else hi = mid;
-            }
-            m = lo;
-            float t[9];
-            load_tri(tris, i, t);
-            const Box b = tri_box(t);
-            tb[2ull * i] = make_float4(b.mn[0], b.mn[1], b.mn[2], 0.0f);
-            tb[2ull * i + 1] = make_float4(b.mx[0], b.mx[1], b.mx[2], 0.0f);
-            ids[i] = i;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float c = (b.mn[k] + b.mx[k]) * 0.5f;
-                e[k] = float_to_ordered(-b.mn[k]);
-                e[3 + k] = float_to_ordered(b.mx[k]);
-                e[6 + k] = float_to_ordered(-c);
-                e[9 + k] = float_to_ordered(c);
-            }
+        for (int k = 0; k < 3; ++k) {
+            const float c = (b.mn[k] + b.mx[k]) * 0.5f;
+            e[k] = float_to_ordered(-b.mn[k]);
+            e[3 + k] = float_to_ordered(b.mx[k]);
+            e[6 + k] = float_to_ordered(-c);
+            e[9 + k] = float_to_ordered(c);
         }
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, m);
-#pragma unroll
-        for (int k = 0; k < 12; ++k) e[k] = __reduce_max_sync(peers, e[k]);
-        if (valid && (threadIdx.x & 31) == (uint32_t)(__ffs(peers) - 1))
-            for (int k = 0; k < 12; ++k) atomicMax(root_ord + 16ull * m + k, e[k]);
-    }
+    });
 }
 
 // One root task per mesh (one warp each): triangles [off[m], off[m + 1]),
