@@ -5,9 +5,10 @@
 // row order) traverse together: a node's children are visited when any ray
 // of the packet hits the node's box, and the packet counts one test per node
 // box.  Every pixel of the packet gets (tests / k) / 200 in the heatmap.  On
-// the GPU a packet is k lanes of a warp (32 / k packets per warp); "any ray"
-// is a ballot over the packet's lanes, so the lanes of a packet take one path
-// and keep identical stacks.
+// the GPU a warp walks 4 packets from one pool (sq_walk_dev.cuh): a lane
+// tests a node against the rays of the packet that visits it.  The packets
+// that a bundle leaves alone (below) are 8 lanes each: "any ray" is a ballot
+// over the packet's lanes, so they take one path and keep identical stacks.
 //
 // trace_bundle<k> (src/tracer.cpp:292-362, traverse_bundle 126-156,
 // intersect_bundle_aabb src/tracer.h:37-80): a tile of k = 16 or 64 rays
@@ -24,7 +25,9 @@
 // early), so the stack order need not be the reference's.  The heatmap bytes
 // are the reference's exactly.
 #include "sq_common.cuh"
-#include "sq_trace_dev.cuh"
+#include "sq_walk_dev.cuh"
+
+#include <algorithm>
 
 namespace {
 
@@ -64,42 +67,64 @@ __device__ uint32_t packet_tests(const Node* __restrict__ nodes, uint32_t nn, ui
     return tests;
 }
 
+// Packets of one warp's pool (sq_walk_dev.cuh): enough that the pool holds a
+// range for every lane most of the time, few enough that an image still
+// makes several rounds of warps.
+constexpr int kPoolPackets = 4;
+
 template <int K>
-__global__ void __launch_bounds__(128) k_trace_packet(const sqk::TraceArgs a)
+__global__ void __launch_bounds__(32) k_trace_packet(const sqk::TraceArgs a)
 {
     constexpr int KX = (K == 1 || K == 2) ? 1 : 2;  // floor(sqrt(k))
     constexpr int KY = K / KX;
-    constexpr int PPW = 32 / K;  // packets per warp
-    const int lane = (int)(threadIdx.x & 31u);
-    const int m = lane % K;      // ray of the packet (row order in the block)
-    const uint32_t pmask = (K == 32 ? 0xFFFFFFFFu : ((1u << K) - 1u)) << (lane - m);
+    constexpr int PW = kPoolPackets;
+    __shared__ WalkPool<K, PW, false> pool;
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t bw = a.width / KX;
     const uint32_t total = bw * (a.height / KY);
+    const float org[3] = {a.cam[0], a.cam[1], a.cam[2]};
     uint64_t tests_sum = 0;
     for (;;) {
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(a.work, (uint32_t)PPW);
+        if (lane == 0) base = atomicAdd(a.work, (uint32_t)PW);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
         if (base >= total) break;
-        const uint32_t pk = base + (uint32_t)(lane / K);
-        if (pk < total) {
-            const uint32_t x = (pk % bw) * KX + (uint32_t)(m % KX);
-            const uint32_t y = (pk / bw) * KY + (uint32_t)(m / KX);
+        const uint32_t count = min((uint32_t)PW, total - base);
+        // ray m of packet p: pixel (m % KX, m / KX) of the packet's block
+        for (uint32_t j = lane; j < count * K; j += 32) {
+            const uint32_t p = j / K, m = j % K, pk = base + p;
             Ray r;
-            gen_reference_camera(x, y, a.width, a.height, a.cam, r);
-            const float inv[3] = {1.0f / r.d[0], 1.0f / r.d[1], 1.0f / r.d[2]};
-            bool fault = false;
-            const uint32_t t = packet_tests(a.nodes, a.node_count, a.root, 1u, r.o, inv, pmask, &fault);
-            if (fault && m == 0) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
-            write_heat(a.heat + 3ull * ((size_t)y * a.width + x), (float)t / (float)K, a.heat_ramp);
-            if (m == 0) tests_sum += t;
+            gen_reference_camera((pk % bw) * KX + m % KX, (pk / bw) * KY + m / KX, a.width, a.height, a.cam, r);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) pool.inv[c][m][p] = 1.0f / r.d[c];
         }
+        WalkStats st = {0u, false, false};
+        walk_pool<K, PW, false>(pool, count >= 32u ? 0xFFFFFFFFu : (1u << count) - 1u, a.nodes, a.node_count, a.tri_count,
+                                a.root, 1u, org, st, [](uint32_t, const float*, const float*) { return false; });
+        if (st.overflow || st.bad) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
+        for (uint32_t j = lane; j < count * K; j += 32) {
+            const uint32_t p = j / K, m = j % K, pk = base + p;
+            const uint32_t x = (pk % bw) * KX + m % KX, y = (pk / bw) * KY + m / KX;
+            write_heat(a.heat + 3ull * ((size_t)y * a.width + x), (float)pool.cnt[p] / (float)K, a.heat_ramp);
+        }
+        if (lane < count) tests_sum += pool.cnt[lane];
+        __syncwarp();  // the pool is used again for the warp's next packets
     }
     if (a.stats) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) tests_sum += __shfl_xor_sync(0xFFFFFFFFu, tests_sum, o);
         if (lane == 0) atomicAdd(a.stats, (unsigned long long)tests_sum);
     }
+}
+
+template <int K>
+void launch_packets(const sqk::TraceArgs& a, cudaStream_t s)
+{
+    static PerDevice<int> cache;
+    const uint32_t grid = (uint32_t)(cache.get([] { return blocks_per_sm(k_trace_packet<K>, 32); }) * sm_count());
+    const uint64_t packets = (uint64_t)a.width * a.height / K;
+    const uint64_t need = (packets + kPoolPackets - 1) / kPoolPackets;
+    k_trace_packet<K><<<(uint32_t)std::min<uint64_t>(grid, need ? need : 1), 32, 0, s>>>(a);
 }
 
 // morton_lut (src/tracer.cpp:18-23): k with bits 1 and 2 exchanged
@@ -265,10 +290,10 @@ void trace_coherent(const TraceArgs& a, uint32_t bundle, uint32_t k, cudaStream_
         return;
     }
     switch (k) {
-    case 1: k_trace_packet<1><<<grid, 128, 0, s>>>(a); break;
-    case 2: k_trace_packet<2><<<grid, 128, 0, s>>>(a); break;
-    case 4: k_trace_packet<4><<<grid, 128, 0, s>>>(a); break;
-    default: k_trace_packet<8><<<grid, 128, 0, s>>>(a); break;
+    case 1: launch_packets<1>(a, s); break;
+    case 2: launch_packets<2>(a, s); break;
+    case 4: launch_packets<4>(a, s); break;
+    default: launch_packets<8>(a, s); break;
     }
 }
 

@@ -245,13 +245,13 @@ inline int sm_count()
     });
 }
 
-// Resident blocks per SM of a kernel at a block size on the current device
-// (at least 1).
+// Resident blocks per SM of a kernel at a block size (and dynamic shared
+// memory) on the current device (at least 1).
 template <class Kernel>
-inline int blocks_per_sm(Kernel kernel, int threads)
+inline int blocks_per_sm(Kernel kernel, int threads, size_t smem = 0)
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
     return n > 0 ? n : 1;
 }
 

@@ -7,11 +7,13 @@
 // rays from a global counter (8x4 pixel tiles for camera rays, 32
 // consecutive rays for explicit ones), traces them, writes the results and
 // takes the next batch until the counter passes the end; the counter is
-// never waited on.  Each lane runs a stack traversal over Node1 records:
+// never waited on.  Each lane runs a stack traversal over Node1 records
+// (REF: the warp together):
 //
 //   SQ_TRACE_REF      the reference's semantics: every child box of every hit
 //                     inner node is tested and counted, no ordering, no early
-//                     exit, Moller-Trumbore hit flag (stack of node groups).
+//                     exit, Moller-Trumbore hit flag; the warp's rays share
+//                     one pool of node ranges (sq_walk_dev.cuh).
 //   SQ_TRACE_CLOSEST  near-child order: all children boxes of a node are
 //                     tested (and counted), hits are ordered by entry
 //                     distance (ties: slot order), the nearest is visited
@@ -25,7 +27,7 @@
 // The arithmetic is operation-for-operation that of oracle/sq_oracle.c
 // (compiled with -fmad=false), so results are bit-identical to it.
 #include "sq_common.cuh"
-#include "sq_trace_dev.cuh"
+#include "sq_walk_dev.cuh"
 
 namespace {
 
@@ -183,51 +185,37 @@ struct Result {
     bool bad;  // an index outside the node or triangle array
 };
 
+// REF mode, 32 rays a warp (sq_walk_dev.cuh).
+using RefPool = WalkPool<1, 32, true>;
+
 // traverse(hierarchy, index, count, ray, attributes) (src/tracer.cpp:47-65)
-// from the node group [root, root + group): every node of the group is
-// tested in turn, then the groups of the hit inner nodes, depth first.
-__device__ Result trace_ref(const Node* __restrict__ nodes, uint32_t nn, uint32_t nt, uint32_t root,
-                            const float* __restrict__ tris, const Ray& r, uint32_t group = 1u)
+// from the node group [root, root + group) for the ray of each lane (all 32
+// call it; `active`: the lane has one).  res.tri_tests is the number of
+// triangles that the lane tested, of any ray.
+__device__ __forceinline__ void trace_ref(const Node* __restrict__ nodes, uint32_t nn, uint32_t nt, uint32_t root,
+                                          uint32_t group, const float* __restrict__ tris, const Ray& r, bool active,
+                                          RefPool& pool, Result& res)
 {
-    float inv[3] = {1.0f / r.d[0], 1.0f / r.d[1], 1.0f / r.d[2]};
-    uint32_t st_child[kStack], st_count[kStack];
-    int sp = 0;
-    uint32_t cnt = 0, tcnt = 0;
-    bool hit = false, overflow = false;
-    bool bad = false;
-    uint32_t gidx = root, gcnt = group;
-    for (;;) {
-        if ((uint64_t)gidx + gcnt > nn) { bad = true; break; }
-        for (uint32_t i = 0; i < gcnt; ++i) {
-            const NodeRec nd = load_node(nodes, gidx + i);
-            cnt++;
-            if (box_ref(nd, r.o, inv, r.tmax)) {
-                if (node_is_leaf(nd.cf)) {
-                    const uint32_t c = node_count(nd.cf);
-                    if ((uint64_t)nd.child + c > nt) { bad = true; break; }
-                    for (uint32_t k = 0; k < c; ++k) hit |= tri_ref(tris, nd.child + k, r.o, r.d);
-                    tcnt += c;
-                } else {
-                    if (sp >= kStack) { overflow = true; break; }
-                    st_child[sp] = nd.child;
-                    st_count[sp] = node_count(nd.cf);
-                    sp++;
-                }
-            }
+    const uint32_t lane = threadIdx.x & 31u;
+    if (active) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            pool.o[a][lane] = r.o[a];
+            pool.d[a][lane] = r.d[a];
+            pool.inv[a][0][lane] = 1.0f / r.d[a];
         }
-        if (overflow || bad || sp == 0) break;
-        --sp;
-        gidx = st_child[sp];
-        gcnt = st_count[sp];
+        pool.tmax[lane] = r.tmax;
     }
-    Result res;
-    res.id = hit ? 0u : kNoHit;
+    WalkStats st = {0u, false, false};
+    walk_pool<1, 32, true>(pool, __ballot_sync(0xFFFFFFFFu, active), nodes, nn, nt, root, group, nullptr, st,
+                           [&](uint32_t tri, const float* o, const float* d) { return tri_ref(tris, tri, o, d); });
+    res.id = (pool.hit >> lane) & 1u ? 0u : kNoHit;
     res.t = 0.0f;
-    res.tests = cnt;
-    res.tri_tests = tcnt;
-    res.overflow = overflow;
-    res.bad = bad;
-    return res;
+    res.tests = active ? pool.cnt[lane] : 0u;
+    res.tri_tests = st.tri_tests;
+    res.overflow = st.overflow;
+    res.bad = st.bad;
+    __syncwarp();  // the pool is used again for the warp's next rays
 }
 
 // One ray's closest-hit (or any-hit) traversal, resumable one inner node at
@@ -479,6 +467,7 @@ __global__ void __launch_bounds__(128) k_trace(const sqk::TraceArgs a, uint32_t 
     const bool camera = a.ray_kind != SQ_RAYS_EXPLICIT;
     const uint32_t tiles_x = (a.width + 7u) >> 3;
     __shared__ WarpStats s_stats[4];
+    extern __shared__ __align__(16) unsigned char s_pools[];  // REF: one RefPool per warp
     WarpStats& ws = s_stats[threadIdx.x >> 5];
     ws.reset(lane);
     for (;;) {
@@ -511,20 +500,20 @@ __global__ void __launch_bounds__(128) k_trace(const sqk::TraceArgs a, uint32_t 
         Result res;
         res.tests = 0;
         res.tri_tests = 0;
-        if (active) {
-            if (MODE == SQ_TRACE_REF) res = trace_ref(a.nodes, a.node_count, a.tri_count, a.root, a.tris, r,
-                                                      a.root_group);
-            else res = trace_closest<MODE == SQ_TRACE_ANYHIT>(a.nodes, a.node_count, a.tri_count, a.root, a.tris, r);
-            if (res.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
-            if (res.bad) raise_error(a.err, SQ_DEVERR_TOPOLOGY);
-        }
+        res.overflow = res.bad = false;
+        if (MODE == SQ_TRACE_REF)
+            trace_ref(a.nodes, a.node_count, a.tri_count, a.root, a.root_group, a.tris, r, active,
+                      reinterpret_cast<RefPool*>(s_pools)[threadIdx.x >> 5], res);
+        else if (active)
+            res = trace_closest<MODE == SQ_TRACE_ANYHIT>(a.nodes, a.node_count, a.tri_count, a.root, a.tris, r);
+        if (res.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
+        if (res.bad) raise_error(a.err, SQ_DEVERR_TOPOLOGY);
         if (a.stats) {
             // requested bytes: ray in (explicit rays), hit record + heatmap out,
             // 32 B per node record tested, 36 B per triangle tested
             unsigned long long bt = res.tests, tt = res.tri_tests;
-            unsigned long long by = active ? (unsigned long long)(camera ? 0u : 32u) + (a.hits ? 12u : 0u) +
-                                                 (a.heat ? 3u : 0u) + 32ull * res.tests + 36ull * res.tri_tests
-                                           : 0ull;
+            unsigned long long by = 32ull * res.tests + 36ull * res.tri_tests;
+            if (active) by += (unsigned long long)(camera ? 0u : 32u) + (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u);
             ws.add(lane, bt, tt, by, bt);
         }
         if (!active) continue;
@@ -644,6 +633,13 @@ __global__ void __launch_bounds__(128) k_trace_refill(const sqk::TraceArgs a, ui
     }
 }
 
+// Dynamic shared memory of a tiles kernel: the pools of REF mode.
+template <int MODE>
+constexpr size_t pool_bytes(int block)
+{
+    return MODE == SQ_TRACE_REF ? sizeof(RefPool) * (size_t)(block / 32) : 0;
+}
+
 template <int MODE>
 void launch(const sqk::TraceArgs& a, cudaStream_t s)
 {
@@ -652,19 +648,22 @@ void launch(const sqk::TraceArgs& a, cudaStream_t s)
     else batches = ((a.width + 7u) / 8u) * ((a.height + 3u) / 4u);
     if (batches == 0) return;
     const bool refill = a.refill && MODE != SQ_TRACE_REF;
+    // REF: one warp per block, so that a block's place is free as soon as its
+    // warp is done
+    constexpr int kBlock = MODE == SQ_TRACE_REF ? 32 : 128;
     static PerDevice<std::array<int, 2>> cache;
     const std::array<int, 2> per_sm = cache.get([] {
-        return std::array<int, 2>{blocks_per_sm(k_trace<MODE>, 128),
+        return std::array<int, 2>{blocks_per_sm(k_trace<MODE>, kBlock, pool_bytes<MODE>(kBlock)),
                                   blocks_per_sm(k_trace_refill<MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE>, 128)};
     });
     uint32_t grid = (uint32_t)(per_sm[refill ? 1 : 0] * sm_count());
-    const uint32_t need = (batches + 3u) / 4u;
+    const uint32_t need = refill ? (batches + 3u) / 4u : (batches + kBlock / 32 - 1u) / (kBlock / 32);
     if (grid > need) grid = need;
     if (refill) {
         const uint32_t total = a.ray_kind == SQ_RAYS_EXPLICIT ? a.ray_count : batches * 32u;
         k_trace_refill<MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE><<<grid, 128, 0, s>>>(a, total);
     } else {
-        k_trace<MODE><<<grid, 128, 0, s>>>(a, batches);
+        k_trace<MODE><<<grid, kBlock, pool_bytes<MODE>(kBlock), s>>>(a, batches);
     }
 }
 
@@ -675,6 +674,7 @@ __global__ void __launch_bounds__(256) k_trace_batch(const sqk::BatchTraceArgs a
 {
     const uint32_t lane = threadIdx.x & 31u;
     __shared__ WarpStats s_stats[8];
+    extern __shared__ __align__(16) unsigned char s_pools[];  // REF: one RefPool per warp
     WarpStats& ws = s_stats[threadIdx.x >> 5];
     ws.reset(lane);
     for (;;) {
@@ -711,19 +711,21 @@ __global__ void __launch_bounds__(256) k_trace_batch(const sqk::BatchTraceArgs a
         Result res;
         res.tests = 0;
         res.tri_tests = 0;
-        if (active) {
-            if (MODE == SQ_TRACE_REF) res = trace_ref(a.nodes, a.node_count, a.tri_count, job.root, a.tris, r);
-            else res = trace_closest<MODE == SQ_TRACE_ANYHIT>(a.nodes, a.node_count, a.tri_count, job.root, a.tris, r);
-            if (res.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
-            if (res.bad) raise_error(a.err, SQ_DEVERR_TOPOLOGY);
-            if (MODE != SQ_TRACE_REF && res.id != kNoHit) res.id -= job.tri_offset;
-        }
+        res.overflow = res.bad = false;
+        if (MODE == SQ_TRACE_REF)
+            trace_ref(a.nodes, a.node_count, a.tri_count, job.root, 1u, a.tris, r, active,
+                      reinterpret_cast<RefPool*>(s_pools)[threadIdx.x >> 5], res);
+        else if (active)
+            res = trace_closest<MODE == SQ_TRACE_ANYHIT>(a.nodes, a.node_count, a.tri_count, job.root, a.tris, r);
+        if (res.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
+        if (res.bad) raise_error(a.err, SQ_DEVERR_TOPOLOGY);
+        if (MODE != SQ_TRACE_REF && active && res.id != kNoHit) res.id -= job.tri_offset;
         if (a.stats) {
             unsigned long long bt = res.tests, tt = res.tri_tests;
-            unsigned long long by = active ? (unsigned long long)(job.ray_kind == SQ_RAYS_EXPLICIT ? 32u : 0u) +
-                                                 (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u) + 32ull * res.tests +
-                                                 36ull * res.tri_tests
-                                           : 0ull;
+            unsigned long long by = 32ull * res.tests + 36ull * res.tri_tests;
+            if (active)
+                by += (unsigned long long)(job.ray_kind == SQ_RAYS_EXPLICIT ? 32u : 0u) + (a.hits ? 12u : 0u) +
+                      (a.heat ? 3u : 0u);
             ws.add(lane, bt, tt, by, bt);
         }
         if (!active) continue;
@@ -862,8 +864,14 @@ void launch_batch(const sqk::BatchTraceArgs& a, int block, cudaStream_t s)
     constexpr int RM = MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE;  // refill: closest / any-hit only
     static PerDevice<std::array<int, 6>> cache;
     const std::array<int, 6> per_sm = cache.get([] {
-        return std::array<int, 6>{blocks_per_sm(k_trace_batch<MODE>, 64), blocks_per_sm(k_trace_batch<MODE>, 128),
-                                  blocks_per_sm(k_trace_batch<MODE>, 256), blocks_per_sm(k_trace_batch_refill<RM>, 64),
+        // above 48 KB of dynamic shared memory is a per-device opt-in
+        if (MODE == SQ_TRACE_REF)
+            cudaFuncSetAttribute(k_trace_batch<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)pool_bytes<MODE>(256));
+        return std::array<int, 6>{blocks_per_sm(k_trace_batch<MODE>, 64, pool_bytes<MODE>(64)),
+                                  blocks_per_sm(k_trace_batch<MODE>, 128, pool_bytes<MODE>(128)),
+                                  blocks_per_sm(k_trace_batch<MODE>, 256, pool_bytes<MODE>(256)),
+                                  blocks_per_sm(k_trace_batch_refill<RM>, 64),
                                   blocks_per_sm(k_trace_batch_refill<RM>, 128),
                                   blocks_per_sm(k_trace_batch_refill<RM>, 256)};
     });
@@ -873,7 +881,7 @@ void launch_batch(const sqk::BatchTraceArgs& a, int block, cudaStream_t s)
     const uint32_t need = (a.total_batches + (uint32_t)(block / 32) - 1) / (uint32_t)(block / 32);
     if (grid > need) grid = need;
     if (refill) k_trace_batch_refill<RM><<<grid, block, 0, s>>>(a);
-    else k_trace_batch<MODE><<<grid, block, 0, s>>>(a);
+    else k_trace_batch<MODE><<<grid, block, pool_bytes<MODE>(block), s>>>(a);
 }
 
 }  // namespace

@@ -1,0 +1,165 @@
+// sq_walk_dev.cuh -- the order-free traversals of the reference, a warp's
+// rays or packets from one pool of node ranges.
+//
+// trace() / traverse() (src/tracer.cpp:47-65, 195-230) and trace_packet<k>
+// (src/tracer.cpp:88-123, 232-281) test every child of every node that a ray
+// (any ray of a packet) hits, in no order that matters and with no early
+// exit: the result is a count and a hit flag.  So a ray's node ranges need
+// not be walked by the ray's own lane.  The warp keeps one pool of (node
+// range, owner) entries in shared memory, and each step every lane takes an
+// entry of any owner, tests up to two nodes against the owner's K rays (a
+// node counts once a packet, so the first ray that hits ends its test) and
+// puts the hit nodes' child ranges back.  Triangles of hit leaves go to a
+// second pool and are tested 32 at a time.
+//
+// What bounds it: with a ray per lane the kernel waited for its longest rays
+// (a ray through the middle of the 2M-triangle soup tests thousands of boxes,
+// its neighbours in the warp tens): 14 of 32 lanes busy and 30% of the warps
+// resident on average.
+#pragma once
+
+#include "sq_trace_dev.cuh"
+
+namespace sq {
+
+constexpr uint32_t kPoolCap = 768;      // node ranges in a warp's pool
+constexpr uint32_t kPoolReserve = 128;  // kept for the one-at-a-time walk below
+constexpr uint32_t kTriCap = 128;       // 31 waiting + 64 of one step fit
+constexpr uint32_t kCountBits = 27;     // an entry: node, owner << 27 | node count
+constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
+
+// K rays per owner, PW owners per warp (at most 32).
+template <int K, int PW, bool TRI>
+struct WalkPool {
+    uint2 node[kPoolCap];
+    uint2 tri[TRI ? kTriCap : 1];
+    float inv[3][K][PW];                      // reciprocal directions
+    float o[3][TRI ? PW : 1], d[3][TRI ? PW : 1], tmax[TRI ? PW : 1];
+    uint32_t cnt[PW];                         // box tests of each owner
+    uint32_t hit;                             // bit per owner: a triangle was hit
+};
+
+struct WalkStats {
+    uint32_t tri_tests;  // this lane's
+    bool overflow, bad;  // pool full; an index outside the node or triangle array
+};
+
+// Walks nodes [root, root + group) for every owner in `owners` (a mask, the
+// same in all lanes); pool.inv (and o, d, tmax with TRI) hold the owners'
+// rays.  Without TRI all rays start at `org` and end at 10000.  hit_tri(tri, o, d)
+// tests one triangle.  Afterwards pool.cnt and pool.hit have the results.
+//
+// The pool grows by at most two ranges per entry taken, so as it fills fewer
+// entries are taken a step, down to one at a time where fewer than
+// kPoolReserve places are left: a depth-first walk of one subtree, which needs
+// no more places than the 64 pending ranges a ray's own stack would hold.
+template <int K, int PW, bool TRI, class HitTri>
+__device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI>& pool, uint32_t owners, const Node* __restrict__ nodes,
+                                          uint32_t nn, uint32_t nt, uint32_t root, uint32_t group, const float* org,
+                                          WalkStats& st, HitTri hit_tri)
+{
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    if (lane < (uint32_t)PW) pool.cnt[lane] = 0;
+    if (lane == 0) pool.hit = 0;
+    // a range of 2^26 nodes or more (no node has one, a caller's root group
+    // may) is walked in pieces
+    for (uint32_t g0 = 0; g0 < group;) {
+        const uint32_t piece = min(group - g0, 1u << 26);
+        if ((owners >> lane) & 1u)
+            pool.node[__popc(owners & lt)] = make_uint2(root + g0, piece | (lane << kCountBits));
+        g0 += piece;
+        uint32_t size = __popc(owners), tris = 0;
+        __syncwarp();
+        for (;;) {
+            if (TRI && (tris >= 32u || (size == 0u && tris))) {
+                const uint32_t take = min(32u, tris);
+                uint2 e = make_uint2(0u, 0u);
+                if (lane < take) e = pool.tri[tris - 1u - lane];
+                tris -= take;
+                const uint32_t w = e.y >> kCountBits, c = e.y & kCountMask;
+                if (lane < take) {
+                    const float o[3] = {pool.o[0][w], pool.o[1][w], pool.o[2][w]};
+                    const float d[3] = {pool.d[0][w], pool.d[1][w], pool.d[2][w]};
+                    bool hit = false;
+                    for (uint32_t k = 0; k < c; ++k) hit |= hit_tri(e.x + k, o, d);
+                    st.tri_tests += c;
+                    if (hit) atomicOr(&pool.hit, 1u << w);
+                }
+                __syncwarp();
+                continue;
+            }
+            if (size == 0) break;
+            const uint32_t room = size + kPoolReserve < kPoolCap ? (kPoolCap - kPoolReserve - size) / 2u : 0u;
+            const uint32_t take = min(min(32u, size), max(room, 1u));
+            if (size + 2u > kPoolCap) {
+                st.overflow = true;
+                break;
+            }
+            uint2 e = make_uint2(0u, 0u);
+            if (lane < take) e = pool.node[size - 1u - lane];
+            size -= take;
+            const uint32_t w = e.y >> kCountBits;
+            uint32_t c = e.y & kCountMask;
+            if ((uint64_t)e.x + c > nn) {
+                st.bad = true;
+                c = 0;
+            }
+            // up to two nodes now, the rest of the range back to the pool; a
+            // long range is halved instead
+            const bool halve = c > 16u;
+            const uint32_t k = halve ? 0u : min(c, 2u);
+            uint2 put[3];
+            bool has[3] = {halve, halve, !halve && c > 2u}, leaf[2] = {false, false};
+            put[0] = make_uint2(e.x, (c >> 1) | (w << kCountBits));
+            put[1] = make_uint2(e.x + (c >> 1), (c - (c >> 1)) | (w << kCountBits));
+            put[2] = make_uint2(e.x + 2u, (c - 2u) | (w << kCountBits));
+            if (k) {
+                float o[3], tmax;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) o[a] = TRI ? pool.o[a][w] : org[a];
+                tmax = TRI ? pool.tmax[w] : 10000.0f;
+                const NodeRec n0 = load_node(nodes, e.x), n1 = load_node(nodes, e.x + (k > 1u ? 1u : 0u));
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (q && k < 2u) break;
+                    const NodeRec& nd = q ? n1 : n0;
+                    bool hit = false;
+                    for (int m = 0; m < K && !hit; ++m) {
+                        const float inv[3] = {pool.inv[0][m][w], pool.inv[1][m][w], pool.inv[2][m][w]};
+                        hit = box_ref(nd, o, inv, tmax);
+                    }
+                    const uint32_t cc = node_count(nd.cf);
+                    if (hit && cc) {
+                        put[q] = make_uint2(nd.child, cc | (w << kCountBits));
+                        if (!node_is_leaf(nd.cf)) has[q] = true;
+                        else if (TRI) {
+                            if ((uint64_t)nd.child + cc > nt) st.bad = true;
+                            else leaf[q] = true;
+                        }
+                    }
+                }
+                atomicAdd(&pool.cnt[w], k);
+            }
+            __syncwarp();  // every lane has its entry before any is overwritten
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const uint32_t b = __ballot_sync(FULL, has[q]);
+                if (has[q]) pool.node[size + __popc(b & lt)] = put[q];
+                size += __popc(b);
+            }
+            if (TRI) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const uint32_t b = __ballot_sync(FULL, leaf[q]);
+                    if (leaf[q]) pool.tri[tris + __popc(b & lt)] = put[q];
+                    tris += __popc(b);
+                }
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+    }
+}
+
+}  // namespace sq
