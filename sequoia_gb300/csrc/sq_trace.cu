@@ -218,17 +218,93 @@ __device__ __forceinline__ void trace_ref(const Node* __restrict__ nodes, uint32
     __syncwarp();  // the pool is used again for the warp's next rays
 }
 
+// Closest-hit / any-hit stack entries hold what the visit of the child needs
+// -- its first child or triangle and how many -- so that popping one does not
+// wait for the node's own record (a visit used to be two dependent loads: the
+// popped record, then its children).  One million any-hit rays against the
+// 500k soup took 2.04 ms against 2.60 ms with node indices on the stack.
+//
+//   narrow  8 bytes: bit 31 leaf, bits 27-30 count (1 to 15; 0: the low bits
+//           are the node's index and its record is read after all), bits 0-26
+//           first child or triangle; entry distance.  Trees of up to 2^27
+//           records and triangles.
+//   wide    16 bytes: first child or triangle, count and leaf bit (31), entry
+//           distance.  Larger trees.
+template <bool WIDE>
+struct Entry {
+    uint32_t x, y;  // y: wide only
+};
+template <bool WIDE>
+struct StackSlot {
+    uint2 v;
+};
+template <>
+struct StackSlot<true> {
+    uint4 v;
+};
+constexpr uint32_t kNarrowMask = 0x07FFFFFFu;
+
+template <bool WIDE>
+__device__ __forceinline__ Entry<WIDE> make_entry(uint32_t index, const NodeRec& nd)
+{
+    const uint32_t c = node_count(nd.cf), leaf = node_is_leaf(nd.cf) ? 0x80000000u : 0u;
+    Entry<WIDE> e;
+    e.y = 0;
+    if (WIDE) { e.x = nd.child; e.y = c | leaf; }
+    else e.x = c - 1u < 15u ? leaf | (c << 27) | nd.child : index;
+    return e;
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void put_slot(StackSlot<WIDE>& s, const Entry<WIDE>& e, float t)
+{
+    if constexpr (WIDE) s.v = make_uint4(e.x, e.y, __float_as_uint(t), 0u);
+    else s.v = make_uint2(e.x, __float_as_uint(t));
+}
+template <bool WIDE>
+__device__ __forceinline__ Entry<WIDE> get_slot(const StackSlot<WIDE>& s, float& t)
+{
+    Entry<WIDE> e;
+    e.x = s.v.x;
+    e.y = 0;
+    if constexpr (WIDE) { e.y = s.v.y; t = __uint_as_float(s.v.z); }
+    else t = __uint_as_float(s.v.y);
+    return e;
+}
+
+// First child (or triangle), count and leaf flag of an entry.
+template <bool WIDE>
+__device__ __forceinline__ void open_entry(const Entry<WIDE>& e, const Node* __restrict__ nodes, uint32_t& first,
+                                           uint32_t& count, bool& leaf)
+{
+    if (WIDE) {
+        first = e.x;
+        count = e.y & 0xFFFFu;
+        leaf = (e.y >> 31) != 0u;
+        return;
+    }
+    first = e.x & kNarrowMask;
+    count = (e.x >> 27) & 0xFu;
+    leaf = (e.x >> 31) != 0u;
+    if (count == 0) {
+        const NodeRec nd = load_node(nodes, first);
+        first = nd.child;
+        count = node_count(nd.cf);
+        leaf = node_is_leaf(nd.cf);
+    }
+}
+
 // One ray's closest-hit (or any-hit) traversal, resumable one inner node at
 // a time so that a warp can refill a finished lane with a new ray while the
-// others continue.  Stack entries: node index, or (triangle index |
-// 0x80000000) for a leaf record whose triangle is still to be tested.
+// others continue.
 struct Lane2 {
     RayPre rp;
     float best_t;
     uint32_t best;
-    uint32_t cnt, tcnt;  // box tests, triangle tests
-    uint32_t cur;        // inner node to visit next; kNoHit when the ray is done
+    uint32_t cnt, tcnt;        // box tests, triangle tests
+    uint32_t first, children;  // the children to test next
     int sp;
+    bool more;                 // there are such children (else the ray is done)
     bool overflow, bad;
 };
 
@@ -257,71 +333,97 @@ __device__ __forceinline__ void lane2_start(Lane2& L, const Node* __restrict__ n
     L.sp = 0;
     L.overflow = false;
     L.bad = false;
-    L.cur = kNoHit;
+    L.more = false;
     float tn;
     if (root >= nn) { L.bad = true; return; }
     const NodeRec rn = load_node(nodes, root);
     if (!box_robust(rn, L.rp, L.best_t, tn)) return;
-    if (!node_is_leaf(rn.cf)) { L.cur = root; return; }
     const uint32_t c = node_count(rn.cf);
+    if (!node_is_leaf(rn.cf)) {
+        L.first = rn.child;
+        L.children = c;
+        L.more = true;
+        return;
+    }
     if ((uint64_t)rn.child + c > nt) { L.bad = true; return; }
     for (uint32_t k = 0; k < c; ++k)
         if (lane2_tri<ANY>(L, tris, rn.child + k)) return;
 }
 
-// Visit L.cur (an inner node that passed its box test and the cull test):
-// test all its children's boxes, order the hits by entry distance (ties:
-// slot order), push them, then pop until an inner node survives the cull
-// test, testing leaf triangles on the way.  Leaves L.cur at that node, or at
-// kNoHit when the ray is done.
-template <bool ANY>
+// Test the boxes of children [L.first, L.first + L.children), take the
+// nearest hit next and push the others (ties: slot order), then pop until an
+// inner node survives the cull test, testing leaf triangles on the way.
+// Leaves L at that node's children, or with L.more false when the ray is
+// done.  A node's two children, by far the most frequent case, are loaded
+// together and ordered without the hit list.
+template <bool ANY, bool WIDE>
 __device__ __forceinline__ void visit2(Lane2& L, const Node* __restrict__ nodes, uint32_t nn, uint32_t nt,
-                                       const float* __restrict__ tris, uint32_t* st_node, float* st_tn)
+                                       const float* __restrict__ tris, StackSlot<WIDE>* st)
 {
-    const NodeRec nd = load_node(nodes, L.cur);
-    L.cur = kNoHit;
-    const uint32_t c = node_count(nd.cf);
-    if ((uint64_t)nd.child + c > nn) { L.bad = true; return; }
-    uint32_t hn[8];
-    float ht[8];
-    int nh = 0;
-    for (uint32_t i = 0; i < c; ++i) {
-        const NodeRec ch = load_node(nodes, nd.child + i);
-        L.cnt++;
-        float t;
-        if (box_robust(ch, L.rp, L.best_t, t)) {
-            if (nh >= 8) { L.overflow = true; return; }
-            if (node_is_leaf(ch.cf) && (uint64_t)ch.child + node_count(ch.cf) > nt) { L.bad = true; return; }
-            const uint32_t ent = (node_is_leaf(ch.cf) && node_count(ch.cf) == 1u) ? (ch.child | 0x80000000u)
-                                                                                  : (nd.child + i);
-            // insertion by (tn, slot): equal distances keep slot order
-            int b = nh - 1;
-            while (b >= 0 && ht[b] > t) { hn[b + 1] = hn[b]; ht[b + 1] = ht[b]; --b; }
-            hn[b + 1] = ent;
-            ht[b + 1] = t;
-            nh++;
+    const uint32_t first = L.first, c = L.children;
+    L.more = false;
+    if ((uint64_t)first + c > nn) { L.bad = true; return; }
+    Entry<WIDE> e;
+    e.x = e.y = 0;
+    bool have = false;  // e is the entry to take next
+    if (c == 2u) {
+        const NodeRec n0 = load_node(nodes, first), n1 = load_node(nodes, first + 1u);
+        float t0, t1;
+        L.cnt += 2u;
+        const bool h0 = box_robust(n0, L.rp, L.best_t, t0), h1 = box_robust(n1, L.rp, L.best_t, t1);
+        if ((h0 && node_is_leaf(n0.cf) && (uint64_t)n0.child + node_count(n0.cf) > nt) ||
+            (h1 && node_is_leaf(n1.cf) && (uint64_t)n1.child + node_count(n1.cf) > nt)) {
+            L.bad = true;
+            return;
         }
+        if (L.sp + (int)h0 + (int)h1 > kStack) { L.overflow = true; return; }
+        const bool near1 = h1 && (!h0 || t1 < t0);
+        have = h0 || h1;
+        e = near1 ? make_entry<WIDE>(first + 1u, n1) : make_entry<WIDE>(first, n0);
+        if (h0 && h1) put_slot(st[L.sp++], near1 ? make_entry<WIDE>(first, n0) : make_entry<WIDE>(first + 1u, n1), near1 ? t0 : t1);
+    } else {
+        Entry<WIDE> he[8];
+        float ht[8];
+        int nh = 0;
+        for (uint32_t i = 0; i < c; ++i) {
+            const NodeRec ch = load_node(nodes, first + i);
+            L.cnt++;
+            float t;
+            if (box_robust(ch, L.rp, L.best_t, t)) {
+                if (nh >= 8) { L.overflow = true; return; }
+                if (node_is_leaf(ch.cf) && (uint64_t)ch.child + node_count(ch.cf) > nt) { L.bad = true; return; }
+                // insertion by (t, slot): equal distances keep slot order
+                int b = nh - 1;
+                while (b >= 0 && ht[b] > t) { he[b + 1] = he[b]; ht[b + 1] = ht[b]; --b; }
+                he[b + 1] = make_entry<WIDE>(first + i, ch);
+                ht[b + 1] = t;
+                nh++;
+            }
+        }
+        if (L.sp + nh > kStack) { L.overflow = true; return; }
+        for (int a = nh - 1; a >= 1; --a) put_slot(st[L.sp++], he[a], ht[a]);
+        have = nh > 0;
+        if (have) e = he[0];
     }
-    if (L.sp + nh > kStack) { L.overflow = true; return; }
-    for (int a = nh - 1; a >= 0; --a) { st_node[L.sp] = hn[a]; st_tn[L.sp] = ht[a]; L.sp++; }
-    while (L.sp > 0) {
-        --L.sp;
-        const uint32_t e = st_node[L.sp];
-        if (st_tn[L.sp] > L.best_t * kRobust) continue;
-        if (e & 0x80000000u) {
-            if (lane2_tri<ANY>(L, tris, e & 0x7FFFFFFFu)) return;
-            continue;
+    for (;;) {
+        if (!have) {
+            if (L.sp == 0) return;
+            float t;
+            e = get_slot(st[--L.sp], t);
+            if (t > L.best_t * kRobust) continue;
         }
-        const NodeRec lr = load_node(nodes, e);
-        if (node_is_leaf(lr.cf)) {
-            // leaf record holding several triangles
-            const uint32_t lc = node_count(lr.cf);
-            for (uint32_t k = 0; k < lc; ++k)
-                if (lane2_tri<ANY>(L, tris, lr.child + k)) return;
-            continue;
+        have = false;
+        uint32_t f, k;
+        bool leaf;
+        open_entry<WIDE>(e, nodes, f, k, leaf);
+        if (!leaf) {
+            L.first = f;
+            L.children = k;
+            L.more = true;
+            return;
         }
-        L.cur = e;
-        return;
+        for (uint32_t q = 0; q < k; ++q)
+            if (lane2_tri<ANY>(L, tris, f + q)) return;
     }
 }
 
@@ -338,10 +440,14 @@ __device__ __forceinline__ Result lane2_result(const Lane2& L)
 }
 
 // One ray traced to the end (the tiles kernels): the same traversal as
-// lane2_start + visit2 above, written as one loop, which the compiler fits
-// in fewer registers (48 against 56) -- the per-lane refill kernel needs the
-// resumable form, the tiles kernels do not.  The tests compare the two
-// schedules ray for ray (ids, t and box-test counts).
+// lane2_start + visit2 above, written as one loop over node indices, which
+// the compiler fits in fewer registers (48 against 56): neighbouring rays
+// share their node records in L1, so the second load costs them little and
+// the lanes of a warp, in step by a vote, waited 7% longer (the 2M soup at
+// 1080p 1,877 us against 1,737).  The per-lane refill kernels need the
+// resumable form.  The tests compare the two schedules ray for ray (ids, t
+// and box-test counts).  Stack entries: node index, or (triangle index |
+// 0x80000000) for a leaf record whose triangle is still to be tested.
 template <bool ANY>
 __device__ Result trace_closest(const Node* __restrict__ nodes, uint32_t nn, uint32_t nt, uint32_t root,
                                 const float* __restrict__ tris, const Ray& ray)
@@ -537,17 +643,16 @@ __global__ void __launch_bounds__(128) k_trace(const sqk::TraceArgs a, uint32_t 
 // visit order as in k_trace, so results are identical; only the assignment
 // of rays to lanes changes.  Ray g is explicit ray g, or pixel (g mod 32) of
 // 8x4 tile g / 32 for camera rays.
-template <int MODE>
+template <int MODE, bool WIDE>
 __global__ void __launch_bounds__(128) k_trace_refill(const sqk::TraceArgs a, uint32_t total)
 {
     constexpr bool ANY = MODE == SQ_TRACE_ANYHIT;
     const uint32_t lane = threadIdx.x & 31u;
     const bool camera = a.ray_kind != SQ_RAYS_EXPLICIT;
     const uint32_t tiles_x = (a.width + 7u) >> 3;
-    uint32_t st_node[kStack];
-    float st_tn[kStack];
+    StackSlot<WIDE> st[kStack];
     Lane2 L;
-    L.cur = kNoHit;
+    L.more = false;
     bool has = false, exhausted = false;
     uint32_t rid = 0;
     unsigned long long s_bt = 0, s_tt = 0, s_by = 0;
@@ -596,8 +701,8 @@ __global__ void __launch_bounds__(128) k_trace_refill(const sqk::TraceArgs a, ui
             continue;
         }
         if (has) {
-            if (L.cur != kNoHit) visit2<ANY>(L, a.nodes, a.node_count, a.tri_count, a.tris, st_node, st_tn);
-            if (L.cur == kNoHit) {
+            if (L.more) visit2<ANY, WIDE>(L, a.nodes, a.node_count, a.tri_count, a.tris, st);
+            if (!L.more) {
                 has = false;
                 const Result res = lane2_result(L);
                 if (res.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
@@ -640,7 +745,10 @@ constexpr size_t pool_bytes(int block)
     return MODE == SQ_TRACE_REF ? sizeof(RefPool) * (size_t)(block / 32) : 0;
 }
 
-template <int MODE>
+// Trees whose records and triangles a narrow stack entry can address.
+bool narrow_tree(uint32_t nodes, uint32_t tris) { return nodes <= kNarrowMask && tris <= kNarrowMask; }
+
+template <int MODE, bool WIDE>
 void launch(const sqk::TraceArgs& a, cudaStream_t s)
 {
     uint32_t batches;
@@ -654,14 +762,14 @@ void launch(const sqk::TraceArgs& a, cudaStream_t s)
     static PerDevice<std::array<int, 2>> cache;
     const std::array<int, 2> per_sm = cache.get([] {
         return std::array<int, 2>{blocks_per_sm(k_trace<MODE>, kBlock, pool_bytes<MODE>(kBlock)),
-                                  blocks_per_sm(k_trace_refill<MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE>, 128)};
+                                  blocks_per_sm(k_trace_refill<MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE, WIDE>, 128)};
     });
     uint32_t grid = (uint32_t)(per_sm[refill ? 1 : 0] * sm_count());
     const uint32_t need = refill ? (batches + 3u) / 4u : (batches + kBlock / 32 - 1u) / (kBlock / 32);
     if (grid > need) grid = need;
     if (refill) {
         const uint32_t total = a.ray_kind == SQ_RAYS_EXPLICIT ? a.ray_count : batches * 32u;
-        k_trace_refill<MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE><<<grid, 128, 0, s>>>(a, total);
+        k_trace_refill<MODE == SQ_TRACE_REF ? SQ_TRACE_CLOSEST : MODE, WIDE><<<grid, 128, 0, s>>>(a, total);
     } else {
         k_trace<MODE><<<grid, kBlock, pool_bytes<MODE>(kBlock), s>>>(a, batches);
     }
@@ -747,16 +855,15 @@ __global__ void __launch_bounds__(256) k_trace_batch(const sqk::BatchTraceArgs a
 // k_trace_refill over the job table's ray slots (slot g: lane g mod 32 of
 // the job's 32-ray batch g / 32); a lane keeps its current job's batch range
 // and searches the table only when a slot leaves it.
-template <int MODE>
+template <int MODE, bool WIDE>
 __global__ void __launch_bounds__(256) k_trace_batch_refill(const sqk::BatchTraceArgs a)
 {
     constexpr bool ANY = MODE == SQ_TRACE_ANYHIT;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t total = a.total_batches * 32u;
-    uint32_t st_node[kStack];
-    float st_tn[kStack];
+    StackSlot<WIDE> st[kStack];
     Lane2 L;
-    L.cur = kNoHit;
+    L.more = false;
     bool has = false, exhausted = false, explicit_rays = false;
     uint32_t out = 0, tri_offset = 0;
     uint32_t cj = 0, jlo = 1, jhi = 0;
@@ -821,8 +928,8 @@ __global__ void __launch_bounds__(256) k_trace_batch_refill(const sqk::BatchTrac
             continue;
         }
         if (has) {
-            if (L.cur != kNoHit) visit2<ANY>(L, a.nodes, a.node_count, a.tri_count, a.tris, st_node, st_tn);
-            if (L.cur == kNoHit) {
+            if (L.more) visit2<ANY, WIDE>(L, a.nodes, a.node_count, a.tri_count, a.tris, st);
+            if (!L.more) {
                 has = false;
                 Result res = lane2_result(L);
                 if (res.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
@@ -857,7 +964,7 @@ __global__ void __launch_bounds__(256) k_trace_batch_refill(const sqk::BatchTrac
     }
 }
 
-template <int MODE>
+template <int MODE, bool WIDE>
 void launch_batch(const sqk::BatchTraceArgs& a, int block, cudaStream_t s)
 {
     if (a.total_batches == 0) return;
@@ -871,16 +978,16 @@ void launch_batch(const sqk::BatchTraceArgs& a, int block, cudaStream_t s)
         return std::array<int, 6>{blocks_per_sm(k_trace_batch<MODE>, 64, pool_bytes<MODE>(64)),
                                   blocks_per_sm(k_trace_batch<MODE>, 128, pool_bytes<MODE>(128)),
                                   blocks_per_sm(k_trace_batch<MODE>, 256, pool_bytes<MODE>(256)),
-                                  blocks_per_sm(k_trace_batch_refill<RM>, 64),
-                                  blocks_per_sm(k_trace_batch_refill<RM>, 128),
-                                  blocks_per_sm(k_trace_batch_refill<RM>, 256)};
+                                  blocks_per_sm(k_trace_batch_refill<RM, WIDE>, 64),
+                                  blocks_per_sm(k_trace_batch_refill<RM, WIDE>, 128),
+                                  blocks_per_sm(k_trace_batch_refill<RM, WIDE>, 256)};
     });
     const bool refill = a.refill && MODE != SQ_TRACE_REF;
     const int bi = block <= 64 ? 0 : (block <= 128 ? 1 : 2);
     uint32_t grid = (uint32_t)(per_sm[(refill ? 3 : 0) + bi] * sm_count());
     const uint32_t need = (a.total_batches + (uint32_t)(block / 32) - 1) / (uint32_t)(block / 32);
     if (grid > need) grid = need;
-    if (refill) k_trace_batch_refill<RM><<<grid, block, 0, s>>>(a);
+    if (refill) k_trace_batch_refill<RM, WIDE><<<grid, block, 0, s>>>(a);
     else k_trace_batch<MODE><<<grid, block, pool_bytes<MODE>(block), s>>>(a);
 }
 
@@ -891,16 +998,20 @@ namespace sqk {
 void trace_batch(const BatchTraceArgs& a, int block, cudaStream_t s)
 {
     if (block != 64 && block != 128 && block != 256) block = 128;
-    if (a.mode == SQ_TRACE_REF) launch_batch<SQ_TRACE_REF>(a, block, s);
-    else if (a.mode == SQ_TRACE_CLOSEST) launch_batch<SQ_TRACE_CLOSEST>(a, block, s);
-    else launch_batch<SQ_TRACE_ANYHIT>(a, block, s);
+    const bool narrow = narrow_tree(a.node_count, a.tri_count);
+    if (a.mode == SQ_TRACE_REF) launch_batch<SQ_TRACE_REF, false>(a, block, s);
+    else if (a.mode == SQ_TRACE_CLOSEST)
+        narrow ? launch_batch<SQ_TRACE_CLOSEST, false>(a, block, s) : launch_batch<SQ_TRACE_CLOSEST, true>(a, block, s);
+    else narrow ? launch_batch<SQ_TRACE_ANYHIT, false>(a, block, s) : launch_batch<SQ_TRACE_ANYHIT, true>(a, block, s);
 }
 
 void trace(const TraceArgs& a, cudaStream_t s)
 {
-    if (a.mode == SQ_TRACE_REF) launch<SQ_TRACE_REF>(a, s);
-    else if (a.mode == SQ_TRACE_CLOSEST) launch<SQ_TRACE_CLOSEST>(a, s);
-    else launch<SQ_TRACE_ANYHIT>(a, s);
+    const bool narrow = narrow_tree(a.node_count, a.tri_count);
+    if (a.mode == SQ_TRACE_REF) launch<SQ_TRACE_REF, false>(a, s);
+    else if (a.mode == SQ_TRACE_CLOSEST)
+        narrow ? launch<SQ_TRACE_CLOSEST, false>(a, s) : launch<SQ_TRACE_CLOSEST, true>(a, s);
+    else narrow ? launch<SQ_TRACE_ANYHIT, false>(a, s) : launch<SQ_TRACE_ANYHIT, true>(a, s);
 }
 
 }  // namespace sqk
