@@ -28,8 +28,8 @@ struct Ray8 {
 };
 
 struct Pre8 {
-    float o[3], inv[3], tmin, tmax;
-    int kx, ky, kz;
+    float o[3], inv[3], tmin;
+    uint32_t axes;  // kx | ky << 2 | kz << 4: the triangle test's axes
     float sx, sy, sz;
 };
 
@@ -38,7 +38,6 @@ __device__ __forceinline__ void prep8(const Ray8& r, Pre8& p)
 #pragma unroll
     for (int k = 0; k < 3; ++k) { p.o[k] = r.o[k]; p.inv[k] = 1.0f / r.d[k]; }
     p.tmin = r.tmin;
-    p.tmax = r.tmax;
     const float ax = fabsf(r.d[0]), ay = fabsf(r.d[1]), az = fabsf(r.d[2]);
     int kz = 0;
     float m = ax;
@@ -48,7 +47,7 @@ __device__ __forceinline__ void prep8(const Ray8& r, Pre8& p)
     int ky = kx + 1; if (ky == 3) ky = 0;
     const float dkz = r.d[kz];
     if (dkz < 0.0f) { const int t = kx; kx = ky; ky = t; }
-    p.kx = kx; p.ky = ky; p.kz = kz;
+    p.axes = (uint32_t)(kx | (ky << 2) | (kz << 4));
     p.sx = r.d[kx] / dkz;
     p.sy = r.d[ky] / dkz;
     p.sz = 1.0f / dkz;
@@ -110,10 +109,11 @@ __device__ __forceinline__ bool tri8(const float4* __restrict__ t8, uint32_t k, 
     float A[3] = {a.x - r.o[0], a.y - r.o[1], a.z - r.o[2]};
     float B[3] = {b.x - r.o[0], b.y - r.o[1], b.z - r.o[2]};
     float C[3] = {c.x - r.o[0], c.y - r.o[1], c.z - r.o[2]};
-    const float Akz = sel3(A, r.kz), Bkz = sel3(B, r.kz), Ckz = sel3(C, r.kz);
-    const float Ax = sel3(A, r.kx) - r.sx * Akz, Ay = sel3(A, r.ky) - r.sy * Akz;
-    const float Bx = sel3(B, r.kx) - r.sx * Bkz, By = sel3(B, r.ky) - r.sy * Bkz;
-    const float Cx = sel3(C, r.kx) - r.sx * Ckz, Cy = sel3(C, r.ky) - r.sy * Ckz;
+    const int kx = (int)(r.axes & 3u), ky = (int)((r.axes >> 2) & 3u), kz = (int)(r.axes >> 4);
+    const float Akz = sel3(A, kz), Bkz = sel3(B, kz), Ckz = sel3(C, kz);
+    const float Ax = sel3(A, kx) - r.sx * Akz, Ay = sel3(A, ky) - r.sy * Akz;
+    const float Bx = sel3(B, kx) - r.sx * Bkz, By = sel3(B, ky) - r.sy * Bkz;
+    const float Cx = sel3(C, kx) - r.sx * Ckz, Cy = sel3(C, ky) - r.sy * Ckz;
     float U = Cx * By - Cy * Bx;
     float V = Ax * Cy - Ay * Cx;
     float W = Bx * Ay - By * Ax;
@@ -415,9 +415,9 @@ struct Res8 {
 // the current closest distance).
 template <bool ANY, bool SIGNED>
 __device__ Res8 trace8_impl(const Node8* __restrict__ nodes, uint32_t root, const float4* __restrict__ t8,
-                            const Pre8& rp)
+                            const Pre8& rp, float tmax)
 {
-    float best_t = rp.tmax;
+    float best_t = tmax;
     uint32_t best = kNoHit;
     uint32_t tests = 0, ttests = 0, nvis = 0;
     bool overflow = false;
@@ -458,11 +458,15 @@ __device__ Res8 trace8_impl(const Node8* __restrict__ nodes, uint32_t root, cons
         if (aff) scan(std::true_type{});
         else scan(std::false_type{});
         if (sp + nh > kStack8) { overflow = true; break; }
-        for (int a = nh - 1; a >= 0; --a) st[sp++] = make_uint2(hn[a], __float_as_uint(ht[a]));
+        // the nearest is taken without a trip over the stack
+        for (int a = nh - 1; a >= 1; --a) st[sp++] = make_uint2(hn[a], __float_as_uint(ht[a]));
+        uint32_t near_e = nh ? hn[0] : kNoHit;
         have = false;
         bool done = false;
-        while (sp > 0) {
-            const uint2 o = st[--sp];
+        while (near_e != kNoHit || sp > 0) {
+            uint2 o = make_uint2(near_e, 0xFF800000u);  // -infinity: never culled
+            if (near_e == kNoHit) o = st[--sp];
+            near_e = kNoHit;
             const uint32_t e = o.x;
             if (__uint_as_float(o.y) > best_t * kRobust) continue;
             if (e & 0x80000000u) {
@@ -500,8 +504,8 @@ __device__ Res8 trace8(const Node8* __restrict__ nodes, uint32_t root, const flo
 {
     Pre8 rp;
     prep8(ray, rp);
-    if (no_nan_slabs(rp)) return trace8_impl<ANY, true>(nodes, root, t8, rp);
-    return trace8_impl<ANY, false>(nodes, root, t8, rp);
+    if (no_nan_slabs(rp)) return trace8_impl<ANY, true>(nodes, root, t8, rp, ray.tmax);
+    return trace8_impl<ANY, false>(nodes, root, t8, rp, ray.tmax);
 }
 
 // ---------------------------------------------------------------------------
@@ -512,19 +516,25 @@ __device__ Res8 trace8(const Node8* __restrict__ nodes, uint32_t root, const flo
 //            warp takes the next batch when all its lanes are done.  This
 //            keeps neighbouring primary rays in one warp and their node
 //            fetches shared -- the choice for camera rays;
-//   refill   one ray per lane as a state machine that visits one wide node
-//            per loop iteration (visit8); a lane whose ray has finished takes
+//   refill   one ray per lane as a state machine that visits one wide node or
+//            leaf per loop iteration (step8); a lane whose ray has finished takes
 //            the next unprocessed ray at once (one atomic per warp for all
 //            lanes that need one), so a warp never idles behind its slowest
 //            ray -- the choice for explicit (typically incoherent) rays.
 // Both visit children in the same order (ascending entry distance, then
 // slot), so they count the same box tests for the same ray.
 
+// Totals of a lane over all its rays (32 bits are hours of them); the rays
+// themselves only carry their box tests.
+struct Totals8 {
+    uint32_t tests = 0, tris = 0, nodes = 0, rays = 0, explicit_rays = 0;
+};
+
 struct Lane8 {
     Pre8 rp;
     float best_t;
-    uint32_t best, tests, ttests, nvis;
-    uint32_t cur;  // next wide node to visit, or kNoHit when the ray is finished
+    uint32_t best, tests;
+    uint32_t cur;  // next entry (wide node or leaf range), or kNoHit when the ray is finished
     int sp;
     bool overflow;
 };
@@ -532,23 +542,39 @@ struct Lane8 {
 __device__ __forceinline__ void lane_start(Lane8& L, const Ray8& ray, uint32_t root)
 {
     prep8(ray, L.rp);
-    L.best_t = L.rp.tmax;
+    L.best_t = ray.tmax;
     L.best = kNoHit;
-    L.tests = L.ttests = L.nvis = 0;
+    L.tests = 0;
     L.cur = root;
     L.sp = 0;
     L.overflow = false;
 }
 
+// Add a warp's totals to the trace statistics: requested bytes are 32 per
+// explicit ray, `out` per ray, 80 per node and 48 per triangle.
+__device__ __forceinline__ void add_totals(const Totals8& sum, uint32_t out, unsigned long long* stats)
+{
+    unsigned long long v[4] = {sum.tests, sum.tris,
+                               32ull * sum.explicit_rays + (unsigned long long)out * sum.rays + 80ull * sum.nodes +
+                                   48ull * sum.tris,
+                               sum.nodes};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xFFFFFFFFu, v[k], o);
+        if ((threadIdx.x & 31u) == 0) atomicAdd(stats + k, v[k]);
+    }
+}
+
 // Test a leaf entry's triangles; returns true when an any-hit ray is done.
 template <bool ANY>
-__device__ __forceinline__ bool leaf8(Lane8& L, const float4* __restrict__ t8, uint32_t e)
+__device__ __forceinline__ bool leaf8(Lane8& L, const float4* __restrict__ t8, uint32_t e, Totals8& sum)
 {
     const uint32_t cnt = (e >> 27) & 0xFu, first = e & 0x07FFFFFFu;
     for (uint32_t j = 0; j < cnt; ++j) {
         float t;
         uint32_t id;
-        L.ttests++;
+        sum.tris++;
         if (tri8(t8, first + j, L.rp, L.best_t, t, id)) {
             if (t < L.best_t || (t == L.best_t && id < L.best)) { L.best_t = t; L.best = id; }
             if (ANY) return true;
@@ -557,36 +583,52 @@ __device__ __forceinline__ bool leaf8(Lane8& L, const float4* __restrict__ t8, u
     return false;
 }
 
-// Visit node L.cur; afterwards L.cur is the next node, or kNoHit when the
-// ray has finished (stack empty, any-hit found, or stack overflow: of a
-// node's hits all but the nearest are pushed).
-template <bool ANY, bool SIGNED>
-__device__ __forceinline__ void visit8(Lane8& L, const Node8* __restrict__ nodes, const float4* __restrict__ t8,
-                                       uint2* st, float* __restrict__ s_n)
+// The next entry of the lane's stack that is not beyond the closest hit, or
+// kNoHit when the stack is empty.
+__device__ __forceinline__ uint32_t pop8(Lane8& L, const uint2* st)
 {
-    // the next node: the nearest child, else the stack (leaves tested on the way)
-    uint32_t e = visit_children<SIGNED>(nodes, L.cur, L.rp, L.best_t * kRobust, s_n, st, L.sp, L.tests);
-    L.nvis++;
-    if (L.sp > kStack8) {
-        L.overflow = true;
+    while (L.sp) {
+        const uint2 o = st[--L.sp];
+        if (!(__uint_as_float(o.y) > L.best_t * kRobust)) return o.x;
+    }
+    return kNoHit;
+}
+
+// One step of a lane that holds a ray: a visit of its inner node, or the test
+// of its leaf's triangles, then the next entry (kNoHit: the ray has finished
+// -- stack empty, any-hit found, or stack overflow: of a node's hits all but
+// the nearest are pushed).  Testing a leaf is a step of its own, so the lanes
+// of a warp that reach leaves in the same step test together; in a loop
+// inside the visit they came one after another (one bounce off the 4.2M
+// terrain 608 -> 571 us, 2^24 incoherent rays 22.8 -> 22.1 ms).  Holding
+// lanes back until 2 to 20 wait at leaves was slower on small ray counts and
+// no faster than 2% on large ones.
+template <bool ANY>
+__device__ __forceinline__ void step8(Lane8& L, bool has, const Node8* __restrict__ nodes,
+                                      const float4* __restrict__ t8, uint2* st, float* __restrict__ s_n, Totals8& sum)
+{
+    const bool leaf = has && (L.cur & 0x80000000u);
+    bool pop = false;
+    if (has && !leaf) {
+        // slab form chosen per ray, as trace8 does (sign-selected planes for a
+        // ray that cannot produce NaN), so a ray's box tests do not depend on
+        // the rays it shares a warp with
+        const float lim = L.best_t * kRobust;
+        L.cur = no_nan_slabs(L.rp) ? visit_children<true>(nodes, L.cur, L.rp, lim, s_n, st, L.sp, L.tests)
+                                   : visit_children<false>(nodes, L.cur, L.rp, lim, s_n, st, L.sp, L.tests);
+        sum.nodes++;
+        if (L.sp > kStack8) {
+            L.overflow = true;
+            L.cur = kNoHit;
+            L.sp = 0;
+        }
+        pop = L.cur == kNoHit;
+    }
+    if (leaf) {
+        pop = !leaf8<ANY>(L, t8, L.cur, sum);
         L.cur = kNoHit;
-        return;
     }
-    for (;;) {
-        if (e == kNoHit) {
-            if (L.sp == 0) { L.cur = kNoHit; return; }
-            const uint2 o = st[--L.sp];
-            if (__uint_as_float(o.y) > L.best_t * kRobust) continue;
-            e = o.x;
-        }
-        if (e & 0x80000000u) {
-            if (leaf8<ANY>(L, t8, e)) { L.cur = kNoHit; return; }
-            e = kNoHit;
-            continue;
-        }
-        L.cur = e;
-        return;
-    }
+    if (pop) L.cur = pop8(L, st);
 }
 
 // Camera rays, tiles: a warp takes one 8x4 pixel tile, each lane runs its
@@ -700,11 +742,10 @@ __global__ void __launch_bounds__(kTilesBlock, 32) k_trace8_tiles(const sqk::Tra
     if (a.stats) ws.flush(lane, a.stats);
 }
 
-// Seven blocks per SM (72 registers): one bounce off the 4.2M-triangle
-// terrain took 0.62 ms against 0.65-0.67 ms with six (80 registers) and 0.63
-// ms with eight (64).
+// Eight blocks per SM (64 registers): one bounce off the 4.2M-triangle
+// terrain took 552 us against 571 us with seven.
 template <int MODE>
-__global__ void __launch_bounds__(128, 7) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
+__global__ void __launch_bounds__(128, 8) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
 {
     constexpr bool ANY = MODE == SQ_TRACE_ANYHIT;
     const uint32_t lane = threadIdx.x & 31u;
@@ -717,7 +758,7 @@ __global__ void __launch_bounds__(128, 7) k_trace8_refill(const sqk::Trace8Args 
     L.cur = kNoHit;
     bool has = false, exhausted = false;
     uint32_t rid = 0;
-    unsigned long long s_bt = 0, s_tt = 0, s_by = 0, s_nv = 0;
+    Totals8 sum;
     for (;;) {
         // refill: every lane without a ray takes the next one
         const uint32_t need = __ballot_sync(0xFFFFFFFFu, !has && !exhausted);
@@ -761,22 +802,13 @@ __global__ void __launch_bounds__(128, 7) k_trace8_refill(const sqk::Trace8Args 
             if (__all_sync(0xFFFFFFFFu, exhausted)) break;
             continue;
         }
+        step8<ANY>(L, has, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane, sum);
         if (has) {
-            // slab form chosen per ray, as trace8 does (sign-selected planes
-            // for a ray that cannot produce NaN), so a ray's box tests do not
-            // depend on the rays it shares a warp with
-            if (no_nan_slabs(L.rp)) visit8<ANY, true>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
-            else visit8<ANY, false>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
             if (L.cur == kNoHit) {
                 has = false;
                 if (L.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
-                if (a.stats) {
-                    s_bt += L.tests;
-                    s_tt += L.ttests;
-                    s_nv += L.nvis;
-                    s_by += (camera ? 0u : 32u) + (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u) + 80ull * L.nvis +
-                            48ull * L.ttests;
-                }
+                sum.tests += L.tests;
+                sum.rays++;
                 if (a.hits) {
                     uint32_t* h = reinterpret_cast<uint32_t*>(a.hits) + 3ull * rid;
                     h[0] = L.best;
@@ -789,18 +821,8 @@ __global__ void __launch_bounds__(128, 7) k_trace8_refill(const sqk::Trace8Args 
             }
         }
     }
-    if (a.stats) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s_bt += __shfl_xor_sync(0xFFFFFFFFu, s_bt, o);
-            s_tt += __shfl_xor_sync(0xFFFFFFFFu, s_tt, o);
-            s_by += __shfl_xor_sync(0xFFFFFFFFu, s_by, o);
-            s_nv += __shfl_xor_sync(0xFFFFFFFFu, s_nv, o);
-        }
-        if (lane == 0) {
-            atomicAdd(a.stats, s_bt); atomicAdd(a.stats + 1, s_tt); atomicAdd(a.stats + 2, s_by); atomicAdd(a.stats + 3, s_nv);
-        }
-    }
+    sum.explicit_rays = camera ? 0u : sum.rays;
+    if (a.stats) add_totals(sum, (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u), a.stats);
 }
 
 template <int MODE>
@@ -895,8 +917,9 @@ __global__ void __launch_bounds__(256) k_trace8_batch_tiles(const sqk::BatchTrac
     if (a.stats) ws.flush(lane, a.stats);
 }
 
-// Launch bounds of 28 warps per SM whatever the block shape: the same
-// register budget (72) as k_trace8_refill, whose occupancy it needs.
+// Launch bounds of 28 warps per SM whatever the block shape (72 registers):
+// the job search needs more than k_trace8_refill's 64 (2^24 incoherent rays
+// 22.1 ms against 23.6 ms at 32 warps).
 template <int MODE, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(const sqk::BatchTraceArgs a)
 {
@@ -914,7 +937,7 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(cons
     // takes consecutive slots, so the job search runs only when a slot
     // leaves the range
     uint32_t cj = 0, jlo = 1, jhi = 0;
-    unsigned long long s_bt = 0, s_tt = 0, s_by = 0, s_nv = 0;
+    Totals8 sum;
     for (;;) {
         const uint32_t need = __ballot_sync(0xFFFFFFFFu, !has && !exhausted);
         if (need) {
@@ -971,19 +994,14 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(cons
             if (__all_sync(0xFFFFFFFFu, exhausted)) break;
             continue;
         }
+        step8<ANY>(L, has, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane, sum);
         if (has) {
-            if (no_nan_slabs(L.rp)) visit8<ANY, true>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
-            else visit8<ANY, false>(L, nodes, a.tris8, st, s_n[threadIdx.x >> 5] + lane);
             if (L.cur == kNoHit) {
                 has = false;
                 if (L.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
-                if (a.stats) {
-                    s_bt += L.tests;
-                    s_tt += L.ttests;
-                    s_nv += L.nvis;
-                    s_by += (explicit_rays ? 32u : 0u) + (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u) + 80ull * L.nvis +
-                            48ull * L.ttests;
-                }
+                sum.tests += L.tests;
+                sum.rays++;
+                sum.explicit_rays += explicit_rays ? 1u : 0u;
                 const uint32_t id = L.best == kNoHit ? kNoHit : L.best - tri_offset;
                 if (a.hits) {
                     uint32_t* h = reinterpret_cast<uint32_t*>(a.hits) + 3ull * out;
@@ -997,18 +1015,7 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(cons
             }
         }
     }
-    if (a.stats) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s_bt += __shfl_xor_sync(0xFFFFFFFFu, s_bt, o);
-            s_tt += __shfl_xor_sync(0xFFFFFFFFu, s_tt, o);
-            s_by += __shfl_xor_sync(0xFFFFFFFFu, s_by, o);
-            s_nv += __shfl_xor_sync(0xFFFFFFFFu, s_nv, o);
-        }
-        if (lane == 0) {
-            atomicAdd(a.stats, s_bt); atomicAdd(a.stats + 1, s_tt); atomicAdd(a.stats + 2, s_by); atomicAdd(a.stats + 3, s_nv);
-        }
-    }
+    if (a.stats) add_totals(sum, (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u), a.stats);
 }
 
 template <int MODE>
