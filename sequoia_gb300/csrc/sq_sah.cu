@@ -19,7 +19,7 @@
 // result is record-for-record the oracle's.
 //
 // Schedule:
-//   large nodes (> kSmall triangles): level by level, two kernels a level.
+//   large nodes (> kMid triangles): level by level, two kernels a level.
 //     k_large_split  one warp per node picks the plane from the node's bins,
 //                    places the children and scans the left counts of the
 //                    node's chunks;
@@ -29,6 +29,8 @@
 //                    next level's split finds its bins ready.
 //     A triangle's box is read once a level: the bin it falls in is kept as a
 //     byte beside its id, and the next partition needs only that byte.
+//   middle nodes (> kSmall, at most kMid triangles): one block per subtree, in
+//     shared memory, down to the small nodes.
 //   small nodes: one warp per subtree, smaller child first (stack depth
 //     O(log n)), binning and partitioning with warp intrinsics only.
 #include "sq_common.cuh"
@@ -48,12 +50,13 @@ constexpr uint32_t kChunk = 2048;
 constexpr uint32_t kChunkSmall = 256;
 constexpr uint32_t kChunkSmallBelow = 1u << 20;
 constexpr uint32_t kSmall = 128;
+constexpr uint32_t kMid = 1024;
 constexpr int kMaxBins = 32;
 constexpr int kBinWords = 13;  // -pmin xyz, pmax xyz, -cmin xyz, cmax xyz (ordered ints), count
 constexpr int kStackDepth = 24;
 // Large-phase levels of the batched build (device-side counts, no host
-// round trip): deeper work is finished by the small phase.
-constexpr uint32_t kBatchLargeLevels = 24;
+// round trip): larger tasks left then are finished by k_small_big.
+constexpr uint32_t kBatchLargeLevels = 20;
 // Large-phase levels a single build queues between two host reads of the
 // task count, after a first group sized to the mesh (build_sah).
 constexpr uint32_t kSahLevelsPerCheck = 4;
@@ -93,10 +96,10 @@ static_assert(sizeof(Part) == 64, "Part is 64 bytes");
 // on the device, so a level needs no host round trip.
 struct Ctl {
     unsigned long long level[3];
-    uint32_t n_small, n_leaf;
-    uint32_t small_pop, pad;  // tasks taken by k_small's warps
+    uint32_t n_mid, n_small, n_leaf;
+    uint32_t mid_pop, small_pop, pad;  // tasks taken by k_mid's blocks and k_small's warps
 };
-static_assert(sizeof(Ctl) == 40, "Ctl is 40 bytes");
+static_assert(sizeof(Ctl) == 48, "Ctl is 48 bytes");
 
 __device__ __forceinline__ float box_sa(const float* mn, const float* mx)
 {
@@ -199,32 +202,47 @@ struct LevelLists {
 // 2048 triangles)
 __host__ __device__ __forceinline__ uint32_t count_words(int nb) { return ((uint32_t)nb + 1u) >> 1; }
 
+// Where the other tasks go.
+struct DoneLists {
+    Task *mid, *small;
+    LeafRange* leaves;
+    Ctl* ctl;
+};
+
+__device__ __forceinline__ bool is_leaf_task(const Task& t, uint32_t leaf_size)
+{
+    return t.count <= leaf_size || !(box_sa(t.cmn, t.cmx) > 0.0f);
+}
+
+__device__ __forceinline__ void list_leaf(const Task& t, const DoneLists& done)
+{
+    LeafRange lr;
+    lr.begin = t.begin; lr.count = t.count; lr.slot = t.slot; lr.flags = t.flags;
+    for (int a = 0; a < 3; ++a) { lr.pmn[a] = t.pmn[a]; lr.pmx[a] = t.pmx[a]; }
+    lr.pad[0] = lr.pad[1] = 0;
+    done.leaves[atomicAdd(&done.ctl->n_leaf, 1u)] = lr;
+}
+
 // Place a task (all lanes of a warp call it with the same task): leaf
 // (recorded in the leaf list), large (listed for the level counted by *cnt),
-// or small.  side: which child of `part` it is, for the large case.  zero:
+// middle or small.  side: which child of `part` it is, for the large case.  zero:
 // the bins are collected with atomics and must start from zero (else one
 // block stores them whole).
 template <uint32_t CHUNK>
 __device__ void place_task(const Task& t, uint32_t leaf_size, int nb, const LevelLists& next, unsigned long long* cnt,
-                           bool zero, Task* __restrict__ small, LeafRange* __restrict__ leaves, Ctl* ctl, Part& part,
-                           int side)
+                           bool zero, const DoneLists& done, Part& part, int side)
 {
     const uint32_t lane = threadIdx.x & 31u;
     part.task[side] = kNone;
-    const bool leaf = t.count <= leaf_size || !(box_sa(t.cmn, t.cmx) > 0.0f);
-    if (leaf) {
-        if (lane == 0) {
-            const uint32_t k = atomicAdd(&ctl->n_leaf, 1u);
-            LeafRange lr;
-            lr.begin = t.begin; lr.count = t.count; lr.slot = t.slot; lr.flags = t.flags;
-            for (int a = 0; a < 3; ++a) { lr.pmn[a] = t.pmn[a]; lr.pmx[a] = t.pmx[a]; }
-            lr.pad[0] = lr.pad[1] = 0;
-            leaves[k] = lr;
-        }
+    if (is_leaf_task(t, leaf_size)) {
+        if (lane == 0) list_leaf(t, done);
         return;
     }
-    if (t.count <= kSmall) {
-        if (lane == 0) small[atomicAdd(&ctl->n_small, 1u)] = t;
+    if (t.count <= kMid) {
+        if (lane == 0) {
+            if (t.count <= kSmall) done.small[atomicAdd(&done.ctl->n_small, 1u)] = t;
+            else done.mid[atomicAdd(&done.ctl->n_mid, 1u)] = t;
+        }
         return;
     }
     const uint32_t chunks = (t.count + CHUNK - 1) / CHUNK;
@@ -257,10 +275,10 @@ __device__ void place_task(const Task& t, uint32_t leaf_size, int nb, const Leve
 // bin it in place (everything on side 0).
 template <uint32_t CHUNK>
 __device__ void place_root(const Task& t, uint32_t leaf_size, int nb, const LevelLists& l0, Part* __restrict__ parts,
-                           Task* __restrict__ small, LeafRange* __restrict__ leaves, Ctl* ctl)
+                           const DoneLists& done)
 {
     Part p;
-    place_task<CHUNK>(t, leaf_size, nb, l0, &ctl->level[0], true, small, leaves, ctl, p, 0);
+    place_task<CHUNK>(t, leaf_size, nb, l0, &done.ctl->level[0], true, done, p, 0);
     if (p.task[0] == kNone) return;
     p.begin = t.begin;
     p.count = p.nl = t.count;
@@ -276,7 +294,7 @@ __device__ void place_root(const Task& t, uint32_t leaf_size, int nb, const Leve
 
 template <uint32_t CHUNK>
 __global__ void k_root_task(const uint32_t* __restrict__ root_ord, uint32_t n, uint32_t leaf_size, int nb,
-                            LevelLists l0, Part* parts, Task* small, LeafRange* leaves, Ctl* ctl, float* scene_out)
+                            LevelLists l0, Part* parts, DoneLists done, float* scene_out)
 {
     Task t;  // one warp
     t.begin = 0; t.count = n; t.slot = 0; t.flags = 2u;
@@ -290,7 +308,7 @@ __global__ void k_root_task(const uint32_t* __restrict__ root_ord, uint32_t n, u
             scene_out[3 + k] = t.pmx[k];
         }
     }
-    place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
+    place_root<CHUNK>(t, leaf_size, nb, l0, parts, done);
 }
 
 // ---------------------------------------------------------------------------
@@ -351,7 +369,7 @@ __global__ void __launch_bounds__(256) k_grid_bin(const float4* __restrict__ tb,
 template <uint32_t CHUNK>
 __global__ void k_grid_tasks(const uint32_t* __restrict__ cell_ord, const uint32_t* __restrict__ root_ord, uint32_t n,
                              uint32_t leaf_size, uint32_t scene_box_cells, int nb, LevelLists l0, Part* parts,
-                             Task* small, LeafRange* leaves, Ctl* ctl, float* scene_out)
+                             DoneLists done, float* scene_out)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -378,7 +396,7 @@ __global__ void k_grid_tasks(const uint32_t* __restrict__ cell_ord, const uint32
         // the plain grid builder gives every cell node the scene box (src/builder.cpp:2173-2174)
         for (int k = 0; k < 3; ++k) { t.pmn[k] = dec_neg(root_ord[k]); t.pmx[k] = dec_pos(root_ord[3 + k]); }
     }
-    place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
+    place_root<CHUNK>(t, leaf_size, nb, l0, parts, done);
 }
 
 // heap of 63 inner nodes above the 64 cell nodes (src/builder.cpp:2181-2188),
@@ -621,7 +639,7 @@ __global__ void __launch_bounds__(128) k_large_split(LevelLists cur, LevelLists 
                                                      uint32_t cur_i, uint32_t next_i, int nb, uint32_t base,
                                                      uint32_t leaf_size, Node* __restrict__ nodes,
                                                      Part* __restrict__ parts, uint32_t* __restrict__ chunk_left,
-                                                     Task* small, LeafRange* leaves, Ctl* ctl)
+                                                     DoneLists done)
 {
     chain_wait();  // a chained launch (enqueue_levels)
     chain_release();
@@ -649,12 +667,7 @@ __global__ void __launch_bounds__(128) k_large_split(LevelLists cur, LevelLists 
             // no plane scored below FLT_MAX: the node becomes a leaf
             p.plane = -1;
             if (lane == 0) {
-                const uint32_t k = atomicAdd(&ctl->n_leaf, 1u);
-                LeafRange lr;
-                lr.begin = tk.begin; lr.count = tk.count; lr.slot = tk.slot; lr.flags = tk.flags;
-                for (int a = 0; a < 3; ++a) { lr.pmn[a] = tk.pmn[a]; lr.pmx[a] = tk.pmx[a]; }
-                lr.pad[0] = lr.pad[1] = 0;
-                leaves[k] = lr;
+                list_leaf(tk, done);
                 parts[t] = p;
             }
             continue;
@@ -668,9 +681,9 @@ __global__ void __launch_bounds__(128) k_large_split(LevelLists cur, LevelLists 
         const uint32_t buf = (tk.flags & 1u) ^ 1u;
         const bool zero = chunks > 1;
         place_task<CHUNK>(child_task(tk.begin, r.nl, base + 2u * q, buf, r.lp, r.lc), leaf_size, nb, next,
-                          &ctl->level[next_i], zero, small, leaves, ctl, p, 0);
+                          &done.ctl->level[next_i], zero, done, p, 0);
         place_task<CHUNK>(child_task(q, tk.count - r.nl, base + 2u * q + 1u, buf, r.rp, r.rc), leaf_size, nb, next,
-                          &ctl->level[next_i], zero, small, leaves, ctl, p, 1);
+                          &done.ctl->level[next_i], zero, done, p, 1);
         if (lane == 0) parts[t] = p;
         // exclusive scan of the chunks' left counts, 128 chunks a round
         uint32_t carry = 0;
@@ -891,6 +904,208 @@ __global__ void k_emit_leaves(const LeafRange* __restrict__ leaves, const Ctl* _
 }
 
 // ---------------------------------------------------------------------------
+// middle phase: one block per subtree of kSmall + 1 to kMid triangles
+//
+// The subtree is staged in shared memory and split level by level, a warp per
+// node for the planes (at most seven nodes of more than kSmall triangles exist
+// at a time), the block's threads over the triangles for binning and the
+// stable partition, until every node is small or a leaf; then the ids go back
+// to their buffer in the final order.  A level here is four block barriers;
+// as a level of the large phase it was two launches of 3 to 15 us, and the
+// lower third of the large levels were these.
+constexpr int kMidNodes = 8;
+static_assert(kMid / (kSmall + 1) < kMidNodes, "a warp per middle node");
+
+struct MidNode {
+    Task t;  // begin relative to the subtree
+    float k1, cmin;
+    int axis, plane;  // plane -1: stays (a leaf)
+    uint32_t nl, lstart, pad[2];
+};
+
+struct MidStage {
+    float4 box[kMid][2];  // min xyz, id; max xyz
+    uint32_t bins[kMidNodes][kMaxBins * kBinWords];
+    MidNode node[2][kMidNodes];
+    uint32_t n_node[2];
+    uint32_t lbits[kMid / 32], lpre[kMid / 32];  // left flags by position, and left triangles before each word
+    uint16_t loc[2][kMid];                       // the triangle at each position
+    uint8_t bin[kMid];
+    uint32_t task;
+};
+
+template <int NBP>
+__global__ void __launch_bounds__(256) k_mid(uint32_t* __restrict__ ids_a, uint32_t* __restrict__ ids_b,
+                                             const float4* __restrict__ tb, int nb, uint32_t leaf_size, uint32_t base,
+                                             Node* __restrict__ nodes, DoneLists done)
+{
+    extern __shared__ __align__(16) unsigned char s_mid[];
+    MidStage& sg = *reinterpret_cast<MidStage*>(s_mid);
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t copy = (lane * NBP) & (kMaxBins - 1);  // first bin of the lane's copy
+    const uint32_t total = done.ctl->n_mid;
+    auto add_node = [&](int p, const Task& t) {
+        MidNode& m = sg.node[p][atomicAdd(&sg.n_node[p], 1u)];
+        m.t = t;
+        m.axis = choose_axis(t.cmn, t.cmx);
+        m.cmin = sel(t.cmn, m.axis);
+        m.k1 = bin_k1(nb, sel(t.cmx, m.axis) - m.cmin);
+    };
+    for (;;) {
+        if (tid == 0) {
+            sg.task = atomicAdd(&done.ctl->mid_pop, 1u);
+            sg.n_node[0] = sg.n_node[1] = 0;
+        }
+        __syncthreads();
+        if (sg.task >= total) return;
+        const Task root = done.mid[sg.task];
+        const uint32_t rb = root.begin, count = root.count, parity = root.flags & 1u;
+        uint32_t* ids = (parity ? ids_b : ids_a) + rb;
+        for (uint32_t j = tid; j < count; j += 256) {
+            const uint32_t id = ids[j];
+            float4 lo = __ldg(tb + 2ull * id);
+            lo.w = __uint_as_float(id);
+            sg.box[j][0] = lo;
+            sg.box[j][1] = __ldg(tb + 2ull * id + 1);
+            sg.loc[0][j] = (uint16_t)j;
+        }
+        if (tid == 0) {
+            Task t = root;
+            t.begin = 0;
+            add_node(0, t);
+        }
+        int cur = 0;
+        for (;; cur ^= 1) {
+            __syncthreads();
+            const uint32_t active = sg.n_node[cur];
+            if (active == 0) break;
+            MidNode* node = sg.node[cur];
+            for (uint32_t j = tid; j < active * (kMaxBins * kBinWords); j += 256) (&sg.bins[0][0])[j] = 0;
+            __syncthreads();
+            // the node of a position (kMidNodes: none, its triangles are done)
+            auto node_at = [&](uint32_t pos) {
+                uint32_t a = kMidNodes;
+                for (uint32_t q = 0; q < active; ++q)
+                    if (pos - node[q].t.begin < node[q].t.count) a = q;
+                return a;
+            };
+            for (uint32_t pos = tid; pos < count; pos += 256) {
+                const uint32_t a = node_at(pos);
+                if (a == kMidNodes) continue;
+                const uint32_t li = sg.loc[cur][pos];
+                const float4 lo = sg.box[li][0], hi = sg.box[li][1];
+                const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
+                float cc[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) cc[k] = (mn[k] + mx[k]) * 0.5f;
+                const uint32_t b = (uint32_t)bin_of(node[a].k1, sel(cc, node[a].axis), node[a].cmin, nb);
+                sg.bin[pos] = (uint8_t)b;
+                uint32_t* w = sg.bins[a] + (copy + b) * kBinWords;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    atomicMax(w + k, float_to_ordered(-mn[k]));
+                    atomicMax(w + 3 + k, float_to_ordered(mx[k]));
+                    atomicMax(w + 6 + k, float_to_ordered(-cc[k]));
+                    atomicMax(w + 9 + k, float_to_ordered(cc[k]));
+                }
+                atomicAdd(w + 12, 1u);
+            }
+            __syncthreads();
+            if (warp < active) {
+                MidNode& m = node[warp];
+                uint32_t w[kBinWords];
+#pragma unroll
+                for (int k = 0; k < kBinWords; ++k) w[k] = 0;
+                if (lane < (uint32_t)NBP) {
+#pragma unroll
+                    for (int q = 0; q < kMaxBins; q += NBP) {
+                        const uint32_t* bw = sg.bins[warp] + (lane + q) * kBinWords;
+#pragma unroll
+                        for (int k = 0; k < 12; ++k) w[k] = max(w[k], bw[k]);
+                        w[12] += bw[12];
+                    }
+                }
+                float p[6], c[6];
+                const uint32_t cnt = load_bin(w, (int)lane < nb, p, c);
+                PlaneResult r;
+                choose_planes<32>(nb, cnt, p, c, r.plane, r.nl, r.lp, r.rp, r.lc, r.rc);
+                if (lane == 0) {
+                    const Task t = m.t;
+                    const bool split = r.plane >= 0 && r.nl != 0 && r.nl != t.count;
+                    m.plane = split ? r.plane : -1;
+                    m.nl = r.nl;
+                    if (!split) {
+                        // no plane scored below FLT_MAX: the node becomes a leaf
+                        Task g = t;
+                        g.begin += rb;
+                        list_leaf(g, done);
+                    } else {
+                        const uint32_t q = rb + t.begin + r.nl;
+                        Box pb;
+                        for (int k = 0; k < 3; ++k) { pb.mn[k] = t.pmn[k]; pb.mx[k] = t.pmx[k]; }
+                        store_node(nodes + t.slot, pb, base + 2u * q, 2u, 0);
+#pragma unroll
+                        for (int side = 0; side < 2; ++side) {
+                            Task ch = side ? child_task(t.begin + r.nl, t.count - r.nl, base + 2u * q + 1u, parity, r.rp, r.rc)
+                                           : child_task(t.begin, r.nl, base + 2u * q, parity, r.lp, r.lc);
+                            const bool leaf = is_leaf_task(ch, leaf_size);
+                            if (!leaf && ch.count > kSmall) {
+                                add_node(cur ^ 1, ch);
+                                continue;
+                            }
+                            ch.begin += rb;
+                            if (leaf) list_leaf(ch, done);
+                            else done.small[atomicAdd(&done.ctl->n_small, 1u)] = ch;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            // partition, stably: left flags by position, their prefix, the moves
+            for (uint32_t w0 = warp * 32u; w0 < count; w0 += 256) {
+                const uint32_t pos = w0 + lane;
+                const uint32_t a = pos < count ? node_at(pos) : (uint32_t)kMidNodes;
+                const uint32_t b = __ballot_sync(FULL, a != kMidNodes && (int)sg.bin[pos] <= node[a].plane);
+                if (lane == 0) sg.lbits[w0 >> 5] = b;
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const uint32_t words = (count + 31u) >> 5;
+                const uint32_t v = lane < words ? (uint32_t)__popc(sg.lbits[lane]) : 0u;
+                uint32_t x = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, x, o);
+                    if (lane >= (uint32_t)o) x += y;
+                }
+                if (lane < words) sg.lpre[lane] = x - v;
+                __syncwarp();
+                if (lane < active) {
+                    const uint32_t s0 = node[lane].t.begin;
+                    node[lane].lstart = sg.lpre[s0 >> 5] + __popc(sg.lbits[s0 >> 5] & ((1u << (s0 & 31u)) - 1u));
+                }
+                if (lane == 0) sg.n_node[cur] = 0;
+            }
+            __syncthreads();
+            for (uint32_t pos = tid; pos < count; pos += 256) {
+                const uint32_t a = node_at(pos), li = sg.loc[cur][pos];
+                uint32_t to = pos;
+                if (a != kMidNodes && node[a].plane >= 0) {
+                    const uint32_t word = sg.lbits[pos >> 5], bit = 1u << (pos & 31u);
+                    const uint32_t lr = sg.lpre[pos >> 5] + __popc(word & (bit - 1u)) - node[a].lstart;
+                    const uint32_t b0 = node[a].t.begin;
+                    to = b0 + ((word & bit) ? lr : node[a].nl + (pos - b0) - lr);
+                }
+                sg.loc[cur ^ 1][to] = (uint16_t)li;
+            }
+        }
+        for (uint32_t j = tid; j < count; j += 256) ids[j] = __float_as_uint(sg.box[sg.loc[cur][j]][0].w);
+        __syncthreads();  // the stage is used again for the block's next task
+    }
+}
+
+// ---------------------------------------------------------------------------
 // small phase: one warp per subtree
 //
 // A subtree of at most kStage triangles (every small task of a single build:
@@ -910,7 +1125,7 @@ __global__ void k_emit_leaves(const LeafRange* __restrict__ leaves, const Ctl* _
 // The large tasks left after a batch's fixed levels are split by k_small_big,
 // one node at a time, in the global buffers.
 constexpr uint32_t kStage = 128;
-static_assert(kSmall <= kStage, "every small task is staged");
+static_assert(kSmall <= kStage && kMid / 32 <= 32, "every small task is staged; one warp scans a middle task's words");
 
 struct SmallNode {
     float p[6], c[6];  // primitive and centroid boxes (min xyz, max xyz)
@@ -1123,6 +1338,8 @@ __global__ void __launch_bounds__(128) k_small(const Task* __restrict__ small, C
                                                Node* __restrict__ nodes, uint32_t leaf0)
 {
     __shared__ __align__(16) SmallStage s_stage[4];
+    chain_wait();  // a chained launch (launch_subtrees)
+    chain_release();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t total = ctl->n_small;
     for (;;) {
@@ -1266,15 +1483,16 @@ struct SahWs {
     uint32_t *ids_a, *ids_b;
     uint8_t *bin_a, *bin_b;
     LevelLists lists[2];
-    Task* small;
+    Task *mid, *small;
     LeafRange* leaves;
     Part* parts;
     uint32_t *chunk_left, *cells, *hist, *root_ord;
     Ctl* ctl;
+    DoneLists done() const { return DoneLists{mid, small, leaves, ctl}; }
 };
 
 // Most large tasks a level can have, and most chunks.
-size_t sah_tasks(uint32_t n) { return n / kSmall + 2; }
+size_t sah_tasks(uint32_t n) { return n / kMid + 2; }
 size_t sah_chunks(uint32_t n) { return (size_t)n / (n < kChunkSmallBelow ? kChunkSmall : kChunk) + sah_tasks(n) + 1; }
 
 // Lays the workspace out at p (null: only the size is wanted) and returns its size.
@@ -1299,6 +1517,7 @@ size_t sah_layout(char* p, uint32_t n, uint32_t meshes, SahWs& w)
         take(l.bins, (size_t)kMaxBins * kBinWords * tasks);
         take(l.counts, (size_t)(kMaxBins / 2) * chunks);
     }
+    take(w.mid, (size_t)n / kSmall + 2);
     take(w.small, (size_t)n / 2 + 2);
     take(w.leaves, (size_t)n + 66 + meshes);  // + 64 empty grid cells, + empty meshes
     take(w.parts, tasks);
@@ -1360,16 +1579,32 @@ void enqueue_levels(const SahWs& w, uint32_t level, uint32_t count, int nb, uint
     for (uint32_t l = level; l < level + count; ++l) {
         launch_chained(k_large_split<CHUNK>, dim3(grid), dim3(128), 0, s, w.lists[l & 1], w.lists[(l + 1) & 1],
                        (const Ctl*)w.ctl, l % 3u, (l + 1) % 3u, nb, base, leaf_size, nodes, w.parts, w.chunk_left,
-                       w.small, w.leaves, w.ctl);
+                       w.done());
         enqueue_move<CHUNK, false>(w, l & 1, (l + 1) & 1, l % 3u, nb, s);
     }
 }
 
-void launch_small(const SahWs& w, int nb, uint32_t leaf_size, uint32_t base, Node* nodes, uint32_t leaf0, cudaStream_t s)
+template <int NBP>
+void launch_subtrees_n(const SahWs& w, int nb, uint32_t leaf_size, uint32_t base, Node* nodes, uint32_t leaf0,
+                       cudaStream_t s)
 {
-    const uint32_t grid = (uint32_t)sms() * 8u;
-    auto kernel = nb <= 8 ? k_small<8> : nb <= 16 ? k_small<16> : k_small<32>;
-    kernel<<<grid, 128, 0, s>>>(w.small, w.ctl, w.ids_a, w.ids_b, w.tb, nb, leaf_size, base, nodes, leaf0);
+    // above 48 KB of dynamic shared memory is a per-device opt-in
+    static PerDevice<int> cache;
+    const int per_sm = cache.get([] {
+        cudaFuncSetAttribute(k_mid<NBP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MidStage));
+        return blocks_per_sm(k_mid<NBP>, 256, sizeof(MidStage));
+    });
+    k_mid<NBP><<<per_sm * sms(), 256, sizeof(MidStage), s>>>(w.ids_a, w.ids_b, w.tb, nb, leaf_size, base, nodes, w.done());
+    launch_chained(k_small<NBP>, dim3(sms() * 8), dim3(128), 0, s, (const Task*)w.small, w.ctl, (const uint32_t*)w.ids_a,
+                   (const uint32_t*)w.ids_b, (const float4*)w.tb, nb, leaf_size, base, nodes, leaf0);
+}
+
+void launch_subtrees(const SahWs& w, int nb, uint32_t leaf_size, uint32_t base, Node* nodes, uint32_t leaf0,
+                     cudaStream_t s)
+{
+    if (nb <= 8) launch_subtrees_n<8>(w, nb, leaf_size, base, nodes, leaf0, s);
+    else if (nb <= 16) launch_subtrees_n<16>(w, nb, leaf_size, base, nodes, leaf0, s);
+    else launch_subtrees_n<32>(w, nb, leaf_size, base, nodes, leaf0, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1404,8 +1639,8 @@ __global__ void __launch_bounds__(256) k_sah_setup_seg(const float* __restrict__
 // record root0 + m.
 template <uint32_t CHUNK>
 __global__ void k_root_tasks_seg(const uint32_t* __restrict__ root_ord, const uint32_t* __restrict__ off, uint32_t M,
-                                 uint32_t leaf_size, uint32_t root0, int nb, LevelLists l0, Part* parts, Task* small,
-                                 LeafRange* leaves, Ctl* ctl)
+                                 uint32_t leaf_size, uint32_t root0, int nb, LevelLists l0, Part* parts,
+                                 DoneLists done)
 {
     const uint32_t m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (m >= M) return;
@@ -1426,7 +1661,7 @@ __global__ void k_root_tasks_seg(const uint32_t* __restrict__ root_ord, const ui
             t.pmx[k] = t.cmx[k] = -FLT_MAX;
         }
     }
-    place_root<CHUNK>(t, leaf_size, nb, l0, parts, small, leaves, ctl);
+    place_root<CHUNK>(t, leaf_size, nb, l0, parts, done);
 }
 
 }  // namespace
@@ -1469,20 +1704,20 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
         constexpr uint32_t CHUNK = decltype(chunk)::value;
         if (grid)
             k_grid_tasks<CHUNK><<<16, 128, 0, s>>>(w.cells, w.root_ord, n, leaf_size, scene_box_cells, (int)nb,
-                                                   w.lists[0], w.parts, w.small, w.leaves, w.ctl, scene_out);
+                                                   w.lists[0], w.parts, w.done(), scene_out);
         else
-            k_root_task<CHUNK><<<1, 32, 0, s>>>(w.root_ord, n, leaf_size, (int)nb, w.lists[0], w.parts, w.small,
-                                                w.leaves, w.ctl, scene_out);
-        if (n > kSmall) enqueue_root_bins<CHUNK>(w, (int)nb, s);
+            k_root_task<CHUNK><<<1, 32, 0, s>>>(w.root_ord, n, leaf_size, (int)nb, w.lists[0], w.parts, w.done(),
+                                                scene_out);
+        if (n > kMid) enqueue_root_bins<CHUNK>(w, (int)nb, s);
     });
     // large phase: levels are queued in groups and the host reads the next
     // level's task count (and waits) only between groups; levels past the
     // tree's depth find no tasks and cost two empty launches.  The first
     // group is a balanced tree's depth and two levels more, which is all of
-    // most meshes' large phase; a mesh of at most kSmall triangles has none.
+    // most meshes' large phase; a mesh of at most kMid triangles has none.
     uint32_t group = 2;
-    while (((uint64_t)kSmall << (group - 2)) < n) ++group;
-    if (n > kSmall)
+    while (((uint64_t)kMid << (group - 2)) < n) ++group;
+    if (n > kMid)
         for (uint32_t level = 0;; group = kSahLevelsPerCheck) {
             with_chunk(n, [&](auto chunk) {
                 enqueue_levels<decltype(chunk)::value>(w, level, group, (int)nb, base, leaf_size, nodes, s);
@@ -1494,7 +1729,7 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
         }
     // small phase and leaves
     const uint32_t sg = (uint32_t)sms() * 8u;
-    launch_small(w, (int)nb, leaf_size, base, nodes, leaf0, s);
+    launch_subtrees(w, (int)nb, leaf_size, base, nodes, leaf0, s);
     k_emit_leaves<<<sg, 256, 0, s>>>(w.leaves, w.ctl, w.ids_a, w.ids_b, w.tb, nodes, leaf0, err);
     if (grid) k_grid_heap<<<1, 32, 0, s>>>(nodes);
     return (int)cudaGetLastError();
@@ -1526,11 +1761,11 @@ int build_sah_batch(const float* tris, uint32_t n, const uint32_t* off, uint32_t
     with_chunk(n, [&](auto chunk) {
         constexpr uint32_t CHUNK = decltype(chunk)::value;
         k_root_tasks_seg<CHUNK><<<(M + 3) / 4, 128, 0, s>>>(w.root_ord, off, M, leaf_size, root0, (int)nb, w.lists[0],
-                                                            w.parts, w.small, w.leaves, w.ctl);
+                                                            w.parts, w.done());
         enqueue_root_bins<CHUNK>(w, (int)nb, s);
         enqueue_levels<CHUNK>(w, 0, kBatchLargeLevels, (int)nb, 0u, leaf_size, nodes, s);
     });
-    launch_small(w, (int)nb, leaf_size, 0u, nodes, leaf0, s);
+    launch_subtrees(w, (int)nb, leaf_size, 0u, nodes, leaf0, s);
     k_small_big<<<sm * 8u, 128, 0, s>>>(w.lists[kBatchLargeLevels & 1].tasks, &w.ctl->level[kBatchLargeLevels % 3],
                                         w.ids_a, w.ids_b, w.tb, (int)nb, leaf_size, 0u, nodes, leaf0, err);
     k_emit_leaves<<<sm * 8u, 256, 0, s>>>(w.leaves, w.ctl, w.ids_a, w.ids_b, w.tb, nodes, leaf0, err);
