@@ -594,22 +594,23 @@ __device__ __forceinline__ uint32_t pop8(Lane8& L, const uint2* st)
     return kNoHit;
 }
 
-// One step of a lane that holds a ray: a visit of its inner node, or the test
-// of its leaf's triangles, then the next entry (kNoHit: the ray has finished
-// -- stack empty, any-hit found, or stack overflow: of a node's hits all but
-// the nearest are pushed).  Testing a leaf is a step of its own, so the lanes
-// of a warp that reach leaves in the same step test together; in a loop
-// inside the visit they came one after another (one bounce off the 4.2M
-// terrain 608 -> 571 us, 2^24 incoherent rays 22.8 -> 22.1 ms).  Holding
-// lanes back until 2 to 20 wait at leaves was slower on small ray counts and
-// no faster than 2% on large ones.
+// One step of a lane that holds a ray: a visit of its inner node, then the
+// test of the leaf's triangles if it has come to a leaf (by that visit or by
+// the step before), then the next entry (kNoHit: the ray has finished --
+// stack empty, any-hit found, or stack overflow: of a node's hits all but the
+// nearest are pushed).  One leaf a step, outside the visit: the lanes of a
+// warp test their leaves together, where a loop inside the visit took them
+// one after another.  A leaf that had a step to itself cost the lane one more
+// pass of the loop, which 20,000 rays that do not fill the GPU cannot hide
+// (600,000-triangle sphere: loop inside 166 us, own step 181, this 165); one
+// bounce off the 4.2M terrain 2025, 1569 and 1480 us, 2^24 incoherent rays
+// 25.1, 19.9 and 20.1 ms.  Holding lanes back until 2 to 20 wait at leaves
+// was slower on small ray counts and no faster than 2% on large ones.
 template <bool ANY>
 __device__ __forceinline__ void step8(Lane8& L, bool has, const Node8* __restrict__ nodes,
                                       const float4* __restrict__ t8, uint2* st, float* __restrict__ s_n, Totals8& sum)
 {
-    const bool leaf = has && (L.cur & 0x80000000u);
-    bool pop = false;
-    if (has && !leaf) {
+    if (has && !(L.cur & 0x80000000u)) {
         // slab form chosen per ray, as trace8 does (sign-selected planes for a
         // ray that cannot produce NaN), so a ray's box tests do not depend on
         // the rays it shares a warp with
@@ -622,13 +623,12 @@ __device__ __forceinline__ void step8(Lane8& L, bool has, const Node8* __restric
             L.cur = kNoHit;
             L.sp = 0;
         }
-        pop = L.cur == kNoHit;
     }
-    if (leaf) {
-        pop = !leaf8<ANY>(L, t8, L.cur, sum);
+    if (has && (L.cur & 0x80000000u) && L.cur != kNoHit) {
+        if (leaf8<ANY>(L, t8, L.cur, sum)) L.sp = 0;
         L.cur = kNoHit;
     }
-    if (pop) L.cur = pop8(L, st);
+    if (has && L.cur == kNoHit) L.cur = pop8(L, st);
 }
 
 // Camera rays, tiles: a warp takes one 8x4 pixel tile, each lane runs its
@@ -742,10 +742,16 @@ __global__ void __launch_bounds__(kTilesBlock, 32) k_trace8_tiles(const sqk::Tra
     if (a.stats) ws.flush(lane, a.stats);
 }
 
-// Eight blocks per SM (64 registers): one bounce off the 4.2M-triangle
-// terrain took 552 us against 571 us with seven.
-template <int MODE>
-__global__ void __launch_bounds__(128, 8) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
+// PER_SM: resident blocks per SM the registers are limited for.  Eight (64
+// registers) hide most latency, seven (72) make a warp's own step shorter:
+// 200,000 rays 294 us
+// with eight and 283 with seven (600,000-triangle sphere), 600,000 off a 1M
+// terrain 478 and 483, 2M off the 4.2M terrain 1480 and 1538, 2^24 incoherent
+// 20.1 and 20.8 ms.  So up to kFewRays8 rays per lane of the GPU take seven.
+constexpr uint32_t kFewRays8 = 4;
+
+template <int MODE, int PER_SM>
+__global__ void __launch_bounds__(128, PER_SM) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
 {
     constexpr bool ANY = MODE == SQ_TRACE_ANYHIT;
     const uint32_t lane = threadIdx.x & 31u;
@@ -832,20 +838,25 @@ void launch8(const sqk::Trace8Args& a, cudaStream_t s)
     if (a.ray_kind == SQ_RAYS_EXPLICIT) batches = (a.ray_count + 31u) / 32u;
     else batches = ((a.width + 7u) / 8u) * ((a.height + 3u) / 4u);
     if (batches == 0) return;
-    static PerDevice<std::array<int, 2>> cache;
-    const std::array<int, 2> per_sm = cache.get([] {
-        return std::array<int, 2>{blocks_per_sm(k_trace8_tiles<MODE>, kTilesBlock),
-                                  blocks_per_sm(k_trace8_refill<MODE>, 128)};
+    static PerDevice<std::array<int, 3>> cache;
+    const std::array<int, 3> per_sm = cache.get([] {
+        return std::array<int, 3>{blocks_per_sm(k_trace8_tiles<MODE>, kTilesBlock),
+                                  blocks_per_sm(k_trace8_refill<MODE, 7>, 128),
+                                  blocks_per_sm(k_trace8_refill<MODE, 8>, 128)};
     });
-    const int v = a.refill ? 1 : 0;
-    uint32_t grid = (uint32_t)(per_sm[v] * sm_count());
-    if (!v && a.tile_end && a.tile_end < batches) batches = a.tile_end;  // a band of the image
-    const uint32_t first = v ? 0u : min(a.tile0, batches);
-    const uint32_t need = v ? (batches + 3u) / 4u : batches - first;
-    if (grid > need) grid = need;
+    if (a.refill) {
+        const uint32_t total = a.ray_kind == SQ_RAYS_EXPLICIT ? a.ray_count : batches * 32u;
+        const bool few = total <= kFewRays8 * 8u * 128u * (uint32_t)sm_count();
+        const uint32_t grid = min((uint32_t)(per_sm[few ? 1 : 2] * sm_count()), (batches + 3u) / 4u);
+        if (few) k_trace8_refill<MODE, 7><<<grid, 128, 0, s>>>(a, total);
+        else k_trace8_refill<MODE, 8><<<grid, 128, 0, s>>>(a, total);
+        return;
+    }
+    if (a.tile_end && a.tile_end < batches) batches = a.tile_end;  // a band of the image
+    const uint32_t first = min(a.tile0, batches);
+    const uint32_t grid = min((uint32_t)(per_sm[0] * sm_count()), batches - first);
     if (grid == 0) return;
-    if (v) k_trace8_refill<MODE><<<grid, 128, 0, s>>>(a, a.ray_kind == SQ_RAYS_EXPLICIT ? a.ray_count : batches * 32u);
-    else k_trace8_tiles<MODE><<<grid, kTilesBlock, 0, s>>>(a, batches);
+    k_trace8_tiles<MODE><<<grid, kTilesBlock, 0, s>>>(a, batches);
 }
 
 // Batch, tiles: as k_trace8_tiles over the job table's 32-ray batches.
