@@ -6,9 +6,7 @@
 // of the packet hits the node's box, and the packet counts one test per node
 // box.  Every pixel of the packet gets (tests / k) / 200 in the heatmap.  On
 // the GPU a warp walks 4 packets from one pool (sq_walk_dev.cuh): a lane
-// tests a node against the rays of the packet that visits it.  The packets
-// that a bundle leaves alone (below) are 8 lanes each: "any ray" is a ballot
-// over the packet's lanes, so they take one path and keep identical stacks.
+// tests a node against the rays of the packet that visits it.
 //
 // trace_bundle<k> (src/tracer.cpp:292-362, traverse_bundle 126-156,
 // intersect_bundle_aabb src/tracer.h:37-80): a tile of k = 16 or 64 rays
@@ -17,9 +15,9 @@
 // bundle's direction bounds (min, max and midpoint) while the midpoint
 // direction hits; where only the bounds can hit, each packet of 8 rays
 // continues alone from that node (the packet tracer above).  A pixel of
-// packet m gets bundle_tests / k + packet_tests[m] / 8.  One warp traces one
-// tile: the bundle part is the same for every lane, and the packets of 8 are
-// 8-lane groups (two rays per lane for k = 64).
+// packet m gets bundle_tests / k + packet_tests[m] / 8.  A warp walks two
+// tiles of 16 rays or one of 64 from one pool, their bundles and packets
+// together.
 //
 // Both counts are independent of the visiting order (nothing terminates
 // early), so the stack order need not be the reference's.  The heatmap bytes
@@ -32,40 +30,6 @@
 namespace {
 
 using namespace sq;
-
-constexpr int kPacketStack = 128;  // the reference's packet stack (src/tracer.cpp:94)
-
-
-// traverse_packet_stack from nodes [index, index + count) for the packet of
-// lanes `pmask` (all of which call this together): returns the packet's box
-// test count; *fault is set on a stack overflow or an index past the array.
-__device__ uint32_t packet_tests(const Node* __restrict__ nodes, uint32_t nn, uint32_t index, uint32_t count,
-                                 const float* o, const float* inv, uint32_t pmask, bool* fault)
-{
-    uint32_t st_i[kPacketStack], st_c[kPacketStack];
-    int sp = 1;
-    uint32_t tests = 0;
-    st_i[0] = index;
-    st_c[0] = count;
-    while (sp > 0) {
-        --sp;
-        const uint32_t bi = st_i[sp], bc = st_c[sp];
-        if ((uint64_t)bi + bc > nn) { *fault = true; break; }
-        for (uint32_t c = 0; c < bc; ++c) {
-            const NodeRec nd = load_node(nodes, bi + c);
-            const bool hit = box_ref(nd, o, inv, 10000.0f);
-            const bool any = __ballot_sync(pmask, hit) != 0u;
-            tests++;
-            if (any && !node_is_leaf(nd.cf)) {
-                if (sp >= kPacketStack) { *fault = true; return tests; }
-                st_i[sp] = nd.child;
-                st_c[sp] = node_count(nd.cf);
-                sp++;
-            }
-        }
-    }
-    return tests;
-}
 
 // Packets of one warp's pool (sq_walk_dev.cuh): enough that the pool holds a
 // range for every lane most of the time, few enough that an image still
@@ -99,7 +63,7 @@ __global__ void __launch_bounds__(32) k_trace_packet(const sqk::TraceArgs a)
             for (int c = 0; c < 3; ++c) pool.inv[c][m][p] = 1.0f / r.d[c];
         }
         WalkStats st = {0u, false, false};
-        walk_pool<K, PW, false>(pool, count >= 32u ? 0xFFFFFFFFu : (1u << count) - 1u, a.nodes, a.node_count, a.tri_count,
+        walk_pool(pool, count >= 32u ? 0xFFFFFFFFu : (1u << count) - 1u, a.nodes, a.node_count, a.tri_count,
                                 a.root, 1u, org, st, [](uint32_t, const float*, const float*) { return false; });
         if (st.overflow || st.bad) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
         for (uint32_t j = lane; j < count * K; j += 32) {
@@ -130,131 +94,73 @@ void launch_packets(const sqk::TraceArgs& a, cudaStream_t s)
 // morton_lut (src/tracer.cpp:18-23): k with bits 1 and 2 exchanged
 __device__ __forceinline__ uint32_t bundle_lut(uint32_t k) { return (k & ~6u) | ((k & 2u) << 1) | ((k & 4u) >> 1); }
 
-// intersect_bundle_aabb (src/tracer.h:37-80)
-__device__ __forceinline__ void bundle_box(const NodeRec& nd, const float* pos, const float* imin, const float* imax,
-                                           const float* imid, bool& any_hit, bool& mid_hit)
-{
-    float tmin_mid[3], tmin_any[3], tmax_mid[3], tmax_any[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float lo = nd.mn[k] - pos[k], hi = nd.mx[k] - pos[k];
-        const float t1a = lo * imin[k], t1b = lo * imax[k], t2a = hi * imin[k], t2b = hi * imax[k];
-        const float t1 = lo * imid[k], t2 = hi * imid[k];
-        const float t1min = ref_min(t1a, t1b), t1max = simd_max(t1a, t1b);
-        const float t2min = ref_min(t2a, t2b), t2max = simd_max(t2a, t2b);
-        tmin_mid[k] = ref_min(t1, t2);
-        tmin_any[k] = ref_min(t1min, t2min);
-        tmax_mid[k] = simd_max(t1, t2);
-        tmax_any[k] = simd_max(t1max, t2max);
-    }
-    const float front_mid = ref_max(ref_max(tmin_mid[0], tmin_mid[1]), tmin_mid[2]);
-    const float front_any = ref_max(ref_max(tmin_any[0], tmin_any[1]), tmin_any[2]);
-    const float back_mid = ref_min(ref_min(tmax_mid[0], tmax_mid[1]), tmax_mid[2]);
-    const float back_any = ref_min(ref_min(tmax_any[0], tmax_any[1]), tmax_any[2]);
-    mid_hit = back_mid >= front_mid;
-    any_hit = back_any >= front_any;
-}
+// Bundles of one warp's pool: one of 64 rays is eight packets already (two:
+// 300k terrain at 1280x720, build included, 970 us against 635), of 16 rays
+// one, two, three and four took 436, 454, 540 and 610 us there and 935, 833,
+// 838 and 858 us on a 300k soup at 1920x1072.  A bundle at a time, its walk
+// repeated on every lane, took 1774 us (64 rays) and 1049 us (16) on the
+// terrain.
+template <int K>
+constexpr int kPoolBundles = K == 16 ? 2 : 1;
 
 template <int K>
-__global__ void __launch_bounds__(128) k_trace_bundle(const sqk::TraceArgs a)
+__global__ void __launch_bounds__(32) k_trace_bundle(const sqk::TraceArgs a)
 {
     constexpr int TW = (K == 16) ? 4 : 8;  // floor(sqrt(k))
     constexpr int TH = K / TW;
-    constexpr int SLOTS = (K + 31) / 32;   // rays per lane
-    const int lane = (int)(threadIdx.x & 31u);
-    const uint32_t gmask = 0xFFu << (lane & 24);  // this lane's 8-lane group (one packet per slot)
+    constexpr int NB = kPoolBundles<K>, PK = K / 8, PW = NB * PK;
+    __shared__ WalkPool<8, PW, false, NB> pool;
+    __shared__ float s_d[3][NB][K];
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t tiles_x = a.width / TW;
     const uint32_t total = tiles_x * (a.height / TH);
+    const float org[3] = {a.cam[0], a.cam[1], a.cam[2]};
     uint64_t tests_sum = 0;
     for (;;) {
-        uint32_t tile = 0;
-        if (lane == 0) tile = atomicAdd(a.work, 1u);
-        tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
-        if (tile >= total) break;
-        const uint32_t i0 = (tile % tiles_x) * TW, j0 = (tile / tiles_x) * TH;
-        // this lane's rays: r = lane + 32 * s
-        float d[SLOTS][3], inv[SLOTS][3];
-        uint32_t px[SLOTS];
-        bool valid[SLOTS];
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            const uint32_t r = (uint32_t)lane + 32u * (uint32_t)s;
-            valid[s] = r < (uint32_t)K;
-            const uint32_t v = bundle_lut(valid[s] ? r : 0u);
-            const uint32_t x = i0 + v % TW, y = j0 + v / TW;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(a.work, (uint32_t)NB);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= total) break;
+        const uint32_t count = min((uint32_t)NB, total - base);
+        // ray r of bundle g: packet r / 8, pixel bundle_lut(r) of the tile
+        for (uint32_t j = lane; j < count * K; j += 32) {
+            const uint32_t g = j / K, r = j % K, tile = base + g, v = bundle_lut(r);
             Ray ray;
-            gen_reference_camera(x, y, a.width, a.height, a.cam, ray);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) { d[s][c] = ray.d[c]; inv[s][c] = 1.0f / ray.d[c]; }
-            px[s] = y * a.width + x;
-        }
-        // the bundle's direction bounds, accumulated in ray order as the
-        // reference does (src/tracer.cpp:331-336)
-        float dmin[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, dmax[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (int r = 0; r < K; ++r) {
+            gen_reference_camera((tile % tiles_x) * TW + v % TW, (tile / tiles_x) * TH + v / TW, a.width, a.height,
+                                 a.cam, ray);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                float v = __shfl_sync(0xFFFFFFFFu, d[0][c], r & 31);
-                if (SLOTS > 1) {
-                    const float v1 = __shfl_sync(0xFFFFFFFFu, d[SLOTS - 1][c], r & 31);
-                    if (r >= 32) v = v1;
-                }
-                dmin[c] = ref_min(dmin[c], v);
-                dmax[c] = ref_max(dmax[c], v);
+                s_d[c][g][r] = ray.d[c];
+                pool.inv[c][r % 8][g * PK + r / 8] = 1.0f / ray.d[c];
             }
         }
-        float imin[3], imax[3], imid[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            imin[c] = 1.0f / dmin[c];
-            imax[c] = 1.0f / dmax[c];
-            imid[c] = 1.0f / ((dmin[c] + dmax[c]) * 0.5f);
-        }
-        // the bundle traversal (the same on every lane)
-        uint32_t btests = 0, ptests[SLOTS];
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) ptests[s] = 0;
-        uint32_t st_i[kPacketStack], st_c[kPacketStack];
-        int sp = 1;
-        st_i[0] = a.root;
-        st_c[0] = 1;
-        bool fault = false;
-        while (sp > 0 && !fault) {
-            --sp;
-            const uint32_t bi = st_i[sp], bc = st_c[sp];
-            if ((uint64_t)bi + bc > a.node_count) { fault = true; break; }
-            for (uint32_t c = 0; c < bc; ++c) {
-                const NodeRec nd = load_node(a.nodes, bi + c);
-                bool any_hit, mid_hit;
-                bundle_box(nd, a.cam, imin, imax, imid, any_hit, mid_hit);
-                btests++;
-                if (mid_hit) {
-                    if (!node_is_leaf(nd.cf)) {
-                        if (sp >= kPacketStack) { fault = true; break; }
-                        st_i[sp] = nd.child;
-                        st_c[sp] = node_count(nd.cf);
-                        sp++;
-                    }
-                } else if (any_hit) {
-                    // each packet of 8 continues alone from this node
-#pragma unroll
-                    for (int s = 0; s < SLOTS; ++s) {
-                        if (valid[s]) ptests[s] += packet_tests(a.nodes, a.node_count, bi + c, 1u, a.cam, inv[s],
-                                                                gmask, &fault);
-                    }
-                }
+        __syncwarp();
+        // the bundle's direction bounds, accumulated in ray order as the
+        // reference does (src/tracer.cpp:331-336)
+        if (lane < 3u * count) {
+            const uint32_t g = lane / 3u, c = lane % 3u;
+            float dmin = FLT_MAX, dmax = -FLT_MAX;
+            for (int r = 0; r < K; ++r) {
+                dmin = ref_min(dmin, s_d[c][g][r]);
+                dmax = ref_max(dmax, s_d[c][g][r]);
             }
-            fault = __any_sync(0xFFFFFFFFu, fault);
+            pool.bun[c][g] = 1.0f / dmin;
+            pool.bun[3 + c][g] = 1.0f / dmax;
+            pool.bun[6 + c][g] = 1.0f / ((dmin + dmax) * 0.5f);
         }
-        if (fault && lane == 0) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
-#pragma unroll
-        for (int s = 0; s < SLOTS; ++s) {
-            if (!valid[s]) continue;
-            const float t = (float)btests / (float)K + (float)ptests[s] / 8.0f;
-            write_heat(a.heat + 3ull * px[s], t, a.heat_ramp);
-            if ((lane & 7) == 0) tests_sum += ptests[s];
+        WalkStats st = {0u, false, false};
+        walk_pool(pool, ((1u << count) - 1u) << PW, a.nodes, a.node_count, a.tri_count, a.root, 1u, org, st,
+                  [](uint32_t, const float*, const float*) { return false; });
+        if (st.overflow || st.bad) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
+        for (uint32_t j = lane; j < count * K; j += 32) {
+            const uint32_t g = j / K, r = j % K, tile = base + g, v = bundle_lut(r);
+            const uint32_t x = (tile % tiles_x) * TW + v % TW, y = (tile / tiles_x) * TH + v / TW;
+            const float t = (float)pool.cnt[PW + g] / (float)K + (float)pool.cnt[g * PK + r / 8] / 8.0f;
+            write_heat(a.heat + 3ull * ((size_t)y * a.width + x), t, a.heat_ramp);
         }
-        if (lane == 0) tests_sum += btests;
+        if (lane < count * PK) tests_sum += pool.cnt[lane];
+        if (lane < count) tests_sum += pool.cnt[PW + lane];
+        __syncwarp();  // the pool is used again for the warp's next bundles
     }
     if (a.stats) {
 #pragma unroll
@@ -263,7 +169,14 @@ __global__ void __launch_bounds__(128) k_trace_bundle(const sqk::TraceArgs a)
     }
 }
 
-int sms() { return sm_count(); }
+template <int K>
+void launch_bundles(const sqk::TraceArgs& a, cudaStream_t s)
+{
+    static PerDevice<int> cache;
+    const uint32_t grid = (uint32_t)(cache.get([] { return blocks_per_sm(k_trace_bundle<K>, 32); }) * sm_count());
+    const uint64_t tiles = (uint64_t)a.width * a.height / K, need = (tiles + kPoolBundles<K> - 1) / kPoolBundles<K>;
+    k_trace_bundle<K><<<(uint32_t)std::min<uint64_t>(grid, need ? need : 1), 32, 0, s>>>(a);
+}
 
 }  // namespace
 
@@ -283,10 +196,9 @@ bool coherent_shape_ok(uint32_t bundle, uint32_t k, uint32_t w, uint32_t h)
 
 void trace_coherent(const TraceArgs& a, uint32_t bundle, uint32_t k, cudaStream_t s)
 {
-    const uint32_t grid = (uint32_t)sms() * 8u;
     if (bundle) {
-        if (k == 16) k_trace_bundle<16><<<grid, 128, 0, s>>>(a);
-        else k_trace_bundle<64><<<grid, 128, 0, s>>>(a);
+        if (k == 16) launch_bundles<16>(a, s);
+        else launch_bundles<64>(a, s);
         return;
     }
     switch (k) {

@@ -12,10 +12,18 @@
 // puts the hit nodes' child ranges back.  Triangles of hit leaves go to a
 // second pool and are tested 32 at a time.
 //
+// trace_bundle<k> (src/tracer.cpp:126-156, 292-362) adds owners that are
+// bundles: tested by their direction bounds, walked while the middle
+// direction hits, and where only the bounds hit, all packets of the bundle go
+// on alone from that node.  Such a node is one entry of a third kind (node,
+// packets [first, first + n)), halved each time it is taken until it is one
+// packet's, so no entry taken puts more than two back.
+//
 // What bounds it: with a ray per lane the kernel waited for its longest rays
 // (a ray through the middle of the 2M-triangle soup tests thousands of boxes,
 // its neighbours in the warp tens): 14 of 32 lanes busy and 30% of the warps
-// resident on average.
+// resident on average.  Bundles waited for one walk after another: the bundle
+// the same on all 32 lanes, its packets 8 lanes each.
 #pragma once
 
 #include "sq_trace_dev.cuh"
@@ -28,14 +36,43 @@ constexpr uint32_t kTriCap = 128;       // 31 waiting + 64 of one step fit
 constexpr uint32_t kCountBits = 27;     // an entry: node, owner << 27 | node count
 constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
 
-// K rays per owner, PW owners per warp (at most 32).
-template <int K, int PW, bool TRI>
+// intersect_bundle_aabb (src/tracer.h:37-80)
+__device__ __forceinline__ void bundle_box(const NodeRec& nd, const float* pos, const float* imin, const float* imax,
+                                           const float* imid, bool& any_hit, bool& mid_hit)
+{
+    float tmin_mid[3], tmin_any[3], tmax_mid[3], tmax_any[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float lo = nd.mn[k] - pos[k], hi = nd.mx[k] - pos[k];
+        const float t1a = lo * imin[k], t1b = lo * imax[k], t2a = hi * imin[k], t2b = hi * imax[k];
+        const float t1 = lo * imid[k], t2 = hi * imid[k];
+        const float t1min = ref_min(t1a, t1b), t1max = simd_max(t1a, t1b);
+        const float t2min = ref_min(t2a, t2b), t2max = simd_max(t2a, t2b);
+        tmin_mid[k] = ref_min(t1, t2);
+        tmin_any[k] = ref_min(t1min, t2min);
+        tmax_mid[k] = simd_max(t1, t2);
+        tmax_any[k] = simd_max(t1max, t2max);
+    }
+    const float front_mid = ref_max(ref_max(tmin_mid[0], tmin_mid[1]), tmin_mid[2]);
+    const float front_any = ref_max(ref_max(tmin_any[0], tmin_any[1]), tmin_any[2]);
+    const float back_mid = ref_min(ref_min(tmax_mid[0], tmax_mid[1]), tmax_mid[2]);
+    const float back_any = ref_min(ref_min(tmax_any[0], tmax_any[1]), tmax_any[2]);
+    mid_hit = back_mid >= front_mid;
+    any_hit = back_any >= front_any;
+}
+
+// K rays per owner, PW owners per warp, and NB bundles of PW / NB owners each
+// (0: the owners start by themselves).  Owner numbers: 0 to PW - 1 the owners,
+// then the bundles, then the bundles' entries of the third kind; at most 32.
+template <int K, int PW, bool TRI, int NB = 0>
 struct WalkPool {
+    static_assert(PW + 2 * NB <= 32, "an owner number has 5 bits");
     uint2 node[kPoolCap];
     uint2 tri[TRI ? kTriCap : 1];
     float inv[3][K][PW];                      // reciprocal directions
     float o[3][TRI ? PW : 1], d[3][TRI ? PW : 1], tmax[TRI ? PW : 1];
-    uint32_t cnt[PW];                         // box tests of each owner
+    float bun[9][NB ? NB : 1];                // bundles: reciprocals of the least, largest and middle direction
+    uint32_t cnt[PW + NB];                    // box tests of each owner and bundle
     uint32_t hit;                             // bit per owner: a triangle was hit
 };
 
@@ -45,7 +82,7 @@ struct WalkStats {
 };
 
 // Walks nodes [root, root + group) for every owner in `owners` (a mask, the
-// same in all lanes); pool.inv (and o, d, tmax with TRI) hold the owners'
+// same in all lanes; with bundles, of bundles); pool.inv (and o, d, tmax with TRI) hold the owners'
 // rays.  Without TRI all rays start at `org` and end at 10000.  hit_tri(tri, o, d)
 // tests one triangle.  Afterwards pool.cnt and pool.hit have the results.
 //
@@ -53,14 +90,14 @@ struct WalkStats {
 // entries are taken a step, down to one at a time where fewer than
 // kPoolReserve places are left: a depth-first walk of one subtree, which needs
 // no more places than the 64 pending ranges a ray's own stack would hold.
-template <int K, int PW, bool TRI, class HitTri>
-__device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI>& pool, uint32_t owners, const Node* __restrict__ nodes,
+template <int K, int PW, bool TRI, int NB, class HitTri>
+__device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI, NB>& pool, uint32_t owners, const Node* __restrict__ nodes,
                                           uint32_t nn, uint32_t nt, uint32_t root, uint32_t group, const float* org,
                                           WalkStats& st, HitTri hit_tri)
 {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    if (lane < (uint32_t)PW) pool.cnt[lane] = 0;
+    if (lane < (uint32_t)(PW + NB)) pool.cnt[lane] = 0;
     if (lane == 0) pool.hit = 0;
     // a range of 2^26 nodes or more (no node has one, a caller's root group
     // may) is walked in pieces
@@ -99,22 +136,63 @@ __device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI>& pool, uint32_t o
             uint2 e = make_uint2(0u, 0u);
             if (lane < take) e = pool.node[size - 1u - lane];
             size -= take;
-            const uint32_t w = e.y >> kCountBits;
-            uint32_t c = e.y & kCountMask;
+            uint32_t w = e.y >> kCountBits, c = e.y & kCountMask;
+            uint32_t fan = 0, fan_first = 0;  // packets that go on alone from node e.x
+            if (NB && w >= (uint32_t)(PW + NB)) {
+                fan = c & 0xFFu;
+                fan_first = c >> 8;
+                c = 1;
+                if (fan == 1u) {
+                    w = fan_first;
+                    fan = 0;
+                }
+            }
             if ((uint64_t)e.x + c > nn) {
                 st.bad = true;
                 c = 0;
             }
             // up to two nodes now, the rest of the range back to the pool; a
             // long range is halved instead
-            const bool halve = c > 16u;
+            const bool halve = c > 16u || (NB && fan);
             const uint32_t k = halve ? 0u : min(c, 2u);
             uint2 put[3];
             bool has[3] = {halve, halve, !halve && c > 2u}, leaf[2] = {false, false};
             put[0] = make_uint2(e.x, (c >> 1) | (w << kCountBits));
             put[1] = make_uint2(e.x + (c >> 1), (c - (c >> 1)) | (w << kCountBits));
             put[2] = make_uint2(e.x + 2u, (c - 2u) | (w << kCountBits));
-            if (k) {
+            if (NB && fan) {
+                const uint32_t h = fan >> 1;
+                put[0] = make_uint2(e.x, h | (fan_first << 8) | (w << kCountBits));
+                put[1] = make_uint2(e.x, (fan - h) | ((fan_first + h) << 8) | (w << kCountBits));
+            }
+            if (NB && k && w >= (uint32_t)PW) {
+                const uint32_t g = w - (uint32_t)PW;
+                const NodeRec n0 = load_node(nodes, e.x), n1 = load_node(nodes, e.x + (k > 1u ? 1u : 0u));
+                float imin[3], imax[3], imid[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    imin[a] = pool.bun[a][g];
+                    imax[a] = pool.bun[3 + a][g];
+                    imid[a] = pool.bun[6 + a][g];
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (q && k < 2u) break;
+                    const NodeRec& nd = q ? n1 : n0;
+                    bool any_hit, mid_hit;
+                    bundle_box(nd, org, imin, imax, imid, any_hit, mid_hit);
+                    const uint32_t cc = node_count(nd.cf);
+                    if (mid_hit) {
+                        has[q] = !node_is_leaf(nd.cf) && cc;
+                        put[q] = make_uint2(nd.child, cc | (w << kCountBits));
+                    } else if (any_hit) {
+                        constexpr uint32_t PK = (uint32_t)(NB ? PW / NB : 1);
+                        has[q] = true;
+                        put[q] = make_uint2(e.x + (uint32_t)q, PK | ((g * PK) << 8) | ((w + (uint32_t)NB) << kCountBits));
+                    }
+                }
+                atomicAdd(&pool.cnt[w], k);
+            } else if (k) {
                 float o[3], tmax;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) o[a] = TRI ? pool.o[a][w] : org[a];
