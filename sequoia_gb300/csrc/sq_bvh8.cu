@@ -398,11 +398,12 @@ constexpr uint32_t kMaxLevels = 64;
 // own: with the level's cluster mark stored beside the counters the collapse
 // of the 2M soup took 858 us instead of 215.
 constexpr uint32_t kWsNodes = 0;               // a 64-bit pair: nodes beyond the roots, triangle slots
-constexpr uint32_t kWsBarrier = 32;            // arrivals, generation
+constexpr uint32_t kWsBarrier = 32;            // arrivals at the level barriers
 constexpr uint32_t kWsCount = 64;              // final node count, then the number of levels
 constexpr uint32_t kWsClusters = 66;           // levels that the deepest cluster node makes
 constexpr uint32_t kWsBefore = 67;             // nodes before the level
-constexpr uint32_t kWsLevel = 96;              // tasks of level l at kWsLevel + l
+constexpr uint32_t kWsOpen = 96;               // a 64-bit word: tasks of the level opened last, its number above
+constexpr uint32_t kWsLevel = 128;             // tasks of level l at kWsLevel + l
 constexpr uint32_t kWsHead = kWsLevel + kMaxLevels + 32;
 
 __host__ __device__ inline CollapseWs collapse_ws(uint32_t* ws, uint32_t capacity)
@@ -464,12 +465,16 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse_level(
 }
 
 // After level `level`, before anything of the next one: a level that made
-// more nodes than tasks made cluster nodes, one level below its own.
-__device__ __forceinline__ void collapse_level_end(uint32_t* head, uint32_t level)
+// more nodes than tasks made cluster nodes, one level below its own.  Returns
+// the next level's tasks.  (Relaxed loads, so they are in flight together: the
+// caller has ordered them after the level's atomics.)
+__device__ __forceinline__ uint32_t collapse_level_end(uint32_t* head, uint32_t level)
 {
-    const uint32_t nodes = ld_acquire_u32(head + kWsNodes), tasks = ld_acquire_u32(head + kWsLevel + level + 1);
-    if (nodes - ld_acquire_u32(head + kWsBefore) > tasks) st_relaxed_u32(head + kWsClusters, level + 2u);
+    const uint32_t nodes = ld_relaxed_u32(head + kWsNodes), tasks = ld_relaxed_u32(head + kWsLevel + level + 1);
+    const uint32_t before = ld_relaxed_u32(head + kWsBefore);
+    if (nodes - before > tasks) st_relaxed_u32(head + kWsClusters, level + 2u);
     st_relaxed_u32(head + kWsBefore, nodes);
+    return tasks;
 }
 
 // The final counts: nodes, and levels (levels of tasks, or one more where the
@@ -505,15 +510,19 @@ __global__ void k_collapse_done(CollapseWs w, uint32_t levels, uint32_t nroots, 
 // the first barrier.
 constexpr uint32_t kBarrierSpins = 1u << 24;
 
-// Grid barrier in two halves.  barrier_arrive: every warp calls it once, when
-// its writes before the barrier are done; the block's last warp arrives for
-// the block, and the grid's last block runs on_last() before any block
-// leaves, with every write of before the barrier visible to it.
-// barrier_wait: the block waits (thread 0 polls), and every thread gets the
-// value of *word, which the blocks changed before the barrier; false when the
-// wait gave up.  s_warps: a shared counter, zero before the first use.
+// Grid barrier of a level in two halves.  barrier_arrive: every warp calls it
+// once, when its writes before the barrier are done; the block's last warp
+// arrives for the block, and the grid's last block (arrivals are counted from
+// the first level on: `target` of them) runs on_last(), with every write of
+// before the barrier visible to it, and opens the next level.  barrier_wait:
+// the block waits (thread 0 polls), and every thread gets the next level's
+// tasks, which are in the polled word; false when the wait gave up.  s_warps:
+// a shared counter, zero before the first use.  Each access that depends on
+// one before it is an L2 round trip, most of a thin level's time: the count
+// reset and the tasks read after the wait took two to three more (2M soup 12 us
+// over 12 levels, 1,280 triangles 3 us over four).
 template <class OnLast>
-__device__ __forceinline__ void barrier_arrive(uint32_t* bar, uint32_t nblocks, uint32_t* s_warps, OnLast on_last)
+__device__ __forceinline__ void barrier_arrive(uint32_t* arrivals, uint32_t target, uint32_t* s_warps, OnLast on_last)
 {
     __syncwarp();
     if ((threadIdx.x & 31u) != 0) return;
@@ -521,23 +530,29 @@ __device__ __forceinline__ void barrier_arrive(uint32_t* bar, uint32_t nblocks, 
     if (atomicAdd(s_warps, 1u) + 1u != (blockDim.x >> 5)) return;
     __threadfence();
     *s_warps = 0;  // every warp of the block has counted; the next use is after barrier_wait's block barrier
-    if (atomicAdd(bar, 1u) + 1u == nblocks) {
-        // last arrival: reset the count, then open the next generation
+    if (atomicAdd(arrivals, 1u) + 1u == target) {
         __threadfence();
         on_last();
-        atomicExch(bar, 0u);
-        __threadfence();
-        atomicAdd(bar + 1, 1u);
     }
 }
 
-__device__ __forceinline__ bool barrier_wait(const uint32_t* bar, uint32_t gen, uint32_t spin_limit, const uint32_t* word,
-                                             uint32_t* err, uint32_t& value)
+__device__ __forceinline__ void open_level(uint32_t* head, uint32_t level, uint32_t tasks)
 {
-    __shared__ uint32_t s_ok, s_value;
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(head + kWsOpen),
+                 "l"(((unsigned long long)level << 32) | tasks)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool barrier_wait(const uint32_t* head, uint32_t level, uint32_t spin_limit, uint32_t* err,
+                                             uint32_t& tasks)
+{
+    __shared__ uint32_t s_ok, s_tasks;
     if (threadIdx.x == 0) {
         uint32_t ok = 1, spins = 0;
-        while (ld_acquire_u32(bar + 1) == gen) {
+        unsigned long long v;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(head + kWsOpen) : "memory");
+            if ((uint32_t)(v >> 32) == level) break;
             if (++spins > spin_limit) {
                 raise_error(err, SQ_DEVERR_SAH_QUEUE);
                 ok = 0;
@@ -546,11 +561,11 @@ __device__ __forceinline__ bool barrier_wait(const uint32_t* bar, uint32_t gen, 
             __nanosleep(32);
         }
         s_ok = ok;
-        s_value = ld_acquire_u32(word);
+        s_tasks = (uint32_t)v;
     }
     __syncthreads();
     const bool ok = s_ok != 0;
-    value = s_value;
+    tasks = s_tasks;
     __syncthreads();  // read by every thread before the next wait writes them
     return ok;
 }
@@ -571,7 +586,6 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
     __syncthreads();
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t* bar = w.head + kWsBarrier;
     uint32_t ntasks = nroots;
     // (an overflow of the node capacity has raised the error word; the lists
     // hold no more than `capacity` tasks)
@@ -580,9 +594,9 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
             if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(err, SQ_DEVERR_SAH_QUEUE);
             return;
         }
-        // the generations are the levels: nobody has opened this one yet
         auto arrive = [&] {
-            barrier_arrive(bar, gridDim.x + barrier_extra, &s_warps, [&] { collapse_level_end(w.head, level); });
+            barrier_arrive(w.head + kWsBarrier, (gridDim.x + barrier_extra) * (level + 1u), &s_warps,
+                           [&] { open_level(w.head, level + 1u, collapse_level_end(w.head, level)); });
         };
         if (4u * wid >= ntasks) arrive();
         for (uint32_t base = 4u * wid; base < ntasks; base += 4u * warps) {
@@ -594,7 +608,7 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
             collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
                           s_group[threadIdx.x >> 5], [&] { if (last) arrive(); });
         }
-        if (!barrier_wait(bar, level, spin_limit, w.head + kWsLevel + level + 1, err, ntasks)) return;
+        if (!barrier_wait(w.head, level + 1u, spin_limit, err, ntasks)) return;
         if (!ntasks && blockIdx.x == 0 && threadIdx.x == 0) collapse_done(w.head, level + 1, nroots, capacity, meta);
     }
 }
