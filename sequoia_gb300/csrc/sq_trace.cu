@@ -227,7 +227,10 @@ __device__ __forceinline__ void trace_ref(const Node* __restrict__ nodes, uint32
 //   narrow  8 bytes: bit 31 leaf, bits 27-30 count (1 to 15; 0: the low bits
 //           are the node's index and its record is read after all), bits 0-26
 //           first child or triangle; entry distance.  Trees of up to 2^27
-//           records and triangles.
+//           records and triangles.  A first child that needs more bits is past
+//           the tree's records (only an imported record can name one): its
+//           entry is the node's index, so that the bad range is met where
+//           every other is, by the visit that would read it.
 //   wide    16 bytes: first child or triangle, count and leaf bit (31), entry
 //           distance.  Larger trees.
 template <bool WIDE>
@@ -251,7 +254,7 @@ __device__ __forceinline__ Entry<WIDE> make_entry(uint32_t index, uint32_t cf, u
     Entry<WIDE> e;
     e.y = 0;
     if (WIDE) { e.x = child; e.y = c | leaf; }
-    else e.x = c - 1u < 15u ? leaf | (c << 27) | child : index;
+    else e.x = c - 1u < 15u && child <= kNarrowMask ? leaf | (c << 27) | child : index;
     return e;
 }
 
