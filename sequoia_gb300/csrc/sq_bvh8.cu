@@ -169,6 +169,10 @@ __device__ __forceinline__ void write_tri8(float4* __restrict__ d, const float* 
 // is called by the whole warp once that is done: what follows (the node's
 // planes and the triangle copies) is of no matter to the next level.  sm: this
 // warp's staging area.
+// A node that cannot be made (a record of more than eight children, a leaf of
+// more than 15 triangles, no room for its children) is refused: the error word
+// is set and the node is written without children, so that neither the cluster
+// pass nor a trace before the error is seen meets a node that nothing wrote.
 template <class Alloc, class Publish, class Published>
 __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0, const float* __restrict__ tris,
                                     bool active, uint32_t rec_i, uint32_t node_i, Node8* __restrict__ nodes8,
@@ -181,6 +185,7 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
     const int g = lane >> 3;  // group (node) of this lane
     const int gs = lane & ~7; // first lane of the group
     auto gballot = [&](bool pr) -> uint32_t { return (__ballot_sync(FULL, pr) >> gs) & 0xFFu; };
+    const bool owns = active;
     Node self;
     uint32_t c0 = 0, cn = 0;
     if (active) {
@@ -274,8 +279,8 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
     // children's in the high half (at most 64 and 120)
     const uint32_t cntk = leafc ? e_cnt : 0u;
     const uint32_t both = cntk | (inner && own_node ? e_cnt << 16 : 0u);
-    const uint32_t imask = gballot(inner);
-    const uint32_t valid = gballot(ok);
+    uint32_t imask = gballot(inner);
+    uint32_t valid = gballot(ok);
     const uint32_t tmask = gballot(inner && !own_node);
     const uint32_t leafrec = gballot(k < nc && node_is_leaf(e_node.count_flags));
     uint32_t incl = both;
@@ -304,9 +309,6 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
     const uint32_t child_base = __shfl_sync(FULL, node_base, 0) + (pre_nt & 0xFFFFu);
     tri_base = __shfl_sync(FULL, tri_base, 0) + pre_t;
     task_base = __shfl_sync(FULL, task_base, 0) + (pre_nt >> 16);
-    sm.off[g][k] = tri_off;
-    sm.cnt[g][k] = cntk;
-    sm.child[g][k] = e_node.child;
     if (active && inner) {
         const uint32_t node = child_base + __popc(imask & ((1u << k) - 1u));
         if (!own_node) publish(task_base + __popc(tmask & ((1u << k) - 1u)), node, e_rec);
@@ -314,7 +316,12 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
             *placeholder_of(nodes8 + node) = make_uint4(e_rec, tri_base + n_tris + ((incl - both) >> 16), 0u, kPlaceholder);
     }
     published();
-    write_node8(active, k, g, self, e_node, ok, imask, valid, child_base, tri_base, sm, nodes8 + node_i);
+    if (imask && child_base + __popc(imask) > capacity) active = false;
+    if (!active) imask = valid = 0;
+    sm.off[g][k] = tri_off;
+    sm.cnt[g][k] = active ? cntk : 0u;
+    sm.child[g][k] = e_node.child;
+    write_node8(owns, k, g, self, e_node, ok && active, imask, valid, child_base, tri_base, sm, nodes8 + node_i);
     if (active) {
         // leaf triangles, spread over the group: triangle t of the node
         // belongs to the leaf slot whose [off, off + cnt) holds it
@@ -334,8 +341,12 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
 // The cluster nodes, four per warp: lane k of a group has the cluster's
 // triangle k, its box from its leaf record.  One pass over the node array
 // (80 B a node read or written, the leaf records and the triangles gathered):
-// bound by those gathers.
-__global__ void __launch_bounds__(256) k_collapse_clusters(const Node* __restrict__ rec, const float* __restrict__ tris,
+// bound by those gathers.  A placeholder is taken only where its record and
+// its triangle slots are inside the arrays (ntris triangles, leaf records from
+// leaf0 on): where the collapse ran out of room, the last counted nodes were
+// written by nothing.
+__global__ void __launch_bounds__(256) k_collapse_clusters(const Node* __restrict__ rec, uint32_t leaf0,
+                                                           const float* __restrict__ tris, uint32_t ntris,
                                                            const uint32_t* __restrict__ count,
                                                            Node8* __restrict__ nodes8, float4* __restrict__ tris8)
 {
@@ -354,12 +365,14 @@ __global__ void __launch_bounds__(256) k_collapse_clusters(const Node* __restric
         Node self, child;
         bool ok = false;
         uint32_t id = 0;
-        if (active) {
+        if (active && ph.x < leaf0) {
             self = rec[ph.x];
-            if (k < (int)node_count(self.count_flags)) {
+            const uint32_t c = node_count(self.count_flags);
+            if (k < (int)c && c <= 8u && self.child >= leaf0 && (uint64_t)self.child + c <= (uint64_t)leaf0 + ntris &&
+                (uint64_t)ph.y + c <= ntris) {
                 child = rec[self.child + (uint32_t)k];
                 id = child.child;
-                ok = child.mnx <= child.mxx && child.mny <= child.mxy && child.mnz <= child.mxz;
+                ok = id < ntris && child.mnx <= child.mxx && child.mny <= child.mxy && child.mnz <= child.mxz;
             }
         }
         const uint32_t valid = (__ballot_sync(FULL, ok) >> gs) & 0xFFu;
@@ -435,8 +448,10 @@ __device__ __forceinline__ void collapse_task(const Node* __restrict__ rec, uint
         if (kj) jb = atomicAdd(head + kWsLevel + level + 1, kj);
         alloc_nodes_tris(head + kWsNodes, kn, kt, nroots, capacity, err, nb, tb);
     };
+    // (a node past the capacity is listed too: its task is counted, and the
+    // next level passes it over)
     auto publish = [&](uint32_t j, uint32_t node, uint32_t record) {
-        if (node >= capacity || j >= capacity) return;
+        if (j >= capacity) return;
         next_rec[j] = record;
         next_node[j] = node;
     };
@@ -457,9 +472,10 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse_level(
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (4u * warp >= ntasks) return;  // whole warps
     const uint32_t i = 4u * warp + ((threadIdx.x & 31u) >> 3);
-    const bool active = i < ntasks;
-    const uint32_t rec_i = !active ? 0u : (level ? w.rec[level & 1][i] : root + i);
-    const uint32_t node_i = !active ? 0u : (level ? w.node[level & 1][i] : i);
+    const bool listed = i < ntasks;
+    const uint32_t rec_i = !listed ? 0u : (level ? w.rec[level & 1][i] : root + i);
+    const uint32_t node_i = !listed ? 0u : (level ? w.node[level & 1][i] : i);
+    const bool active = listed && node_i < capacity;
     collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
                   s_group[threadIdx.x >> 5], [] {});
 }
@@ -601,9 +617,10 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
         if (4u * wid >= ntasks) arrive();
         for (uint32_t base = 4u * wid; base < ntasks; base += 4u * warps) {
             const uint32_t i = base + ((threadIdx.x & 31u) >> 3);
-            const bool active = i < ntasks;
-            const uint32_t rec_i = !active ? 0u : (level ? __ldcg(w.rec[level & 1] + i) : root + i);
-            const uint32_t node_i = !active ? 0u : (level ? __ldcg(w.node[level & 1] + i) : i);
+            const bool listed = i < ntasks;
+            const uint32_t rec_i = !listed ? 0u : (level ? __ldcg(w.rec[level & 1] + i) : root + i);
+            const uint32_t node_i = !listed ? 0u : (level ? __ldcg(w.node[level & 1] + i) : i);
+            const bool active = listed && node_i < capacity;
             const bool last = ntasks - base <= 4u * warps;
             collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
                           s_group[threadIdx.x >> 5], [&] { if (last) arrive(); });
@@ -638,12 +655,12 @@ static int coop_blocks()
     });
 }
 
-static cudaError_t launch_clusters(const Node* rec, const float* tris, const CollapseWs& w, void* nodes8, void* tris8,
-                                   cudaStream_t s)
+static cudaError_t launch_clusters(const Node* rec, uint32_t leaf0, const float* tris, uint32_t n, const CollapseWs& w,
+                                   void* nodes8, void* tris8, cudaStream_t s)
 {
     static PerDevice<int> cache;
     const int grid = cache.get([] { return blocks_per_sm(k_collapse_clusters, 256) * sm_count(); });
-    k_collapse_clusters<<<grid, 256, 0, s>>>(rec, tris, w.head + kWsCount, static_cast<Node8*>(nodes8),
+    k_collapse_clusters<<<grid, 256, 0, s>>>(rec, leaf0, tris, n, w.head + kWsCount, static_cast<Node8*>(nodes8),
                                              static_cast<float4*>(tris8));
     return cudaGetLastError();
 }
@@ -669,7 +686,7 @@ static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, con
         ntasks = std::min(host_ctl[0], capacity);
     }
     k_collapse_done<<<1, 1, 0, s>>>(w, level, 1u, capacity);
-    if ((e = launch_clusters(rec, tris, w, nodes8, tris8, s)) != cudaSuccess) return (int)e;
+    if ((e = launch_clusters(rec, leaf0, tris, n, w, nodes8, tris8, s)) != cudaSuccess) return (int)e;
     uint32_t m[2];
     if ((e = cudaMemcpyAsync(m, w.head + kWsCount, sizeof m, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
@@ -696,7 +713,7 @@ static cudaError_t enqueue_collapse(const Node* rec, uint32_t root, uint32_t nro
     const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_collapse_coop, dim3(per_sm * sm_count()), dim3(256),
                                                       args, 0, s);
     if (e != cudaSuccess) return e;
-    return launch_clusters(rec, tris, w, nodes8, tris8, s);
+    return launch_clusters(rec, leaf0, tris, n, w, nodes8, tris8, s);
 }
 
 int build_bvh8_queue(const Node* rec, uint32_t root0, uint32_t nroots, uint32_t leaf0, const float* tris, uint32_t n,
