@@ -884,10 +884,13 @@ __device__ void warp_emit_leaf(const uint32_t* __restrict__ ids, uint32_t b, uin
         if (c == 1 && !(flags & 2u)) store_node(nodes + slot, bb, id, 1u, kLeafFlag);
     }
     if (lane == 0 && (c != 1 || (flags & 2u))) {
-        if (c > 65535u) { raise_error(err, SQ_DEVERR_NODE_COUNT); return; }
+        // a record counts to 65535: a larger range is refused, its record empty
+        // (the collapse and the traversals read it before the error is seen)
+        const bool fits = c <= 65535u;
+        if (!fits) raise_error(err, SQ_DEVERR_NODE_COUNT);
         Box pb;
         for (int a = 0; a < 3; ++a) { pb.mn[a] = pmn[a]; pb.mx[a] = pmx[a]; }
-        store_node(nodes + slot, pb, leaf0 + b, c, 0);
+        store_node(nodes + slot, pb, leaf0 + b, fits ? c : 0u, 0);
     }
 }
 

@@ -98,3 +98,34 @@ def test_refused_batch(lib_built):
     assert np.array_equal(got["id"], want["id"]) and np.array_equal(got["t"], want["t"])
     b.free()
     ctx.close()
+
+
+@pytest.mark.parametrize("builder", ["sah", "grid"])
+@pytest.mark.parametrize("wide", [False, True])
+def test_range_past_the_record_count(lib_built, builder, wide):
+    """A leaf range of more than 65535 triangles, which no record can hold."""
+    import sequoia_gb300 as sq
+    from sequoia_gb300 import scenes
+    ctx = sq.Context(0)
+    soup = scenes.gaussian_soup(500, 2, seed=33)
+    lo, hi = scenes.scene_box(soup)
+    rays = scenes.random_rays(2000, lo, hi, seed=8)
+    far = soup[:1] + np.float32(1000)
+    alone = ctx.build(soup, builder, wide=wide)
+    want, _ = ctx.trace(alone, "closest", rays=rays)
+    for tris in (np.concatenate([soup, np.repeat(far, 70_000, 0)]), np.repeat(far, 70_000, 0)):
+        fill_cache(ctx, NONE)
+        bvh = ctx.build(np.ascontiguousarray(tris), builder, wide=wide)
+        assert raw_sync(ctx) == (ERR_DEVICE, NODE_COUNT)
+        for sched in ("tiles", "refill"):
+            got, _ = ctx.trace(bvh, "closest", rays=rays, sched=sched)
+            if len(tris) > 70_000:
+                assert np.array_equal(got["id"], want["id"]) and np.array_equal(got["t"], want["t"])
+            else:
+                assert (got["id"] == NONE).all()
+        ref, _ = ctx.trace(bvh, "ref", rays=rays)
+        assert len(tris) > 70_000 or (ref["id"] == NONE).all()
+        assert raw_sync(ctx) == (0, 0)
+        bvh.free()
+    alone.free()
+    ctx.close()
