@@ -30,8 +30,7 @@
 
 namespace sq {
 
-constexpr uint32_t kPoolCap = 768;      // node ranges in a warp's pool
-constexpr uint32_t kPoolReserve = 128;  // kept for the one-at-a-time walk below
+constexpr uint32_t kPoolOpen = 640;     // node ranges in a warp's pool beside the reserve
 constexpr uint32_t kTriCap = 128;       // 31 waiting + 64 of one step fit
 constexpr uint32_t kCountBits = 27;     // an entry: node, owner << 27 | node count
 constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
@@ -67,7 +66,13 @@ __device__ __forceinline__ void bundle_box(const NodeRec& nd, const float* pos, 
 template <int K, int PW, bool TRI, int NB = 0>
 struct WalkPool {
     static_assert(PW + 2 * NB <= 32, "an owner number has 5 bits");
-    uint2 node[kPoolCap];
+    // places kept for the one-at-a-time walk (walk_pool): the deepest walk of
+    // one ray or packet that is asked for has 128 pending ranges, one of a
+    // bundle 128 more, and a range, a fan and the places checked for come on
+    // top
+    static constexpr uint32_t kReserve = NB ? 272u : 136u;
+    static constexpr uint32_t kCap = kPoolOpen + kReserve;
+    uint2 node[kCap];
     uint2 tri[TRI ? kTriCap : 1];
     float inv[3][K][PW];                      // reciprocal directions
     float o[3][TRI ? PW : 1], d[3][TRI ? PW : 1], tmax[TRI ? PW : 1];
@@ -87,9 +92,12 @@ struct WalkStats {
 // tests one triangle.  Afterwards pool.cnt and pool.hit have the results.
 //
 // The pool grows by at most two ranges per entry taken, so as it fills fewer
-// entries are taken a step, down to one at a time where fewer than
-// kPoolReserve places are left: a depth-first walk of one subtree, which needs
-// no more places than the 64 pending ranges a ray's own stack would hold.
+// entries are taken a step, down to one at a time where only the reserve is
+// left: the rest of the range goes above the children that were found, and a
+// bundle's packets above both, so this is the reference's own order (all of a
+// group, then the last hit child's; src/tracer.cpp:47-65, 126-156) and needs
+// the places of the reference's own stack.  (Halving long ranges here too left
+// half a group behind at every level of a chain of groups of 17 nodes.)
 template <int K, int PW, bool TRI, int NB, class HitTri>
 __device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI, NB>& pool, uint32_t owners, const Node* __restrict__ nodes,
                                           uint32_t nn, uint32_t nt, uint32_t root, uint32_t group, const float* org,
@@ -127,9 +135,10 @@ __device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI, NB>& pool, uint32
                 continue;
             }
             if (size == 0) break;
-            const uint32_t room = size + kPoolReserve < kPoolCap ? (kPoolCap - kPoolReserve - size) / 2u : 0u;
-            const uint32_t take = min(min(32u, size), max(room, 1u));
-            if (size + 2u > kPoolCap) {
+            const uint32_t room = size < kPoolOpen ? (kPoolOpen - size) / 2u : 0u;
+            const bool one = room == 0u;
+            const uint32_t take = one ? 1u : min(min(32u, size), room);
+            if (size + 2u > WalkPool<K, PW, TRI, NB>::kCap) {
                 st.overflow = true;
                 break;
             }
@@ -153,13 +162,14 @@ __device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI, NB>& pool, uint32
             }
             // up to two nodes now, the rest of the range back to the pool; a
             // long range is halved instead
-            const bool halve = c > 16u || (NB && fan);
-            const uint32_t k = halve ? 0u : min(c, 2u);
+            const bool halve = (c > 16u && !one) || (NB && fan);
+            const uint32_t two = NB && one ? 1u : 2u;
+            const uint32_t k = halve ? 0u : min(c, two);
             uint2 put[3];
-            bool has[3] = {halve, halve, !halve && c > 2u}, leaf[2] = {false, false};
+            bool has[3] = {halve, halve, !halve && c > two}, leaf[2] = {false, false};
             put[0] = make_uint2(e.x, (c >> 1) | (w << kCountBits));
             put[1] = make_uint2(e.x + (c >> 1), (c - (c >> 1)) | (w << kCountBits));
-            put[2] = make_uint2(e.x + 2u, (c - 2u) | (w << kCountBits));
+            put[2] = make_uint2(e.x + two, (c - two) | (w << kCountBits));
             if (NB && fan) {
                 const uint32_t h = fan >> 1;
                 put[0] = make_uint2(e.x, h | (fan_first << 8) | (w << kCountBits));
@@ -189,6 +199,11 @@ __device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI, NB>& pool, uint32
                         constexpr uint32_t PK = (uint32_t)(NB ? PW / NB : 1);
                         has[q] = true;
                         put[q] = make_uint2(e.x + (uint32_t)q, PK | ((g * PK) << 8) | ((w + (uint32_t)NB) << kCountBits));
+                        if (one && has[2]) {  // on top of the rest of the range
+                            const uint2 rest = put[2];
+                            put[2] = put[0];
+                            put[0] = rest;
+                        }
                     }
                 }
                 atomicAdd(&pool.cnt[w], k);
