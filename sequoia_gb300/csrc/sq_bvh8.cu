@@ -344,17 +344,26 @@ __device__ void collapse_node_group(const Node* __restrict__ rec, uint32_t leaf0
 // bound by those gathers.  A placeholder is taken only where its record and
 // its triangle slots are inside the arrays (ntris triangles, leaf records from
 // leaf0 on): where the collapse ran out of room, the last counted nodes were
-// written by nothing.
+// written by nothing.  A collapse that gave up (a barrier wait that ran out,
+// too many levels) left no count: its trees become empty roots, so that a
+// trace before the error is seen, as in a batch, reads nothing else.
 __global__ void __launch_bounds__(256) k_collapse_clusters(const Node* __restrict__ rec, uint32_t leaf0,
                                                            const float* __restrict__ tris, uint32_t ntris,
-                                                           const uint32_t* __restrict__ count,
-                                                           Node8* __restrict__ nodes8, float4* __restrict__ tris8)
+                                                           const uint32_t* __restrict__ count, uint32_t nroots,
+                                                           uint32_t* __restrict__ meta, Node8* __restrict__ nodes8,
+                                                           float4* __restrict__ tris8)
 {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     __shared__ GroupSmem s_group[8];
     GroupSmem& sm = s_group[threadIdx.x >> 5];
     const int lane = (int)(threadIdx.x & 31u), k = lane & 7, g = lane >> 3, gs = lane & ~7;
     const uint32_t n = *count;
+    if (n == 0) {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 5u * nroots; i += gridDim.x * blockDim.x)
+            reinterpret_cast<uint4*>(nodes8)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (meta && blockIdx.x == 0 && threadIdx.x < 2) meta[threadIdx.x] = 1u;
+        return;
+    }
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t base = 4u * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < n; base += 4u * warps) {
         const uint32_t i = base + (uint32_t)g;
@@ -656,12 +665,12 @@ static int coop_blocks()
 }
 
 static cudaError_t launch_clusters(const Node* rec, uint32_t leaf0, const float* tris, uint32_t n, const CollapseWs& w,
-                                   void* nodes8, void* tris8, cudaStream_t s)
+                                   uint32_t nroots, uint32_t* meta, void* nodes8, void* tris8, cudaStream_t s)
 {
     static PerDevice<int> cache;
     const int grid = cache.get([] { return blocks_per_sm(k_collapse_clusters, 256) * sm_count(); });
-    k_collapse_clusters<<<grid, 256, 0, s>>>(rec, leaf0, tris, n, w.head + kWsCount, static_cast<Node8*>(nodes8),
-                                             static_cast<float4*>(tris8));
+    k_collapse_clusters<<<grid, 256, 0, s>>>(rec, leaf0, tris, n, w.head + kWsCount, nroots, meta,
+                                             static_cast<Node8*>(nodes8), static_cast<float4*>(tris8));
     return cudaGetLastError();
 }
 
@@ -686,7 +695,7 @@ static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, con
         ntasks = std::min(host_ctl[0], capacity);
     }
     k_collapse_done<<<1, 1, 0, s>>>(w, level, 1u, capacity);
-    if ((e = launch_clusters(rec, leaf0, tris, n, w, nodes8, tris8, s)) != cudaSuccess) return (int)e;
+    if ((e = launch_clusters(rec, leaf0, tris, n, w, 1u, nullptr, nodes8, tris8, s)) != cudaSuccess) return (int)e;
     uint32_t m[2];
     if ((e = cudaMemcpyAsync(m, w.head + kWsCount, sizeof m, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
@@ -713,7 +722,7 @@ static cudaError_t enqueue_collapse(const Node* rec, uint32_t root, uint32_t nro
     const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_collapse_coop, dim3(per_sm * sm_count()), dim3(256),
                                                       args, 0, s);
     if (e != cudaSuccess) return e;
-    return launch_clusters(rec, leaf0, tris, n, w, nodes8, tris8, s);
+    return launch_clusters(rec, leaf0, tris, n, w, nroots, meta, nodes8, tris8, s);
 }
 
 int build_bvh8_queue(const Node* rec, uint32_t root0, uint32_t nroots, uint32_t leaf0, const float* tris, uint32_t n,

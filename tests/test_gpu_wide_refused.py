@@ -129,3 +129,27 @@ def test_range_past_the_record_count(lib_built, builder, wide):
         bvh.free()
     alone.free()
     ctx.close()
+
+
+def test_collapse_that_gave_up_is_an_empty_tree(lib_built):
+    import sequoia_gb300 as sq
+    import torch
+    from sequoia_gb300 import scenes
+    ctx = sq.Context(0)
+    tris = scenes.gaussian_soup(20_000, 4, seed=35)
+    lo, hi = scenes.scene_box(tris)
+    rays = scenes.random_rays(3000, lo, hi, seed=9)
+    for word in (NONE, 0x7FFFFFFF):
+        fill_cache(ctx, word)
+        ctx.debug_inject("stall_barrier", 256)
+        bvh = ctx.build(tris, "morton", wide=True)
+        out = torch.ones(3 * len(rays), dtype=torch.int32, device="cuda")
+        ctx.trace(bvh, "closest", rays=rays, hits=out)
+        st, bits = raw_sync(ctx)
+        assert st == ERR_DEVICE and bits == 0x8
+        got = out.cpu().numpy().view(np.uint32).reshape(-1, 3)
+        assert (got[:, 0] == NONE).all() and (got[:, 2] == 0).all()
+        info = bvh.info()
+        assert (info.wide_nodes, info.wide_levels) == (1, 1)
+        bvh.free()
+    ctx.close()
