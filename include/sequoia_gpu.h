@@ -426,15 +426,20 @@ sq_status sq_last_trace_stats(sq_ctx* ctx, uint64_t stats[4]);
  *   SQ_DEBUG_FAIL_ALLOC      device allocation number `limit` from now (0 =
  *                            the next one) fails as if the GPU were out of
  *                            memory; the call reports SQ_ERR_OOM.
+ *   SQ_DEBUG_FORCE           from now on, take the paths of `limit` (SQ_FORCE_*
+ *                            bits) that this device or size would not: the
+ *                            results are valid and the same.
  *   SQ_DEBUG_OFF             disarm all of them.
  * No injection faults or hangs the GPU: a wait that gives up returns, the
  * kernel finishes, and the context stays usable (the error word is reported
  * and cleared by the next sq_sync).  The results of the call that carried
- * the injection are not valid.                                               */
+ * the injection are not valid (SQ_DEBUG_FORCE aside).                        */
 #define SQ_DEBUG_OFF 0u
 #define SQ_DEBUG_STALL_LOOKBACK 1u
 #define SQ_DEBUG_STALL_BARRIER 2u
 #define SQ_DEBUG_FAIL_ALLOC 3u
+#define SQ_DEBUG_FORCE 4u
+#define SQ_FORCE_LEVEL_COLLAPSE 1u /* 8-wide collapse: a launch per level, as without cooperative launches */
 sq_status sq_debug_inject(sq_ctx* ctx, uint32_t what, uint32_t limit);
 /* Device memory the context holds in its caching allocator: out[0] / out[1]
  * = blocks / bytes held by live objects (BVHs, batches, buffers of a call in

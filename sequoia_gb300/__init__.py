@@ -427,7 +427,8 @@ class Context:
         return h_arr
 
     # failure-detection test hooks (sq_debug_inject / sq_debug_memory)
-    INJECT = {"off": 0, "stall_lookback": 1, "stall_barrier": 2, "fail_alloc": 3}
+    INJECT = {"off": 0, "stall_lookback": 1, "stall_barrier": 2, "fail_alloc": 3, "force": 4}
+    FORCE_LEVEL_COLLAPSE = 1
 
     def debug_inject(self, what, limit=0):
         self._check(load_library().sq_debug_inject(self.handle, self.INJECT[what], int(limit)))

@@ -354,7 +354,8 @@ sq_status build_wide(sq_ctx* c, sq_bvh* b)
     const bool stalled = c->stall_barrier != 0;
     c->stall_barrier = 0;
     const int rc = sqk::build_bvh8(b->nodes, b->root, b->leaf0, b->tris, n, b->nodes8, b->tris8, b->ws8, c->host_ctl,
-                                   c->ctrl, c->stream, b->meta8, stalled ? &stall : nullptr);
+                                   c->ctrl, c->stream, b->meta8, stalled ? &stall : nullptr,
+                                   (c->force & SQ_FORCE_LEVEL_COLLAPSE) != 0);
     if (rc != 0) return fail(c, SQ_ERR_CUDA, "8-wide collapse: %s", cudaGetErrorString((cudaError_t)rc));
     b->launches8 = c->host_ctl[4];
     if (!c->host_ctl[5]) {
@@ -1101,8 +1102,12 @@ sq_status sq_debug_inject(sq_ctx* c, uint32_t what, uint32_t limit)
     if (!c) return SQ_ERR_INVALID;
     switch (what) {
     case SQ_DEBUG_OFF:
-        c->stall_lookback = c->stall_barrier = 0;
+        c->stall_lookback = c->stall_barrier = c->force = 0;
         c->fail_alloc_in = -1;
+        return SQ_OK;
+    case SQ_DEBUG_FORCE:
+        if (limit & ~SQ_FORCE_LEVEL_COLLAPSE) return fail(c, SQ_ERR_INVALID, "sq_debug_inject: unknown path 0x%x", limit);
+        c->force = limit;
         return SQ_OK;
     case SQ_DEBUG_STALL_LOOKBACK:
     case SQ_DEBUG_STALL_BARRIER:

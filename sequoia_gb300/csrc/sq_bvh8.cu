@@ -444,17 +444,19 @@ __host__ __device__ inline CollapseWs collapse_ws(uint32_t* ws, uint32_t capacit
 // The work of one task group of level `level`: allocation from the head's
 // counters, open-record children to the next level's list.  Wide node r
 // (r < nroots) is the tree of record root + r; the other nodes follow.
+// next_count: the next level's task counter.
 template <class Published>
 __device__ __forceinline__ void collapse_task(const Node* __restrict__ rec, uint32_t leaf0,
                                               const float* __restrict__ tris, bool active, uint32_t rec_i,
-                                              uint32_t node_i, uint32_t level, uint32_t nroots, const CollapseWs& w,
+                                              uint32_t node_i, uint32_t level, uint32_t* next_count, uint32_t nroots,
+                                              const CollapseWs& w,
                                               Node8* __restrict__ nodes8, float4* __restrict__ tris8, uint32_t capacity,
                                               uint32_t* err, GroupSmem& sm, Published published)
 {
     uint32_t* head = w.head;
     uint32_t *next_rec = w.rec[(level + 1) & 1], *next_node = w.node[(level + 1) & 1];
     auto alloc = [&](uint32_t kn, uint32_t kt, uint32_t kj, uint32_t& nb, uint32_t& tb, uint32_t& jb) {
-        if (kj) jb = atomicAdd(head + kWsLevel + level + 1, kj);
+        if (kj) jb = atomicAdd(next_count, kj);
         alloc_nodes_tris(head + kWsNodes, kn, kt, nroots, capacity, err, nb, tb);
     };
     // (a node past the capacity is listed too: its task is counted, and the
@@ -469,8 +471,11 @@ __device__ __forceinline__ void collapse_task(const Node* __restrict__ rec, uint
 }
 
 // One level per launch (where a cooperative launch is not possible): group i
-// (four per warp) takes task i of the level's list.
+// (four per warp) takes task i of the level's list.  The task counts of four
+// levels take turns, so the depth has no limit here.
 constexpr int kCollapseBlock = 128;
+
+__device__ __forceinline__ uint32_t* level_slot(uint32_t* head, uint32_t level) { return head + kWsLevel + (level & 3u); }
 
 __global__ void __launch_bounds__(kCollapseBlock) k_collapse_level(
     const Node* __restrict__ rec, uint32_t leaf0, const float* __restrict__ tris, uint32_t root, uint32_t nroots,
@@ -485,17 +490,17 @@ __global__ void __launch_bounds__(kCollapseBlock) k_collapse_level(
     const uint32_t rec_i = !listed ? 0u : (level ? w.rec[level & 1][i] : root + i);
     const uint32_t node_i = !listed ? 0u : (level ? w.node[level & 1][i] : i);
     const bool active = listed && node_i < capacity;
-    collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
-                  s_group[threadIdx.x >> 5], [] {});
+    collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, level_slot(w.head, level + 1u), nroots, w, nodes8, tris8,
+                  capacity, err, s_group[threadIdx.x >> 5], [] {});
 }
 
 // After level `level`, before anything of the next one: a level that made
 // more nodes than tasks made cluster nodes, one level below its own.  Returns
 // the next level's tasks.  (Relaxed loads, so they are in flight together: the
 // caller has ordered them after the level's atomics.)
-__device__ __forceinline__ uint32_t collapse_level_end(uint32_t* head, uint32_t level)
+__device__ __forceinline__ uint32_t collapse_level_end(uint32_t* head, uint32_t level, const uint32_t* next_count)
 {
-    const uint32_t nodes = ld_relaxed_u32(head + kWsNodes), tasks = ld_relaxed_u32(head + kWsLevel + level + 1);
+    const uint32_t nodes = ld_relaxed_u32(head + kWsNodes), tasks = ld_relaxed_u32(next_count);
     const uint32_t before = ld_relaxed_u32(head + kWsBefore);
     if (nodes - before > tasks) st_relaxed_u32(head + kWsClusters, level + 2u);
     st_relaxed_u32(head + kWsBefore, nodes);
@@ -516,7 +521,11 @@ __device__ __forceinline__ void collapse_done(uint32_t* head, uint32_t levels, u
     }
 }
 
-__global__ void k_collapse_level_end(CollapseWs w, uint32_t level) { collapse_level_end(w.head, level); }
+__global__ void k_collapse_level_end(CollapseWs w, uint32_t level)
+{
+    collapse_level_end(w.head, level, level_slot(w.head, level + 1u));
+    *level_slot(w.head, level) = 0;
+}
 
 __global__ void k_collapse_done(CollapseWs w, uint32_t levels, uint32_t nroots, uint32_t capacity)
 {
@@ -619,9 +628,10 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
             if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(err, SQ_DEVERR_SAH_QUEUE);
             return;
         }
+        uint32_t* next_count = w.head + kWsLevel + level + 1u;
         auto arrive = [&] {
             barrier_arrive(w.head + kWsBarrier, (gridDim.x + barrier_extra) * (level + 1u), &s_warps,
-                           [&] { open_level(w.head, level + 1u, collapse_level_end(w.head, level)); });
+                           [&] { open_level(w.head, level + 1u, collapse_level_end(w.head, level, next_count)); });
         };
         if (4u * wid >= ntasks) arrive();
         for (uint32_t base = 4u * wid; base < ntasks; base += 4u * warps) {
@@ -631,8 +641,8 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
             const uint32_t node_i = !listed ? 0u : (level ? __ldcg(w.node[level & 1] + i) : i);
             const bool active = listed && node_i < capacity;
             const bool last = ntasks - base <= 4u * warps;
-            collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, nroots, w, nodes8, tris8, capacity, err,
-                          s_group[threadIdx.x >> 5], [&] { if (last) arrive(); });
+            collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, next_count, nroots, w, nodes8, tris8, capacity,
+                          err, s_group[threadIdx.x >> 5], [&] { if (last) arrive(); });
         }
         if (!barrier_wait(w.head, level + 1u, spin_limit, err, ntasks)) return;
         if (!ntasks && blockIdx.x == 0 && threadIdx.x == 0) collapse_done(w.head, level + 1, nroots, capacity, meta);
@@ -675,8 +685,9 @@ static cudaError_t launch_clusters(const Node* rec, uint32_t leaf0, const float*
 }
 
 // The collapse as one kernel launch per level of tasks (the host reads each
-// level's task count), where a cooperative launch does not fit.  The node
-// count is host_ctl[0] and the number of levels host_ctl[3].
+// level's task count), where a cooperative launch does not fit (by_level: the
+// tests ask for it).  The node count is host_ctl[0] and the number of levels
+// host_ctl[3].
 static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n,
                              void* nodes8, void* tris8, const CollapseWs& w, uint32_t* host_ctl, uint32_t* err,
                              cudaStream_t s)
@@ -684,12 +695,13 @@ static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, con
     const uint32_t capacity = bvh8_capacity(n) + 1u;
     cudaError_t e;
     uint32_t ntasks = 1, level = 0;
-    for (; ntasks && level + 1 < kMaxLevels; ++level) {
+    for (; ntasks; ++level) {
         k_collapse_level<<<(ntasks + 15) / 16, kCollapseBlock, 0, s>>>(rec, leaf0, tris, root, 1u, level, ntasks, w, capacity,
                                                                static_cast<Node8*>(nodes8), static_cast<float4*>(tris8),
                                                                err);
         k_collapse_level_end<<<1, 1, 0, s>>>(w, level);
-        if ((e = cudaMemcpyAsync(host_ctl, w.head + kWsLevel + level + 1, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+        if ((e = cudaMemcpyAsync(host_ctl, w.head + kWsLevel + ((level + 1u) & 3u), 4, cudaMemcpyDeviceToHost, s)) !=
+            cudaSuccess)
             return (int)e;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
         ntasks = std::min(host_ctl[0], capacity);
@@ -737,12 +749,12 @@ int build_bvh8_queue(const Node* rec, uint32_t root0, uint32_t nroots, uint32_t 
 
 int build_bvh8(const Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n, void* nodes8, void* tris8,
                uint32_t* ws, uint32_t* host_ctl, uint32_t* err, cudaStream_t s, uint32_t* meta,
-               const BarrierStall* stall)
+               const BarrierStall* stall, bool by_level)
 {
     host_ctl[5] = 0;
     cudaError_t e;
     if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * kWsHead, s)) != cudaSuccess) return (int)e;
-    const int per_sm = coop_blocks();
+    const int per_sm = by_level ? 0 : coop_blocks();
     if (per_sm == 0)
         return build_bvh8_levels(rec, root, leaf0, tris, n, nodes8, tris8, collapse_ws(ws, bvh8_capacity(n) + 1u),
                                  host_ctl, err, s);

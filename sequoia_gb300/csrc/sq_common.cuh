@@ -450,9 +450,10 @@ size_t bvh8_tri_bytes(uint32_t n);
 struct BarrierStall {
     uint32_t spin_limit;
 };
+// by_level: the collapse as where no cooperative launch is possible.
 int build_bvh8(const sq::Node* rec, uint32_t root, uint32_t leaf0, const float* tris, uint32_t n, void* nodes8,
                void* tris8, uint32_t* ws, uint32_t* host_ctl, uint32_t* err, cudaStream_t s, uint32_t* meta,
-               const BarrierStall* stall = nullptr);
+               const BarrierStall* stall = nullptr, bool by_level = false);
 void trace8(const Trace8Args& a, cudaStream_t s);
 
 // batched trace over many BVHs and ray tiles (sq_trace.cu, sq_bvh8_trace.cu)

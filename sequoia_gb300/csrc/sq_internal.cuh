@@ -25,6 +25,7 @@ struct sq_ctx {
     // else the wait's poll limit + 1; fail_alloc_in: allocations to let
     // through before one fails (-1 = off)
     uint32_t stall_lookback = 0, stall_barrier = 0;
+    uint32_t force = 0;  // SQ_FORCE_* paths (sq_debug_inject), until disarmed
     int64_t fail_alloc_in = -1;
     // banded camera traces into page-locked host memory (created on first
     // use): two streams the bands alternate on, so a band starts while the
