@@ -240,7 +240,8 @@ sq_status enqueue_run(sq_batch* b)
     const bool wide = b->params.wide != 0;
     if (wide) {
         const int rc = sqk::build_bvh8_queue(b->d_nodes, 3u * N + 2u, M, 2u * N + 2u, b->d_tris, N, b->d_nodes8,
-                                             b->d_tris8, b->d_ws8, c->ctrl, s);
+                                             b->d_tris8, b->d_ws8, c->ctrl, s,
+                                             (c->force & SQ_FORCE_LEVEL_COLLAPSE) != 0);
         if (rc) return fail(c, SQ_ERR_CUDA, "batch collapse: %s", cudaGetErrorString((cudaError_t)rc));
     }
     // trace

@@ -471,27 +471,29 @@ __device__ __forceinline__ void collapse_task(const Node* __restrict__ rec, uint
 }
 
 // One level per launch (where a cooperative launch is not possible): group i
-// (four per warp) takes task i of the level's list.  The task counts of four
-// levels take turns, so the depth has no limit here.
+// (four per warp) takes task i of the level's list and so on in strides of the
+// grid.  The task counts of four levels take turns, so the depth has no limit
+// here.
 constexpr int kCollapseBlock = 128;
 
 __device__ __forceinline__ uint32_t* level_slot(uint32_t* head, uint32_t level) { return head + kWsLevel + (level & 3u); }
 
 __global__ void __launch_bounds__(kCollapseBlock) k_collapse_level(
     const Node* __restrict__ rec, uint32_t leaf0, const float* __restrict__ tris, uint32_t root, uint32_t nroots,
-    uint32_t level, uint32_t ntasks, CollapseWs w, uint32_t capacity, Node8* __restrict__ nodes8,
-    float4* __restrict__ tris8, uint32_t* err)
+    uint32_t level, CollapseWs w, uint32_t capacity, Node8* __restrict__ nodes8, float4* __restrict__ tris8, uint32_t* err)
 {
     __shared__ GroupSmem s_group[kCollapseBlock / 32];
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (4u * warp >= ntasks) return;  // whole warps
-    const uint32_t i = 4u * warp + ((threadIdx.x & 31u) >> 3);
-    const bool listed = i < ntasks;
-    const uint32_t rec_i = !listed ? 0u : (level ? w.rec[level & 1][i] : root + i);
-    const uint32_t node_i = !listed ? 0u : (level ? w.node[level & 1][i] : i);
-    const bool active = listed && node_i < capacity;
-    collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, level_slot(w.head, level + 1u), nroots, w, nodes8, tris8,
-                  capacity, err, s_group[threadIdx.x >> 5], [] {});
+    const uint32_t ntasks = level ? min(*level_slot(w.head, level), capacity) : nroots;
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t base = 4u * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); base < ntasks; base += 4u * warps) {
+        const uint32_t i = base + ((threadIdx.x & 31u) >> 3);
+        const bool listed = i < ntasks;
+        const uint32_t rec_i = !listed ? 0u : (level ? w.rec[level & 1][i] : root + i);
+        const uint32_t node_i = !listed ? 0u : (level ? w.node[level & 1][i] : i);
+        const bool active = listed && node_i < capacity;
+        collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, level_slot(w.head, level + 1u), nroots, w, nodes8,
+                      tris8, capacity, err, s_group[threadIdx.x >> 5], [] {});
+    }
 }
 
 // After level `level`, before anything of the next one: a level that made
@@ -527,9 +529,12 @@ __global__ void k_collapse_level_end(CollapseWs w, uint32_t level)
     *level_slot(w.head, level) = 0;
 }
 
-__global__ void k_collapse_done(CollapseWs w, uint32_t levels, uint32_t nroots, uint32_t capacity)
+// (tasks left after the last level that was launched: no count, so the trees
+// are empty)
+__global__ void k_collapse_done(CollapseWs w, uint32_t levels, uint32_t nroots, uint32_t capacity, uint32_t* err)
 {
-    collapse_done(w.head, levels, nroots, capacity, nullptr);
+    if (*level_slot(w.head, levels)) raise_error(err, SQ_DEVERR_SAH_QUEUE);
+    else collapse_done(w.head, levels, nroots, capacity, nullptr);
 }
 
 // All levels in one cooperative launch (every block is resident): a
@@ -696,7 +701,7 @@ static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, con
     cudaError_t e;
     uint32_t ntasks = 1, level = 0;
     for (; ntasks; ++level) {
-        k_collapse_level<<<(ntasks + 15) / 16, kCollapseBlock, 0, s>>>(rec, leaf0, tris, root, 1u, level, ntasks, w, capacity,
+        k_collapse_level<<<(ntasks + 15) / 16, kCollapseBlock, 0, s>>>(rec, leaf0, tris, root, 1u, level, w, capacity,
                                                                static_cast<Node8*>(nodes8), static_cast<float4*>(tris8),
                                                                err);
         k_collapse_level_end<<<1, 1, 0, s>>>(w, level);
@@ -706,7 +711,7 @@ static int build_bvh8_levels(const Node* rec, uint32_t root, uint32_t leaf0, con
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return (int)e;
         ntasks = std::min(host_ctl[0], capacity);
     }
-    k_collapse_done<<<1, 1, 0, s>>>(w, level, 1u, capacity);
+    k_collapse_done<<<1, 1, 0, s>>>(w, level, 1u, capacity, err);
     if ((e = launch_clusters(rec, leaf0, tris, n, w, 1u, nullptr, nodes8, tris8, s)) != cudaSuccess) return (int)e;
     uint32_t m[2];
     if ((e = cudaMemcpyAsync(m, w.head + kWsCount, sizeof m, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return (int)e;
@@ -738,12 +743,27 @@ static cudaError_t enqueue_collapse(const Node* rec, uint32_t root, uint32_t nro
 }
 
 int build_bvh8_queue(const Node* rec, uint32_t root0, uint32_t nroots, uint32_t leaf0, const float* tris, uint32_t n,
-                     void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s)
+                     void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s, bool by_level)
 {
-    const int per_sm = coop_blocks();
-    if (per_sm == 0) return (int)cudaErrorCooperativeLaunchTooLarge;
+    const int per_sm = by_level ? 0 : coop_blocks();
     cudaError_t e;
     if ((e = cudaMemsetAsync(ws, 0, sizeof(uint32_t) * kWsHead, s)) != cudaSuccess) return (int)e;
+    if (per_sm == 0) {
+        // a fixed number of levels, as many as the cooperative kernel takes:
+        // a level without tasks returns at once
+        static PerDevice<int> cache;
+        const int grid = cache.get([] { return blocks_per_sm(k_collapse_level, kCollapseBlock) * sm_count(); });
+        const uint32_t capacity = bvh8_capacity(n) + nroots;
+        const CollapseWs w = collapse_ws(ws, capacity);
+        for (uint32_t level = 0; level + 1 < kMaxLevels; ++level) {
+            k_collapse_level<<<grid, kCollapseBlock, 0, s>>>(rec, leaf0, tris, root0, nroots, level, w, capacity,
+                                                             static_cast<Node8*>(nodes8), static_cast<float4*>(tris8),
+                                                             err);
+            k_collapse_level_end<<<1, 1, 0, s>>>(w, level);
+        }
+        k_collapse_done<<<1, 1, 0, s>>>(w, kMaxLevels - 1, nroots, capacity, err);
+        return (int)launch_clusters(rec, leaf0, tris, n, w, nroots, nullptr, nodes8, tris8, s);
+    }
     return (int)enqueue_collapse(rec, root0, nroots, leaf0, tris, n, nodes8, tris8, ws, nullptr, err, per_sm, nullptr, s);
 }
 

@@ -496,7 +496,8 @@ void trace8_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);
 // be captured in a CUDA graph.  ws: bvh8_ws_words(n, nroots) words.  Wide node
 // k (k < nroots) is the tree of record root0 + k.
 int build_bvh8_queue(const sq::Node* rec, uint32_t root0, uint32_t nroots, uint32_t leaf0, const float* tris,
-                     uint32_t n, void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s);
+                     uint32_t n, void* nodes8, void* tris8, uint32_t* ws, uint32_t* err, cudaStream_t s,
+                     bool by_level = false);
 
 }  // namespace sqk
 

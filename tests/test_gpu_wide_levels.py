@@ -1,6 +1,6 @@
 """The 8-wide collapse as one launch per level, the path of a device without
-cooperative launches: the same tree as the cooperative kernel's (node and
-level counts, hits, distances, box tests)."""
+cooperative launches: the same trees as the cooperative kernel's (node and
+level counts, hits, distances, box tests), in single builds and batches."""
 import numpy as np
 import pytest
 
@@ -52,3 +52,25 @@ def test_unknown_path_is_refused(lctx):
     with pytest.raises(sq.SequoiaError) as e:
         lctx.debug_inject("force", 1 << 30)
     assert e.value.status == 1
+
+
+@pytest.mark.parametrize("builder", ["morton", "sah"])
+@pytest.mark.parametrize("graph", [False, True])
+def test_batch(lctx, builder, graph):
+    from sequoia_gb300 import scenes
+    from test_gpu_batch import separate
+    meshes = []
+    for j, n in enumerate([0, 1, 7, 40_000, 300, 0, 2500] + list(range(1, 30))):
+        tris = scenes.gaussian_soup(n, 1, seed=600 + j) if n else np.zeros((0, 9), np.float32)
+        lo, hi = scenes.scene_box(tris) if n else (np.zeros(3, np.float32), np.ones(3, np.float32))
+        meshes.append(dict(tris=tris, rays=scenes.random_rays(60 + j, lo, hi, seed=j)))
+    want = separate(lctx, meshes, "closest", True, builder)
+    lctx.debug_inject("force", lctx.FORCE_LEVEL_COLLAPSE)
+    b = lctx.batch(meshes, mode="closest", wide=True, builder=builder, graph=graph)
+    for _ in range(2):
+        got, _ = b.run()
+        for key in ("id", "t", "tests"):
+            assert np.array_equal(got[key], want[key]), key
+    lctx.debug_inject("off")
+    assert lctx.sync() == 0
+    b.free()
