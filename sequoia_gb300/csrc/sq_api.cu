@@ -797,6 +797,7 @@ sq_status sq_trace(sq_ctx* c, const sq_bvh* b, const sq_ray_source* rays, uint32
     a.refill = sched_refill ? 1u : 0u;  // the binary tree: 32-ray batches per warp unless asked
     a.heat_ramp = heat_ramp ? 1u : 0u;
     a.root_group = 1u;
+    a.wide_entries = (c->force & SQ_FORCE_WIDE_ENTRIES) ? 1u : 0u;
     uint64_t count = 0;
     float* rays_own = nullptr;
     if (rays->kind == SQ_RAYS_REFERENCE_CAMERA || rays->kind == SQ_RAYS_PINHOLE) {
@@ -1078,6 +1079,7 @@ sq_status sq_trace_batches(sq_ctx* c, const sq_bvh* b, const sq_ray_source* batc
     // per-lane refill by default when most rays are explicit (incoherent)
     a.refill = sched_refill ? 1u : (sched_tiles ? 0u : (2ull * xrays > rays ? 1u : 0u));
     a.heat_ramp = heat_ramp;
+    a.wide_entries = (c->force & SQ_FORCE_WIDE_ENTRIES) ? 1u : 0u;
     if ((e = cudaMemsetAsync(c->ctrl + 1, 0, 11 * sizeof(uint32_t), s)) != cudaSuccess) return cuda_fail(e, "reset");
     if ((e = cudaEventRecord(c->ev[4], s)) != cudaSuccess) return cuda_fail(e, "event");
     if (rays) {
@@ -1106,7 +1108,8 @@ sq_status sq_debug_inject(sq_ctx* c, uint32_t what, uint32_t limit)
         c->fail_alloc_in = -1;
         return SQ_OK;
     case SQ_DEBUG_FORCE:
-        if (limit & ~SQ_FORCE_LEVEL_COLLAPSE) return fail(c, SQ_ERR_INVALID, "sq_debug_inject: unknown path 0x%x", limit);
+        if (limit & ~(SQ_FORCE_LEVEL_COLLAPSE | SQ_FORCE_WIDE_ENTRIES))
+            return fail(c, SQ_ERR_INVALID, "sq_debug_inject: unknown path 0x%x", limit);
         c->force = limit;
         return SQ_OK;
     case SQ_DEBUG_STALL_LOOKBACK:

@@ -408,6 +408,7 @@ struct TraceArgs {
     uint32_t refill;      // closest / any-hit: 1 = per-lane ray refill, 0 = 32-ray batches per warp
     uint32_t heat_ramp;   // heatmap pixels: 0 = grey, 1 = the reference's colour ramp (write_heat)
     uint32_t root_group;  // REF mode: start from the node group [root, root + root_group) (1 = the root)
+    uint32_t wide_entries;  // refill: 16-byte stack entries whatever the tree's size (else by the size)
 };
 void trace(const TraceArgs& a, cudaStream_t s);
 // packet / bundle tracers of the reference (sq_coherent.cu): heatmap only
@@ -488,6 +489,7 @@ struct BatchTraceArgs {
     unsigned long long* stats;
     uint32_t refill;       // 8-wide kernel: 1 = per-lane ray refill (see sq_bvh8_trace.cu)
     uint32_t heat_ramp;    // heatmap pixels: 0 = grey, 1 = colour ramp (write_heat)
+    uint32_t wide_entries;  // binary refill: as TraceArgs
 };
 void trace_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);
 void trace8_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);

@@ -1010,7 +1010,7 @@ namespace sqk {
 void trace_batch(const BatchTraceArgs& a, int block, cudaStream_t s)
 {
     if (block != 64 && block != 128 && block != 256) block = 128;
-    const bool narrow = narrow_tree(a.node_count, a.tri_count);
+    const bool narrow = !a.wide_entries && narrow_tree(a.node_count, a.tri_count);
     if (a.mode == SQ_TRACE_REF) launch_batch<SQ_TRACE_REF, false>(a, block, s);
     else if (a.mode == SQ_TRACE_CLOSEST)
         narrow ? launch_batch<SQ_TRACE_CLOSEST, false>(a, block, s) : launch_batch<SQ_TRACE_CLOSEST, true>(a, block, s);
@@ -1019,7 +1019,7 @@ void trace_batch(const BatchTraceArgs& a, int block, cudaStream_t s)
 
 void trace(const TraceArgs& a, cudaStream_t s)
 {
-    const bool narrow = narrow_tree(a.node_count, a.tri_count);
+    const bool narrow = !a.wide_entries && narrow_tree(a.node_count, a.tri_count);
     if (a.mode == SQ_TRACE_REF) launch<SQ_TRACE_REF, false>(a, s);
     else if (a.mode == SQ_TRACE_CLOSEST)
         narrow ? launch<SQ_TRACE_CLOSEST, false>(a, s) : launch<SQ_TRACE_CLOSEST, true>(a, s);
