@@ -423,6 +423,8 @@ sq_status sq_last_trace_stats(sq_ctx* ctx, uint64_t stats[4]);
  *                            for one block more than the grid: every block
  *                            gives up after `limit` polls and raises
  *                            SQ_DEVERR_SAH_QUEUE.
+ *   SQ_DEBUG_STALL_BARRIER_TIME  as SQ_DEBUG_STALL_BARRIER, but the blocks give
+ *                            up when a real wait would: after half a second.
  *   SQ_DEBUG_FAIL_ALLOC      device allocation number `limit` from now (0 =
  *                            the next one) fails as if the GPU were out of
  *                            memory; the call reports SQ_ERR_OOM.
@@ -439,6 +441,7 @@ sq_status sq_last_trace_stats(sq_ctx* ctx, uint64_t stats[4]);
 #define SQ_DEBUG_STALL_BARRIER 2u
 #define SQ_DEBUG_FAIL_ALLOC 3u
 #define SQ_DEBUG_FORCE 4u
+#define SQ_DEBUG_STALL_BARRIER_TIME 5u
 #define SQ_FORCE_LEVEL_COLLAPSE 1u /* 8-wide collapse: a launch per level, as without cooperative launches */
 #define SQ_FORCE_WIDE_ENTRIES 2u   /* binary refill: the 16-byte stack entries of trees above 2^27 records */
 sq_status sq_debug_inject(sq_ctx* ctx, uint32_t what, uint32_t limit);

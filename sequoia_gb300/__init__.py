@@ -427,7 +427,8 @@ class Context:
         return h_arr
 
     # failure-detection test hooks (sq_debug_inject / sq_debug_memory)
-    INJECT = {"off": 0, "stall_lookback": 1, "stall_barrier": 2, "fail_alloc": 3, "force": 4}
+    INJECT = {"off": 0, "stall_lookback": 1, "stall_barrier": 2, "fail_alloc": 3, "force": 4,
+              "stall_barrier_time": 5}
     FORCE_LEVEL_COLLAPSE, FORCE_WIDE_ENTRIES = 1, 2
 
     def debug_inject(self, what, limit=0):

@@ -1107,6 +1107,9 @@ sq_status sq_debug_inject(sq_ctx* c, uint32_t what, uint32_t limit)
         c->stall_lookback = c->stall_barrier = c->force = 0;
         c->fail_alloc_in = -1;
         return SQ_OK;
+    case SQ_DEBUG_STALL_BARRIER_TIME:
+        c->stall_barrier = 1u;
+        return SQ_OK;
     case SQ_DEBUG_FORCE:
         if (limit & ~(SQ_FORCE_LEVEL_COLLAPSE | SQ_FORCE_WIDE_ENTRIES))
             return fail(c, SQ_ERR_INVALID, "sq_debug_inject: unknown path 0x%x", limit);

@@ -540,14 +540,24 @@ __global__ void k_collapse_done(CollapseWs w, uint32_t levels, uint32_t nroots, 
 // All levels in one cooperative launch (every block is resident): a
 // grid-stride loop over a level's tasks, a grid barrier, the next level.  No
 // host round trip per level, and a CUDA graph can hold it.  The barrier's
-// wait is bounded: a block that polls more than kBarrierSpins times raises
-// SQ_DEVERR_SAH_QUEUE and returns (the other blocks then time out at their
-// next barrier too).  Task lists are read through L2 (__ldcg): the same lists
-// are rewritten every other level, so an SM's L1 may hold stale lines of
-// them.  The failure-detection tests pass a small poll limit and one phantom
-// block (barrier_extra = 1) that never arrives: every block then gives up at
-// the first barrier.
-constexpr uint32_t kBarrierSpins = 1u << 24;
+// wait is bounded (barrier_wait): a block that gives up raises
+// SQ_DEVERR_SAH_QUEUE and returns (the other blocks then give up at their next
+// barrier too).  Task lists are read through L2 (__ldcg): the same lists are
+// rewritten every other level, so an SM's L1 may hold stale lines of them.
+// The failure-detection tests pass one phantom block (barrier_extra = 1) that
+// never arrives: every block then gives up at the first barrier.
+//
+// The bound is half a second of polling, which no level of 2^27 triangles comes
+// near (8 million take less than a millisecond in all); polls alone are not
+// counted, since how long one takes depends on what else the GPU does (2^24 of
+// them, at a sleep and an L2 round trip each, are ten seconds or more).  A poll
+// adds at most 0.1 ms, so the time that the kernel is not on the GPU at all
+// does not count.
+struct BarrierLimit {
+    uint32_t polls, ns;  // polls before the time starts, and the time
+};
+constexpr BarrierLimit kBarrierLimit = {1u << 10, 500000000u};
+constexpr uint32_t kBarrierPollNs = 100000u;
 
 // Grid barrier of a level in two halves.  barrier_arrive: every warp calls it
 // once, when its writes before the barrier are done; the block's last warp
@@ -582,20 +592,33 @@ __device__ __forceinline__ void open_level(uint32_t* head, uint32_t level, uint3
                  : "memory");
 }
 
-__device__ __forceinline__ bool barrier_wait(const uint32_t* head, uint32_t level, uint32_t spin_limit, uint32_t* err,
+// Low word of the GPU's nanosecond clock (differences of up to four seconds).
+__device__ __forceinline__ uint32_t global_ns()
+{
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+    return t;
+}
+
+__device__ __forceinline__ bool barrier_wait(const uint32_t* head, uint32_t level, BarrierLimit limit, uint32_t* err,
                                              uint32_t& tasks)
 {
     __shared__ uint32_t s_ok, s_tasks;
     if (threadIdx.x == 0) {
-        uint32_t ok = 1, spins = 0;
+        uint32_t ok = 1, polls = 0, waited = 0, last = 0;
         unsigned long long v;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(head + kWsOpen) : "memory");
             if ((uint32_t)(v >> 32) == level) break;
-            if (++spins > spin_limit) {
-                raise_error(err, SQ_DEVERR_SAH_QUEUE);
-                ok = 0;
-                break;
+            if (++polls > limit.polls) {
+                const uint32_t now = global_ns();
+                if (polls > limit.polls + 1u) waited += min(now - last, kBarrierPollNs);
+                last = now;
+                if (waited >= limit.ns) {
+                    raise_error(err, SQ_DEVERR_SAH_QUEUE);
+                    ok = 0;
+                    break;
+                }
             }
             __nanosleep(32);
         }
@@ -617,7 +640,7 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
                                                        const float* __restrict__ tris, uint32_t root, uint32_t nroots,
                                                        CollapseWs w, uint32_t capacity, Node8* __restrict__ nodes8,
                                                        float4* __restrict__ tris8, uint32_t* meta, uint32_t* err,
-                                                       uint32_t barrier_extra, uint32_t spin_limit)
+                                                       uint32_t barrier_extra, BarrierLimit limit)
 {
     __shared__ GroupSmem s_group[8];
     __shared__ uint32_t s_warps;
@@ -649,7 +672,7 @@ __global__ void __launch_bounds__(256) k_collapse_coop(const Node* __restrict__ 
             collapse_task(rec, leaf0, tris, active, rec_i, node_i, level, next_count, nroots, w, nodes8, tris8, capacity,
                           err, s_group[threadIdx.x >> 5], [&] { if (last) arrive(); });
         }
-        if (!barrier_wait(w.head, level + 1u, spin_limit, err, ntasks)) return;
+        if (!barrier_wait(w.head, level + 1u, limit, err, ntasks)) return;
         if (!ntasks && blockIdx.x == 0 && threadIdx.x == 0) collapse_done(w.head, level + 1, nroots, capacity, meta);
     }
 }
@@ -733,9 +756,9 @@ static cudaError_t enqueue_collapse(const Node* rec, uint32_t root, uint32_t nro
     uint32_t capacity = bvh8_capacity(n) + nroots;
     CollapseWs w = collapse_ws(ws, capacity);
     const uint32_t extra = stall ? 1u : 0u;
-    const uint32_t spins = stall ? stall->spin_limit : kBarrierSpins;
+    const BarrierLimit limit = stall && stall->spin_limit ? BarrierLimit{stall->spin_limit, 0u} : kBarrierLimit;
     void* args[] = {(void*)&rec, (void*)&leaf0, (void*)&tris, (void*)&root, (void*)&nroots, (void*)&w, (void*)&capacity,
-                    (void*)&nodes8, (void*)&tris8, (void*)&meta, (void*)&err, (void*)&extra, (void*)&spins};
+                    (void*)&nodes8, (void*)&tris8, (void*)&meta, (void*)&err, (void*)&extra, (void*)&limit};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_collapse_coop, dim3(per_sm * sm_count()), dim3(256),
                                                       args, 0, s);
     if (e != cudaSuccess) return e;

@@ -447,7 +447,8 @@ size_t bvh8_tri_bytes(uint32_t n);
 // host_ctl[4]: kernel launches.
 // Fault injection for the failure-detection tests: the cooperative
 // collapse's grid barrier waits for one block more than the grid, so every
-// block gives up after spin_limit polls (SQ_DEVERR_SAH_QUEUE) and returns.
+// block gives up after spin_limit polls (0: when a real wait would) and
+// returns (SQ_DEVERR_SAH_QUEUE).
 struct BarrierStall {
     uint32_t spin_limit;
 };
