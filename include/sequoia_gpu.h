@@ -444,6 +444,7 @@ sq_status sq_last_trace_stats(sq_ctx* ctx, uint64_t stats[4]);
 #define SQ_DEBUG_STALL_BARRIER_TIME 5u
 #define SQ_FORCE_LEVEL_COLLAPSE 1u /* 8-wide collapse: a launch per level, as without cooperative launches */
 #define SQ_FORCE_WIDE_ENTRIES 2u   /* binary refill: the 16-byte stack entries of trees above 2^27 records */
+#define SQ_FORCE_SMALL_TOTALS 4u   /* 8-wide refill: lanes hand their statistics on at 64 tests, not 2^28 */
 sq_status sq_debug_inject(sq_ctx* ctx, uint32_t what, uint32_t limit);
 /* Device memory the context holds in its caching allocator: out[0] / out[1]
  * = blocks / bytes held by live objects (BVHs, batches, buffers of a call in

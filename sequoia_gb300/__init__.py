@@ -429,7 +429,7 @@ class Context:
     # failure-detection test hooks (sq_debug_inject / sq_debug_memory)
     INJECT = {"off": 0, "stall_lookback": 1, "stall_barrier": 2, "fail_alloc": 3, "force": 4,
               "stall_barrier_time": 5}
-    FORCE_LEVEL_COLLAPSE, FORCE_WIDE_ENTRIES = 1, 2
+    FORCE_LEVEL_COLLAPSE, FORCE_WIDE_ENTRIES, FORCE_SMALL_TOTALS = 1, 2, 4
 
     def debug_inject(self, what, limit=0):
         self._check(load_library().sq_debug_inject(self.handle, self.INJECT[what], int(limit)))

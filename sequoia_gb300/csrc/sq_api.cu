@@ -876,6 +876,7 @@ sq_status sq_trace(sq_ctx* c, const sq_bvh* b, const sq_ray_source* rays, uint32
             w.err = a.err;
             w.stats = a.stats;
             w.heat_ramp = a.heat_ramp;
+            w.totals_limit = (c->force & SQ_FORCE_SMALL_TOTALS) ? 64u : sqk::kTotalsLimit;
             // default: explicit rays refill lanes; camera rays keep coherent
             // 8x4 tiles per warp
             w.refill = sched_refill ? 1u : (sched_tiles ? 0u : (a.ray_kind == SQ_RAYS_EXPLICIT ? 1u : 0u));
@@ -1079,6 +1080,7 @@ sq_status sq_trace_batches(sq_ctx* c, const sq_bvh* b, const sq_ray_source* batc
     // per-lane refill by default when most rays are explicit (incoherent)
     a.refill = sched_refill ? 1u : (sched_tiles ? 0u : (2ull * xrays > rays ? 1u : 0u));
     a.heat_ramp = heat_ramp;
+    a.totals_limit = (c->force & SQ_FORCE_SMALL_TOTALS) ? 64u : sqk::kTotalsLimit;
     a.wide_entries = (c->force & SQ_FORCE_WIDE_ENTRIES) ? 1u : 0u;
     if ((e = cudaMemsetAsync(c->ctrl + 1, 0, 11 * sizeof(uint32_t), s)) != cudaSuccess) return cuda_fail(e, "reset");
     if ((e = cudaEventRecord(c->ev[4], s)) != cudaSuccess) return cuda_fail(e, "event");
@@ -1111,7 +1113,7 @@ sq_status sq_debug_inject(sq_ctx* c, uint32_t what, uint32_t limit)
         c->stall_barrier = 1u;
         return SQ_OK;
     case SQ_DEBUG_FORCE:
-        if (limit & ~(SQ_FORCE_LEVEL_COLLAPSE | SQ_FORCE_WIDE_ENTRIES))
+        if (limit & ~(SQ_FORCE_LEVEL_COLLAPSE | SQ_FORCE_WIDE_ENTRIES | SQ_FORCE_SMALL_TOTALS))
             return fail(c, SQ_ERR_INVALID, "sq_debug_inject: unknown path 0x%x", limit);
         c->force = limit;
         return SQ_OK;

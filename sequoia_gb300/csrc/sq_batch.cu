@@ -267,6 +267,7 @@ sq_status enqueue_run(sq_batch* b)
     // per-lane ray refill when most rays are explicit (incoherent); camera
     // tiles keep whole 32-ray batches per warp
     a.refill = 2ull * b->explicit_rays > (uint64_t)b->rays ? 1u : 0u;
+    a.totals_limit = (c->force & SQ_FORCE_SMALL_TOTALS) ? 64u : sqk::kTotalsLimit;
     a.wide_entries = (c->force & SQ_FORCE_WIDE_ENTRIES) ? 1u : 0u;
     const int block = b->params.block_threads ? (int)b->params.block_threads : 128;
     if (wide && a.mode != SQ_TRACE_REF) sqk::trace8_batch(a, block, s);

@@ -524,8 +524,10 @@ __device__ Res8 trace8(const Node8* __restrict__ nodes, uint32_t root, const flo
 // Both visit children in the same order (ascending entry distance, then
 // slot), so they count the same box tests for the same ray.
 
-// Totals of a lane over all its rays (32 bits are hours of them); the rays
-// themselves only carry their box tests.
+// Totals of a lane over its rays; the rays themselves only carry their box
+// tests.  32 bits are ten minutes or so of one launch, so a lane adds what it
+// has to the statistics long before (spill_totals) and starts again: 64-bit
+// sums would cost the refill kernels their occupancy step.
 struct Totals8 {
     uint32_t tests = 0, tris = 0, nodes = 0, rays = 0, explicit_rays = 0;
 };
@@ -564,6 +566,23 @@ __device__ __forceinline__ void add_totals(const Totals8& sum, uint32_t out, uns
         for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xFFFFFFFFu, v[k], o);
         if ((threadIdx.x & 31u) == 0) atomicAdd(stats + k, v[k]);
     }
+}
+
+// The same for one lane, once its box tests have reached `limit`.  (A slot that
+// was tested leads to at most 15 triangles and one node, so at kTotalsLimit
+// tests neither of those sums is full.)
+__device__ __forceinline__ void spill_totals(Totals8& sum, uint32_t limit, uint32_t explicit_rays, uint32_t out,
+                                             unsigned long long* stats)
+{
+    if (sum.tests < limit) return;
+    if (stats) {
+        atomicAdd(stats, (unsigned long long)sum.tests);
+        atomicAdd(stats + 1, (unsigned long long)sum.tris);
+        atomicAdd(stats + 2, 32ull * explicit_rays + (unsigned long long)out * sum.rays + 80ull * sum.nodes +
+                                 48ull * sum.tris);
+        atomicAdd(stats + 3, (unsigned long long)sum.nodes);
+    }
+    sum = Totals8{};
 }
 
 // Test a leaf entry's triangles; returns true when an any-hit ray is done.
@@ -815,6 +834,7 @@ __global__ void __launch_bounds__(128, PER_SM) k_trace8_refill(const sqk::Trace8
                 if (L.overflow) raise_error(a.err, SQ_DEVERR_STACK_OVERFLOW);
                 sum.tests += L.tests;
                 sum.rays++;
+                spill_totals(sum, a.totals_limit, camera ? 0u : sum.rays, (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u), a.stats);
                 if (a.hits) {
                     uint32_t* h = reinterpret_cast<uint32_t*>(a.hits) + 3ull * rid;
                     h[0] = L.best;
@@ -1014,6 +1034,7 @@ __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(cons
                 sum.tests += L.tests;
                 sum.rays++;
                 sum.explicit_rays += explicit_rays ? 1u : 0u;
+                spill_totals(sum, a.totals_limit, sum.explicit_rays, (a.hits ? 12u : 0u) + (a.heat ? 3u : 0u), a.stats);
                 const uint32_t id = L.best == kNoHit ? kNoHit : L.best - tri_offset;
                 if (a.hits) {
                     uint32_t* h = reinterpret_cast<uint32_t*>(a.hits) + 3ull * out;

@@ -433,7 +433,9 @@ struct Trace8Args {
     // camera rays, tiles schedule: only tiles [tile0, tile_end) of the image
     // (tile_end 0: to the last tile), so an image can be traced in row bands
     uint32_t tile0, tile_end;
+    uint32_t totals_limit;  // refill: box tests at which a lane adds its 32-bit totals to `stats`
 };
+constexpr uint32_t kTotalsLimit = 1u << 28;
 // Triangles an 8-wide BVH can address: a traversal stack entry holds the
 // first triangle of a leaf range in 27 bits (and its count in 4).
 constexpr uint32_t kWide8MaxTris = 1u << 27;
@@ -491,6 +493,7 @@ struct BatchTraceArgs {
     uint32_t refill;       // 8-wide kernel: 1 = per-lane ray refill (see sq_bvh8_trace.cu)
     uint32_t heat_ramp;    // heatmap pixels: 0 = grey, 1 = colour ramp (write_heat)
     uint32_t wide_entries;  // binary refill: as TraceArgs
+    uint32_t totals_limit;  // 8-wide refill: as Trace8Args
 };
 void trace_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);
 void trace8_batch(const BatchTraceArgs& a, int block_threads, cudaStream_t s);
