@@ -5,7 +5,7 @@
 // row order) traverse together: a node's children are visited when any ray
 // of the packet hits the node's box, and the packet counts one test per node
 // box.  Every pixel of the packet gets (tests / k) / 200 in the heatmap.  On
-// the GPU a warp walks 4 packets from one pool (sq_walk_dev.cuh): a lane
+// the GPU a warp walks 4 to 32 packets from one pool (sq_walk_dev.cuh): a lane
 // tests a node against the rays of the packet that visits it.
 //
 // trace_bundle<k> (src/tracer.cpp:292-362, traverse_bundle 126-156,
@@ -26,34 +26,52 @@
 #include "sq_walk_dev.cuh"
 
 #include <algorithm>
+#include <array>
 
 namespace {
 
 using namespace sq;
 
-// Packets of one warp's pool (sq_walk_dev.cuh): enough that the pool holds a
-// range for every lane most of the time, few enough that an image still
-// makes several rounds of warps.
-constexpr int kPoolPackets = 4;
+// Packets of one warp's pool (sq_walk_dev.cuh).  Four are enough that the pool
+// holds a range for every lane most of the time and few enough that the warps
+// of a small image or a deep tree end together; an image of many packets in a
+// small tree wants 32, since a packet is then soon done and fetching it, its
+// rays and the pool's start are what costs.  So above kFewPackets packets a
+// resident warp, each takes a share of what is left, from 32 down to 4
+// packets; the larger the tree (the longer the packets), the smaller the share
+// (packet_share).  1920x1072, packets of 1 / 2 / 4 / 8 rays, us with four each
+// time and with shares:
+//   200 triangles     355 / 199 / 116 /  80     79 /  59 /  56 /  56
+//   1,500             361 / 202 / 118 /  86     86 /  75 /  80 /  76
+//   30,000            373 / 212 / 134 / 127    138 / 110 / 104 / 120
+//   2M                581 / 412 / 387 / 540    490 / 395 / 376 / 554
+// Packets of 8 in trees from kLargeTree triangles on stay at four (2M at
+// 3840x2160: 929 us, with shares 1,054).
+constexpr int kPoolPackets = 4, kManyPackets = 32;
+constexpr uint32_t kFewPackets = 16;
+constexpr uint32_t kSmallTree = 4096, kMediumTree = 1u << 17, kLargeTree = 1u << 20;
+uint32_t packet_share(uint32_t tris) { return tris < kSmallTree ? 4u : (tris < kMediumTree ? 8u : 16u); }
 
-template <int K>
-__global__ void __launch_bounds__(32) k_trace_packet(const sqk::TraceArgs a)
+// share: a warp takes 1 / share of the packets left, kPoolPackets to PW of them
+template <int K, int PW>
+__global__ void __launch_bounds__(32) k_trace_packet(const sqk::TraceArgs a, uint32_t share)
 {
     constexpr int KX = (K == 1 || K == 2) ? 1 : 2;  // floor(sqrt(k))
     constexpr int KY = K / KX;
-    constexpr int PW = kPoolPackets;
     __shared__ WalkPool<K, PW, false> pool;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t bw = a.width / KX;
     const uint32_t total = bw * (a.height / KY);
     const float org[3] = {a.cam[0], a.cam[1], a.cam[2]};
     uint64_t tests_sum = 0;
+    uint32_t base = 0;
     for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(a.work, (uint32_t)PW);
+        const uint32_t take = PW == kPoolPackets ? (uint32_t)PW
+                                                 : min(max((total - base) / share, (uint32_t)kPoolPackets), (uint32_t)PW);
+        if (lane == 0) base = atomicAdd(a.work, take);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
         if (base >= total) break;
-        const uint32_t count = min((uint32_t)PW, total - base);
+        const uint32_t count = min(take, total - base);
         // ray m of packet p: pixel (m % KX, m / KX) of the packet's block
         for (uint32_t j = lane; j < count * K; j += 32) {
             const uint32_t p = j / K, m = j % K, pk = base + p;
@@ -84,11 +102,20 @@ __global__ void __launch_bounds__(32) k_trace_packet(const sqk::TraceArgs a)
 template <int K>
 void launch_packets(const sqk::TraceArgs& a, cudaStream_t s)
 {
-    static PerDevice<int> cache;
-    const uint32_t grid = (uint32_t)(cache.get([] { return blocks_per_sm(k_trace_packet<K>, 32); }) * sm_count());
+    static PerDevice<std::array<int, 2>> cache;
+    const std::array<int, 2> per_sm = cache.get([] {
+        return std::array<int, 2>{blocks_per_sm(k_trace_packet<K, kPoolPackets>, 32),
+                                  blocks_per_sm(k_trace_packet<K, kManyPackets>, 32)};
+    });
     const uint64_t packets = (uint64_t)a.width * a.height / K;
+    const uint32_t many = (uint32_t)(per_sm[1] * sm_count());
+    if (packets > (uint64_t)kFewPackets * many && !(K == 8 && a.tri_count >= kLargeTree)) {
+        k_trace_packet<K, kManyPackets><<<many, 32, 0, s>>>(a, many * packet_share(a.tri_count));
+        return;
+    }
     const uint64_t need = (packets + kPoolPackets - 1) / kPoolPackets;
-    k_trace_packet<K><<<(uint32_t)std::min<uint64_t>(grid, need ? need : 1), 32, 0, s>>>(a);
+    const uint32_t grid = (uint32_t)(per_sm[0] * sm_count());
+    k_trace_packet<K, kPoolPackets><<<(uint32_t)std::min<uint64_t>(grid, need ? need : 1), 32, 0, s>>>(a, 1u);
 }
 
 // morton_lut (src/tracer.cpp:18-23): k with bits 1 and 2 exchanged
