@@ -621,8 +621,8 @@ __device__ __forceinline__ uint32_t pop8(Lane8& L, const uint2* st)
 // warp test their leaves together, where a loop inside the visit took them
 // one after another.  A leaf that had a step to itself cost the lane one more
 // pass of the loop, which 20,000 rays that do not fill the GPU cannot hide
-// (600,000-triangle sphere: loop inside 166 us, own step 181, this 165); one
-// bounce off the 4.2M terrain 2025, 1569 and 1480 us, 2^24 incoherent rays
+// (600,000-triangle sphere: loop inside 166 us, own step 181, this 165, and 157
+// with seven blocks an SM, see k_trace8_refill); one bounce off the 4.2M terrain 2025, 1569 and 1480 us, 2^24 incoherent rays
 // 25.1, 19.9 and 20.1 ms.  Holding lanes back until 2 to 20 wait at leaves
 // was slower on small ray counts and no faster than 2% on large ones.
 template <bool ANY>
@@ -762,12 +762,16 @@ __global__ void __launch_bounds__(kTilesBlock, 32) k_trace8_tiles(const sqk::Tra
 }
 
 // PER_SM: resident blocks per SM the registers are limited for.  Eight (64
-// registers) hide most latency, seven (72) make a warp's own step shorter:
-// 200,000 rays 294 us
-// with eight and 283 with seven (600,000-triangle sphere), 600,000 off a 1M
-// terrain 478 and 483, 2M off the 4.2M terrain 1480 and 1538, 2^24 incoherent
-// 20.1 and 20.8 ms.  So up to kFewRays8 rays per lane of the GPU take seven.
-constexpr uint32_t kFewRays8 = 4;
+// registers) hide most latency, seven (72) make a warp's own step shorter.
+// Random rays against the 2M soup, seven and eight: 200,000 rays 528 and 579
+// us, 600,000 812 and 853, 900,000 1,052 and 1,076, 2M 1,888 and 1,887, 4M
+// 3,427 and 3,390 (327,680-triangle sphere: 600,000 379 and 383, 900,000 448
+// and 446, 2M 845 and 827).  So up to kFewRays8 rays per lane of the GPU
+// (934,000 rays) take seven.  Camera rays take seven whatever their number:
+// neighbouring rays share their nodes, so there is less latency to hide
+// (sphere at 1920x1072 300 and 317 us, at 3840x2160 571 and 588; with eight an
+// 81,920-triangle sphere was slower than before these kernels).
+constexpr uint32_t kFewRays8 = 6;
 
 template <int MODE, int PER_SM>
 __global__ void __launch_bounds__(128, PER_SM) k_trace8_refill(const sqk::Trace8Args a, uint32_t total)
@@ -866,7 +870,7 @@ void launch8(const sqk::Trace8Args& a, cudaStream_t s)
     });
     if (a.refill) {
         const uint32_t total = a.ray_kind == SQ_RAYS_EXPLICIT ? a.ray_count : batches * 32u;
-        const bool few = total <= kFewRays8 * 8u * 128u * (uint32_t)sm_count();
+        const bool few = a.ray_kind != SQ_RAYS_EXPLICIT || total <= kFewRays8 * 8u * 128u * (uint32_t)sm_count();
         const uint32_t grid = min((uint32_t)(per_sm[few ? 1 : 2] * sm_count()), (batches + 3u) / 4u);
         if (few) k_trace8_refill<MODE, 7><<<grid, 128, 0, s>>>(a, total);
         else k_trace8_refill<MODE, 8><<<grid, 128, 0, s>>>(a, total);
@@ -948,10 +952,12 @@ __global__ void __launch_bounds__(256) k_trace8_batch_tiles(const sqk::BatchTrac
     if (a.stats) ws.flush(lane, a.stats);
 }
 
-// Launch bounds of 28 warps per SM whatever the block shape (72 registers):
-// the job search needs more than k_trace8_refill's 64 (2^24 incoherent rays
-// in 64 batches 21.4 ms, 22.6 ms at 32 warps, 23.3 ms at 24; 800,000 rays in
-// 8 batches on a 60k sphere 357, 384 and 374 us).
+// Launch bounds of 28 warps per SM (72 registers) for blocks of 64 and 128, of
+// 24 (80 registers) for 256, which does not divide 28: the job search needs
+// more than k_trace8_refill's 64 (blocks of 128, 2^24 incoherent rays in 64
+// batches 21.4 ms, 22.6 ms at 32 warps, 23.3 ms at 24; 800,000 rays in 8
+// batches on a 60k sphere 357, 384 and 374 us).  Blocks of 256 are taken where
+// a batch asks for them or its autotuner finds them fastest.
 template <int MODE, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace8_batch_refill(const sqk::BatchTraceArgs a)
 {
