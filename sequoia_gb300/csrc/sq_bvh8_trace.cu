@@ -622,9 +622,10 @@ __device__ __forceinline__ uint32_t pop8(Lane8& L, const uint2* st)
 // one after another.  A leaf that had a step to itself cost the lane one more
 // pass of the loop, which 20,000 rays that do not fill the GPU cannot hide
 // (600,000-triangle sphere: loop inside 166 us, own step 181, this 165, and 157
-// with seven blocks an SM, see k_trace8_refill); one bounce off the 4.2M terrain 2025, 1569 and 1480 us, 2^24 incoherent rays
-// 25.1, 19.9 and 20.1 ms.  Holding lanes back until 2 to 20 wait at leaves
-// was slower on small ray counts and no faster than 2% on large ones.
+// with seven blocks an SM, see k_trace8_refill); one bounce off the 4.2M
+// terrain 2025, 1569 and 1480 us, 2^24 incoherent rays 25.1, 19.9 and 20.1 ms.
+// Holding lanes back until 2 to 20 wait at leaves was slower on small ray
+// counts and no faster than 2% on large ones.
 template <bool ANY>
 __device__ __forceinline__ void step8(Lane8& L, bool has, const Node8* __restrict__ nodes,
                                       const float4* __restrict__ t8, uint2* st, float* __restrict__ s_n, Totals8& sum)
