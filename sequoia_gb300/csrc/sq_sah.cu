@@ -97,7 +97,8 @@ static_assert(sizeof(Part) == 64, "Part is 64 bytes");
 struct Ctl {
     unsigned long long level[3];
     uint32_t n_mid, n_small, n_leaf;
-    uint32_t mid_pop, small_pop, pad;  // tasks taken by k_mid's blocks and k_small's warps
+    uint32_t mid_pop, small_pop;  // tasks taken by k_mid's blocks and k_small's warps
+    uint32_t odd;                 // a triangle with a NaN bound is among them (encode_boxes)
 };
 static_assert(sizeof(Ctl) == 48, "Ctl is 48 bytes");
 
@@ -145,13 +146,51 @@ __device__ __forceinline__ void load_box(const float4* __restrict__ tb, uint32_t
 
 __device__ __forceinline__ float sel(const float* v, int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); }
 
+// The twelve words of a triangle in a bin: order-preserving integers of
+// (-pmin, pmax, -cmin, cmax), so that a bin is their maxima.  A NaN bound is
+// passed over, as in the reference's comparisons (src/vec3.h:179-180): it gives
+// 0, below every number.  (float_to_ordered of a NaN is whatever the compiler
+// makes of its sign operations.)  ODD: look for one.  The setup kernels leave
+// in Ctl::odd whether the build has any, and the binning kernels are compiled
+// both ways: a look for each triangle, or at the flag, took 3% of k_small and
+// 8% of k_large_move.
+template <bool ODD>
+__device__ __forceinline__ void encode_boxes(const float* mn, const float* mx, const float* c, uint32_t* e)
+{
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        e[a] = float_to_ordered(-mn[a]);
+        e[3 + a] = float_to_ordered(mx[a]);
+        e[6 + a] = float_to_ordered(-c[a]);
+        e[9 + a] = float_to_ordered(c[a]);
+    }
+    if (ODD) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (isnan(mn[a])) e[a] = 0u;
+            if (isnan(mx[a])) e[3 + a] = 0u;
+            if (isnan(c[a])) e[6 + a] = e[9 + a] = 0u;
+        }
+    }
+}
+
+// A triangle with a NaN bound has a NaN centroid.  (Infinities of both signs
+// only cost the look.)
+__device__ __forceinline__ bool odd_box(const float* c)
+{
+    const float sum = (c[0] + c[1]) + c[2];
+    return sum != sum;
+}
+
 // ---------------------------------------------------------------------------
 // setup: triangle boxes, identity ids, root boxes
 
 __global__ void __launch_bounds__(256) k_sah_setup(const float* __restrict__ tris, uint32_t n, float4* __restrict__ tb,
-                                                   uint32_t* __restrict__ ids, uint32_t* __restrict__ root_ord)
+                                                   uint32_t* __restrict__ ids, uint32_t* __restrict__ root_ord,
+                                                   Ctl* __restrict__ ctl)
 {
     float v[12];
+    bool odd = false;
 #pragma unroll
     for (int k = 0; k < 12; ++k) v[k] = -FLT_MAX;  // max of (-pmin, pmax, -cmin, cmax)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -161,15 +200,18 @@ __global__ void __launch_bounds__(256) k_sah_setup(const float* __restrict__ tri
         tb[2ull * i] = make_float4(b.mn[0], b.mn[1], b.mn[2], 0.0f);
         tb[2ull * i + 1] = make_float4(b.mx[0], b.mx[1], b.mx[2], 0.0f);
         ids[i] = i;
+        float c[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const float c = (b.mn[k] + b.mx[k]) * 0.5f;
+            c[k] = (b.mn[k] + b.mx[k]) * 0.5f;
             v[k] = fmaxf(v[k], -b.mn[k]);
             v[3 + k] = fmaxf(v[3 + k], b.mx[k]);
-            v[6 + k] = fmaxf(v[6 + k], -c);
-            v[9 + k] = fmaxf(v[9 + k], c);
+            v[6 + k] = fmaxf(v[6 + k], -c[k]);
+            v[9 + k] = fmaxf(v[9 + k], c[k]);
         }
+        odd = odd || odd_box(c);
     }
+    if (odd) ctl->odd = 1u;
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
 #pragma unroll
@@ -187,8 +229,11 @@ __global__ void __launch_bounds__(256) k_sah_setup(const float* __restrict__ tri
     }
 }
 
-__device__ __forceinline__ float dec_neg(uint32_t u) { return -ordered_to_float(u); }
-__device__ __forceinline__ float dec_pos(uint32_t u) { return ordered_to_float(u); }
+// A bound from its word (0: no triangle had one, with NaN bounds only).
+template <bool ODD = true>
+__device__ __forceinline__ float dec_neg(uint32_t u) { return !ODD || u ? -ordered_to_float(u) : FLT_MAX; }
+template <bool ODD = true>
+__device__ __forceinline__ float dec_pos(uint32_t u) { return !ODD || u ? ordered_to_float(u) : -FLT_MAX; }
 
 // Where the large tasks of one level are listed: the tasks, each task's
 // first chunk, the task of each chunk, and the bins and per-chunk bin counts
@@ -345,12 +390,10 @@ __global__ void __launch_bounds__(256) k_grid_bin(const float4* __restrict__ tb,
         const uint32_t m = cell_slot(g[0], g[1], g[2]);
         keys[i] = m;
         uint32_t* cb = s_cell + m * kBinWords;
-        for (int a = 0; a < 3; ++a) {
-            atomicMax(cb + a, float_to_ordered(-mn[a]));
-            atomicMax(cb + 3 + a, float_to_ordered(mx[a]));
-            atomicMax(cb + 6 + a, float_to_ordered(-c[a]));
-            atomicMax(cb + 9 + a, float_to_ordered(c[a]));
-        }
+        uint32_t e[12];
+        encode_boxes<true>(mn, mx, c, e);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) atomicMax(cb + k, e[k]);
         atomicAdd(cb + 12, 1u);
     }
     __syncthreads();
@@ -425,13 +468,7 @@ __device__ __forceinline__ void warp_bin_add(uint32_t* __restrict__ wb, int bin,
 {
     const int lane = threadIdx.x & 31;
     uint32_t e[12];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        e[a] = float_to_ordered(-mn[a]);
-        e[3 + a] = float_to_ordered(mx[a]);
-        e[6 + a] = float_to_ordered(-c[a]);
-        e[9 + a] = float_to_ordered(c[a]);
-    }
+    encode_boxes<true>(mn, mx, c, e);
     const int b0 = __shfl_sync(0xFFFFFFFFu, bin, 0);
     if (__all_sync(0xFFFFFFFFu, bin == b0)) {
         // the whole warp in one bin: full-warp reductions and one writer
@@ -576,6 +613,7 @@ __device__ __forceinline__ void choose_planes(int nb, uint32_t cnt, const float*
 }
 
 // A bin's boxes from its encoded words (FLT_MAX boxes when it is empty).
+template <bool ODD>
 __device__ __forceinline__ uint32_t load_bin(const uint32_t* bin, bool in_range, float* p, float* c)
 {
     const uint32_t cnt = in_range ? bin[12] : 0u;
@@ -584,8 +622,8 @@ __device__ __forceinline__ uint32_t load_bin(const uint32_t* bin, bool in_range,
         p[a] = c[a] = FLT_MAX;
         p[3 + a] = c[3 + a] = -FLT_MAX;
         if (cnt) {
-            p[a] = dec_neg(bin[a]); p[3 + a] = dec_pos(bin[3 + a]);
-            c[a] = dec_neg(bin[6 + a]); c[3 + a] = dec_pos(bin[9 + a]);
+            p[a] = dec_neg<ODD>(bin[a]); p[3 + a] = dec_pos<ODD>(bin[3 + a]);
+            c[a] = dec_neg<ODD>(bin[6 + a]); c[3 + a] = dec_pos<ODD>(bin[9 + a]);
         }
     }
     return cnt;
@@ -598,7 +636,7 @@ __device__ __forceinline__ PlaneResult warp_choose_plane(const uint32_t* __restr
     const int lane = threadIdx.x & 31;
     PlaneResult r;
     float p[6], c[6];
-    const uint32_t cnt = load_bin(bins + lane * kBinWords, lane < nb, p, c);
+    const uint32_t cnt = load_bin<true>(bins + lane * kBinWords, lane < nb, p, c);
     choose_planes<32>(nb, cnt, p, c, r.plane, r.nl, r.lp, r.rp, r.lc, r.rc);
     return r;
 }
@@ -728,20 +766,22 @@ __global__ void __launch_bounds__(128) k_large_split(LevelLists cur, LevelLists 
 // bin.
 constexpr int kSlots = 32;
 
-template <uint32_t CHUNK, int NBP, bool ROOT>
-__global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ parts, LevelLists cur, LevelLists next,
-                                                    uint32_t cur_i, uint32_t* __restrict__ ids_a,
-                                                    uint32_t* __restrict__ ids_b, uint8_t* __restrict__ bin_a,
-                                                    uint8_t* __restrict__ bin_b, const uint32_t* __restrict__ chunk_left,
-                                                    const float4* __restrict__ tb, int nb, Ctl* ctl)
+struct MoveSmem {
+    uint32_t bins[2 * kSlots * kBinWords];
+    uint32_t cnt[2][2][kSlots];
+    uint32_t w[8];
+};
+
+template <uint32_t CHUNK, int NBP, bool ROOT, bool ODD>
+__device__ __forceinline__ void move_chunks(MoveSmem& sm, uint32_t chunks, const Part* __restrict__ parts,
+                                            const LevelLists& cur, const LevelLists& next, uint32_t* __restrict__ ids_a,
+                                            uint32_t* __restrict__ ids_b, uint8_t* __restrict__ bin_a,
+                                            uint8_t* __restrict__ bin_b, const uint32_t* __restrict__ chunk_left,
+                                            const float4* __restrict__ tb, int nb)
 {
-    chain_wait();  // a chained launch (enqueue_levels)
-    chain_release();
-    __shared__ uint32_t s_bins[2 * kSlots * kBinWords];
-    __shared__ uint32_t s_cnt[2][2][kSlots];
-    __shared__ uint32_t s_w[8];
-    if (!ROOT && blockIdx.x == 0 && threadIdx.x == 0) ctl->level[(cur_i + 2u) % 3u] = 0;
-    const uint32_t chunks = (uint32_t)(ctl->level[cur_i] >> 32);
+    uint32_t* s_bins = sm.bins;
+    uint32_t (&s_cnt)[2][2][kSlots] = sm.cnt;
+    uint32_t* s_w = sm.w;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t copy = (lane * NBP) & (kSlots - 1);  // first bin of the lane's copy
@@ -807,13 +847,7 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
                                      left ? P.cmin[0] : P.cmin[1], nb);
                 bin_out[to] = (uint8_t)b;
                 key = side * kSlots + (uint32_t)b;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    e[a] = float_to_ordered(-mn[a]);
-                    e[3 + a] = float_to_ordered(mx[a]);
-                    e[6 + a] = float_to_ordered(-cc[a]);
-                    e[9 + a] = float_to_ordered(cc[a]);
-                }
+                encode_boxes<ODD>(mn, mx, cc, e);
                 atomicAdd(&s_cnt[side][pos / CHUNK - (left ? first[0] : first[1])][copy + (uint32_t)b], 1u);
             }
             const uint32_t key0 = __shfl_sync(0xFFFFFFFFu, key, 0);
@@ -865,6 +899,22 @@ __global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ par
         }
         __syncthreads();  // the shared bins are cleared for the next chunk
     }
+}
+
+template <uint32_t CHUNK, int NBP, bool ROOT>
+__global__ void __launch_bounds__(256) k_large_move(const Part* __restrict__ parts, LevelLists cur, LevelLists next,
+                                                    uint32_t cur_i, uint32_t* __restrict__ ids_a,
+                                                    uint32_t* __restrict__ ids_b, uint8_t* __restrict__ bin_a,
+                                                    uint8_t* __restrict__ bin_b, const uint32_t* __restrict__ chunk_left,
+                                                    const float4* __restrict__ tb, int nb, Ctl* ctl)
+{
+    chain_wait();  // a chained launch (enqueue_levels)
+    chain_release();
+    __shared__ MoveSmem sm;
+    if (!ROOT && blockIdx.x == 0 && threadIdx.x == 0) ctl->level[(cur_i + 2u) % 3u] = 0;
+    const uint32_t chunks = (uint32_t)(ctl->level[cur_i] >> 32);
+    if (ctl->odd) move_chunks<CHUNK, NBP, ROOT, true>(sm, chunks, parts, cur, next, ids_a, ids_b, bin_a, bin_b, chunk_left, tb, nb);
+    else move_chunks<CHUNK, NBP, ROOT, false>(sm, chunks, parts, cur, next, ids_a, ids_b, bin_a, bin_b, chunk_left, tb, nb);
 }
 
 // ---------------------------------------------------------------------------
@@ -948,6 +998,7 @@ __global__ void __launch_bounds__(256) k_mid(uint32_t* __restrict__ ids_a, uint3
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t copy = (lane * NBP) & (kMaxBins - 1);  // first bin of the lane's copy
     const uint32_t total = done.ctl->n_mid;
+    const bool odd = done.ctl->odd != 0u;
     auto add_node = [&](int p, const Task& t) {
         MidNode& m = sg.node[p][atomicAdd(&sg.n_node[p], 1u)];
         m.t = t;
@@ -993,27 +1044,31 @@ __global__ void __launch_bounds__(256) k_mid(uint32_t* __restrict__ ids_a, uint3
                     if (pos - node[q].t.begin < node[q].t.count) a = q;
                 return a;
             };
-            for (uint32_t pos = tid; pos < count; pos += 256) {
-                const uint32_t a = node_at(pos);
-                if (a == kMidNodes) continue;
-                const uint32_t li = sg.loc[cur][pos];
-                const float4 lo = sg.box[li][0], hi = sg.box[li][1];
-                const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
-                float cc[3];
+            auto bin_all = [&](auto form) {
+                for (uint32_t pos = tid; pos < count; pos += 256) {
+                    const uint32_t a = node_at(pos);
+                    if (a == kMidNodes) continue;
+                    const uint32_t li = sg.loc[cur][pos];
+                    const float4 lo = sg.box[li][0], hi = sg.box[li][1];
+                    const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
+                    float cc[3];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) cc[k] = (mn[k] + mx[k]) * 0.5f;
-                const uint32_t b = (uint32_t)bin_of(node[a].k1, sel(cc, node[a].axis), node[a].cmin, nb);
-                sg.bin[pos] = (uint8_t)b;
-                uint32_t* w = sg.bins[a] + (copy + b) * kBinWords;
+                    for (int k = 0; k < 3; ++k) cc[k] = (mn[k] + mx[k]) * 0.5f;
+                    const uint32_t b = (uint32_t)bin_of(node[a].k1, sel(cc, node[a].axis), node[a].cmin, nb);
+                    sg.bin[pos] = (uint8_t)b;
+                    uint32_t* w = sg.bins[a] + (copy + b) * kBinWords;
+                    uint32_t e[12];
+                    encode_boxes<decltype(form)::value>(mn, mx, cc, e);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    atomicMax(w + k, float_to_ordered(-mn[k]));
-                    atomicMax(w + 3 + k, float_to_ordered(mx[k]));
-                    atomicMax(w + 6 + k, float_to_ordered(-cc[k]));
-                    atomicMax(w + 9 + k, float_to_ordered(cc[k]));
+                    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+                        for (int k = a; k < 12; k += 3) atomicMax(w + k, e[k]);
+                    }
+                    atomicAdd(w + 12, 1u);
                 }
-                atomicAdd(w + 12, 1u);
-            }
+            };
+            if (odd) bin_all(std::true_type{});
+            else bin_all(std::false_type{});
             __syncthreads();
             if (warp < active) {
                 MidNode& m = node[warp];
@@ -1030,7 +1085,7 @@ __global__ void __launch_bounds__(256) k_mid(uint32_t* __restrict__ ids_a, uint3
                     }
                 }
                 float p[6], c[6];
-                const uint32_t cnt = load_bin(w, (int)lane < nb, p, c);
+                const uint32_t cnt = load_bin<true>(w, (int)lane < nb, p, c);
                 PlaneResult r;
                 choose_planes<32>(nb, cnt, p, c, r.plane, r.nl, r.lp, r.rp, r.lc, r.rc);
                 if (lane == 0) {
@@ -1145,7 +1200,7 @@ struct SmallStage {
 };
 
 // One small task from the stage.
-template <int NBP>
+template <int NBP, bool ODD>
 __device__ void staged_subtree(const Task& root, SmallStage& sg, const uint32_t* __restrict__ ids,
                                const float4* __restrict__ tb, int nb, uint32_t leaf_size, uint32_t base,
                                Node* __restrict__ nodes, uint32_t leaf0)
@@ -1222,12 +1277,12 @@ __device__ void staged_subtree(const Task& root, SmallStage& sg, const uint32_t*
                     const uint32_t bin = (uint32_t)bin_of(kk, sel(cc, ax), cm, nb);
                     el[it] = li | (bin << 8) | (ge << 16);
                     uint32_t* w = sg.bins + (ge * NBP + bin) * kBinWords;
+                    uint32_t e[12];
+                    encode_boxes<ODD>(mn, mx, cc, e);
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        atomicMax(w + a, float_to_ordered(-mn[a]));
-                        atomicMax(w + 3 + a, float_to_ordered(mx[a]));
-                        atomicMax(w + 6 + a, float_to_ordered(-cc[a]));
-                        atomicMax(w + 9 + a, float_to_ordered(cc[a]));
+#pragma unroll
+                        for (int k = a; k < 12; k += 3) atomicMax(w + k, e[k]);
                     }
                     atomicAdd(w + 12, 1u);
                 }
@@ -1240,7 +1295,7 @@ __device__ void staged_subtree(const Task& root, SmallStage& sg, const uint32_t*
         float lp[6], rp[6], lc[6], rc[6];
         {
             float p[6], c[6];
-            const uint32_t cnt = load_bin(sg.bins + lane * kBinWords, act && (int)b < nb, p, c);
+            const uint32_t cnt = load_bin<ODD>(sg.bins + lane * kBinWords, act && (int)b < nb, p, c);
             choose_planes<NBP>(nb, cnt, p, c, plane, nl, lp, rp, lc, rc);
         }
         // the node's records and its children: lane 0 of a group has the
@@ -1345,13 +1400,16 @@ __global__ void __launch_bounds__(128) k_small(const Task* __restrict__ small, C
     chain_release();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t total = ctl->n_small;
+    const bool odd = ctl->odd != 0u;
     for (;;) {
         uint32_t ti = 0;
         if (lane == 0) ti = atomicAdd(&ctl->small_pop, 1u);
         ti = __shfl_sync(0xFFFFFFFFu, ti, 0);
         if (ti >= total) return;
         const Task t = small[ti];
-        staged_subtree<NBP>(t, s_stage[warp], (t.flags & 1u) ? ids_b : ids_a, tb, nb, leaf_size, base, nodes, leaf0);
+        const uint32_t* ids = (t.flags & 1u) ? ids_b : ids_a;
+        if (odd) staged_subtree<NBP, true>(t, s_stage[warp], ids, tb, nb, leaf_size, base, nodes, leaf0);
+        else staged_subtree<NBP, false>(t, s_stage[warp], ids, tb, nb, leaf_size, base, nodes, leaf0);
     }
 }
 
@@ -1618,7 +1676,7 @@ void launch_subtrees(const SahWs& w, int nb, uint32_t leaf_size, uint32_t base, 
 __global__ void __launch_bounds__(256) k_sah_setup_seg(const float* __restrict__ tris, uint32_t n,
                                                        const uint32_t* __restrict__ off, uint32_t M,
                                                        float4* __restrict__ tb, uint32_t* __restrict__ ids,
-                                                       uint32_t* __restrict__ root_ord)
+                                                       uint32_t* __restrict__ root_ord, Ctl* __restrict__ ctl)
 {
     seg_maxima<12>(n, off, M, root_ord, 16u, [&](uint32_t i, uint32_t* e) {
         float t[9];
@@ -1627,14 +1685,11 @@ __global__ void __launch_bounds__(256) k_sah_setup_seg(const float* __restrict__
         tb[2ull * i] = make_float4(b.mn[0], b.mn[1], b.mn[2], 0.0f);
         tb[2ull * i + 1] = make_float4(b.mx[0], b.mx[1], b.mx[2], 0.0f);
         ids[i] = i;
+        float c[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float c = (b.mn[k] + b.mx[k]) * 0.5f;
-            e[k] = float_to_ordered(-b.mn[k]);
-            e[3 + k] = float_to_ordered(b.mx[k]);
-            e[6 + k] = float_to_ordered(-c);
-            e[9 + k] = float_to_ordered(c);
-        }
+        for (int k = 0; k < 3; ++k) c[k] = (b.mn[k] + b.mx[k]) * 0.5f;
+        if (odd_box(c)) ctl->odd = 1u;
+        encode_boxes<true>(b.mn, b.mx, c, e);
     });
 }
 
@@ -1693,7 +1748,7 @@ int build_sah(const float* tris, uint32_t n, uint32_t nb, uint32_t leaf_size, in
     SQ_TRY(cudaMemsetAsync(w.root_ord, 0, sizeof(uint32_t) * 16, s));
     SQ_TRY(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), s));
     const uint32_t g = min((n + 255) / 256, (uint32_t)sms() * 8u);
-    k_sah_setup<<<g, 256, 0, s>>>(tris, n, w.tb, w.ids_a, w.root_ord);
+    k_sah_setup<<<g, 256, 0, s>>>(tris, n, w.tb, w.ids_a, w.root_ord, w.ctl);
     if (grid) {
         // bin into 64 cells keyed by Morton slot, then stable sort by slot
         k_grid_bin<<<g, 256, 0, s>>>(w.tb, n, w.root_ord, sort_keys, w.cells, w.hist);
@@ -1759,7 +1814,7 @@ int build_sah_batch(const float* tris, uint32_t n, const uint32_t* off, uint32_t
     const uint32_t sm = (uint32_t)sms();
     if (n > 0) {
         const uint32_t g = min((n + 255) / 256, sm * 8u);
-        k_sah_setup_seg<<<g, 256, 0, s>>>(tris, n, off, M, w.tb, w.ids_a, w.root_ord);
+        k_sah_setup_seg<<<g, 256, 0, s>>>(tris, n, off, M, w.tb, w.ids_a, w.root_ord, w.ctl);
     }
     with_chunk(n, [&](auto chunk) {
         constexpr uint32_t CHUNK = decltype(chunk)::value;
