@@ -30,7 +30,7 @@
 
 namespace sq {
 
-constexpr uint32_t kPoolOpen = 640;     // node ranges in a warp's pool beside the reserve
+constexpr uint32_t kPoolCap = 768;      // node ranges in a warp's pool (more cost resident warps)
 constexpr uint32_t kTriCap = 128;       // 31 waiting + 64 of one step fit
 constexpr uint32_t kCountBits = 27;     // an entry: node, owner << 27 | node count
 constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
@@ -70,9 +70,8 @@ struct WalkPool {
     // one ray or packet that is asked for has 128 pending ranges, one of a
     // bundle 128 more, and a range, a fan and the places checked for come on
     // top
-    static constexpr uint32_t kReserve = NB ? 272u : 136u;
-    static constexpr uint32_t kCap = kPoolOpen + kReserve;
-    uint2 node[kCap];
+    static constexpr uint32_t kOpen = kPoolCap - (NB ? 272u : 136u);
+    uint2 node[kPoolCap];
     uint2 tri[TRI ? kTriCap : 1];
     float inv[3][K][PW];                      // reciprocal directions
     float o[3][TRI ? PW : 1], d[3][TRI ? PW : 1], tmax[TRI ? PW : 1];
@@ -135,10 +134,11 @@ __device__ __forceinline__ void walk_pool(WalkPool<K, PW, TRI, NB>& pool, uint32
                 continue;
             }
             if (size == 0) break;
-            const uint32_t room = size < kPoolOpen ? (kPoolOpen - size) / 2u : 0u;
+            constexpr uint32_t kOpen = WalkPool<K, PW, TRI, NB>::kOpen;
+            const uint32_t room = size < kOpen ? (kOpen - size) / 2u : 0u;
             const bool one = room == 0u;
             const uint32_t take = one ? 1u : min(min(32u, size), room);
-            if (size + 2u > WalkPool<K, PW, TRI, NB>::kCap) {
+            if (size + 2u > kPoolCap) {
                 st.overflow = true;
                 break;
             }
