@@ -43,13 +43,14 @@ using namespace sq;
 // time and with shares:
 //   200 triangles     355 / 199 / 116 /  80     79 /  59 /  56 /  56
 //   1,500             361 / 202 / 118 /  86     86 /  75 /  80 /  76
-//   30,000            373 / 212 / 134 / 127    138 / 110 / 104 / 120
-//   2M                581 / 412 / 387 / 540    490 / 395 / 376 / 554
-// Packets of 8 in trees from kLargeTree triangles on stay at four (2M at
-// 3840x2160: 929 us, with shares 1,054).
+//   30,000            373 / 212 / 134          138 / 110 / 104
+//   2M                581 / 412 / 387          490 / 395 / 376
+// Packets of 8, which take longest, have shares in small trees only: in larger
+// ones they gain at 3840x2160 (20,000 triangles 338 and 283 us) and lose below
+// (1920x1072 126 and 133; 2M at 3840x2160 929 and 1,054).
 constexpr int kPoolPackets = 4, kManyPackets = 32;
 constexpr uint32_t kFewPackets = 16;
-constexpr uint32_t kSmallTree = 4096, kMediumTree = 1u << 17, kLargeTree = 1u << 20;
+constexpr uint32_t kSmallTree = 4096, kMediumTree = 1u << 15;
 uint32_t packet_share(uint32_t tris) { return tris < kSmallTree ? 4u : (tris < kMediumTree ? 8u : 16u); }
 
 // share: a warp takes 1 / share of the packets left, kPoolPackets to PW of them
@@ -109,7 +110,7 @@ void launch_packets(const sqk::TraceArgs& a, cudaStream_t s)
     });
     const uint64_t packets = (uint64_t)a.width * a.height / K;
     const uint32_t many = (uint32_t)(per_sm[1] * sm_count());
-    if (packets > (uint64_t)kFewPackets * many && !(K == 8 && a.tri_count >= kLargeTree)) {
+    if (packets > (uint64_t)kFewPackets * many && (K < 8 || a.tri_count < kSmallTree)) {
         k_trace_packet<K, kManyPackets><<<many, 32, 0, s>>>(a, many * packet_share(a.tri_count));
         return;
     }
